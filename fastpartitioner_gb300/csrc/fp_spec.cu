@@ -83,12 +83,36 @@ __device__ __forceinline__ unsigned long long cand_entry(int p, int c, unsigned 
          (f & 0xfffffull);
 }
 
+// A sighting key (32-bit, of a vertex one warp or CTA tallied) or a 64-bit key
+// of absolute net indexes as (net index << 32 | slot).
+__device__ __forceinline__ unsigned long long key64(unsigned f, int sb) { return wide_key(f, sb, 0); }
+__device__ __forceinline__ unsigned long long key64(unsigned long long f, int) { return f; }
+__device__ __forceinline__ unsigned min_key(unsigned f) { return __reduce_min_sync(kAll, f); }
+__device__ __forceinline__ unsigned long long min_key(unsigned long long f) { return warp_min_u64(f); }
+
+// Smallest size, then the smallest key among its holders (one warp, each lane
+// one (size, key, part); part < 0: none); returns the part, -1 if no lane has one.
+template <class F>
+__device__ __forceinline__ int least_size_first(int size, F first, int part) {
+  const int ms = __reduce_min_sync(kAll, part >= 0 ? size : 0x7fffffff);
+  const F mf = min_key(part >= 0 && size == ms ? first : ~(F)0);
+  const unsigned m = __ballot_sync(kAll, part >= 0 && size == ms && first == mf);
+  return m ? __shfl_sync(kAll, part, __ffs(m) - 1) : -1;
+}
+
 // One warp.  The tallied parts (count > 0, no stale TV marker) are first
 // compacted, in ascending order, into list (K ints of warp scratch); cand /
 // *ncand (if cand is not null) receive their re-check entries and scan (if not
 // null) TV's scanned-part bits.  The bound, exact and slack passes then walk
 // only the compacted parts.
-__device__ int ldg_decide(const DevInstance& I, const RoundCtx& R, const int* cnt, const unsigned long long* first,
+//
+// Near parts with one common count need no FP64: with equal counts the score
+// falls (weakly: division, subtraction and product round monotonically) as the
+// size grows, and equal scores go to the smaller size, so the smallest size,
+// then the first sighting, wins.  A score in double takes 722 cycles here; two
+// redux.sync take 44.
+template <class F>
+__device__ int ldg_decide(const DevInstance& I, const RoundCtx& R, const int* cnt, const F* first, int sb,
                           int metric, int v, int own, bool first_of_window, int* list, unsigned long long* cand,
                           int* ncand, uint32_t* scan, bool* special, int* slack_out) {
   const int lane = threadIdx.x & 31;
@@ -109,7 +133,7 @@ __device__ int ldg_decide(const DevInstance& I, const RoundCtx& R, const int* cn
       const int i = nc + __popc(m & below);
       list[i] = p;
       if (cand) {
-        const unsigned long long f = first[p];
+        const unsigned long long f = key64(first[p], sb);
         wide |= c > 0xffff || (f >> 32) > 0xffffull;
         cand[i] = cand_entry(p, c - (p == own ? 1 : 0), f);
       }
@@ -136,16 +160,18 @@ __device__ int ldg_decide(const DevInstance& I, const RoundCtx& R, const int* cn
       any |= f + t > 0.0f;
     }
   }
-  for (int off = 16; off; off >>= 1) fb = fmaxf(fb, __shfl_xor_sync(kAll, fb, off));
+  fb = warp_max_nonneg(fb);
   LdgKey best{-1.0, 0, -1, ~0ull};
   float sbest = 0.0f;   // a lower bound of the winner's exact score, in float
   if (__any_sync(kAll, any)) {
     // Parts whose upper bound reaches the largest lower bound: the argmax and
     // all its ties are among them.  A single one with a positive lower bound
-    // is the argmax outright (every other score lies below fb); otherwise the
-    // exact double scores (TV/partition.cpp:103-104) and tie-breaks decide.
-    int nnear = 0, np = -1;
-    float nlo = 0.0f;
+    // is the argmax outright (every other score lies below fb); several of one
+    // count, one of them positive for sure, are ordered by size and sighting;
+    // otherwise the exact double scores (TV/partition.cpp:103-104) and
+    // tie-breaks decide.
+    int nnear = 0, np = -1, nsz = 0, cmin = 0x7fffffff, cmax = 0;
+    F nf = ~(F)0;
     for (int i = lane; i < nc; i += 32) {
       const int p = list[i];
       const int cc = cnt[p] - (p == own ? 1 : 0);
@@ -154,16 +180,23 @@ __device__ int ldg_decide(const DevInstance& I, const RoundCtx& R, const int* cn
       const float f = __fmul_rn((float)cc, pf), t = score_tol(cc, pf);
       if (!(f + t > 0.0f) || f + t < fb) continue;
       nnear++;
-      np = p;
-      nlo = f - t;
+      cmin = min(cmin, cc);
+      cmax = max(cmax, cc);
+      const int sz = R.sizes[p];
+      const F fp = first[p];
+      if (np < 0 || sz < nsz || (sz == nsz && fp < nf)) {
+        np = p;
+        nsz = sz;
+        nf = fp;
+      }
     }
-    const int tot = __reduce_add_sync(kAll, nnear);
-    const unsigned hn = __ballot_sync(kAll, nnear > 0);
-    const int src = __ffs(hn) - 1;
-    const float lo1 = __shfl_sync(kAll, nlo, src);
-    if (tot == 1 && lo1 > 0.0f) {
-      best.part = __shfl_sync(kAll, np, src);
-      sbest = lo1;
+    const int tot = warp_sum(nnear);
+    cmin = warp_min(cmin);
+    cmax = warp_max(cmax);
+    if (fb > 0.0f && (tot == 1 || cmin == cmax)) {
+      best.part = least_size_first<F>(nsz, nf, np);
+      const float pf = R.penf[best.part];
+      sbest = __fmul_rn((float)cmax, pf) - score_tol(cmax, pf);
     } else {
       for (int i = lane; i < nc; i += 32) {
         const int p = list[i];
@@ -173,7 +206,7 @@ __device__ int ldg_decide(const DevInstance& I, const RoundCtx& R, const int* cn
         const float f = __fmul_rn((float)cc, pf), t = score_tol(cc, pf);
         if (!(f + t > 0.0f) || f + t < fb) continue;   // cannot be a positive best
         const double pen = __dsub_rn(1.0, __ddiv_rn((double)R.sizes[p], I.C));   // TV/partition.cpp:103-104
-        LdgKey k{__dmul_rn((double)cc, pen), R.sizes[p], p, first[p]};
+        LdgKey k{__dmul_rn((double)cc, pen), R.sizes[p], p, key64(first[p], sb)};
         if (ldg_better(k, best)) best = k;
       }
       best = warp_ldg_argmax(best);
@@ -253,40 +286,54 @@ __device__ int ldg_recheck(const DevInstance& I, const RoundCtx& R, const SpecBu
   if (nc < 0) return -1;   // no list (65536 nets or more): the caller cuts
   // Float scores first: the float penalty 1 - sz / C is off by less than
   // 4e-7 * (1 + sz / C), so a score of count c by less than c times that; the
-  // bound used is 1e-6 * c * (1 + sz / C).  Exact double scores only for
-  // candidates whose upper bound reaches the largest lower bound.
+  // bound used is 1e-6 * c * (1 + sz / C).  The near candidates are then ordered
+  // as in ldg_decide (one left, or one count: by size and first sighting;
+  // otherwise exact double scores).  The first 32 entries stay in registers.
   const float Cf = R.Cf;
+  const unsigned long long e0 = lane < nc ? lds(&cl[lane]) : 0;
+  auto ent_at = [&](int i) { return i < 32 ? e0 : lds(&cl[i]); };
+  auto size_of = [&](int p) { return R.sizes[p] + dsz[p]; };
   float fb = 0.0f;
   for (int i = lane; i < nc; i += 32) {
-    const unsigned long long ent = lds(&cl[i]);
-    const int p = (int)(ent >> 52);
+    const unsigned long long ent = ent_at(i);
     const int c = (int)((ent >> 36) & 0xffffull);
-    const float xf = __fdiv_rn((float)(R.sizes[p] + dsz[p]), Cf);
+    const float xf = __fdiv_rn((float)size_of((int)(ent >> 52)), Cf);
     fb = fmaxf(fb, __fmul_rn((float)c, 1.0f - xf) - (float)c * 1e-6f * (1.0f + fabsf(xf)));
   }
-  for (int off = 16; off; off >>= 1) fb = fmaxf(fb, __shfl_xor_sync(kAll, fb, off));
-  // a single part reaching fb > 0 is the argmax outright (as in ldg_decide)
-  int nnear = 0, np = -1;
+  fb = warp_max_nonneg(fb);
+  int nnear = 0, np = -1, nsz = 0, cmin = 0x7fffffff, cmax = 0;
+  unsigned long long nf = ~0ull;   // the entry's low 36 bits order like the first sighting
   for (int i = lane; i < nc; i += 32) {
-    const unsigned long long ent = lds(&cl[i]);
+    const unsigned long long ent = ent_at(i);
     const int p = (int)(ent >> 52);
     const int c = (int)((ent >> 36) & 0xffffull);
-    const float xf = __fdiv_rn((float)(R.sizes[p] + dsz[p]), Cf);
-    if (__fmul_rn((float)c, 1.0f - xf) + (float)c * 1e-6f * (1.0f + fabsf(xf)) < fb) continue;   // cannot be best
+    const int sz = size_of(p);
+    const float xf = __fdiv_rn((float)sz, Cf);
+    if (c == 0 || __fmul_rn((float)c, 1.0f - xf) + (float)c * 1e-6f * (1.0f + fabsf(xf)) < fb) continue;
     nnear++;
-    np = p;
+    cmin = min(cmin, c);
+    cmax = max(cmax, c);
+    const unsigned long long f = ent & 0xfffffffffull;
+    if (np < 0 || sz < nsz || (sz == nsz && f < nf)) {
+      np = p;
+      nsz = sz;
+      nf = f;
+    }
   }
+  const int tot = warp_sum(nnear);
+  cmin = warp_min(cmin);
+  cmax = warp_max(cmax);
   LdgKey best{-1.0, 0, -1, ~0ull};
-  if (fb > 0.0f && __reduce_add_sync(kAll, nnear) == 1) {
-    best.part = __shfl_sync(kAll, np, __ffs(__ballot_sync(kAll, nnear > 0)) - 1);
-  } else {
+  if (fb > 0.0f && (tot == 1 || cmin == cmax)) {
+    best.part = least_size_first<unsigned long long>(nsz, nf, np);
+  } else if (tot > 0) {
     for (int i = lane; i < nc; i += 32) {
-      const unsigned long long ent = lds(&cl[i]);
+      const unsigned long long ent = ent_at(i);
       const int p = (int)(ent >> 52);
       const int c = (int)((ent >> 36) & 0xffffull);
-      const int sz = R.sizes[p] + dsz[p];
+      const int sz = size_of(p);
       const float xf = __fdiv_rn((float)sz, Cf);
-      if (__fmul_rn((float)c, 1.0f - xf) + (float)c * 1e-6f * (1.0f + fabsf(xf)) < fb) continue;   // cannot be best
+      if (c == 0 || __fmul_rn((float)c, 1.0f - xf) + (float)c * 1e-6f * (1.0f + fabsf(xf)) < fb) continue;
       const unsigned long long f = (((ent >> 20) & 0xffffull) << 32) | (ent & 0xfffffull);
       const double pen = __dsub_rn(1.0, __ddiv_rn((double)sz, I.C));
       LdgKey k{__dmul_rn((double)c, pen), sz, p, f};
@@ -298,15 +345,10 @@ __device__ int ldg_recheck(const DevInstance& I, const RoundCtx& R, const SpecBu
   if (d0 < 0) {
     unsigned long long mk = ~0ull;
     for (int p = lane; p < K; p += 32) {
-      const int sz = R.sizes[p] + dsz[p];
-      const unsigned long long key = ((unsigned long long)((unsigned)sz ^ 0x80000000u) << 32) | (unsigned)p;
+      const unsigned long long key = ((unsigned long long)((unsigned)size_of(p) ^ 0x80000000u) << 32) | (unsigned)p;
       mk = key < mk ? key : mk;
     }
-    for (int off = 16; off; off >>= 1) {
-      const unsigned long long x = __shfl_xor_sync(kAll, mk, off);
-      mk = x < mk ? x : mk;
-    }
-    d0 = (int)(mk & 0xffffffffu);
+    d0 = (int)(warp_min_u64(mk) & 0xffffffffu);
   }
   int d = d0;
   if (metric == kTV) {
@@ -577,10 +619,11 @@ __device__ __forceinline__ int block_reduce_min(int x, int* scr) {
 
 // Evaluation of a medium vertex at position z by the whole CTA: the warps split
 // the tally, warp 0 decides, the warps split the locate pass and the gain /
-// loss terms.  Writes the same per-position record as a warp evaluation (flag
-// bit 2 marks it).
+// loss terms.  All warps add to one set of K-sized arrays (native 32-bit
+// shared-memory atomics): nothing is merged per warp.  Writes the same
+// per-position record as a warp evaluation (flag bit 2 marks it).
 __device__ void cta_eval_ldg(const DevInstance& I, const SpecBuf& B, const RoundCtx& R, int metric, int z, int pos,
-                             int par, int q, int* cnt_b, unsigned long long* first_b, int* gains_b, int* losses_b,
+                             int par, int q, int sb, int* cnt_b, unsigned* first_b, int* gains_b, int* losses_b,
                              int* adelta_b, int* iscr, int* s_mw, int* s_mv, int* loc_b, bool logp) {
   __shared__ int sh[4];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -592,31 +635,19 @@ __device__ void cta_eval_ldg(const DevInstance& I, const SpecBuf& B, const Round
   const int own = lds(&I.part_vec[v]);
   const uint32_t base = __ldg(&I.vptr[v]);
   const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
-  int* cnt = cnt_b + (size_t)wib * K;
-  unsigned long long* first = first_b + (size_t)wib * K;
   const long long t0 = clock64();
-  for (int p = lane; p < K; p += 32) { cnt[p] = 0; first[p] = ~0ull; }
-  __syncwarp();
-  int c1 = 0;
-  {
-    int n0, n1;
-    net_range(deg, wib, kSWarps, &n0, &n1);
-    for (int nb = n0; nb < n1; nb += 32) c1 += tally_batch(I, own, base, nb, n1, cnt, first);
-  }
-  c1 = warp_sum(c1);
-  __syncthreads();
-  if (lane == 0) iscr[wib] = c1;
   for (int p = threadIdx.x; p < K; p += blockDim.x) {
-    int c = 0;
-    unsigned long long f = ~0ull;
-    for (int x = 0; x < kSWarps; x++) {
-      c += cnt_b[(size_t)x * K + p];
-      const unsigned long long fx = first_b[(size_t)x * K + p];
-      f = fx < f ? fx : f;
-    }
-    cnt_b[p] = c;
-    first_b[p] = f;
+    cnt_b[p] = 0;
+    first_b[p] = ~0u;
+    if (vol) { gains_b[p] = 0; losses_b[p] = 0; adelta_b[p] = 0; }
   }
+  __syncthreads();
+  int c1 = 0;
+  int n0, n1;
+  net_range(deg, wib, kSWarps, &n0, &n1);
+  for (int nb = n0; nb < n1; nb += 32) c1 += tally_batch(I, own, base, nb, n1, 0, sb, cnt_b, first_b);
+  c1 = warp_sum(c1);
+  if (lane == 0) iscr[wib] = c1;
   __syncthreads();
   int c1t = 0;
   for (int x = 0; x < kSWarps; x++) c1t += iscr[x];
@@ -624,7 +655,7 @@ __device__ void cta_eval_ldg(const DevInstance& I, const SpecBuf& B, const Round
   if (wib == 0) {
     bool special;
     int slack;
-    const int d = ldg_decide(I, R, cnt_b, first_b, metric, v, own, z == pos, gains_b, B.cand + (size_t)o * K,
+    const int d = ldg_decide(I, R, cnt_b, first_b, sb, metric, v, own, z == pos, cnt_b + K, B.cand + (size_t)o * K,
                              &B.ncand[o], metric == kTV ? B.scan + (size_t)o * words : nullptr, &special, &slack);
     if (lane == 0) {
       sh[0] = d;
@@ -650,28 +681,9 @@ __device__ void cta_eval_ldg(const DevInstance& I, const SpecBuf& B, const Round
     const bool need = metric == kTV ? c1t >= deg - cnt_b[d] : true;
     mover = metric == kTV && need;
     {   // records for every decision that moves: own's slot per net serves the validation
-      int* gains = gains_b + (size_t)wib * K;
-      int* losses = losses_b + (size_t)wib * K;
-      int* adelta = adelta_b + (size_t)wib * K;
-      if (vol) {
-        for (int p = lane; p < K; p += 32) { gains[p] = 0; losses[p] = 0; adelta[p] = 0; }
-        __syncwarp();
-      }
-      locate_all(I, B, metric, v, own, d, base, deg, wib, kSWarps, loc_b + wib * 96, gains, losses, adelta);
+      locate_all(I, B, metric, v, own, d, base, deg, wib, kSWarps, loc_b + wib * 96, gains_b, losses_b, adelta_b);
       __syncthreads();
       if (vol) {
-        for (int p = threadIdx.x; p < K; p += blockDim.x) {
-          int g = 0, l = 0, a = 0;
-          for (int x = 0; x < kSWarps; x++) {
-            g += gains_b[(size_t)x * K + p];
-            l += losses_b[(size_t)x * K + p];
-            a += adelta_b[(size_t)x * K + p];
-          }
-          gains_b[p] = g;
-          losses_b[p] = l;
-          adelta_b[p] = a;
-        }
-        __syncthreads();
         const AcceptPart a = accept_partial(R, gains_b, losses_b, adelta_b, K, rv, threadIdx.x, blockDim.x);
         const bool fM = __syncthreads_or(a.failM);
         const bool fN = __syncthreads_or(a.failN);
@@ -888,12 +900,16 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
   int* vol_s = cv.take<int>(K);
   int* mark_s = cv.take<int>(K);
   int* cnt_b = cv.take<int>((size_t)K * kSWarps);                    // per-warp arrays, warp x at x*K
-  unsigned long long* first_b = cv.take<unsigned long long>((size_t)K * kSWarps);
+  // sighting keys: the warps' 32-bit ones (warp x at x*K), or the 64-bit ones of
+  // the window's whole-grid vertices (vertex j at j*K)
+  unsigned long long* first64_b = cv.take<unsigned long long>((size_t)K * kSWarps);
+  unsigned* first_b = reinterpret_cast<unsigned*>(first64_b);
   int* gains_b = cv.take<int>((size_t)K * kSWarps);
   int* losses_b = cv.take<int>((size_t)K * kSWarps);
   int* adelta_b = cv.take<int>((size_t)K * kSWarps);
   int* cnt = cnt_b + (size_t)wib * K;
-  unsigned long long* first = first_b + (size_t)wib * K;
+  unsigned* first = first_b + (size_t)wib * K;
+  const int sb = slot_bits(K);
   int* gains = gains_b + (size_t)wib * K;
   int* losses = losses_b + (size_t)wib * K;
   int* adelta = adelta_b + (size_t)wib * K;
@@ -1031,31 +1047,40 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         const uint32_t base_s = s_gb[j];
         int* hcnt = B.hcnt + hslot(j);
         unsigned long long* hfirst = B.hfirst + hslot(j);
-        for (int p = lane; p < K; p += 32) { cnt[p] = 0; first[p] = ~0ull; }
-        __syncwarp();
-        int c1 = 0;
-        {
-          int n0, n1;
-          net_range(deg_s, gw, nwarps, &n0, &n1);
-          for (int nb = n0; nb < n1; nb += 32) c1 += tally_batch(I, own_s, base_s, nb, n1, cnt, first);
-        }
-        c1 = warp_sum(c1);
-        __syncthreads();
-        for (int p = threadIdx.x; p < K; p += blockDim.x) {
-          int c = 0;
-          unsigned long long f = ~0ull;
-          for (int x = 0; x < kSWarps; x++) {
-            c += cnt_b[(size_t)x * K + p];
-            const unsigned long long fx = first_b[(size_t)x * K + p];
-            f = fx < f ? fx : f;
+        // a warp's share in pieces whose sighting keys fit 32 bits (all but always one)
+        const int share = (deg_s + nwarps - 1) / nwarps, piece = key_nets(sb);
+        for (int a0 = 0; a0 < share; a0 += piece) {
+          for (int p = lane; p < K; p += 32) { cnt[p] = 0; first[p] = ~0u; }
+          __syncwarp();
+          int c1 = 0;
+          {
+            int n0, n1;
+            net_range(deg_s, gw, nwarps, &n0, &n1);
+            const int b0 = min(n0 + a0, n1), b1 = min(b0 + piece, n1);
+            for (int nb = b0; nb < b1; nb += 32) c1 += tally_batch(I, own_s, base_s, nb, b1, b0, sb, cnt, first);
           }
-          if (c) {
-            atomicAdd(&hcnt[p], c);
-            atomicMin(&hfirst[p], f);
+          c1 = warp_sum(c1);
+          __syncthreads();
+          for (int p = threadIdx.x; p < K; p += blockDim.x) {
+            int c = 0;
+            unsigned long long f = ~0ull;
+            for (int x = 0; x < kSWarps; x++) {
+              const int cx = cnt_b[(size_t)x * K + p];
+              if (cx && f == ~0ull) {   // the warps' shares ascend: the first that saw p saw it first
+                int n0, n1;
+                net_range(deg_s, blockIdx.x * kSWarps + x, nwarps, &n0, &n1);
+                f = wide_key(first_b[(size_t)x * K + p], sb, n0 + a0);
+              }
+              c += cx;
+            }
+            if (c) {
+              atomicAdd(&hcnt[p], c);
+              atomicMin(&hfirst[p], f);
+            }
           }
+          if (lane == 0 && c1) atomicAdd(&B.hmisc[hmslot(j)], c1);
+          __syncthreads();   // the per-warp arrays serve the next vertex and the evaluations below
         }
-        if (lane == 0 && c1) atomicAdd(&B.hmisc[hmslot(j)], c1);
-        __syncthreads();   // the per-warp arrays serve the next vertex and the evaluations below
       }
       if (kTimingStats && ns && threadIdx.x == 0) atomicMax(&B.stats[38], gtimer() - tR);
       // ---- A: evaluate
@@ -1071,10 +1096,10 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         if (__ldg(&B.vclass[v]) != 0) continue;   // medium vertex: evaluated by the whole CTA below
         const long long cz = clock64();
         const int own = lds(&I.part_vec[v]);
-        for (int p = lane; p < K; p += 32) { cnt[p] = 0; first[p] = ~0ull; }
+        for (int p = lane; p < K; p += 32) { cnt[p] = 0; first[p] = ~0u; }
         __syncwarp();
         int c1 = 0;
-        for (int nb = 0; nb < deg; nb += 32) c1 += tally_batch(I, own, base, nb, deg, cnt, first);
+        for (int nb = 0; nb < deg; nb += 32) c1 += tally_batch(I, own, base, nb, deg, 0, sb, cnt, first);
         __syncwarp();
         c1 = warp_sum(c1);
         const long long cT = clock64();
@@ -1082,7 +1107,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         int slack;
         // candidates (part, count, first sighting) for an exact re-check of the
         // decision if the part sizes drift beyond its slack; TV's scanned parts
-        const int d = ldg_decide(I, R, cnt, first, metric, v, own, z == pos, gains, B.cand + (size_t)o * K,
+        const int d = ldg_decide(I, R, cnt, first, sb, metric, v, own, z == pos, gains, B.cand + (size_t)o * K,
                                  &B.ncand[o], metric == kTV ? B.scan + (size_t)o * words : nullptr, &special, &slack);
         const long long cD = clock64();
         // An isolated vertex (no nets, weight 0) changes nothing a later position
@@ -1170,7 +1195,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
       for (int mi = lower_bound_pos(B.mid_pos, B.nmid, cz0); mi < B.nmid; mi++) {
         const int z = __ldg(&B.mid_pos[mi]);
         if (z >= cz1) break;
-        cta_eval_ldg(I, B, R, metric, z, pos, par, q, cnt_b, first_b, gains_b, losses_b, adelta_b, iscr, s_mw, s_mv,
+        cta_eval_ldg(I, B, R, metric, z, pos, par, q, sb, cnt_b, first_b, gains_b, losses_b, adelta_b, iscr, s_mw, s_mv,
                      loc_b, logp);
       }
       __syncthreads();
@@ -1189,7 +1214,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
           const size_t hs = hslot(j);
           for (int p = threadIdx.x; p < K; p += blockDim.x) {
             cnt_b[(size_t)j * K + p] = lds(&B.hcnt[hs + p]);
-            first_b[(size_t)j * K + p] = lds(&B.hfirst[hs + p]);
+            first64_b[(size_t)j * K + p] = lds(&B.hfirst[hs + p]);
           }
         }
         __syncthreads();
@@ -1197,13 +1222,13 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
           const int j = wib;
           const int zs = s_gz[j], vsup = s_gv[j], own_s = s_go[j];
           const int* cj = cnt_b + (size_t)j * K;
-          const unsigned long long* fj = first_b + (size_t)j * K;
+          const unsigned long long* fj = first64_b + (size_t)j * K;
           bool special;
           int slack;
           // block 0 keeps the candidates for an exact re-check, TV's scanned parts
           const int os = zs - pos;
           const bool b0 = blockIdx.x == 0;
-          const int d = ldg_decide(I, R, cj, fj, metric, vsup, own_s, zs == pos, gains_b + (size_t)j * K,
+          const int d = ldg_decide(I, R, cj, fj, sb, metric, vsup, own_s, zs == pos, gains_b + (size_t)j * K,
                                    b0 ? B.cand + (size_t)os * K : nullptr, b0 ? &B.ncand[os] : nullptr,
                                    b0 && metric == kTV ? B.scan + (size_t)os * words : nullptr, &special, &slack);
           if (lane == 0) { s_gdec[j] = d; s_gspec[j] = special ? 1 : 0; s_gslk[j] = slack; }

@@ -96,17 +96,20 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, int* status) {
   return s_ok != 0;
 }
 
-__device__ __forceinline__ int warp_sum(int x) {
-  for (int off = 16; off; off >>= 1) x += __shfl_xor_sync(kAll, x, off);
-  return x;
+// 32-bit warp reductions are one redux.sync (22 cycles measured, against about
+// 180 for five dependent shuffles).
+__device__ __forceinline__ int warp_sum(int x) { return __reduce_add_sync(kAll, x); }
+__device__ __forceinline__ int warp_min(int x) { return __reduce_min_sync(kAll, x); }
+__device__ __forceinline__ int warp_max(int x) { return __reduce_max_sync(kAll, x); }
+// Maximum of non-negative floats (their bit patterns order like the values).
+__device__ __forceinline__ float warp_max_nonneg(float x) {
+  return __uint_as_float(__reduce_max_sync(kAll, __float_as_uint(x)));
 }
-__device__ __forceinline__ int warp_min(int x) {
-  for (int off = 16; off; off >>= 1) x = min(x, __shfl_xor_sync(kAll, x, off));
-  return x;
-}
-__device__ __forceinline__ int warp_max(int x) {
-  for (int off = 16; off; off >>= 1) x = max(x, __shfl_xor_sync(kAll, x, off));
-  return x;
+// Minimum of a 64-bit key: the high words, then the low words of their holders.
+__device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long x) {
+  const unsigned hi = __reduce_min_sync(kAll, (unsigned)(x >> 32));
+  const unsigned lo = __reduce_min_sync(kAll, (unsigned)(x >> 32) == hi ? (unsigned)x : ~0u);
+  return ((unsigned long long)hi << 32) | lo;
 }
 __device__ __forceinline__ long long warp_sum64(long long x) {
   for (int off = 16; off; off >>= 1) x += __shfl_xor_sync(kAll, x, off);
@@ -149,13 +152,28 @@ __device__ __forceinline__ void net_range(int deg, int wi, int nw, int* b, int* 
   *e = min(*b + g, deg);
 }
 
-// Adds to the warp's part tally the nets [nb, min(nb + 32, deg)) of a vertex
-// (base: its offset in vnets; deg: the end of the warp's nets): for every listed part, the number of
-// nets listing it (cnt) and the (net index, slot) of its first sighting (first);
-// returns this lane's count of nets where `own` has exactly one pin.  Slots of
-// the 32 nets are flattened across the warp (inclusive scan of list lengths).
-__device__ __forceinline__ int tally_batch(const DevInstance& I, int own, uint32_t base, int nb, int deg, int* cnt,
-                                           unsigned long long* first) {
+// Sighting keys: the reference breaks ties by the part seen first, in (net,
+// slot) order.  A key is the net's index from the start of the tallied range
+// above the slot, in 32 bits: shared-memory atomicMin has a native 32-bit form
+// (about 50 cycles), the 64-bit one is a compare-and-swap loop (146 cycles
+// uncontended).  The slot takes slot_bits(K) bits, so a range holds at most
+// key_nets(sb) nets: more than a vertex evaluated by one warp or CTA has (65535
+// nets, K <= 4096); a longer share of a whole-grid vertex is tallied in pieces,
+// and the pieces meet in 64-bit keys of absolute net indexes (wide_key).
+__device__ __forceinline__ int slot_bits(int K) { return 32 - __clz(K - 1); }
+__device__ __forceinline__ int key_nets(int sb) { return sb <= 1 ? 0x7fffffff : (int)(1u << (32 - sb)); }
+__device__ __forceinline__ unsigned long long wide_key(unsigned f, int sb, int n0) {
+  return ((unsigned long long)((unsigned)n0 + (f >> sb)) << 32) | (f & ((1u << sb) - 1u));
+}
+
+// Adds to the part tally the nets [nb, min(nb + 32, deg)) of a vertex (base:
+// its offset in vnets; deg: the end of the range of nets; n0: its start): for
+// every listed part, the number of nets listing it (cnt) and the sighting key
+// of its first one (first); returns this lane's count of nets where `own` has
+// exactly one pin.  Slots of the 32 nets are flattened across the warp
+// (inclusive scan of list lengths).
+__device__ __forceinline__ int tally_batch(const DevInstance& I, int own, uint32_t base, int nb, int deg, int n0,
+                                           int sb, int* cnt, unsigned* first) {
   const int lane = threadIdx.x & 31;
   const int K = I.K;
   const int k = nb + lane;
@@ -178,7 +196,8 @@ __device__ __forceinline__ int tally_batch(const DevInstance& I, int own, uint32
   // keeps kU requests per lane in flight (the walk is latency-bound otherwise).
   constexpr int kU = 4;
   for (int f0 = 0; f0 < total; f0 += 32 * kU) {
-    int aa[kU], key_net[kU], key_slot[kU], pp[kU];
+    int aa[kU], pp[kU];
+    unsigned key[kU];
 #pragma unroll
     for (int u = 0; u < kU; u++) {
       const int f = f0 + u * 32 + lane;
@@ -193,8 +212,7 @@ __device__ __forceinline__ int tally_batch(const DevInstance& I, int own, uint32
       const int nl = __shfl_sync(kAll, n, lo);
       const int il = __shfl_sync(kAll, incl, lo);
       const int j = f - (il - nl);              // slot within net nb + lo
-      key_net[u] = nb + lo;
-      key_slot[u] = j;
+      key[u] = ((unsigned)(nb - n0 + lo) << sb) | (unsigned)j;
       aa[u] = f < total ? sl + j : -1;          // slot address, -1 past the end
     }
     int cc[kU];
@@ -213,7 +231,7 @@ __device__ __forceinline__ int tally_batch(const DevInstance& I, int own, uint32
         continue;
       }
       atomicAdd(&cnt[p], 1);
-      atomicMin(&first[p], ((unsigned long long)key_net[u] << 32) | (unsigned)key_slot[u]);
+      atomicMin(&first[p], key[u]);
       if (p == own && cc[u] == 1) c1++;
     }
   }
@@ -491,10 +509,7 @@ __device__ __forceinline__ void block_min_part(const int* sizes, int K, unsigned
     const unsigned long long key = ((unsigned long long)((unsigned)sizes[p] ^ 0x80000000u) << 32) | (unsigned)p;
     mk = key < mk ? key : mk;
   }
-  for (int off = 16; off; off >>= 1) {
-    const unsigned long long o = __shfl_xor_sync(kAll, mk, off);
-    mk = o < mk ? o : mk;
-  }
+  mk = warp_min_u64(mk);
   __syncthreads();
   if (lane == 0) scr[wib] = mk;
   __syncthreads();

@@ -61,8 +61,8 @@ constexpr int kMSRV = 5;
 // CN's tally of the nets [nb, min(nb + 32, deg)) of a vertex: the part of
 // every net with exactly one listed part, the number of such nets per part and
 // the first such net (CN/partition.cpp:150-170).
-__device__ __forceinline__ void tally_uncut(const DevInstance& I, uint32_t base, int nb, int deg, int* cnt,
-                                            unsigned long long* first) {
+__device__ __forceinline__ void tally_uncut(const DevInstance& I, uint32_t base, int nb, int deg, int n0, int sb,
+                                            int* cnt, unsigned* first) {
   const int k = nb + (threadIdx.x & 31);
   if (k >= deg) return;
   const int e = (int)__ldg(&I.vnets[base + k]);
@@ -73,14 +73,15 @@ __device__ __forceinline__ void tally_uncut(const DevInstance& I, uint32_t base,
     return;
   }
   atomicAdd(&cnt[p], 1);
-  atomicMin(&first[p], (unsigned long long)k << 32);
+  atomicMin(&first[p], (unsigned)(k - n0) << sb);
 }
 
-// The stream's tally of nets [nb, min(nb + 32, deg)) into cnt / first.
-__device__ __forceinline__ void tally_stream(const DevInstance& I, bool cn, uint32_t base, int nb, int deg, int* cnt,
-                                             unsigned long long* first) {
-  if (cn) tally_uncut(I, base, nb, deg, cnt, first);
-  else tally_batch(I, -1, base, nb, deg, cnt, first);
+// The stream's tally of nets [nb, min(nb + 32, deg)) of the range from n0 into
+// cnt / first (tally_batch's sighting keys).
+__device__ __forceinline__ void tally_stream(const DevInstance& I, bool cn, uint32_t base, int nb, int deg, int n0,
+                                             int sb, int* cnt, unsigned* first) {
+  if (cn) tally_uncut(I, base, nb, deg, n0, sb, cnt, first);
+  else tally_batch(I, -1, base, nb, deg, n0, sb, cnt, first);
 }
 
 __device__ __forceinline__ unsigned long long skey(int round, int pos) {
@@ -215,8 +216,7 @@ __device__ __forceinline__ void place_net(const DevInstance& I, int e, int d, in
 // least-loaded part minpart when no part scores); writes cand, ncand, dec, wt
 // and the weight's mlist entry.  One warp; returns the decision.
 __device__ int decide_position(const DevInstance& I, const SpecBuf& B, const int* sizes_s, int minpart,
-                               const int* cnt, const unsigned long long* first, int o, int wv, int par,
-                               int* nc_out) {
+                               const int* cnt, const unsigned* first, int sb, int o, int wv, int par, int* nc_out) {
   const int lane = threadIdx.x & 31;
   const int K = I.K;
   unsigned long long* cl = B.cand + (size_t)o * K;
@@ -227,8 +227,9 @@ __device__ int decide_position(const DevInstance& I, const SpecBuf& B, const int
     const int c = p < K ? cnt[p] : 0;
     const unsigned m = __ballot_sync(kAll, c > 0);
     if (c > 0) {
-      cl[nc + __popc(m & ((1u << lane) - 1u))] = sc_entry(p, c, first[p]);
-      const LdgKey k{ldg_score(c, sizes_s[p], I.C), sizes_s[p], p, first[p]};
+      const unsigned long long f = wide_key(first[p], sb, 0);
+      cl[nc + __popc(m & ((1u << lane) - 1u))] = sc_entry(p, c, f);
+      const LdgKey k{ldg_score(c, sizes_s[p], I.C), sizes_s[p], p, f};
       if (ldg_better(k, best)) best = k;
     }
     nc += __popc(m);
@@ -343,10 +344,11 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
   int* sizes_s = cv.take<int>(K);
   int* dsz_cta = cv.take<int>(K);
   int* cnt_b = cv.take<int>((size_t)K * kSWarps);
-  unsigned long long* first_b = cv.take<unsigned long long>((size_t)K * kSWarps);
+  unsigned* first_b = reinterpret_cast<unsigned*>(cv.take<unsigned long long>((size_t)K * kSWarps));
   int* sd_b = cv.take<int>(32 * kSWarps);
   int* cnt = cnt_b + (size_t)wib * K;
-  unsigned long long* first = first_b + (size_t)wib * K;
+  unsigned* first = first_b + (size_t)wib * K;
+  const int sb = slot_bits(K);
   int* sd = sd_b + 32 * wib;
   const bool stats = blockIdx.x == 0 && threadIdx.x == 0;
   unsigned long long t0 = stats ? gtimer() : 0ull;
@@ -373,26 +375,36 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
       const int v = __ldg(&S.porder[pos]);
       const uint32_t base = __ldg(&I.vptr[v]);
       const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
-      for (int p = lane; p < K; p += 32) { cnt[p] = 0; first[p] = ~0ull; }
-      __syncwarp();
-      {
-        int n0, n1;
-        net_range(deg, gw, nwarps, &n0, &n1);
-        for (int nb = n0; nb < n1; nb += 32) tally_stream(I, cn, base, nb, n1, cnt, first);
-      }
-      __syncthreads();
-      for (int p = threadIdx.x; p < K; p += blockDim.x) {
-        int c = 0;
-        unsigned long long f = ~0ull;
-        for (int x = 0; x < kSWarps; x++) {
-          c += cnt_b[(size_t)x * K + p];
-          const unsigned long long fx = first_b[(size_t)x * K + p];
-          f = fx < f ? fx : f;
+      // a warp's share in pieces whose sighting keys fit 32 bits (all but always one)
+      const int share = (deg + nwarps - 1) / nwarps, piece = key_nets(sb);
+      for (int a0 = 0; a0 < share; a0 += piece) {
+        for (int p = lane; p < K; p += 32) { cnt[p] = 0; first[p] = ~0u; }
+        __syncwarp();
+        {
+          int n0, n1;
+          net_range(deg, gw, nwarps, &n0, &n1);
+          const int b0 = min(n0 + a0, n1), b1 = min(b0 + piece, n1);
+          for (int nb = b0; nb < b1; nb += 32) tally_stream(I, cn, base, nb, b1, b0, sb, cnt, first);
         }
-        if (c) {
-          atomicAdd(&B.hcnt[p], c);
-          atomicMin(&B.hfirst[p], f);
+        __syncthreads();
+        for (int p = threadIdx.x; p < K; p += blockDim.x) {
+          int c = 0;
+          unsigned long long f = ~0ull;
+          for (int x = 0; x < kSWarps; x++) {
+            const int cx = cnt_b[(size_t)x * K + p];
+            if (cx && f == ~0ull) {   // the warps' shares ascend: the first that saw p saw it first
+              int n0, n1;
+              net_range(deg, blockIdx.x * kSWarps + x, nwarps, &n0, &n1);
+              f = wide_key(first_b[(size_t)x * K + p], sb, n0 + a0);
+            }
+            c += cx;
+          }
+          if (c) {
+            atomicAdd(&B.hcnt[p], c);
+            atomicMin(&B.hfirst[p], f);
+          }
         }
+        __syncthreads();
       }
       if (!grid_barrier(B.bar, I.status)) return;
       if (blockIdx.x == 0) {
@@ -475,12 +487,12 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
       const int v = __ldg(&S.porder[z]);
       const uint32_t base = __ldg(&I.vptr[v]);
       const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
-      for (int p = lane; p < K; p += 32) { cnt[p] = 0; first[p] = ~0ull; }
+      for (int p = lane; p < K; p += 32) { cnt[p] = 0; first[p] = ~0u; }
       __syncwarp();
-      for (int nb = 0; nb < deg; nb += 32) tally_stream(I, cn, base, nb, deg, cnt, first);
+      for (int nb = 0; nb < deg; nb += 32) tally_stream(I, cn, base, nb, deg, 0, sb, cnt, first);
       __syncwarp();
       int nc;
-      const int d = decide_position(I, B, sizes_s, s_minpart, cnt, first, o, __ldg(&I.w[v]), par, &nc);
+      const int d = decide_position(I, B, sizes_s, s_minpart, cnt, first, sb, o, __ldg(&I.w[v]), par, &nc);
       // CN: a position without candidates decides by the sizes alone; it
       // claims all its nets, so that a changed decision adds no claim
       const int napp = record_slots(I, B, S, base, 0, deg, d, round, z, sd, cn && nc == 0);
@@ -499,25 +511,14 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
         int n0, n1;
         net_range(deg, wib, kSWarps, &n0, &n1);
         __syncthreads();   // the tallies of the CTA's previous position are read
-        for (int p = lane; p < K; p += 32) { cnt[p] = 0; first[p] = ~0ull; }
-        __syncwarp();
-        for (int nb = n0; nb < n1; nb += 32) tally_stream(I, cn, base, nb, n1, cnt, first);
+        // one set of arrays for the CTA's warps (a vertex here has fewer than kStreamHeavy nets)
+        for (int p = threadIdx.x; p < K; p += blockDim.x) { cnt_b[p] = 0; first_b[p] = ~0u; }
         __syncthreads();
-        for (int p = threadIdx.x; p < K; p += blockDim.x) {   // warp 0's arrays hold the sums
-          int c = 0;
-          unsigned long long f = ~0ull;
-          for (int x = 0; x < kSWarps; x++) {
-            c += cnt_b[(size_t)x * K + p];
-            const unsigned long long fx = first_b[(size_t)x * K + p];
-            f = fx < f ? fx : f;
-          }
-          cnt_b[p] = c;
-          first_b[p] = f;
-        }
+        for (int nb = n0; nb < n1; nb += 32) tally_stream(I, cn, base, nb, n1, 0, sb, cnt_b, first_b);
         __syncthreads();
         if (wib == 0) {
           int nc;
-          const int d = decide_position(I, B, sizes_s, s_minpart, cnt_b, first_b, o, __ldg(&I.w[v]), par, &nc);
+          const int d = decide_position(I, B, sizes_s, s_minpart, cnt_b, first_b, sb, o, __ldg(&I.w[v]), par, &nc);
           if (lane == 0) {
             s_dec = d;
             s_nc = nc;
