@@ -1056,7 +1056,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
           {
             int n0, n1;
             net_range(deg_s, gw, nwarps, &n0, &n1);
-            const int b0 = min(n0 + a0, n1), b1 = min(b0 + piece, n1);
+            const int b0 = n0 + min(a0, n1 - n0), b1 = b0 + min(piece, n1 - b0);
             for (int nb = b0; nb < b1; nb += 32) c1 += tally_batch(I, own_s, base_s, nb, b1, b0, sb, cnt, first);
           }
           c1 = warp_sum(c1);

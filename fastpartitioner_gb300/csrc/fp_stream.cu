@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
         {
           int n0, n1;
           net_range(deg, gw, nwarps, &n0, &n1);
-          const int b0 = min(n0 + a0, n1), b1 = min(b0 + piece, n1);
+          const int b0 = n0 + min(a0, n1 - n0), b1 = b0 + min(piece, n1 - b0);
           for (int nb = b0; nb < b1; nb += 32) tally_stream(I, cn, base, nb, b1, b0, sb, cnt, first);
         }
         __syncthreads();
