@@ -86,6 +86,7 @@ int default_grid_verts(int metric) {
   }
 }
 constexpr int kMaxSpecWarps = 16384;
+constexpr int kCtlWords = 12;   // SpecBuf::ctl
 cudaError_t launch_metrics(const DevInstance& I, void* scratch, long long* out, int num_sms, cudaStream_t st,
                            int* launches);
 }  // namespace fp
@@ -563,7 +564,7 @@ static int build_positions(fp_instance* in) {
   // windows end every few dozen positions (max-volume changes, in-window
   // fixes) and a window of compacted positions wastes more evaluations past
   // its cut -- so only TV walks compacted positions.
-  compact = compact && any_iso && pb.metric == FP_METRIC_TV;
+  compact = compact && any_iso;
   for (int z = 0; z < g.nov; z++) {
     const int v = pb.order[z];
     if (compact && g.vptr[v + 1] == g.vptr[v]) {
@@ -697,7 +698,6 @@ int fp_instance_create(fp_ctx* ctx, const fp_hypergraph* h, int32_t K, int32_t m
     const bool msg = metric == FP_METRIC_TM || metric == FP_METRIC_MSM;
     const bool cn = metric == FP_METRIC_CN;
     const bool ldg = !msg && !cn;
-    const bool vfix = metric == FP_METRIC_MSV || metric == FP_METRIC_MSRV;   // in-window decision fixes
     // exact count claims of the LDG engine: a table well above the entries of a
     // round (two per count-only net of a window's movers)
     size_t ctab = 4096;
@@ -713,7 +713,7 @@ int fp_instance_create(fp_ctx* ctx, const fp_hypergraph* h, int32_t K, int32_t m
         (rc = dalloc(in, &d.zrow, msg ? K * words : 1)) || (rc = dalloc(in, &d.zcol, msg ? K * words : 1)) ||
         (rc = dalloc(in, &d.c1row, msg ? K * words : 1)) || (rc = dalloc(in, &d.c1col, msg ? K * words : 1)) ||
         (rc = dalloc(in, &d.moves, kMaxPasses)) || (rc = dalloc(in, &d.status, 1)) ||
-        (rc = dalloc(in, &in->sb.ctl, 8)) || (rc = dalloc(in, &in->sb.bar, 4)) || (rc = dalloc(in, &in->sb.stats, kNumStats)) || (rc = dalloc(in, &in->sb.dec, std::max(kSpecWindow, kMsgWindow))) ||
+        (rc = dalloc(in, &in->sb.ctl, kCtlWords)) || (rc = dalloc(in, &in->sb.bar, 4)) || (rc = dalloc(in, &in->sb.stats, kNumStats)) || (rc = dalloc(in, &in->sb.dec, std::max(kSpecWindow, kMsgWindow))) ||
         (rc = dalloc(in, &in->sb.flag, kSpecWindow)) || (rc = dalloc(in, &in->sb.slack, kSpecWindow)) ||
         (rc = dalloc(in, &in->sb.vslack, kSpecWindow)) || (rc = dalloc(in, &in->sb.wt, kSpecWindow)) ||
         (rc = dalloc(in, &in->sb.vd, kSpecWindow)) || (rc = dalloc(in, &in->sb.scan, (size_t)kSpecWindow * words)) ||
@@ -723,14 +723,14 @@ int fp_instance_create(fp_ctx* ctx, const fp_hypergraph* h, int32_t K, int32_t m
         (rc = dalloc(in, &in->sb.ctab_key, ldg ? ctab : 1)) || (rc = dalloc(in, &in->sb.ctab_pos, ldg ? ctab : 1)) ||
         (rc = dalloc(in, &in->sb.ctab_cnt, ldg ? ctab : 1)) ||
         (rc = dalloc(in, &in->sb.ctab_over, 2)) || (rc = dalloc(in, &in->sb.dfix, kSpecWindow)) ||
-        (rc = dalloc(in, &in->sb.rec_slot2, vfix ? g.pins : 1)) ||
+        (rc = dalloc(in, &in->sb.rec_slot2, ldg ? g.pins : 1)) ||
         (rc = dalloc(in, &in->sb.cn_moved, cn ? g.pins : 1)) || (rc = dalloc(in, &in->sb.cn_kcnt, cn ? g.noe : 1)) ||
         (rc = dalloc(in, &in->sb.cn_nets, cn ? g.noe : 1)) || (rc = dalloc(in, &in->sb.cn_cnt, 4)) ||
         (rc = dalloc(in, &in->sb.cn_wit, cn ? g.nov : 1)) || (rc = dalloc(in, &in->vclass_d, g.nov)) ||
         (rc = dalloc(in, &in->sb.cand, (size_t)kSpecWindow * K)) || (rc = dalloc(in, &in->sb.ncand, kSpecWindow)) ||
         (rc = dalloc(in, &in->sb.mlist, kSpecWindow)) || (rc = dalloc(in, &in->sb.midx, kSpecWindow)) ||
         (rc = dalloc(in, &in->sb.mcnt, 2)) ||
-        (rc = dalloc(in, &in->sb.wsum, kMaxSpecWarps)) || (rc = dalloc(in, &in->sb.vsum, kMaxSpecWarps)) ||
+        (rc = dalloc(in, &in->sb.acc, kSpecWindow)) ||
         (rc = dalloc(in, &in->sb.claim_m, g.noe)) || (rc = dalloc(in, &in->sb.claim64, g.noe)) || (rc = dalloc(in, &in->sb.claim_c, g.noe)) ||
         (rc = dalloc(in, &in->sb.mask_c, g.noe)) || (rc = dalloc(in, &in->sb.hcnt, 2 * kMaxGridVerts * K)) ||
         (rc = dalloc(in, &in->sb.hfirst, 2 * kMaxGridVerts * K)) ||
@@ -846,7 +846,6 @@ int fp_instance_footprint(int32_t nov, int32_t noe, int64_t pins, int32_t K, int
     const bool msg = metric == FP_METRIC_TM || metric == FP_METRIC_MSM;
     const bool cn = metric == FP_METRIC_CN;
     const bool ldg = !msg && !cn;
-    const bool vfix = metric == FP_METRIC_MSV || metric == FP_METRIC_MSRV;
     size_t ctab = 4096;
     while (ctab < (size_t)2 * noe && ctab < ((size_t)1 << 21)) ctab <<= 1;
     const size_t P = (size_t)pins, V = (size_t)nov, E = (size_t)noe, G2K = 2 * (size_t)kMaxGridVerts * K;
@@ -861,18 +860,18 @@ int fp_instance_footprint(int32_t nov, int32_t noe, int64_t pins, int32_t K, int
     for (int k = 0; k < 4; k++) add(msg ? K * words : 1, 4);  // zero and conn == 1 masks
     add(kMaxPasses, 8); add(1, 4);                           // moves, status
     // speculation scratch
-    add(8, 4); add(4, 4); add(kNumStats, 8); add(std::max(kSpecWindow, kMsgWindow), 4);
+    add(kCtlWords, 4); add(4, 4); add(kNumStats, 8); add(std::max(kSpecWindow, kMsgWindow), 4);
     add(W, 1); add(W, 4); add(W, 4); add(W, 4); add(W, 4);   // flag, slack, vslack, wt, vd
     add(W * words, 4);                                       // scan
     add(std::max(kSpecWindow, kMsgWindow), 4); add(std::max(kSpecWindow, kMsgWindow), 4);   // rgain, rloss
     add(ldg ? P : 1, 4); add(ldg ? P : 1, 8);                // rec, rec_slot
     add(ldg ? ctab : 1, 8); add(ldg ? ctab : 1, 4); add(ldg ? ctab : 1, 4);
     add(2, 4); add(W, 4);                                    // ctab_over, dfix
-    add(vfix ? P : 1, 8);                                    // rec_slot2
+    add(ldg ? P : 1, 8);                                     // rec_slot2
     add(cn ? P : 1, 8); add(cn ? E : 1, 4); add(cn ? E : 1, 8); add(4, 4); add(cn ? V : 1, 4);
     add(V, 1);                                               // vertex classes
     add(W * K, 8); add(W, 4); add(W, 16); add(W, 4); add(2, 4);   // cand, ncand, mlist, midx, mcnt
-    add(kMaxSpecWarps, 4); add(kMaxSpecWarps, 4);            // wsum, vsum
+    add(W, 4);                                               // acc
     add(E, 4); add(E, 8); add(E, 4); add(E, 4);              // claim_m, claim64, claim_c, mask_c
     add(G2K, 4); add(G2K, 8); add(G2K, 4); add(G2K, 4); add(G2K, 4);
     add(16 * (size_t)kMaxGridVerts, 4); add(K, 8);           // hmisc, mlast
@@ -924,8 +923,8 @@ static int device_stream(fp_instance* in) {
   const HostGraph& g = in->g;
   const int K = in->pb.K;
   DevInstance& d = in->d;
-  static const int none[8] = {0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff,
-                              0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff};
+  static const int none[kCtlWords] = {0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff,
+                                      0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff};
   cudaError_t e = cudaMemsetAsync(d.part_vec, 0xff, sizeof(int) * g.nov, s);
   auto zero = [&](void* p, size_t bytes, int val) {
     if (e == cudaSuccess && bytes) e = cudaMemsetAsync(p, val, bytes, s);
@@ -1069,8 +1068,8 @@ int fp_refine(fp_instance* in, int32_t passes) {
     in->d.recs = spec ? in->recs : nullptr;
     in->recs_valid = false;
     if (spec) {
-      static const int none[8] = {0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff,
-                                  0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff};
+      static const int none[kCtlWords] = {0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff,
+                                      0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff};
       if (e == cudaSuccess) e = cudaMemcpyAsync(in->sb.ctl, none, sizeof(none), cudaMemcpyHostToDevice, s);
       if (e == cudaSuccess) e = cudaMemsetAsync(in->sb.bar, 0, sizeof(unsigned) * 4, s);
       if (e == cudaSuccess && (in->fault_leave_at || in->fault_poll_limit)) {

@@ -94,16 +94,18 @@ constexpr int kMaxGridVerts = 8;
 // instance.
 struct SpecBuf {
   unsigned* bar;         // [4] grid barrier: arrivals, generation, abort
-  int* ctl;              // [8] per-round words: [2,3] first max-touching mover (by round
-                         //     parity), [4,5] cut (by validation pass parity)
+  int* ctl;              // [12] per-round words: [2,3] first max-touching mover, [4,5] cut,
+                         //     [6,7] first changed decision (by round parity), [0,1] the
+                         //     walk's end and changes, [8,9] misprediction (by walk parity)
   int* dec;              // [wmax] (own part << 16) | decision per window offset
   unsigned char* flag;   // [wmax] bit0 mover, bit1 stale-marker risk, bit2 CTA / grid evaluated,
-                         //     bit3 isolated, bit4 accepted, bit5 decision fixed exact in the
-                         //     window, bit6 claims of a replaced move held (rec_slot2)
-  int* dfix;             // [wmax] exact decision of a position whose size check failed
+                         //     bit3 no nets, bit4 accepted, bit5 decision changed in the
+                         //     window, bit6 claims of a replaced move held (rec_slot2),
+                         //     bit7 the last walk changed the decision (dfix)
+  int* dfix;             // [wmax] (predicted mover << 16) | exact decision the walk took
   int* slack;            // [wmax] part-size drift the decision tolerates (-1: none)
   int* vslack;           // [wmax] volume drift the accept/reject outcome tolerates
-  int* wt;               // [wmax] weight moved by a mover (0 otherwise)
+  int* wt;               // [wmax] vertex weight (streams: of the placed vertex)
   int* vd;               // [wmax] largest volume change of one part by a mover
   int* rgain;            // [wmax] decision-record gain / loss of each window offset (with
   int* rloss;            //     the decision log on)
@@ -114,12 +116,12 @@ struct SpecBuf {
                                 //     2: evaluated by the whole grid
   unsigned long long* cand;  // [wmax * K] LDG candidates per window offset (part, count, first)
   int* ncand;            // [wmax]
-  int4* mlist;           // [wmax] the round's movers (any order): window offset, weight,
-                         //     (own part << 16) | destination
+  int4* mlist;           // [wmax] the round's movers (streams: placements), any order: window
+                         //     offset, weight, (own part << 16) | destination, volume change
   int* midx;             // [wmax] index of a mover's mlist entry, by window offset
   int* mcnt;             // [2] their count, double-buffered by round parity
-  int* wsum;             // [max_warps] per-warp sums of wt
-  int* vsum;             // [max_warps] per-warp sums of vd
+  int* acc;              // [wmax] TV: leave gain minus the vertex's nets (it moves to d iff
+                         //     acc + the nets listing d >= 0)
   unsigned long long* claim64;  // [noe] (round << 32) | ~position of the first claim (CN)
   int2* cn_moved;        // [pins] CN: (pin, window offset of its acting net) of pins to move
   int* cn_kcnt;          // [noe] CN: pins of the round's moves per net (zero between rounds)
@@ -133,7 +135,7 @@ struct SpecBuf {
   int* ctab_pos;         // [ctab_mask + 1] first position of a count-only mover with that (net, part)
   int* ctab_cnt;         // [ctab_mask + 1] count-only movers of the round on that (net, part)
   uint2* rec_slot;       // [pins] table slots of a count-only move's (net, own) and (net, new part)
-  uint2* rec_slot2;      // [pins] (MSV / MSRV) those of a move replaced by an in-window fix
+  uint2* rec_slot2;      // [pins] those of a move that a changed decision replaced
   int* ctab_over;        // [2] a probe ran past its bound this round (by round parity)
   unsigned ctab_mask;
   const int* heavy_pos;  // positions (visiting order, ascending) of vertices evaluated by
@@ -152,7 +154,7 @@ struct SpecBuf {
   int gmax;              // whole-grid vertices one window may hold (1 .. kMaxGridVerts)
   int wgrow;             // LDG window after a cut: this many times the last valid length,
   int wmin;              //   at least this many positions
-  int maxfix;            // in-window decision fixes per window (MSV / MSRV)
+  int maxfix;            // walks per window (mispredicted outcomes start another)
   // LDG engine positions: the vertices walked in windows, in visiting order.
   // When every vertex without nets weighs 0 they are left out of the
   // positions (porder holds the others) and decided after each window:

@@ -36,6 +36,8 @@
 
 #include "fp_spec_common.cuh"
 
+#include <algorithm>
+
 namespace fp {
 
 namespace {
@@ -75,18 +77,22 @@ __device__ __forceinline__ int slack_divf(float a, float b) {
 }
 
 // Candidate entry of a part for the exact re-check: part (12 bits), count
-// without the vertex itself (16 bits), first sighting (net index, 16 bits;
-// slot, 20 bits).  A vertex whose count or first net index does not fit (one
-// with 65536 nets or more) stores no list: ncand = -1.
-__device__ __forceinline__ unsigned long long cand_entry(int p, int c, unsigned long long f) {
-  return ((unsigned long long)p << 52) | ((unsigned long long)c << 36) | (((f >> 32) & 0xffffull) << 20) |
-         (f & 0xfffffull);
+// without the vertex itself (16 bits), 32-bit sighting key.  A vertex whose
+// count or first net index does not fit (one with 65536 nets or more) stores
+// no list: ncand = -1.
+__device__ __forceinline__ unsigned long long cand_entry(int p, int c, unsigned f) {
+  return ((unsigned long long)p << 52) | ((unsigned long long)c << 36) | f;
 }
 
 // A sighting key (32-bit, of a vertex one warp or CTA tallied) or a 64-bit key
 // of absolute net indexes as (net index << 32 | slot).
 __device__ __forceinline__ unsigned long long key64(unsigned f, int sb) { return wide_key(f, sb, 0); }
 __device__ __forceinline__ unsigned long long key64(unsigned long long f, int) { return f; }
+__device__ __forceinline__ unsigned key32(unsigned f, int, bool*) { return f; }
+__device__ __forceinline__ unsigned key32(unsigned long long f, int sb, bool* wide) {
+  *wide |= (f >> 32) > 0xffffull;
+  return ((unsigned)(f >> 32) << sb) | (unsigned)f;
+}
 __device__ __forceinline__ unsigned min_key(unsigned f) { return __reduce_min_sync(kAll, f); }
 __device__ __forceinline__ unsigned long long min_key(unsigned long long f) { return warp_min_u64(f); }
 
@@ -133,9 +139,8 @@ __device__ int ldg_decide(const DevInstance& I, const RoundCtx& R, const int* cn
       const int i = nc + __popc(m & below);
       list[i] = p;
       if (cand) {
-        const unsigned long long f = key64(first[p], sb);
-        wide |= c > 0xffff || (f >> 32) > 0xffffull;
-        cand[i] = cand_entry(p, c - (p == own ? 1 : 0), f);
+        wide |= c > 0xffff;
+        cand[i] = cand_entry(p, c - (p == own ? 1 : 0), key32(first[p], sb, &wide));
       }
     }
     if (scan) {
@@ -261,104 +266,6 @@ __device__ int ldg_decide(const DevInstance& I, const RoundCtx& R, const int* cn
   return d;
 }
 
-// The LDG decision of the vertex at window offset o again, from its stored
-// candidates and the exact part sizes at that position: round-start sizes plus
-// the moves of the window's movers before o -- those before offset o_from
-// already summed per part in dsz_cta (the CTA's share), the rest read from the
-// window records -- gathered in the warp's K-int scratch dsz.  One warp.
-// Returns -1 if the vertex has no candidate list (65536 nets or more).
-__device__ int ldg_recheck(const DevInstance& I, const RoundCtx& R, const SpecBuf& B, int o, int own, int metric,
-                           int* dsz, const int* dsz_cta, int o_from) {
-  const int lane = threadIdx.x & 31;
-  const int K = I.K;
-  for (int p = lane; p < K; p += 32) dsz[p] = dsz_cta[p];
-  __syncwarp();
-  for (int o2 = o_from + lane; o2 < o; o2 += 32) {
-    const int w = lds(&B.wt[o2]);   // 0 unless a mover
-    const int pk = lds(&B.dec[o2]);
-    if (w == 0) continue;
-    atomicAdd(&dsz[pk & 0xffff], w);
-    atomicAdd(&dsz[pk >> 16], -w);
-  }
-  __syncwarp();
-  const unsigned long long* cl = B.cand + (size_t)o * K;
-  const int nc = lds(&B.ncand[o]);
-  if (nc < 0) return -1;   // no list (65536 nets or more): the caller cuts
-  // Float scores first: the float penalty 1 - sz / C is off by less than
-  // 4e-7 * (1 + sz / C), so a score of count c by less than c times that; the
-  // bound used is 1e-6 * c * (1 + sz / C).  The near candidates are then ordered
-  // as in ldg_decide (one left, or one count: by size and first sighting;
-  // otherwise exact double scores).  The first 32 entries stay in registers.
-  const float Cf = R.Cf;
-  const unsigned long long e0 = lane < nc ? lds(&cl[lane]) : 0;
-  auto ent_at = [&](int i) { return i < 32 ? e0 : lds(&cl[i]); };
-  auto size_of = [&](int p) { return R.sizes[p] + dsz[p]; };
-  float fb = 0.0f;
-  for (int i = lane; i < nc; i += 32) {
-    const unsigned long long ent = ent_at(i);
-    const int c = (int)((ent >> 36) & 0xffffull);
-    const float xf = __fdiv_rn((float)size_of((int)(ent >> 52)), Cf);
-    fb = fmaxf(fb, __fmul_rn((float)c, 1.0f - xf) - (float)c * 1e-6f * (1.0f + fabsf(xf)));
-  }
-  fb = warp_max_nonneg(fb);
-  int nnear = 0, np = -1, nsz = 0, cmin = 0x7fffffff, cmax = 0;
-  unsigned long long nf = ~0ull;   // the entry's low 36 bits order like the first sighting
-  for (int i = lane; i < nc; i += 32) {
-    const unsigned long long ent = ent_at(i);
-    const int p = (int)(ent >> 52);
-    const int c = (int)((ent >> 36) & 0xffffull);
-    const int sz = size_of(p);
-    const float xf = __fdiv_rn((float)sz, Cf);
-    if (c == 0 || __fmul_rn((float)c, 1.0f - xf) + (float)c * 1e-6f * (1.0f + fabsf(xf)) < fb) continue;
-    nnear++;
-    cmin = min(cmin, c);
-    cmax = max(cmax, c);
-    const unsigned long long f = ent & 0xfffffffffull;
-    if (np < 0 || sz < nsz || (sz == nsz && f < nf)) {
-      np = p;
-      nsz = sz;
-      nf = f;
-    }
-  }
-  const int tot = warp_sum(nnear);
-  cmin = warp_min(cmin);
-  cmax = warp_max(cmax);
-  LdgKey best{-1.0, 0, -1, ~0ull};
-  if (fb > 0.0f && (tot == 1 || cmin == cmax)) {
-    best.part = least_size_first<unsigned long long>(nsz, nf, np);
-  } else if (tot > 0) {
-    for (int i = lane; i < nc; i += 32) {
-      const unsigned long long ent = ent_at(i);
-      const int p = (int)(ent >> 52);
-      const int c = (int)((ent >> 36) & 0xffffull);
-      const int sz = size_of(p);
-      const float xf = __fdiv_rn((float)sz, Cf);
-      if (c == 0 || __fmul_rn((float)c, 1.0f - xf) + (float)c * 1e-6f * (1.0f + fabsf(xf)) < fb) continue;
-      const unsigned long long f = (((ent >> 20) & 0xffffull) << 32) | (ent & 0xfffffull);
-      const double pen = __dsub_rn(1.0, __ddiv_rn((double)sz, I.C));
-      LdgKey k{__dmul_rn((double)c, pen), sz, p, f};
-      if (ldg_better(k, best)) best = k;
-    }
-    best = warp_ldg_argmax(best);
-  }
-  int d0 = best.part;
-  if (d0 < 0) {
-    unsigned long long mk = ~0ull;
-    for (int p = lane; p < K; p += 32) {
-      const unsigned long long key = ((unsigned long long)((unsigned)size_of(p) ^ 0x80000000u) << 32) | (unsigned)p;
-      mk = key < mk ? key : mk;
-    }
-    d0 = (int)(warp_min_u64(mk) & 0xffffffffu);
-  }
-  int d = d0;
-  if (metric == kTV) {
-    if (R.sizes[d] + dsz[d] > I.max_pw) d = own;
-    if (R.sizes[d] + dsz[d] < I.min_pw) d = own;
-  }
-  __syncwarp();
-  return d;
-}
-
 // The reference's gains / losses of the move own -> d on net e
 // (MGV/partition.cpp:294-337, MSRV/partition.cpp:303-350) and the exact change
 // of every part's volume that commit_rec will make (adelta), from the net's
@@ -413,17 +320,21 @@ __device__ __forceinline__ void net_terms(const DevInstance& I, bool rv, int v, 
 // Records of v's nets for the move own -> d; warp wi of a group of nw warps
 // takes a contiguous share of the nets (net_range).  With volumes (MSV / MSRV) the
 // gain / loss / volume terms are added to the warp's arrays.  loc: the warp's
-// 96 ints of scratch.
-__device__ void locate_all(const DevInstance& I, const SpecBuf& B, int metric, int v, int own, int d,
+// 96 ints of scratch.  Returns this lane's counts of nets the move takes own
+// off (low 16 bits) and appends d to (high 16), TV's leave gain and arrival loss.
+__device__ int locate_all(const DevInstance& I, const SpecBuf& B, int metric, int v, int own, int d,
                            uint32_t base, int deg, int wi, int nw, int* loc, int* gains, int* losses, int* adelta) {
   const bool vol = metric != kTV, rv = metric == kMSRV;
   int n0, n1;
   net_range(deg, wi, nw, &n0, &n1);
+  int ra = 0;
   for (int nb = n0; nb < n1; nb += 32) {
     int e;
     const uint32_t r = locate_batch(I, B.rec, v, own, d, base, nb, n1, loc, loc + 32, loc + 64, &e);
+    if (e >= 0) ra += (rec_rem(r) ? 1 : 0) + (rec_add(r) ? 1 << 16 : 0);
     if (vol && e >= 0) net_terms(I, rv, v, own, d, e, r, gains, losses, adelta);
   }
+  return ra;
 }
 
 // Count claims, exactly: an open-addressed table from (net, part) to the first
@@ -491,10 +402,11 @@ __device__ __forceinline__ void claim_nets(const DevInstance& I, const SpecBuf& 
   }
 }
 
-// Appends a mover of window offset o to the round's list.
-__device__ __forceinline__ void list_mover(const SpecBuf& B, int par, int o, int wv, int pk) {
+// Appends a mover of window offset o (weight wv, largest volume change vd) to
+// the round's list.
+__device__ __forceinline__ void list_mover(const SpecBuf& B, int par, int o, int wv, int pk, int vd) {
   const int i = atomicAdd(&B.mcnt[par], 1);
-  B.mlist[i] = make_int4(o, wv, pk, 0);
+  B.mlist[i] = make_int4(o, wv, pk, vd);
   B.midx[o] = i;
 }
 
@@ -623,8 +535,8 @@ __device__ __forceinline__ int block_reduce_min(int x, int* scr) {
 // shared-memory atomics): nothing is merged per warp.  Writes the same
 // per-position record as a warp evaluation (flag bit 2 marks it).
 __device__ void cta_eval_ldg(const DevInstance& I, const SpecBuf& B, const RoundCtx& R, int metric, int z, int pos,
-                             int par, int q, int sb, int* cnt_b, unsigned* first_b, int* gains_b, int* losses_b,
-                             int* adelta_b, int* iscr, int* s_mw, int* s_mv, int* loc_b, bool logp) {
+                             int par, int sb, int* cnt_b, unsigned* first_b, int* gains_b, int* losses_b,
+                             int* adelta_b, int* iscr, int* loc_b, bool logp) {
   __shared__ int sh[4];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int K = I.K;
@@ -708,17 +620,17 @@ __device__ void cta_eval_ldg(const DevInstance& I, const SpecBuf& B, const Round
     claim_nets(I, B, vol, z, own, d, base, deg, threadIdx.x, blockDim.x, par);
     if (threadIdx.x == 0) {
       if (mt) atomicMin(&B.ctl[2 + par], z);
-      list_mover(B, par, o, __ldg(&I.w[v]), (own << 16) | d);
+      list_mover(B, par, o, __ldg(&I.w[v]), (own << 16) | d, vdd);
     }
   }
   if (threadIdx.x == 0) {
-    const int wv = mover ? __ldg(&I.w[v]) : 0;
     if (logp) { B.rgain[o] = rg; B.rloss[o] = rl; }
     B.dec[o] = (own << 16) | d;
     B.flag[o] = (unsigned char)((mover ? 1 : 0) | (special ? 2 : 0) | 4);
     B.slack[o] = slack;
     B.vslack[o] = vs;
-    B.wt[o] = wv;
+    B.wt[o] = __ldg(&I.w[v]);
+    B.acc[o] = c1t - deg;
     B.vd[o] = mover ? vdd : 0;
     // CTA evaluation statistics (cycles): tally and merge / decision / the rest
     const long long t3 = clock64();
@@ -728,138 +640,610 @@ __device__ void cta_eval_ldg(const DevInstance& I, const SpecBuf& B, const Round
       atomicAdd(&B.stats[31], (unsigned long long)(t3 - t2));
       atomicAdd(&B.stats[40], 1ull);
     }
-    const int owner = o / q - (int)blockIdx.x * kSWarps;   // warp of this CTA owning position z
-    s_mw[owner] += wv;
-    s_mv[owner] += mover ? vdd : 0;
   }
   __syncthreads();
 }
 
-// Validation of a medium vertex by the whole CTA (the warp validation's rules).
-__device__ void cta_validate_ldg(const DevInstance& I, const SpecBuf& B, const RoundCtx& R, int metric, int z, int pos,
-                                 int q, int par, int mtpos, long long pre_w, long long pre_v, const int* cw,
-                                 const int* cv, int* dsz, const int* dsz_cta, int o_from, bool check_nets,
-                                 int* cut) {
-  __shared__ long long shd[2];
-  __shared__ int shw;
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int o = z - pos;
-  const int fl = lds(&B.flag[o]);
-  const int pk = lds(&B.dec[o]);
-  const int own = pk >> 16, d = pk & 0xffff;
-  const int v = __ldg(&B.porder[z]);
-  if (wib == 0) {
-    // drift before z: earlier CTAs, this CTA's warps before the owner (cw / cv),
-    // the owner's positions before z
-    const int owner = o / q;
-    long long D = 0, V = 0;
-    for (int x = lane; x < owner - (int)blockIdx.x * kSWarps; x += 32) {
-      D += cw[x];
-      V += cv[x];
+// The window's positions as the walk stages them in shared memory: the words of
+// up to kWalkLoad positions, per 32 of them what a drift of the sizes has to
+// exceed to matter, and the first kWalkRow candidate entries of kWalkSub
+// positions (rows padded so that four rows read side by side meet no bank
+// conflict).
+constexpr int kWalkLoad = 1024, kWalkSub = 128, kWalkRow = 64, kWalkStride = kWalkRow + 8;
+struct WalkSmem {
+  unsigned long long ent[kWalkSub * kWalkStride];
+  int4 meta[kWalkLoad];      // (own << 16) | decision, weight, acc, (ncand << 8) | flag
+  int margin[kWalkLoad];     // drift at its group's start the position tolerates (-1: always taken again)
+  int gmin[kWalkLoad / 32];  // per group of 32: the smallest margin,
+  unsigned gsum[kWalkLoad / 32];   //   the weight its movers move
+  int nd[32], nslack[32];    // decisions taken again: (nets listing it << 13) | part (-1: no list), drift tolerated
+  unsigned drift;            // largest change of one part's size so far (an upper bound)
+  int group;                 // group to decide again (-1: none left), and its positions
+  unsigned need;
+};
+
+// Least-loaded part of sz, lowest index on ties (one warp); *ms its size.
+__device__ __forceinline__ int warp_least_loaded(const int* sz, int K, int* ms_out) {
+  const int lane = threadIdx.x & 31;
+  int ms = 0x7fffffff, mp = 0x7fffffff;
+  for (int p = lane; p < K; p += 32) {
+    const int x = sz[p];
+    if (x < ms || mp == 0x7fffffff) { ms = x; mp = p; }
+  }
+  const int m = warp_min(ms);
+  *ms_out = m;
+  return warp_min(mp != 0x7fffffff && ms == m ? mp : 0x7fffffff);
+}
+
+// Penalty of a part as the walk scores it: 1 - size / C from the rounded 1 / C,
+// off by less than 4e-7 * (1 + size / C), and the bound 1e-6 * (1 + size / C)
+// used for it (per count of nets).
+__device__ __forceinline__ float2 walk_pen(int size, float rC) {
+  const float xf = __fmul_rn((float)size, rC);
+  return make_float2(1.0f - xf, 1e-6f * (1.0f + fabsf(xf)));
+}
+// Drift bound floor(a / b) - 2 at least, from below, capped; -1 if not positive.
+__device__ __forceinline__ int walk_slack(float a, float b) {
+  const float x = __fdividef(a, b) * (1.0f - 2e-5f) - 2.0f;
+  return !(x > -1.0f) ? -1 : x > 1.0e9f ? kBig : (int)x;
+}
+
+// One warp decides a position again with the sizes sz, whatever its candidates:
+// mt its words, cl all of its entries; exact double scores (TV/partition.cpp:
+// 103-104) unless the near ones share a count.  Returns the decision before
+// TV's clamps, (nets listing it << 13) | part; it tolerates no drift.
+__device__ __noinline__ int walk_pick_any(const DevInstance& I, float rC, const int* sz, int nc,
+                                          const unsigned long long* cl) {
+  const int lane = threadIdx.x & 31;
+  const int K = I.K;
+  const unsigned long long e0 = lane < nc ? lds(&cl[lane]) : 0;   // the first 32 stay in registers
+  float fb = 0.0f;
+  for (int i = lane; i < nc; i += 32) {
+    const unsigned long long e = i < 32 ? e0 : lds(&cl[i]);
+    const int c = (int)((e >> 36) & 0xffffull);
+    const float2 w = walk_pen(sz[(int)(e >> 52)], rC);
+    fb = fmaxf(fb, (float)c * w.x - (float)c * w.y);
+  }
+  fb = warp_max_nonneg(fb);
+  int np = -1, nsz = 0, cmin = 0x7fffffff, cmax = 0;
+  unsigned nf = ~0u;
+  for (int i = lane; i < nc; i += 32) {
+    const unsigned long long e = i < 32 ? e0 : lds(&cl[i]);
+    const int p = (int)(e >> 52), c = (int)((e >> 36) & 0xffffull), s = sz[p];
+    const float2 w = walk_pen(s, rC);
+    if (c == 0 || (float)c * w.x + (float)c * w.y < fb) continue;
+    cmin = min(cmin, c);
+    cmax = max(cmax, c);
+    if (np < 0 || s < nsz || (s == nsz && (unsigned)e < nf)) { np = p; nsz = s; nf = (unsigned)e; }
+  }
+  cmin = warp_min(cmin);
+  cmax = warp_max(cmax);
+  int dn = -1, cd = 0;
+  if (fb > 0.0f && cmin == cmax) {
+    dn = least_size_first<unsigned>(nsz, nf, np);
+    cd = cmax;
+  } else if (cmax > 0) {
+    LdgKey best{-1.0, 0, -1, ~0ull};
+    int bc = 0;
+    for (int i = lane; i < nc; i += 32) {
+      const unsigned long long e = i < 32 ? e0 : lds(&cl[i]);
+      const int p = (int)(e >> 52), c = (int)((e >> 36) & 0xffffull), s = sz[p];
+      const float2 w = walk_pen(s, rC);
+      if (c == 0 || (float)c * w.x + (float)c * w.y < fb) continue;
+      const LdgKey k{ldg_score(c, s, I.C), s, p, e & 0xffffffffull};
+      if (ldg_better(k, best)) { best = k; bc = c; }
     }
-    for (int o2 = owner * q + lane; o2 < o; o2 += 32) {
-      D += lds(&B.wt[o2]);
-      V += lds(&B.vd[o2]);
-    }
-    D = warp_sum64(D);
-    V = warp_sum64(V);
-    if (lane == 0) {
-      shd[0] = pre_w + D;
-      shd[1] = pre_v + V;
-      shw = ((fl & 2) && z != pos) ? 1 : 0;
+    const int mine = best.part;
+    best = warp_ldg_argmax(best);
+    if (best.part >= 0) {
+      dn = best.part;
+      cd = __shfl_sync(kAll, bc, __ffs(__ballot_sync(kAll, mine == dn)) - 1);
     }
   }
+  if (dn < 0) {
+    // no part scores: the least-loaded one, and the nets listing it all the same
+    int ms, cx = 0;
+    dn = warp_least_loaded(sz, K, &ms);
+    for (int i = lane; i < nc; i += 32) {
+      const unsigned long long e = i < 32 ? e0 : lds(&cl[i]);
+      if ((int)(e >> 52) == dn) cx = (int)((e >> 36) & 0xffffull);
+    }
+    cd = warp_max(cx);
+  }
+  return (cd << 13) | dn;
+}
+
+// A position's decision taken again with the sizes sz, TV's clamps included
+// (-1: it has no candidate list).  One warp.
+__device__ __forceinline__ int recheck(const DevInstance& I, float rC, const int* sz, int nc,
+                                       const unsigned long long* cl, bool tv, int own) {
+  if (nc < 0) return -1;
+  int d = walk_pick_any(I, rC, sz, nc, cl) & 0x1fff;
+  if (tv) {
+    if (sz[d] > I.max_pw) d = own;
+    if (sz[d] < I.min_pw) d = own;
+  }
+  __syncwarp();
+  return d;
+}
+
+// The marked positions of a group decided again with the sizes sz by the whole
+// CTA, eight lanes to a position: a lane keeps the best lower bound of its
+// candidates' scores and the largest upper bound of the others, three shuffles
+// meet them.  One candidate clear of the rest wins and tolerates the drift
+// that leaves it so; with none above zero the least-loaded part does.
+// Near-ties and long lists go to walk_pick_any, a warp each.
+__device__ __forceinline__ void walk_eval(const DevInstance& I, const SpecBuf& B, const RoundCtx& R, bool tv, float rC,
+                                          const int* sz, const float2* pen, WalkSmem& S, int i0, int sc, int ol) {
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const unsigned need = S.need >> (4 * wib);
+  if (!(need & 15u)) return;
+  const int K = I.K;
+  const int q = lane >> 3, l = 4 * wib + q;
+  const bool marked = (need >> q) & 1u;
+  const int4 mt = marked ? S.meta[i0 + l] : make_int4(0, 0, 0, 8);
+  const int nc = mt.w >> 8, of = mt.x >> 16;
+  const bool todo = marked && !(mt.w & 8);
+  const bool staged = todo && nc >= 0 && nc <= kWalkRow;
+  const unsigned long long* row = S.ent + (size_t)(i0 - sc + l) * kWalkStride;
+  constexpr float kLow = -1e30f;
+  float blo = kLow, bhi = kLow, oh = kLow, up = kLow;
+  unsigned be = 0;
+  int cm = 0;
+  const int ncl = staged ? nc : 0;
+  for (int x = lane & 7; x < ncl; x += 8) {
+    const unsigned long long e = row[x];
+    const unsigned hi32 = (unsigned)(e >> 32);
+    const int p = (int)(hi32 >> 20), c = (int)((hi32 >> 4) & 0xffffu);
+    const float2 w = pen[p];
+    const float cf = (float)c;
+    const float v = cf * w.x;
+    const float lo = v - cf * w.y, hi = v + cf * w.y;
+    if (c > 0) {
+      up = fmaxf(up, w.x + w.y);
+      cm = max(cm, c);
+      if (lo > blo) {
+        oh = fmaxf(oh, bhi);
+        blo = lo;
+        bhi = hi;
+        be = ((unsigned)c << 13) | (unsigned)p;
+      } else {
+        oh = fmaxf(oh, hi);
+      }
+    }
+  }
+#pragma unroll
+  for (int off = 1; off < 8; off <<= 1) {
+    const float xl = __shfl_xor_sync(kAll, blo, off), xh = __shfl_xor_sync(kAll, bhi, off);
+    const float xo = __shfl_xor_sync(kAll, oh, off);
+    const unsigned xe = __shfl_xor_sync(kAll, be, off);
+    oh = fmaxf(fmaxf(oh, xo), xl > blo ? bhi : xh);
+    if (xl > blo) {
+      blo = xl;
+      bhi = xh;
+      be = xe;
+    }
+    up = fmaxf(up, __shfl_xor_sync(kAll, up, off));
+    cm = max(cm, __shfl_xor_sync(kAll, cm, off));
+  }
+  const bool one = staged && blo > 0.0f && oh < blo;
+  const bool none = staged && !(fmaxf(bhi, oh) > 0.0f);
+  int nd = nc < 0 ? -1 : 0, sl = -1;
+  if (one) {
+    nd = (int)be;
+    const int cd = (int)(be >> 13);
+    const float diff = blo - oh - 1e-6f * (fabsf(blo) + fabsf(oh));
+    sl = min(walk_slack(diff * R.Cf, (float)(cd + cm)), walk_slack(blo * (1.0f - 1e-6f) * R.Cf, (float)cd));
+  }
+  if (__any_sync(kAll, none)) {
+    int ms, s2 = 0x7fffffff;
+    const int am = warp_least_loaded(sz, K, &ms);
+    for (int p = lane; p < K; p += 32)
+      if (p != am) s2 = min(s2, sz[p]);
+    s2 = warp_min(s2);
+    int cd = 0;
+    if (tv) {
+      for (int x = lane & 7; x < ncl; x += 8) {
+        const unsigned hi32 = (unsigned)(row[x] >> 32);
+        if ((int)(hi32 >> 20) == am) cd = (int)((hi32 >> 4) & 0xffffu);
+      }
+#pragma unroll
+      for (int off = 1; off < 8; off <<= 1) cd = max(cd, __shfl_xor_sync(kAll, cd, off));
+    }
+    if (none) {
+      nd = (cd << 13) | am;
+      sl = min((s2 - ms - 1) / 2, up <= kLow ? kBig : walk_slack(-up * R.Cf, 1.0f));
+    }
+  }
+  const bool slow = todo && nc >= 0 && !one && !none;
+  for (unsigned sm = __ballot_sync(kAll, slow && (lane & 7) == 0); sm; sm &= sm - 1) {
+    const int src = __ffs(sm) - 1;
+    const int r = walk_pick_any(I, rC, sz, __shfl_sync(kAll, nc, src),
+                                B.cand + (size_t)(ol + i0 + 4 * wib + (src >> 3)) * K);
+    if ((lane >> 3) == (src >> 3)) nd = r;
+  }
+  if (todo && nc >= 0 && tv) {
+    int dn = nd & 0x1fff;
+    const int s0 = sz[dn];
+    sl = min(sl, s0 > I.max_pw ? s0 - I.max_pw - 1 : I.max_pw - s0);
+    if (s0 > I.max_pw) dn = of;
+    const int s1 = sz[dn];
+    sl = min(sl, s1 < I.min_pw ? I.min_pw - s1 - 1 : s1 - I.min_pw);
+    if (s1 < I.min_pw) dn = of;
+    nd = (nd & ~0x1fff) | dn;
+  }
+  if (todo && (lane & 7) == 0) {
+    S.nd[l] = nd;
+    S.nslack[l] = max(sl, 0);
+  }
+}
+
+// The walk (block 0, every thread).  The positions [zs, end_w) are visited in
+// order with the exact sizes each would see: the window-start sizes plus the
+// moves before it (the window's movers before zs are in mlist).  A position is
+// decided again if the sizes may have drifted beyond its slack; the others
+// keep their decision.  A changed decision goes to dfix with the predicted
+// outcome: exact for TV (its accept test is a count of nets) and for vertices
+// without nets, else the old decision's, or a move (MSV) / no move (MSRV) if
+// that one stayed home.  The walk ends (ctl[0]) at a stale-marker risk or at a
+// changed vertex of a CTA or of the grid; ctl[1] counts the changes.
+//
+// It is bound by the latency of dependent instructions (about 5 cycles each in
+// a lone warp), so it speculates once more, inside the CTA: groups of 32
+// positions that no drift reaches are skipped whole; the positions to decide
+// again of a group are decided side by side with the sizes at hand, each with
+// the drift it tolerates from there; the first warp then takes them in order
+// up to the first one that the moves before it may have changed, from which
+// the rest of the group is decided again (on 16K vertices of unit weight, K =
+// 8, about 9 positions stand per step).  A vertex without nets takes the
+// least-loaded part, which its own kind moves with every step: those the
+// first warp decides one by one.
+__device__ void walk_window(const DevInstance& I, const SpecBuf& B, const RoundCtx& R, int metric, int pos, int zs,
+                            int end_w, int nm, WalkSmem& S, int* sz, float2* pen) {
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int K = I.K;
+  const bool tv = metric == kTV;
+  const float rC = __fdiv_rn(1.0f, R.Cf);
+  for (int p = threadIdx.x; p < K; p += blockDim.x) sz[p] = R.sizes[p];
   __syncthreads();
-  const long long D = shd[0], V = shd[1];
-  const bool recheck = shw == 0 && D > max(lds(&B.slack[o]), 0);
-  __syncthreads();   // every thread has read shw before warp 0 may change it
-  if (recheck) {
-    if (wib == 0) {
-      const int d2 = ldg_recheck(I, R, B, o, own, metric, dsz, dsz_cta, o_from);
-      if (lane == 0 && d2 != d) shw = 2;
+  for (int i = threadIdx.x; i < nm; i += blockDim.x) {
+    const int4 m = lds(&B.mlist[i]);
+    if (m.x >= zs - pos || m.y == 0) continue;
+    atomicAdd(&sz[m.z & 0xffff], m.y);
+    atomicAdd(&sz[m.z >> 16], -m.y);
+  }
+  __syncthreads();
+  for (int p = threadIdx.x; p < K; p += blockDim.x) pen[p] = walk_pen(sz[p], rC);
+  if (threadIdx.x == 0) S.drift = 0xffffffffu;   // not known: the first group takes it
+  int hard = kNone, nchg = 0;   // warp 0
+  bool stop = false;
+  for (int zl = zs; zl < end_w && !stop; zl += kWalkLoad) {
+    const int n = min(kWalkLoad, end_w - zl), ol = zl - pos;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+      const int o = ol + i;
+      const int nc = lds(&B.ncand[o]);
+      S.meta[i] = make_int4(lds(&B.dec[o]), lds(&B.wt[o]), lds(&B.acc[o]), (nc << 8) | (int)lds(&B.flag[o]));
+      S.margin[i] = max(lds(&B.slack[o]), 0);
     }
     __syncthreads();
+    const int ng = (n + 31) >> 5;
+    for (int g = wib; g < ng; g += kSWarps) {
+      const int i = g * 32 + lane;
+      const bool in = i < n;
+      const int4 m = in ? S.meta[i] : make_int4(0, 0, 0, 0);
+      const unsigned x = (m.w & 1) ? (unsigned)m.y : 0u;
+      unsigned incl = x;
+      if (__any_sync(kAll, x != 0))
+        for (int off = 1; off < 32; off <<= 1) {
+          const unsigned t = __shfl_up_sync(kAll, incl, off);
+          if (lane >= off) incl += t;
+        }
+      const bool always = (m.w & 32) || ((m.w & 2) && zl + i != pos);
+      const unsigned slk = in ? (unsigned)S.margin[i] : 0x7fffffffu;
+      const int mg = always || slk < incl - x ? -1 : (int)(slk - (incl - x));
+      if (in) S.margin[i] = mg;
+      const int gm = warp_min(mg);
+      if (lane == 31) {
+        S.gmin[g] = gm;
+        S.gsum[g] = incl;
+      }
+    }
+    __syncthreads();
+    for (int sc = 0; sc < n && !stop; sc += kWalkSub) {
+      const int ns = min(kWalkSub, n - sc);
+      const int g1 = (sc + ns + 31) >> 5;
+      unsigned pot = 0;   // groups a drift may reach
+      {
+        unsigned d = S.drift;
+        for (int g = sc >> 5; g < g1; g++) {
+          // (past the first such group, changed decisions may add to the drift)
+          if (pot || S.gmin[g] < 0 || d > (unsigned)S.gmin[g]) pot |= 1u << (g - (sc >> 5));
+          d += S.gsum[g];
+        }
+      }
+      if (pot) {
+        const int row = min(K, kWalkRow);
+        for (int i = threadIdx.x; i < ns * kWalkRow; i += blockDim.x)
+          if ((i & (kWalkRow - 1)) < row && ((pot >> (i / (kWalkRow * 32))) & 1u))
+            S.ent[(i / kWalkRow) * kWalkStride + (i & (kWalkRow - 1))] =
+                lds(&B.cand[(size_t)(ol + sc + i / kWalkRow) * K + (i & (kWalkRow - 1))]);
+      }
+      __syncthreads();   // also: every thread has read S.drift
+      // warp 0: the group at hand, its lanes' positions and their present outcome
+      int g = sc >> 5, j = 0, own = 0, d = 0, w = 0, mg = 0;
+      int4 m = make_int4(0, 0, 0, 0);
+      bool mv = false, in = false, fresh = true;
+      unsigned drift = S.drift, D = 0, extra = 0;
+      // the moves own -> to of the lanes of mm applied
+      auto apply = [&](unsigned mm, int to) {
+        if (!mm) return;
+        const bool me = (mm >> lane) & 1u;
+        if (me) {
+          atomicAdd(&sz[to], w);
+          atomicAdd(&sz[own], -w);
+        }
+        __syncwarp();
+        if (me) {
+          pen[to] = walk_pen(sz[to], rC);
+          pen[own] = walk_pen(sz[own], rC);
+        }
+        __syncwarp();
+      };
+      while (true) {
+        if (wib == 0) {
+          // on to the next group with positions to decide again
+          int task = -1;
+          unsigned need = 0;
+          for (; g < g1 && hard == kNone; g++) {
+            const int i0 = g * 32;
+            const int nl = min(32, n - i0);
+            if (fresh) {
+              in = lane < nl;
+              m = in ? S.meta[i0 + lane] : make_int4(0, 0, 0, 0);
+              own = m.x >> 16;
+              d = m.x & 0xffff;
+              w = m.y;
+              mv = (m.w & 1) != 0;
+              j = 0;
+              extra = 0;
+              const bool reach = S.gmin[g] < 0 || drift > (unsigned)S.gmin[g];
+              if (reach) {   // the exact drift here
+                int D0 = 0;
+                for (int p = lane; p < K; p += 32) D0 = max(D0, abs(sz[p] - R.sizes[p]));
+                drift = (unsigned)warp_max(D0);
+              }
+              mg = in && reach ? S.margin[i0 + lane] : 0x7fffffff;
+              D = drift;
+              fresh = false;
+            }
+            need = __ballot_sync(kAll, in && lane >= j && (mg < 0 || D > (unsigned)mg));
+            if (need) {
+              task = g;
+              break;
+            }
+            // the rest of the group keeps its outcome
+            apply(__ballot_sync(kAll, mv && lane >= j), d);
+            drift += S.gsum[g] + extra;   // what the group's movers moved bounds the drift from here on
+            fresh = true;
+          }
+          if (lane == 0) {
+            S.group = task;
+            S.need = need;
+          }
+        }
+        __syncthreads();
+        const int tg = S.group;
+        if (tg < 0) break;
+        walk_eval(I, B, R, tv, rC, sz, pen, S, tg * 32, sc, ol);
+        __syncthreads();
+        if (wib == 0) {
+          // ---- take them in order
+          const unsigned need = S.need;
+          const int i0 = g * 32, nl = min(32, n - i0);
+          const bool again = (need >> lane) & 1u, iso = (m.w & 8) != 0;
+          const int nd = again && !iso ? S.nd[lane] : 0, nsl = again && !iso ? S.nslack[lane] : 0;
+          const bool stale = (m.w & 2) && zl + i0 + lane != pos;
+          const bool hardf = again && (stale || nd < 0);
+          // the outcome of every position decided again, as if its decision stood
+          bool mvn = mv;
+          int dn = d;
+          if (again && !iso && !hardf) {
+            dn = nd & 0x1fff;
+            if (dn != d)
+              mvn = dn != own && (tv ? m.z + (nd >> 13) >= 0 : d != own ? (m.w & 16) != 0 : metric == kMSV);
+          }
+          const bool chg = dn != d;
+          // drift from these sizes before each position, and what the changed
+          // decisions before it add to its group's drift
+          const int x = mvn && lane >= j ? w : 0;
+          const int chgw = mvn == mv || lane < j ? 0 : mvn ? w : -w;
+          unsigned Dn = (unsigned)x;
+          int cn = chgw;
+          if (__any_sync(kAll, x != 0))
+            for (int off = 1; off < 32; off <<= 1) {
+              const unsigned t = __shfl_up_sync(kAll, Dn, off);
+              if (lane >= off) Dn += t;
+            }
+          Dn -= (unsigned)x;
+          if (__any_sync(kAll, chgw != 0))
+            for (int off = 1; off < 32; off <<= 1) {
+              const int t = __shfl_up_sync(kAll, cn, off);
+              if (lane >= off) cn += t;
+            }
+          cn -= chgw;
+          const long long lim = again ? (long long)nsl - Dn : (long long)mg - (long long)D - cn;
+          int more = 0;   // weight the vertices without nets add to both
+          while (true) {
+            // the first position in doubt: decided again here and reached by the
+            // moves since, or not decided again and reached now
+            const unsigned db = __ballot_sync(
+                kAll, in && lane >= j && ((again && (hardf || iso)) || (long long)more > lim));
+            const int f = db ? __ffs(db) - 1 : nl;
+            // ---- positions [j, f) stand; a changed vertex of a CTA or of the
+            // grid ends the window
+            const bool take = lane >= j && lane < f;
+            const unsigned hm = __ballot_sync(kAll, take && chg && (m.w & 4));
+            const int fe = hm ? __ffs(hm) - 1 : f;
+            const bool keep = lane >= j && lane < fe;
+            const unsigned cm = __ballot_sync(kAll, keep && chg);
+            if (cm) {
+              if (keep && chg) {
+                B.dfix[ol + i0 + lane] = dn | (mvn ? 1 << 16 : 0);
+                B.flag[ol + i0 + lane] = (unsigned char)((m.w & 255) | 128);
+              }
+              nchg += __popc(cm);
+              const unsigned dx = (unsigned)warp_sum(keep ? chgw : 0);
+              extra += dx;
+              D += dx;
+            }
+            apply(__ballot_sync(kAll, keep && mvn), dn);
+            if (hm) {
+              hard = ((zl + i0 + fe) << 3) | 2;
+              break;
+            }
+            j = f;
+            if (f >= nl) break;
+            const bool af = (need >> f) & 1u;
+            if (__shfl_sync(kAll, hardf ? 1 : 0, f)) {
+              hard = ((zl + i0 + f) << 3) | (__shfl_sync(kAll, stale ? 1 : 0, f) ? 1 : 2);
+              break;
+            }
+            if (!af || !(S.meta[i0 + f].w & 8)) break;   // decided again from here
+            // ---- vertices without nets, one by one (and their like after them)
+            do {
+              const int4 mt = S.meta[i0 + j];
+              const int of = mt.x >> 16, df = mt.x & 0xffff, wf = mt.y;
+              int ms;
+              int q = warp_least_loaded(sz, K, &ms);
+              if (tv && (ms > I.max_pw || ms < I.min_pw)) q = of;   // the clamps keep it home
+              bool m2 = (mt.w & 1) != 0;
+              if (q != df) {
+                m2 = q != of && (tv || (mt.w & 16));
+                if (lane == 0) {
+                  B.dfix[ol + i0 + j] = q | (m2 ? 1 << 16 : 0);
+                  B.flag[ol + i0 + j] = (unsigned char)((mt.w & 255) | 128);
+                }
+                nchg++;
+                const int dd = (m2 ? wf : 0) - ((mt.w & 1) ? wf : 0);
+                extra += (unsigned)dd;
+                D += (unsigned)dd;
+                more += dd;
+              }
+              if (m2) {
+                if (lane < 2) {
+                  const int p = lane == 0 ? q : of;
+                  const int s = sz[p] + (lane == 0 ? wf : -wf);
+                  sz[p] = s;
+                  pen[p] = walk_pen(s, rC);
+                }
+                __syncwarp();
+              }
+              j++;
+            } while (j < nl && ((need >> j) & 1u) && (S.meta[i0 + j].w & 8));
+            if (j >= nl) break;
+          }
+          // the positions taken keep what was decided
+          if (lane < j) {
+            mv = mvn;
+            d = dn;
+          }
+          if (hard == kNone && j >= nl) {
+            drift += S.gsum[g] + extra;
+            fresh = true;
+            g++;
+          }
+        }
+      }
+      if (threadIdx.x == 0) S.drift = drift;
+      stop = __syncthreads_or(hard != kNone) != 0;
+    }
   }
-  if (threadIdx.x == 0 && shw == 0) shw = V > max(lds(&B.vslack[o]), 0) ? 3 : (mtpos < z && d != own) ? 4 : 0;
-  __syncthreads();
-  int why = shw;
-  if (why == 0 && check_nets) {
-    const uint32_t base = __ldg(&I.vptr[v]);
-    const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
-    const int conf = conflicts(I, B, metric != kTV, z, own, d != own, fl & 1, base, deg, threadIdx.x, blockDim.x,
-                               lds(&B.ctab_over[par]) != 0);
-    const int c5 = __syncthreads_or(conf == 5), c6 = __syncthreads_or(conf == 6), c7 = __syncthreads_or(conf == 7);
-    why = c5 ? 5 : c6 ? 6 : c7 ? 7 : 0;
+  if (threadIdx.x == 0) {
+    B.ctl[0] = hard;
+    B.ctl[1] = nchg;
   }
-  if (why && threadIdx.x == 0) atomicMin(cut, (z << 3) | why);
-  __syncthreads();
 }
 
-// In-window fix of the light vertex at position z (window offset o) whose size
-// check failed: its decision becomes the exact one (dfix, taken with the sizes
-// the committed prefix leaves), and the move records, the accept test and the
-// claims are redone for it.  The replaced move's claims stay (a superset keeps
-// every later check conservative); their table slots go to rec_slot2 for the
-// commit.  One warp, the warp gw owning position z.
+// The position z (window offset o) whose decision the last walk changed: the
+// move records, the accept test and the claims are redone for the new
+// decision.  The replaced move's claims stay (a superset keeps every later
+// check conservative); their table slots go to rec_slot2 for the commit, so a
+// second replaced move ends the window here instead.  An outcome other than
+// the walk predicted lowers *mis: the positions after it are walked again.
+// One warp, the one owning position z.
 __device__ void fix_position(const DevInstance& I, const SpecBuf& B, const RoundCtx& R, int metric, int z, int o,
-                             int par, int gw, int* loc, int* gains, int* losses, int* adelta, bool logp) {
+                             int fl, int par, int* mis, int* cut, int* loc, int* gains, int* losses, int* adelta,
+                             bool logp) {
   const int lane = threadIdx.x & 31;
   const bool vol = metric != kTV, rv = metric == kMSRV;
   const int K = I.K;
   const int v = __ldg(&B.porder[z]);
   const uint32_t base = __ldg(&I.vptr[v]);
   const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
-  const int fl = lds(&B.flag[o]);
   const int own = lds(&B.dec[o]) >> 16;
-  const int d = lds(&B.dfix[o]);
+  const int fx = lds(&B.dfix[o]);
+  const int d = fx & 0xffff;
   const bool had = (fl & 1) != 0;
+  if (had && (fl & 64)) {
+    if (lane == 0) {
+      atomicMin(cut, (z << 3) | 2);
+      B.flag[o] = (unsigned char)(fl & ~128);
+    }
+    return;
+  }
   if (had) {
     for (int k = lane; k < deg; k += 32)
       B.rec_slot2[base + k] =
           rec_setchange(lds(&B.rec[base + k]), vol) ? make_uint2(~0u, ~0u) : lds(&B.rec_slot[base + k]);
+    __syncwarp();
   }
-  bool mover = false, mt = false, good = false;
+  bool mover = false, mt = false, good = (fl & 16) != 0;
   int vs = kBig, vdd = 0;
-  if (d != own) {
-    for (int p = lane; p < K; p += 32) { gains[p] = 0; losses[p] = 0; adelta[p] = 0; }
+  int rg = 0, rl = 0;
+  if (deg == 0) {
+    mover = d != own && (!vol || good);
+    vs = lds(&B.vslack[o]);
+  } else if (d != own) {
+    if (vol) {
+      for (int p = lane; p < K; p += 32) { gains[p] = 0; losses[p] = 0; adelta[p] = 0; }
+      __syncwarp();
+    }
+    const int ra = locate_all(I, B, metric, v, own, d, base, deg, 0, 1, loc, gains, losses, adelta);
     __syncwarp();
-    locate_all(I, B, metric, v, own, d, base, deg, 0, 1, loc, gains, losses, adelta);
-    __syncwarp();
-    const AcceptPart a = accept_partial(R, gains, losses, adelta, K, rv, lane, 32);
-    const bool fM = __any_sync(kAll, a.failM);
-    const bool fN = __any_sync(kAll, a.failN);
-    accept_final(fM, fN, warp_max(a.fsl), warp_min(a.msl), &good, &vs);
-    mover = good;
-    mt = mover && __any_sync(kAll, a.mt);
-    vdd = warp_max(a.vd);
+    if (vol) {
+      const AcceptPart a = accept_partial(R, gains, losses, adelta, K, rv, lane, 32);
+      const bool fM = __any_sync(kAll, a.failM);
+      const bool fN = __any_sync(kAll, a.failN);
+      accept_final(fM, fN, warp_max(a.fsl), warp_min(a.msl), &good, &vs);
+      mover = good;
+      mt = mover && __any_sync(kAll, a.mt);
+      vdd = warp_max(a.vd);
+      if (logp) {
+        for (int p = lane; p < K; p += 32) { rg += gains[p]; rl += losses[p]; }
+        rg = warp_sum(rg);
+        rl = warp_sum(rl);
+      }
+    } else {
+      rg = warp_sum(ra & 0xffff);
+      rl = warp_sum(ra >> 16);
+      mover = rg >= rl;   // leave gain >= arrival loss (TV/partition.cpp:355-380)
+    }
   }
   __syncwarp();
-  if (logp) {
-    int rg = 0, rl = 0;
-    if (d != own) {
-      for (int p = lane; p < K; p += 32) { rg += gains[p]; rl += losses[p]; }
-      rg = warp_sum(rg);
-      rl = warp_sum(rl);
-    }
-    if (lane == 0) { B.rgain[o] = rg; B.rloss[o] = rl; }
-  }
   if (mover) {
     claim_nets(I, B, vol, z, own, d, base, deg, lane, 32, par);
     if (lane == 0 && mt) atomicMin(&B.ctl[2 + par], z);
   }
   if (lane == 0) {
+    if (logp) { B.rgain[o] = rg; B.rloss[o] = rl; }
+    if (mover != (fx >> 16 != 0)) atomicMin(mis, z);
     const int wv = mover ? __ldg(&I.w[v]) : 0;
-    const int vn = mover ? vdd : 0;
-    if (had) B.mlist[lds(&B.midx[o])] = make_int4(o, wv, (own << 16) | d, 0);   // the replaced mover's entry
-    else if (mover) list_mover(B, par, o, wv, (own << 16) | d);
-    B.wsum[gw] += wv - lds(&B.wt[o]);
-    B.vsum[gw] += vn - lds(&B.vd[o]);
+    if (had) B.mlist[lds(&B.midx[o])] = make_int4(o, wv, (own << 16) | d, mover ? vdd : 0);   // the replaced mover's entry
+    else if (mover) list_mover(B, par, o, wv, (own << 16) | d, vdd);
     B.dec[o] = (own << 16) | d;
-    B.flag[o] = (unsigned char)((fl & 10) | (mover ? 1 : 0) | (good ? 16 : 0) | 32 | (had ? 64 : 0));
-    B.slack[o] = kBig;   // exact: no size check again
+    B.flag[o] = (unsigned char)((fl & (2 | 8 | 64)) | (mover ? 1 : 0) | (good ? 16 : 0) | 32 | (had && deg > 0 ? 64 : 0));
     B.vslack[o] = vs;
-    B.wt[o] = wv;
-    B.vd[o] = vn;
+    B.vd[o] = mover ? vdd : 0;
   }
   __syncwarp();
 }
@@ -879,10 +1263,6 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
   __shared__ int s_gz[kMaxGridVerts], s_gv[kMaxGridVerts], s_go[kMaxGridVerts], s_gd[kMaxGridVerts];
   __shared__ uint32_t s_gb[kMaxGridVerts];
   __shared__ int s_gdec[kMaxGridVerts], s_gspec[kMaxGridVerts], s_gslk[kMaxGridVerts];
-  __shared__ long long s_pre_w, s_pre_v;
-  __shared__ unsigned long long uscr2[kSWarps];
-  __shared__ int s_cw[kSWarps], s_cv[kSWarps], s_mt, s_nm;   // this CTA's warps' sums, round words
-  __shared__ int s_mw[kSWarps], s_mv[kSWarps];
   __shared__ int loc_b[kSWarps * 96];   // per-warp locate scratch
   const int metric = I.metric;
   const bool vol = metric != kTV;
@@ -915,17 +1295,22 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
   int* adelta = adelta_b + (size_t)wib * K;
   int* loc = loc_b + wib * 96;
   Vol V{I.send, rv ? I.recv : nullptr};
+  // the walk's staged positions and penalties lie over the evaluation's arrays,
+  // its exact sizes over the round's penalties (both rebuilt every round)
+  WalkSmem& walk_s = *reinterpret_cast<WalkSmem*>(cnt_b);
+  float2* walk_pn = reinterpret_cast<float2*>(cnt_b + sizeof(WalkSmem) / sizeof(int));
+  const float rC = __fdiv_rn(1.0f, Cf);
+  int* walk_sz = reinterpret_cast<int*>(penf_s);
 
-  const bool vfix = metric == kMSV || metric == kMSRV;
   int round = 0;
   int heavy_round = 0;
-  int vr = 0;   // validation passes (parity selects the cut word)
+  int wr = 0;   // walks (parity selects the misprediction word)
   unsigned long long tA = gtimer();
   for (int it = 0; it < passes; it++) {
     const bool logp = I.recs != nullptr && it == passes - 1;   // decision records of the last pass
     int pos = 0;
     int W = min(nwarps, B.wmax);
-    int hidx = 0;
+    int hidx = 0, midx = 0;
     bool pass_start = true;
     bool prev_maxtouch = false;
     while (pos < B.npos) {
@@ -1012,6 +1397,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
       pass_start = false;
       prev_maxtouch = false;
       while (hidx < B.nheavy && __ldg(&B.heavy_pos[hidx]) < pos) hidx++;
+      midx += lower_bound_pos(B.mid_pos + midx, min(B.nmid - midx, B.wmax), pos);
 
       // ================================================================= round
       // A window holds up to gmax whole-grid vertices and ends before the next
@@ -1084,7 +1470,6 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
       }
       if (kTimingStats && ns && threadIdx.x == 0) atomicMax(&B.stats[38], gtimer() - tR);
       // ---- A: evaluate
-      int wsum = 0, vsum = 0;
       const long long cA = clock64();
       long long cV = 0;
       int nV = 0;
@@ -1110,11 +1495,9 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         const int d = ldg_decide(I, R, cnt, first, sb, metric, v, own, z == pos, gains, B.cand + (size_t)o * K,
                                  &B.ncand[o], metric == kTV ? B.scan + (size_t)o * words : nullptr, &special, &slack);
         const long long cD = clock64();
-        // An isolated vertex (no nets, weight 0) changes nothing a later position
-        // reads; if its decision flips under the window's size drift, validation
-        // corrects it in place instead of cutting.  Its accept outcome does not
-        // depend on the destination (all gains and losses are zero).
-        const bool iso = deg == 0 && __ldg(&I.w[v]) == 0;
+        // The accept outcome of a vertex without nets does not depend on the
+        // destination (all gains and losses are zero).
+        const bool iso = deg == 0;
         bool mover = false, mt = false, good = metric == kTV;
         int vs = kBig, vdd = 0;
         if (metric == kTV) {
@@ -1153,12 +1536,11 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
           }
           if (lane == 0) { B.rgain[o] = rg; B.rloss[o] = rl; }
         }
-        const int wv = mover ? __ldg(&I.w[v]) : 0;
         if (mover) {
           claim_nets(I, B, vol, z, own, d, base, deg, lane, 32, par);
           if (lane == 0) {
             if (mt) atomicMin(&B.ctl[2 + par], z);
-            list_mover(B, par, o, wv, (own << 16) | d);
+            list_mover(B, par, o, __ldg(&I.w[v]), (own << 16) | d, vdd);
           }
         }
         if (lane == 0) {
@@ -1166,11 +1548,10 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
           B.flag[o] = (unsigned char)((mover ? 1 : 0) | (special ? 2 : 0) | (iso ? 8 : 0) | (good ? 16 : 0));
           B.slack[o] = slack;
           B.vslack[o] = vs;
-          B.wt[o] = wv;
+          B.wt[o] = __ldg(&I.w[v]);
+          B.acc[o] = c1 - deg;
           B.vd[o] = mover ? vdd : 0;
         }
-        wsum += wv;
-        vsum += mover ? vdd : 0;
         if (kTimingStats && lane == 0) {
           atomicAdd(&B.stats[41], (unsigned long long)(cT - cz));
           atomicAdd(&B.stats[42], (unsigned long long)(cD - cT));
@@ -1186,18 +1567,16 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         atomicAdd(&B.stats[25], (unsigned long long)cV);
         atomicAdd(&B.stats[26], (unsigned long long)nV);
       }
-      // medium vertices of this CTA's positions: the CTA evaluates them together
-      if (threadIdx.x < kSWarps) { s_mw[threadIdx.x] = 0; s_mv[threadIdx.x] = 0; }
+      // medium vertices of the window: one CTA each, dealt out from the end of
+      // the grid (their positions cluster; the CTAs that own them took up to 15
+      // each on the 1M-vertex Zipf workload while the others waited)
       __syncthreads();
       const long long cM = clock64();
-      const int cz0 = min(pos + blockIdx.x * kSWarps * q, end_w);
-      const int cz1 = min(cz0 + kSWarps * q, end_w);
-      for (int mi = lower_bound_pos(B.mid_pos, B.nmid, cz0); mi < B.nmid; mi++) {
-        const int z = __ldg(&B.mid_pos[mi]);
-        if (z >= cz1) break;
-        cta_eval_ldg(I, B, R, metric, z, pos, par, q, sb, cnt_b, first_b, gains_b, losses_b, adelta_b, iscr, s_mw, s_mv,
-                     loc_b, logp);
-      }
+      const int mend = midx + lower_bound_pos(B.mid_pos + midx, min(B.nmid - midx, span), end_w);
+      const int mi0 = midx + (int)(gridDim.x - 1 - blockIdx.x);
+      for (int mi = mi0; mi < mend; mi += gridDim.x)
+        cta_eval_ldg(I, B, R, metric, __ldg(&B.mid_pos[mi]), pos, par, sb, cnt_b, first_b, gains_b, losses_b,
+                     adelta_b, iscr, loc_b, logp);
       __syncthreads();
       if (kTimingStats && threadIdx.x == 0) {
         const long long dm = clock64() - cM;
@@ -1301,33 +1680,21 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
             }
           }
           if (mover) claim_nets(I, B, vol, zs, own_s, d, base_s, deg_s, gtid, gthreads, par);
-          const int wv = mover ? __ldg(&I.w[vsup]) : 0;
           if (blockIdx.x == 0 && threadIdx.x == 0) {
             if (logp) { B.rgain[os] = rg; B.rloss[os] = rl; }
             B.dec[os] = (own_s << 16) | d;
             B.flag[os] = (unsigned char)((mover ? 1 : 0) | (s_gspec[j] ? 2 : 0) | 4);
             B.slack[os] = s_gslk[j];
             B.vslack[os] = vs;
-            B.wt[os] = wv;
+            B.wt[os] = __ldg(&I.w[vsup]);
+            B.acc[os] = lds(&B.hmisc[hmslot(j)]) - deg_s;
             B.vd[os] = mover ? vdd : 0;
-            if (mover) {
-              if (mt) atomicMin(&B.ctl[2 + par], zs);
-              list_mover(B, par, os, wv, (own_s << 16) | d);
-            }
-          }
-          // the warp owning position zs carries its weight and volume change
-          const int owner = os / q;
-          if (threadIdx.x == 0 && owner / kSWarps == (int)blockIdx.x) {
-            s_mw[owner % kSWarps] += wv;
-            s_mv[owner % kSWarps] += mover ? vdd : 0;
+            if (mover && mt) atomicMin(&B.ctl[2 + par], zs);
+            if (mover) list_mover(B, par, os, __ldg(&I.w[vsup]), (own_s << 16) | d, vdd);
           }
           __syncthreads();
         }
         if (blockIdx.x == 0 && threadIdx.x == 0) B.stats[33] += gtimer() - tG;
-      }
-      if (lane == 0) {
-        B.wsum[gw] = wsum + s_mw[wib];
-        B.vsum[gw] = vsum + s_mv[wib];
       }
       if (!grid_barrier(B.bar, I.status)) return;
       if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1339,172 +1706,222 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         B.stats[23] += B.stats[24];
         B.stats[24] = 0;
       }
-      int cutw;
-      for (int zfix = pos, nfix = 0;; nfix++) {
-        int* const cut_w = &B.ctl[4 + (vr & 1)];
-        // ---- B: validate.  Prefix sums of moved weight and volume drift over the
-        // warps before this one (warps own consecutive position ranges).
-        // Positions before zfix are known valid (an earlier pass of the window).
-        const unsigned long long tV = gtimer();
-        long long Dw, Vw;
-        {
-          // one round of independent loads: the earlier warps' sums, this CTA's
-          // warps' sums, the round words
-          long long pw = 0, pv = 0;
-          const int lim = blockIdx.x * kSWarps;
-          for (int g = threadIdx.x; g < lim; g += blockDim.x) {
-            pw += lds(&B.wsum[g]);
-            pv += lds(&B.vsum[g]);
-          }
-          if (threadIdx.x < kSWarps) {
-            s_cw[threadIdx.x] = lds(&B.wsum[lim + threadIdx.x]);
-            s_cv[threadIdx.x] = lds(&B.vsum[lim + threadIdx.x]);
-          }
-          if (threadIdx.x == 0) {
-            s_mt = lds(&B.ctl[2 + par]);
-            s_nm = lds(&B.mcnt[par]);
-          }
-          pw = warp_sum64(pw);
-          pv = warp_sum64(pv);
-          if (lane == 0) {
-            uscr[wib] = (unsigned long long)pw;
-            uscr2[wib] = (unsigned long long)pv;
-          }
-          __syncthreads();
-          long long a = 0, b = 0;
-          for (int x = 0; x < kSWarps; x++) {
-            a += (long long)uscr[x];
-            b += (long long)uscr2[x];
-          }
-          if (threadIdx.x == 0) {
-            s_pre_w = a;
-            s_pre_v = b;
-          }
-          Dw = a;
-          Vw = b;
-          for (int x = 0; x < wib; x++) {
-            Dw += s_cw[x];
-            Vw += s_cv[x];
-          }
-        }
-        const int mtpos = s_mt;
-        const int nm = s_nm;
-        const unsigned long long tV1 = gtimer();
-        // part-size changes of the window's movers before this CTA's first position
-        // (phase-A scratch gains_b is free now)
-        int* dsz_cta = gains_b;
-        const int cta_o0 = cz0 - pos;
-        for (int p = threadIdx.x; p < K; p += blockDim.x) dsz_cta[p] = 0;
+      // ---- B: validate the positions [zfrom, zto): the lists (conflicts), the
+      // volumes and, with sizes, the part sizes (the decision taken again where
+      // they drifted beyond its slack).  The first position that an earlier
+      // one invalidates lowers *cut_w, the first whose decision the exact sizes
+      // change *flip_w.
+      int* const cut_w = &B.ctl[4 + par];
+      int* const flip_w = &B.ctl[6 + par];
+      const int cta_o0 = min(pos + blockIdx.x * kSWarps * q, end_w) - pos;
+      int* dsz_cta = gains_b;   // (the evaluation's arrays are free here)
+      // the size changes (in dsz) and volume drift (returned) of the window's
+      // movers before offset o; every thread of the CTA
+      auto moved_before = [&](int o, int* dsz) {
+        for (int p = threadIdx.x; p < K; p += blockDim.x) dsz[p] = 0;
         __syncthreads();
+        const int nm = lds(&B.mcnt[par]);
+        long long x = 0;
         for (int i = threadIdx.x; i < nm; i += blockDim.x) {
           const int4 m = lds(&B.mlist[i]);
-          if (m.x >= cta_o0 || m.y == 0) continue;
-          atomicAdd(&dsz_cta[m.z & 0xffff], m.y);
-          atomicAdd(&dsz_cta[m.z >> 16], -m.y);
+          if (m.x >= o) continue;
+          x += m.w;
+          if (m.y == 0) continue;
+          atomicAdd(&dsz[m.z & 0xffff], m.y);
+          atomicAdd(&dsz[m.z >> 16], -m.y);
+        }
+        if (vol) {
+          x = warp_sum64(x);
+          if (lane == 0) uscr[wib] = (unsigned long long)x;
+          __syncthreads();
+          x = 0;
+          for (int y = 0; y < kSWarps; y++) x += (long long)uscr[y];
         }
         __syncthreads();
+        return x;
+      };
+      auto validate = [&](int zfrom, int zto, bool sizes) {
+        const int mtpos = lds(&B.ctl[2 + par]);
         const bool ov = lds(&B.ctab_over[par]) != 0;
-        for (int z = z0; z < z1; z++) {
-          const int o = z - pos;
-          // the position's words in one round of independent loads
-          const int wz = lds(&B.wt[o]), vz = lds(&B.vd[o]);
-          const int fl = lds(&B.flag[o]);
-          const int slk = lds(&B.slack[o]), vslk = lds(&B.vslack[o]);
-          int pk = lds(&B.dec[o]);
-          const int v = __ldg(&B.porder[z]);
-          if (z < zfix || (fl & 4)) {      // valid already / medium vertex, validated by the CTA below
-            Dw += wz;
-            Vw += vz;
-            continue;
+        if (sizes || vol) {
+          // the movers before this warp's first position
+          long long Vw = moved_before(cta_o0, dsz_cta);
+          long long Dw = 0;
+          if (z0 < z1) {
+            int D0 = 0, wi = 0, vi = 0;
+            for (int p = lane; p < K; p += 32) D0 = max(D0, abs(dsz_cta[p]));
+            for (int o = cta_o0 + lane; o < z0 - pos; o += 32) {
+              if (lds(&B.flag[o]) & 1) wi += lds(&B.wt[o]);
+              if (vol) vi += lds(&B.vd[o]);
+            }
+            Dw = (long long)warp_max(D0) + (unsigned)warp_sum(wi);
+            if (vol) Vw += warp_sum(vi);
           }
-          const uint32_t base = __ldg(&I.vptr[v]);
-          const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
-          const int own = pk >> 16;
-          int why = ((fl & 2) && z != pos) ? 1 : 0;
-          if (!why && Dw > max(slk, 0)) {
-            // beyond the slack: decide again with the exact sizes at this position
-            const int d2 = ldg_recheck(I, R, B, o, own, metric, cnt, dsz_cta, cta_o0);
-            if (d2 != (pk & 0xffff)) {
-              if (fl & 8) {
-                // isolated vertex: take the exact decision (no weight, no nets, so
-                // no later position sees the difference)
-                pk = (own << 16) | d2;
-                if (lane == 0) {
-                  B.dec[o] = pk;
-                  B.flag[o] = (unsigned char)((fl & ~1) | ((fl & 16) && d2 != own ? 1 : 0));
-                }
-              } else {
-                why = 2;
-                if (lane == 0) B.dfix[o] = d2;
+          for (int z = z0; z < min(z1, zto); z++) {
+            const int o = z - pos;
+            // the position's words in one round of independent loads
+            const int wz = lds(&B.wt[o]), vz = lds(&B.vd[o]);
+            const int fl = lds(&B.flag[o]);
+            const int slk = lds(&B.slack[o]), vslk = lds(&B.vslack[o]);
+            const int pk = lds(&B.dec[o]);
+            const int v = __ldg(&B.porder[z]);
+            if (z >= zfrom && !(fl & 4)) {      // the others: a CTA or the grid, below
+              const uint32_t base = __ldg(&I.vptr[v]);
+              const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
+              const int own = pk >> 16;
+              if (sizes && Dw > max(slk, 0)) {
+                // the exact sizes here: this CTA's movers before z on top of dsz_cta
+                for (int p = lane; p < K; p += 32) cnt[p] = sizes_s[p] + dsz_cta[p];
+                __syncwarp();
+                for (int o2 = cta_o0 + lane; o2 < o; o2 += 32)
+                  if (lds(&B.flag[o2]) & 1) {
+                    const int w2 = lds(&B.wt[o2]), pk2 = lds(&B.dec[o2]);
+                    atomicAdd(&cnt[pk2 & 0xffff], w2);
+                    atomicAdd(&cnt[pk2 >> 16], -w2);
+                  }
+                __syncwarp();
+                if (recheck(I, rC, cnt, lds(&B.ncand[o]), B.cand + (size_t)o * K, metric == kTV, own) != (pk & 0xffff) &&
+                    lane == 0)
+                  atomicMin(flip_w, (z << 3) | 2);
+              }
+              // the max-volume parts enter only the accept test of a vertex whose
+              // decision leaves its part (MSRV/partition.cpp:308-400,
+              // MGV/partition.cpp:292-362), and they change only with a move
+              int why = ((fl & 2) && z != pos) ? 1 : Vw > max(vslk, 0) ? 3 : (mtpos < z && (pk & 0xffff) != own) ? 4 : 0;
+              if (!why) {
+                const int c = conflicts(I, B, vol, z, own, (pk & 0xffff) != own, fl & 1, base, deg, lane, 32, ov);
+                const int c5 = __any_sync(kAll, c == 5), c6 = __any_sync(kAll, c == 6), c7 = __any_sync(kAll, c == 7);
+                why = c5 ? 5 : c6 ? 6 : c7 ? 7 : 0;
+              }
+              if (why) {
+                if (lane == 0) atomicMin(cut_w, (z << 3) | why);   // position, then cut reason
+                break;
               }
             }
+            if (fl & 1) Dw += wz;
+            if (vol) Vw += vz;
           }
-          // the max-volume parts enter only the accept test of a vertex whose
-          // decision leaves its part (MSRV/partition.cpp:308-400,
-          // MGV/partition.cpp:292-362), and they change only with a move
-          if (!why) why = Vw > max(vslk, 0) ? 3 : (mtpos < z && (pk & 0xffff) != own) ? 4 : 0;
-          if (!why) {
-            const int c = conflicts(I, B, vol, z, own, (pk & 0xffff) != own, fl & 1, base, deg, lane, 32, ov);
-            const int c5 = __any_sync(kAll, c == 5), c6 = __any_sync(kAll, c == 6), c7 = __any_sync(kAll, c == 7);
-            why = c5 ? 5 : c6 ? 6 : c7 ? 7 : 0;
+        } else {
+          for (int z = max(z0, zfrom); z < min(z1, zto); z++) {   // TV, sizes known: the conflicts alone
+            const int o = z - pos;
+            const int fl = lds(&B.flag[o]), pk = lds(&B.dec[o]);
+            if (fl & 4) continue;
+            const int v = __ldg(&B.porder[z]);
+            const uint32_t base = __ldg(&I.vptr[v]);
+            const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
+            const int own = pk >> 16;
+            int why = ((fl & 2) && z != pos) ? 1 : 0;
+            if (!why) {
+              const int c = conflicts(I, B, vol, z, own, (pk & 0xffff) != own, fl & 1, base, deg, lane, 32, ov);
+              const int c5 = __any_sync(kAll, c == 5), c6 = __any_sync(kAll, c == 6), c7 = __any_sync(kAll, c == 7);
+              why = c5 ? 5 : c6 ? 6 : c7 ? 7 : 0;
+            }
+            if (why) {
+              if (lane == 0) atomicMin(cut_w, (z << 3) | why);
+              break;
+            }
           }
-          if (why) {
-            if (lane == 0) atomicMin(cut_w, (z << 3) | why);   // position, then cut reason
-            break;
-          }
-          Dw += wz;
-          Vw += vz;
         }
+        // medium vertices by their CTAs, whole-grid vertices: their nets by every
+        // thread, the rest by one CTA
+        auto check_big = [&](int z, int k0, int kstep, bool rest, bool grid) {
+          const int o = z - pos;
+          const int fl = lds(&B.flag[o]), pk = lds(&B.dec[o]);
+          const int own = pk >> 16;
+          const bool leaves = (pk & 0xffff) != own;
+          const int v = __ldg(&B.porder[z]);
+          const uint32_t base = __ldg(&I.vptr[v]);
+          const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
+          int why = 0;
+          if (rest) {
+            why = ((fl & 2) && z != pos) ? 1 : 0;
+            if (sizes || vol) {
+              __syncthreads();   // dsz_cta and cnt_b are read
+              const long long Vz = moved_before(o, cnt_b);
+              if (!why) why = Vz > max(lds(&B.vslack[o]), 0) ? 3 : (mtpos < z && leaves) ? 4 : 0;
+              if (sizes && wib == 0) {
+                int D0 = 0;
+                for (int p = lane; p < K; p += 32) D0 = max(D0, abs(cnt_b[p]));
+                if (warp_max(D0) > max(lds(&B.slack[o]), 0)) {
+                  for (int p = lane; p < K; p += 32) cnt_b[p] += sizes_s[p];
+                  __syncwarp();
+                  const int nc = lds(&B.ncand[o]);
+                  if ((nc < 0 || recheck(I, rC, cnt_b, nc, B.cand + (size_t)o * K, metric == kTV, own) != (pk & 0xffff)) &&
+                      lane == 0)
+                    atomicMin(flip_w, (z << 3) | 2);
+                }
+              }
+              __syncthreads();
+            }
+          }
+          if (!why || grid) {
+            const int c = conflicts(I, B, vol, z, own, leaves, fl & 1, base, deg, k0, kstep, ov);
+            if (c) atomicMin(cut_w, (z << 3) | c);
+          }
+          if (why && threadIdx.x == 0) atomicMin(cut_w, (z << 3) | why);
+        };
         __syncthreads();
-        const unsigned long long tV2 = gtimer();
-        for (int mi = lower_bound_pos(B.mid_pos, B.nmid, cz0); mi < B.nmid; mi++) {
+        for (int mi = mi0; mi < mend; mi += gridDim.x) {
           const int z = __ldg(&B.mid_pos[mi]);
-          if (z >= cz1) break;
-          if (z < zfix) continue;
-          cta_validate_ldg(I, B, R, metric, z, pos, q, par, mtpos, s_pre_w, s_pre_v, s_cw, s_cv, cnt_b, dsz_cta,
-                           cta_o0, true, cut_w);
+          if (z >= zto) break;
+          if (z >= zfrom) check_big(z, threadIdx.x, blockDim.x, true, false);
         }
         for (int j = 0; j < ns; j++) {
-          // a whole-grid vertex: its nets checked by every thread, the rest by the
-          // CTA owning its position
-          const int zs = s_gz[j], own_s = s_go[j];
-          if (zs < zfix) continue;
-          const int os = zs - pos;
-          const int fl = lds(&B.flag[os]);
-          const int c = conflicts(I, B, vol, zs, own_s, (lds(&B.dec[os]) & 0xffff) != own_s, fl & 1, s_gb[j], s_gd[j],
-                                  gtid, gthreads, lds(&B.ctab_over[par]) != 0);
-          if (c) atomicMin(cut_w, (zs << 3) | c);
-          if (zs >= cz0 && zs < cz1)
-            cta_validate_ldg(I, B, R, metric, zs, pos, q, par, mtpos, s_pre_w, s_pre_v, s_cw, s_cv, cnt_b, dsz_cta,
-                             cta_o0, false, cut_w);
+          const int z = s_gz[j];
+          if (z >= zto) break;
+          if (z >= zfrom) check_big(z, gtid, gthreads, (int)blockIdx.x == j % (int)gridDim.x, true);
         }
-        __syncthreads();
-        if (kTimingStats && threadIdx.x == 0) {
-          const unsigned long long tV3 = gtimer();
-          atomicMax(&B.stats[39], tV3 - tV);
-          // per-pass phase times of this CTA: prefix sums, light positions, the rest
-          atomicAdd(&B.stats[45], tV1 - tV);
-          atomicAdd(&B.stats[46], tV2 - tV1);
-          atomicAdd(&B.stats[47], tV3 - tV2);
+      };
+      validate(pos, end_w, true);
+      if (!grid_barrier(B.bar, I.status)) return;
+      int cutw = lds(cut_w);
+      const int flipw = lds(flip_w);
+      int hard = kNone;
+      if ((flipw >> 3) < (cutw >> 3)) {
+        // ---- decisions change: walk from the first one to the cut with the exact
+        // sizes (block 0); the positions whose decision changed are redone by
+        // their warps, and the window is walked again behind an outcome that
+        // was mispredicted; then the rest of the window is validated again
+        const int zf = flipw >> 3, zc = min(end_w, cutw >> 3);
+        for (int zs = zf, nw = 1;; nw++) {
+          const unsigned long long tW = gtimer();
+          if (blockIdx.x == 0) walk_window(I, B, R, metric, pos, zs, zc, lds(&B.mcnt[par]), walk_s, walk_sz, walk_pn);
+          if (!grid_barrier(B.bar, I.status)) return;
+          hard = lds(&B.ctl[0]);
+          const int nchg = lds(&B.ctl[1]);
+          const unsigned long long tF = gtimer();
+          if (blockIdx.x == 0 && threadIdx.x == 0) {
+            B.stats[44] += nchg;
+            B.stats[45] += tF - tW;
+          }
+          if (nchg == 0) break;
+          int* const mis = &B.ctl[8 + (wr & 1)];
+          for (int z = max(z0, zs); z < z1; z++) {
+            const int fl = lds(&B.flag[z - pos]);
+            if (fl & 128)
+              fix_position(I, B, R, metric, z, z - pos, fl, par, mis, cut_w, loc, gains, losses, adelta, logp);
+          }
+          if (!grid_barrier(B.bar, I.status)) return;
+          const int zm = lds(mis);
+          if (blockIdx.x == 0 && threadIdx.x == 0) {
+            B.ctl[8 + ((wr & 1) ^ 1)] = kNone;   // the next walk's word
+            B.stats[46] += gtimer() - tF;
+          }
+          wr++;
+          if (zm == kNone) break;
+          // the outcome at zm is exact now; what follows it is walked again
+          zs = zm + 1;
+          if (nw == B.maxfix) {
+            hard = min(hard, (zs << 3) | 2);
+            break;
+          }
+          if (zs >= zc) break;
         }
+        const int lim = hard == kNone ? zc : min(hard >> 3, zc);
+        validate(zf, lim, false);
         if (!grid_barrier(B.bar, I.status)) return;
         cutw = lds(cut_w);
-        if (blockIdx.x == 0 && threadIdx.x == 0) B.ctl[4 + ((vr + 1) & 1)] = kNone;   // the next pass's word
-        vr++;
-        // a size flip of a light position (MSV / MSRV): fix it and validate again
-        bool fix = vfix && nfix < B.maxfix && cutw != kNone && (cutw & 7) == 2;
-        const int zc = cutw >> 3;
-        if (fix) fix = zc < end_w && __ldg(&B.vclass[__ldg(&B.porder[zc])]) == 0;
-        if (!fix) break;
-        if (gw == (zc - pos) / q)
-          fix_position(I, B, R, metric, zc, zc - pos, par, gw, loc, gains, losses, adelta, logp);
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-          B.stats[44]++;
-          B.stats[35] += B.stats[39];
-          B.stats[39] = 0;
-        }
-        if (!grid_barrier(B.bar, I.status)) return;
-        zfix = zc;
+        if (hard != kNone && (hard >> 3) < end_w) cutw = min(cutw, hard);
       }
       // ---- C: commit every mover before the cut.
       const int cut = cutw == kNone ? end_w : min(cutw >> 3, end_w);
@@ -1517,10 +1934,8 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         // per-window maxima over CTAs (no CTA writes these again before the next phase A)
         B.stats[32] += B.stats[36];
         B.stats[34] += B.stats[38];
-        B.stats[35] += B.stats[39];
         B.stats[36] = 0;
         B.stats[38] = 0;
-        B.stats[39] = 0;
         B.stats[17] += tB - tA;
         tA = tB;
       }
@@ -1561,9 +1976,8 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         }
         unclaim_nets(I, B, vol, base, deg, lane, 32, fl & 1, fl & 64);
       }
-      for (int mi = lower_bound_pos(B.mid_pos, B.nmid, cz0); mi < B.nmid; mi++) {
+      for (int mi = mi0; mi < mend; mi += gridDim.x) {
         const int z = __ldg(&B.mid_pos[mi]);
-        if (z >= cz1) break;
         const int o = z - pos;
         const int fl = lds(&B.flag[o]);
         if (!(fl & 1)) continue;
@@ -1618,25 +2032,16 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         // exact sizes between the committed positions (MSRV never moves them;
         // there they are walked only for the decision records).
         int* dsz = gains_b;   // the committed movers' size changes before this CTA's first position
-        const int cta_o0 = cz0 - pos;
-        for (int p = threadIdx.x; p < K; p += blockDim.x) dsz[p] = 0;
         __syncthreads();
-        const int nmv = lds(&B.mcnt[par]);
-        for (int i = threadIdx.x; i < nmv; i += blockDim.x) {
-          const int4 m = lds(&B.mlist[i]);
-          if (m.x >= cta_o0 || m.y == 0) continue;
-          atomicAdd(&dsz[m.z & 0xffff], m.y);
-          atomicAdd(&dsz[m.z >> 16], -m.y);
-        }
-        __syncthreads();
+        moved_before(cta_o0, dsz);
         const int zb = min(z1, cut);
         if (z0 < zb) {
           int* sz = cnt;   // this warp's sizes, at its current position
           for (int p = lane; p < K; p += 32) sz[p] = sizes_s[p] + dsz[p];
           __syncwarp();
           for (int o2 = cta_o0 + lane; o2 < z0 - pos; o2 += 32) {
+            if (!(lds(&B.flag[o2]) & 1)) continue;
             const int w = lds(&B.wt[o2]);
-            if (w == 0) continue;
             const int pk = lds(&B.dec[o2]);
             atomicAdd(&sz[pk & 0xffff], w);
             atomicAdd(&sz[pk >> 16], -w);
@@ -1676,7 +2081,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
           for (int z = z0; z < zb; z++) {
             const int o = z - pos;
             const int w = lds(&B.wt[o]);
-            if (w != 0) {
+            if (w != 0 && (lds(&B.flag[o]) & 1)) {
               __syncwarp();
               if (lane == 0) {
                 const int pk = lds(&B.dec[o]);
@@ -1732,15 +2137,17 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
       }
       if (gw == 0 && lane == 0) {
         B.ctl[2 + (par ^ 1)] = kNone;
-        B.ctab_over[par ^ 1] = 0;
+        B.ctl[4 + (par ^ 1)] = kNone;
+        B.ctl[6 + (par ^ 1)] = kNone;
         B.mcnt[par ^ 1] = 0;
+        B.ctab_over[par ^ 1] = 0;
       }
       prev_maxtouch = mt_c < cut;
       if (cut == end_w) {
         if (end_w == pos + W) W = min(2 * W, B.wmax);
       } else {
         // regrow from the last valid length
-        W = min(B.wmax, max(B.wmin > 0 ? B.wmin : nwarps, B.wgrow * (cut - pos)));
+        W = min(B.wmax, max(B.wmin > 0 ? B.wmin : 128, max(W / 4, B.wgrow * (cut - pos))));
       }
       pos = cut;
       round++;
@@ -1766,7 +2173,8 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
 size_t spec_ldg_smem_bytes(int K) {
   auto a = [](size_t n) { return (n + 15) & ~size_t(15); };
   const size_t k4 = a(sizeof(int) * K);
-  return 5 * k4 + 4 * a(sizeof(int) * (size_t)K * kSWarps) + a(sizeof(unsigned long long) * (size_t)K * kSWarps);
+  const size_t eval = 4 * a(sizeof(int) * (size_t)K * kSWarps) + a(sizeof(unsigned long long) * (size_t)K * kSWarps);
+  return 5 * k4 + std::max(eval, sizeof(WalkSmem) + sizeof(float2) * K);
 }
 
 cudaError_t launch_spec_ldg(const DevInstance& I, const SpecBuf& B, int passes, int num_sms, cudaStream_t st,
