@@ -544,9 +544,9 @@ static int build_stream_positions(fp_instance* in) {
 
 // Positions of the LDG engine (TV / MSV / MSRV).  A vertex without nets and
 // with weight 0 reads only the part sizes and changes nothing that a later
-// decision reads; for TV, when every vertex without nets weighs 0 (vertex
-// weight = degree), they are left out of the walked positions and decided
-// after each window from the exact sizes at their place.  Uploads porder, iso_list and
+// decision reads; when every vertex without nets weighs 0 (vertex weight =
+// degree), they are left out of the walked positions and decided after each
+// window from the exact sizes at their place.  Uploads porder, iso_list and
 // iso_before and fills the SpecBuf fields.
 static int build_positions(fp_instance* in) {
   const HostGraph& g = in->g;
@@ -559,11 +559,9 @@ static int build_positions(fp_instance* in) {
       any_iso = true;
       if (pb.w[v] != 0) compact = false;
     }
-  // Measured on the 4M-vertex Zipf workload (degree weights): TV 75 -> 48 ms
-  // per pass; MSV unchanged and MSRV slower (430 vs 318 ms), because their
-  // windows end every few dozen positions (max-volume changes, in-window
-  // fixes) and a window of compacted positions wastes more evaluations past
-  // its cut -- so only TV walks compacted positions.
+  // Measured on Zipf workloads (degree weights): TV 75 -> 48 ms per pass (4M
+  // vertices), MSV 243 -> 207 and MSRV 47.2 -> 45.3 (256K vertices, one and two
+  // passes).
   compact = compact && any_iso;
   for (int z = 0; z < g.nov; z++) {
     const int v = pb.order[z];
@@ -730,7 +728,7 @@ int fp_instance_create(fp_ctx* ctx, const fp_hypergraph* h, int32_t K, int32_t m
         (rc = dalloc(in, &in->sb.cand, (size_t)kSpecWindow * K)) || (rc = dalloc(in, &in->sb.ncand, kSpecWindow)) ||
         (rc = dalloc(in, &in->sb.mlist, kSpecWindow)) || (rc = dalloc(in, &in->sb.midx, kSpecWindow)) ||
         (rc = dalloc(in, &in->sb.mcnt, 2)) ||
-        (rc = dalloc(in, &in->sb.acc, kSpecWindow)) ||
+        (rc = dalloc(in, &in->sb.acc, kSpecWindow)) || (rc = dalloc(in, &in->sb.rel, kSpecWindow)) ||
         (rc = dalloc(in, &in->sb.claim_m, g.noe)) || (rc = dalloc(in, &in->sb.claim64, g.noe)) || (rc = dalloc(in, &in->sb.claim_c, g.noe)) ||
         (rc = dalloc(in, &in->sb.mask_c, g.noe)) || (rc = dalloc(in, &in->sb.hcnt, 2 * kMaxGridVerts * K)) ||
         (rc = dalloc(in, &in->sb.hfirst, 2 * kMaxGridVerts * K)) ||
@@ -776,9 +774,7 @@ int fp_instance_create(fp_ctx* ctx, const fp_hypergraph* h, int32_t K, int32_t m
     // window regrowth after a cut: twice the last valid length for MSV (cuts
     // every few hundred positions), four times for the metrics with rarer cuts
     in->sb.wgrow = metric == FP_METRIC_MSV ? 2 : 4;
-    // at least one position per warp of the grid after a cut: measured on the
-    // 4M-vertex Zipf workload, MSRV 410 -> 355 ms per pass, MSV 912 -> 906,
-    // TV unchanged (against 256)
+    // 0: the kernels' own shortest window after a cut
     in->sb.wmin = 0;
     in->sb.maxfix = 32;
     in->sb.max_warps = kMaxSpecWarps;
@@ -871,7 +867,7 @@ int fp_instance_footprint(int32_t nov, int32_t noe, int64_t pins, int32_t K, int
     add(cn ? P : 1, 8); add(cn ? E : 1, 4); add(cn ? E : 1, 8); add(4, 4); add(cn ? V : 1, 4);
     add(V, 1);                                               // vertex classes
     add(W * K, 8); add(W, 4); add(W, 16); add(W, 4); add(2, 4);   // cand, ncand, mlist, midx, mcnt
-    add(W, 4);                                               // acc
+    add(W, 4); add(W, 4);                                    // acc, rel
     add(E, 4); add(E, 8); add(E, 4); add(E, 4);              // claim_m, claim64, claim_c, mask_c
     add(G2K, 4); add(G2K, 8); add(G2K, 4); add(G2K, 4); add(G2K, 4);
     add(16 * (size_t)kMaxGridVerts, 4); add(K, 8);           // hmisc, mlast
@@ -924,7 +920,7 @@ static int device_stream(fp_instance* in) {
   const int K = in->pb.K;
   DevInstance& d = in->d;
   static const int none[kCtlWords] = {0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff,
-                                      0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff};
+                                      0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0, 0};
   cudaError_t e = cudaMemsetAsync(d.part_vec, 0xff, sizeof(int) * g.nov, s);
   auto zero = [&](void* p, size_t bytes, int val) {
     if (e == cudaSuccess && bytes) e = cudaMemsetAsync(p, val, bytes, s);
@@ -1069,7 +1065,7 @@ int fp_refine(fp_instance* in, int32_t passes) {
     in->recs_valid = false;
     if (spec) {
       static const int none[kCtlWords] = {0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff,
-                                      0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff};
+                                      0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0, 0};
       if (e == cudaSuccess) e = cudaMemcpyAsync(in->sb.ctl, none, sizeof(none), cudaMemcpyHostToDevice, s);
       if (e == cudaSuccess) e = cudaMemsetAsync(in->sb.bar, 0, sizeof(unsigned) * 4, s);
       if (e == cudaSuccess && (in->fault_leave_at || in->fault_poll_limit)) {

@@ -94,16 +94,19 @@ constexpr int kMaxGridVerts = 8;
 // instance.
 struct SpecBuf {
   unsigned* bar;         // [4] grid barrier: arrivals, generation, abort
-  int* ctl;              // [12] per-round words: [2,3] first max-touching mover, [4,5] cut,
-                         //     [6,7] first changed decision (by round parity), [0,1] the
-                         //     walk's end and changes, [8,9] misprediction (by walk parity)
+  int* ctl;              // [12] [2,3] first max-touching mover, [4,5] cut (by round parity),
+                         //     [6,7] first changed decision, [10,11] their number (by
+                         //     validation parity), [0,1] the walk's end and changes, [8]
+                         //     first outcome it mispredicted, [9] first change without room
   int* dec;              // [wmax] (own part << 16) | decision per window offset
   unsigned char* flag;   // [wmax] bit0 mover, bit1 stale-marker risk, bit2 CTA / grid evaluated,
                          //     bit3 no nets, bit4 accepted, bit5 decision changed in the
                          //     window, bit6 claims of a replaced move held (rec_slot2),
-                         //     bit7 the last walk changed the decision (dfix)
-  int* dfix;             // [wmax] (predicted mover << 16) | exact decision the walk took
+                         //     bit7 the decision changes (dfix)
+  int* dfix;             // [wmax] the changed decision; the walk's with (predicted mover << 16)
   int* slack;            // [wmax] part-size drift the decision tolerates (-1: none)
+  int* rel;              // [wmax] drift it tolerates beyond the window's validated movers
+                         //     (-2: its decision changes)
   int* vslack;           // [wmax] volume drift the accept/reject outcome tolerates
   int* wt;               // [wmax] vertex weight (streams: of the placed vertex)
   int* vd;               // [wmax] largest volume change of one part by a mover

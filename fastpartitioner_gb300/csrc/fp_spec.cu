@@ -18,8 +18,11 @@
 //                 volumes stay within its volume slack; if it would leave its
 //                 part, no earlier mover touched a max-volume part; for TV, no
 //                 stale marker can apply.  The first invalid position cuts the
-//                 window (MSV / MSRV fix a position whose decision the size
-//                 drift flipped in place and validate again from it).
+//                 window.  Decisions that the size drift changes do not: they are
+//                 taken again -- a few in a long window all at once, otherwise by
+//                 a walk of one CTA over the positions in order (walk_window) --
+//                 their moves and claims are redone, and the window is validated
+//                 again from the first of them.
 //   C  commit     all movers before the cut are applied at once -- on any net
 //                 they either are alone or only shift counts, which commute --
 //                 and the next window starts at the cut.
@@ -49,7 +52,7 @@ constexpr int kBig = 1000000000;
 
 struct RoundCtx {
   const int* sizes;
-  const float* penf;   // 1 - size / C in float (off by < 4e-7 * (1 + size / C))
+  const float* penf;   // 1 - size / C in float (pen_of)
   const int* marker;
   const int* vol;
   const int* mark;
@@ -57,24 +60,84 @@ struct RoundCtx {
   float Cf;            // C rounded to float
 };
 
-// LDG argmax over the tallied parts (TV/partition.cpp:98-145 with TV's clamps,
-// MGV/partition.cpp:28-65 without), executed by one warp, plus the part-size
-// drift under which the outcome cannot change.
+// LDG scores (TV/partition.cpp:98-145 with TV's clamps, MGV/partition.cpp:28-65
+// without).  They are first formed in float, from the penalty 1 - size / C off
+// by less than 4e-7 * (1 + size / C); a score of count c is bounded within
+// c * 1e-6 * (1 + size / C).  A part whose lower bound clears every other's
+// upper bound is the argmax; near parts with one common count need no FP64
+// either: with equal counts the score falls (weakly: division, subtraction and
+// product round monotonically) as the size grows, and equal scores go to the
+// smaller size, so the smallest size, then the first sighting, wins.  The
+// exact double scores (722 cycles each here, against 22 for a redux.sync)
+// decide what is left.
 //
-// Scores are first formed in float from the float penalty 1 - size / C, which
-// is off by less than 4e-7 * (1 + size / C); a score of count c is bounded
-// within tol = 1e-6 * c * (1 + |size / C|).  The exact double score (the
-// reference's arithmetic) and the tie-breaks are then evaluated only for parts
-// whose upper bound reaches the largest lower bound: a set that holds the
-// exact argmax and all its ties.  The slack bounds use lower bounds of the
-// score gaps (a low bound only costs an exact re-check).
-__device__ __forceinline__ float score_tol(int c, float pf) { return (float)c * 1e-6f * (1.0f + fabsf(1.0f - pf)); }
-__device__ __forceinline__ int slack_divf(float a, float b) {
-  const float x = __fdiv_rn(a, b) * (1.0f - 1e-5f) - 1.0f;
-  if (!(x > -1.0f)) return -1;
-  if (x > 1.0e9f) return kBig;
-  return (int)floorf(x);
+// Penalty of a part and the bound of its error per count, from rC = 1 / C
+// rounded to float.
+__device__ __forceinline__ float tol_of(float pen) { return 1e-6f * (1.0f + fabsf(1.0f - pen)); }
+__device__ __forceinline__ float2 pen_of(int size, float rC) {
+  const float pen = 1.0f - __fmul_rn((float)size, rC);
+  return make_float2(pen, tol_of(pen));
 }
+// A drift below a / b with room for the roundings: floor(a / b) - 2 or less,
+// capped; -1 if not positive.
+__device__ __forceinline__ int slack_of(float a, float b) {
+  const float x = __fdividef(a, b) * (1.0f - 2e-5f) - 2.0f;
+  return !(x > -1.0f) ? -1 : x > 1.0e9f ? kBig : (int)x;
+}
+
+// What one pass over scored parts keeps: the best lower bound (its upper bound,
+// part and count) and the largest upper bound of the others, the largest
+// penalty and count.
+constexpr float kLow = -1e30f;
+struct ScoreAcc {
+  float blo = kLow, bhi = kLow, oh = kLow, up = kLow;
+  unsigned be = 0;   // (count << 13) | part of the best
+  int cm = 0;
+  __device__ __forceinline__ void add(int p, int c, float2 w) {
+    const float cf = (float)c, v = cf * w.x;
+    const float lo = v - cf * w.y, hi = v + cf * w.y;
+    up = fmaxf(up, w.x + w.y);
+    cm = max(cm, c);
+    if (lo > blo) {
+      oh = fmaxf(oh, bhi);
+      blo = lo;
+      bhi = hi;
+      be = ((unsigned)c << 13) | (unsigned)p;
+    } else {
+      oh = fmaxf(oh, hi);
+    }
+  }
+  // meets the accumulators of the lanes whose ids differ in the low bits of
+  // `lanes` - 1 (8 lanes to a position, or the whole warp)
+  __device__ __forceinline__ void meet(int lanes) {
+#pragma unroll
+    for (int off = 1; off < lanes; off <<= 1) {
+      const float xl = __shfl_xor_sync(kAll, blo, off), xh = __shfl_xor_sync(kAll, bhi, off);
+      const float xo = __shfl_xor_sync(kAll, oh, off), xu = __shfl_xor_sync(kAll, up, off);
+      const unsigned xe = __shfl_xor_sync(kAll, be, off);
+      const int xc = __shfl_xor_sync(kAll, cm, off);
+      // equal bounds: the lower packed word on both sides, so that the lanes agree
+      const bool take = xl > blo || (xl == blo && xe < be);
+      oh = fmaxf(fmaxf(oh, xo), take ? bhi : xh);
+      if (take) {
+        blo = xl;
+        bhi = xh;
+        be = xe;
+      }
+      up = fmaxf(up, xu);
+      cm = max(cm, xc);
+    }
+  }
+  __device__ __forceinline__ bool one() const { return blo > 0.0f && oh < blo; }          // the argmax is clear
+  __device__ __forceinline__ bool none() const { return !(fmaxf(bhi, oh) > 0.0f); }       // no part scores
+  // drift of every part's size that leaves the clear argmax, or none, as it is
+  __device__ __forceinline__ int slack_one(float Cf) const {
+    const int cd = (int)(be >> 13);
+    const float diff = blo - oh - 1e-6f * (fabsf(blo) + fabsf(oh));
+    return min(slack_of(diff * Cf, (float)(cd + cm)), slack_of(blo * (1.0f - 1e-6f) * Cf, (float)cd));
+  }
+  __device__ __forceinline__ int slack_none(float Cf) const { return up <= kLow ? kBig : slack_of(-up * Cf, 1.0f); }
+};
 
 // Candidate entry of a part for the exact re-check: part (12 bits), count
 // without the vertex itself (16 bits), 32-bit sighting key.  A vertex whose
@@ -106,20 +169,13 @@ __device__ __forceinline__ int least_size_first(int size, F first, int part) {
   return m ? __shfl_sync(kAll, part, __ffs(m) - 1) : -1;
 }
 
-// One warp.  The tallied parts (count > 0, no stale TV marker) are first
-// compacted, in ascending order, into list (K ints of warp scratch); cand /
-// *ncand (if cand is not null) receive their re-check entries and scan (if not
-// null) TV's scanned-part bits.  The bound, exact and slack passes then walk
-// only the compacted parts.
-//
-// Near parts with one common count need no FP64: with equal counts the score
-// falls (weakly: division, subtraction and product round monotonically) as the
-// size grows, and equal scores go to the smaller size, so the smallest size,
-// then the first sighting, wins.  A score in double takes 722 cycles here; two
-// redux.sync take 44.
+// One warp decides a vertex from its tally.  cand / *ncand (if cand is not null)
+// receive the re-check entries of the tallied parts (count > 0, no stale TV
+// marker) and scan (if not null) TV's scanned-part bits; *slack_out the drift
+// of every part's size under which the decision stands.
 template <class F>
 __device__ int ldg_decide(const DevInstance& I, const RoundCtx& R, const int* cnt, const F* first, int sb,
-                          int metric, int v, int own, bool first_of_window, int* list, unsigned long long* cand,
+                          int metric, int v, int own, bool first_of_window, unsigned long long* cand,
                           int* ncand, uint32_t* scan, bool* special, int* slack_out) {
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
@@ -127,6 +183,8 @@ __device__ int ldg_decide(const DevInstance& I, const RoundCtx& R, const int* cn
   const bool tv = metric == kTV;
   int nc = 0;
   bool sp = false, wide = false;
+  ScoreAcc A;
+  auto usable = [&](int p, int c) { return c > 0 && !(tv && R.marker[p] == v); };
 #pragma unroll 4
   for (int p0 = 0; p0 < K; p0 += 32) {
     const int p = p0 + lane;
@@ -136,12 +194,12 @@ __device__ int ldg_decide(const DevInstance& I, const RoundCtx& R, const int* cn
     const bool ok = c > 0 && !stale;
     const unsigned m = __ballot_sync(kAll, ok);
     if (ok) {
-      const int i = nc + __popc(m & below);
-      list[i] = p;
+      const int cc = c - (p == own ? 1 : 0);
       if (cand) {
         wide |= c > 0xffff;
-        cand[i] = cand_entry(p, c - (p == own ? 1 : 0), key32(first[p], sb, &wide));
+        cand[nc + __popc(m & below)] = cand_entry(p, cc, key32(first[p], sb, &wide));
       }
+      if (cc > 0) A.add(p, cc, make_float2(R.penf[p], tol_of(R.penf[p])));
     }
     if (scan) {
       const unsigned ms = __ballot_sync(kAll, c > 0);
@@ -152,39 +210,26 @@ __device__ int ldg_decide(const DevInstance& I, const RoundCtx& R, const int* cn
   wide = __any_sync(kAll, wide);
   if (cand && lane == 0) *ncand = wide ? -1 : nc;
   *special = __any_sync(kAll, sp) && !first_of_window;
-  __syncwarp();
-  float fb = 0.0f;   // largest lower bound of a score (0: none positive for sure)
-  bool any = false;
-  for (int i = lane; i < nc; i += 32) {
-    const int p = list[i];
-    const int cc = cnt[p] - (p == own ? 1 : 0);
-    if (cc > 0) {
-      const float pf = R.penf[p];
-      const float f = __fmul_rn((float)cc, pf), t = score_tol(cc, pf);
-      fb = fmaxf(fb, f - t);
-      any |= f + t > 0.0f;
-    }
+  A.meet(32);
+  int d0 = R.minpart, sl = -1;
+  if (A.cm >= 1 << 19) {   // beyond the packed word (whole-grid vertices): exact scores
+    A.blo = A.oh = 1.0f;
   }
-  fb = warp_max_nonneg(fb);
-  LdgKey best{-1.0, 0, -1, ~0ull};
-  float sbest = 0.0f;   // a lower bound of the winner's exact score, in float
-  if (__any_sync(kAll, any)) {
-    // Parts whose upper bound reaches the largest lower bound: the argmax and
-    // all its ties are among them.  A single one with a positive lower bound
-    // is the argmax outright (every other score lies below fb); several of one
-    // count, one of them positive for sure, are ordered by size and sighting;
-    // otherwise the exact double scores (TV/partition.cpp:103-104) and
-    // tie-breaks decide.
-    int nnear = 0, np = -1, nsz = 0, cmin = 0x7fffffff, cmax = 0;
+  if (A.one()) {
+    d0 = (int)(A.be & 0x1fffu);
+    sl = A.slack_one(R.Cf);
+  } else if (A.none()) {
+    sl = min(A.slack_none(R.Cf), (R.second - R.minsize - 1) / 2);   // least-loaded part stays
+  } else {
+    // near parts: those whose upper bound reaches the largest lower bound
+    const float fb = fmaxf(A.cm >= 1 << 19 ? 0.0f : A.blo, 0.0f);
+    int np = -1, nsz = 0, cmin = 0x7fffffff, cmax = 0;
     F nf = ~(F)0;
-    for (int i = lane; i < nc; i += 32) {
-      const int p = list[i];
-      const int cc = cnt[p] - (p == own ? 1 : 0);
-      if (cc <= 0) continue;
-      const float pf = R.penf[p];
-      const float f = __fmul_rn((float)cc, pf), t = score_tol(cc, pf);
-      if (!(f + t > 0.0f) || f + t < fb) continue;
-      nnear++;
+    for (int p = lane; p < K; p += 32) {
+      const int c = cnt[p], cc = c - (p == own ? 1 : 0);
+      if (!usable(p, c) || cc <= 0) continue;
+      const float cf = (float)cc, hi = cf * R.penf[p] + cf * tol_of(R.penf[p]);
+      if (!(hi > 0.0f) || hi < fb) continue;
       cmin = min(cmin, cc);
       cmax = max(cmax, cc);
       const int sz = R.sizes[p];
@@ -195,73 +240,34 @@ __device__ int ldg_decide(const DevInstance& I, const RoundCtx& R, const int* cn
         nf = fp;
       }
     }
-    const int tot = warp_sum(nnear);
     cmin = warp_min(cmin);
     cmax = warp_max(cmax);
-    if (fb > 0.0f && (tot == 1 || cmin == cmax)) {
-      best.part = least_size_first<F>(nsz, nf, np);
-      const float pf = R.penf[best.part];
-      sbest = __fmul_rn((float)cmax, pf) - score_tol(cmax, pf);
+    if (fb > 0.0f && cmin == cmax) {
+      d0 = least_size_first<F>(nsz, nf, np);
     } else {
-      for (int i = lane; i < nc; i += 32) {
-        const int p = list[i];
-        const int cc = cnt[p] - (p == own ? 1 : 0);
-        if (cc <= 0) continue;
-        const float pf = R.penf[p];
-        const float f = __fmul_rn((float)cc, pf), t = score_tol(cc, pf);
-        if (!(f + t > 0.0f) || f + t < fb) continue;   // cannot be a positive best
+      LdgKey best{-1.0, 0, -1, ~0ull};
+      for (int p = lane; p < K; p += 32) {
+        const int c = cnt[p], cc = c - (p == own ? 1 : 0);
+        if (!usable(p, c) || cc <= 0) continue;
+        const float cf = (float)cc, hi = cf * R.penf[p] + cf * tol_of(R.penf[p]);
+        if (!(hi > 0.0f) || hi < fb) continue;   // cannot be a positive best
         const double pen = __dsub_rn(1.0, __ddiv_rn((double)R.sizes[p], I.C));   // TV/partition.cpp:103-104
         LdgKey k{__dmul_rn((double)cc, pen), R.sizes[p], p, key64(first[p], sb)};
         if (ldg_better(k, best)) best = k;
       }
       best = warp_ldg_argmax(best);
-      sbest = (float)best.score;
+      if (best.part >= 0) d0 = best.part;
     }
   }
-  const int d0 = best.part >= 0 ? best.part : R.minpart;
   int d = d0;
-  if (tv) {
-    if (R.sizes[d] > I.max_pw) d = own;
-    if (R.sizes[d] < I.min_pw) d = own;
-  }
-  // Drift margins: every part's size may move by at most D.  All conditions are
-  // monotone in D.
-  int sl = kBig;
-  const float Cf = R.Cf;
-  if (best.part >= 0) {
-    const int w = best.part;
-    const int cw = cnt[w] - (w == own ? 1 : 0);
-    const float Swf = sbest;
-    sl = min(sl, slack_divf(Swf * (1.0f - 1e-6f) * Cf, (float)cw) - 1);   // stays positive
-    for (int i = lane; i < nc; i += 32) {
-      const int q = list[i];
-      if (q == w) continue;
-      const int cq = cnt[q] - (q == own ? 1 : 0);
-      if (cq <= 0) continue;
-      const float pq = R.penf[q];
-      const float fq = __fmul_rn((float)cq, pq) + score_tol(cq, pq);   // above the exact score
-      const float diff = Swf - fq - 1e-6f * (fabsf(Swf) + fabsf(fq));   // below the exact gap
-      if (!(diff > 0.0f)) { sl = -1; continue; }                       // (near) tie: size / order decide
-      sl = min(sl, slack_divf(diff * Cf, (float)(cw + cq)) - 1);
-    }
-  } else {
-    for (int i = lane; i < nc; i += 32) {
-      const int q = list[i];
-      if (cnt[q] - (q == own ? 1 : 0) <= 0) continue;
-      // size - C, shrunk past float rounding of C
-      const float x = (float)R.sizes[q] - Cf - 1e-6f * Cf - 1.0f;
-      sl = min(sl, (!(x > -1.0f) ? -1 : x > 1.0e9f ? kBig : (int)floorf(x)) - 1);   // stays non-positive
-    }
-    sl = min(sl, (R.second - R.minsize - 1) / 2);                 // least-loaded part stays
-  }
   if (tv) {
     const int s0 = R.sizes[d0];
     sl = min(sl, s0 > I.max_pw ? s0 - I.max_pw - 1 : I.max_pw - s0);
-    const int d1 = s0 > I.max_pw ? own : d0;
-    const int s1 = R.sizes[d1];
+    if (s0 > I.max_pw) d = own;
+    const int s1 = R.sizes[d];
     sl = min(sl, s1 < I.min_pw ? I.min_pw - s1 - 1 : s1 - I.min_pw);
+    if (s1 < I.min_pw) d = own;
   }
-  sl = warp_min(sl);
   *slack_out = max(sl, -1);
   return d;
 }
@@ -567,7 +573,7 @@ __device__ void cta_eval_ldg(const DevInstance& I, const SpecBuf& B, const Round
   if (wib == 0) {
     bool special;
     int slack;
-    const int d = ldg_decide(I, R, cnt_b, first_b, sb, metric, v, own, z == pos, cnt_b + K, B.cand + (size_t)o * K,
+    const int d = ldg_decide(I, R, cnt_b, first_b, sb, metric, v, own, z == pos, B.cand + (size_t)o * K,
                              &B.ncand[o], metric == kTV ? B.scan + (size_t)o * words : nullptr, &special, &slack);
     if (lane == 0) {
       sh[0] = d;
@@ -650,14 +656,14 @@ __device__ void cta_eval_ldg(const DevInstance& I, const SpecBuf& B, const Round
 // positions (rows padded so that four rows read side by side meet no bank
 // conflict).
 constexpr int kWalkLoad = 1024, kWalkSub = 128, kWalkRow = 64, kWalkStride = kWalkRow + 8;
+static_assert(kWalkRow == 64, "two entries of a staged row per lane");
 struct WalkSmem {
   unsigned long long ent[kWalkSub * kWalkStride];
   int4 meta[kWalkLoad];      // (own << 16) | decision, weight, acc, (ncand << 8) | flag
-  int margin[kWalkLoad];     // drift at its group's start the position tolerates (-1: always taken again)
-  int gmin[kWalkLoad / 32];  // per group of 32: the smallest margin,
-  unsigned gsum[kWalkLoad / 32];   //   the weight its movers move
+  int margin[kWalkLoad];     // drift the position tolerates (-1: always taken again)
+  int gmin[kWalkLoad / 32];  // per group of 32: the smallest margin
   int nd[32], nslack[32];    // decisions taken again: (nets listing it << 13) | part (-1: no list), drift tolerated
-  unsigned drift;            // largest change of one part's size so far (an upper bound)
+  int drift;                 // largest change of one part's size so far by changed decisions (an upper bound)
   int group;                 // group to decide again (-1: none left), and its positions
   unsigned need;
 };
@@ -675,94 +681,105 @@ __device__ __forceinline__ int warp_least_loaded(const int* sz, int K, int* ms_o
   return warp_min(mp != 0x7fffffff && ms == m ? mp : 0x7fffffff);
 }
 
-// Penalty of a part as the walk scores it: 1 - size / C from the rounded 1 / C,
-// off by less than 4e-7 * (1 + size / C), and the bound 1e-6 * (1 + size / C)
-// used for it (per count of nets).
-__device__ __forceinline__ float2 walk_pen(int size, float rC) {
-  const float xf = __fmul_rn((float)size, rC);
-  return make_float2(1.0f - xf, 1e-6f * (1.0f + fabsf(xf)));
-}
-// Drift bound floor(a / b) - 2 at least, from below, capped; -1 if not positive.
-__device__ __forceinline__ int walk_slack(float a, float b) {
-  const float x = __fdividef(a, b) * (1.0f - 2e-5f) - 2.0f;
-  return !(x > -1.0f) ? -1 : x > 1.0e9f ? kBig : (int)x;
-}
-
 // One warp decides a position again with the sizes sz, whatever its candidates:
-// mt its words, cl all of its entries; exact double scores (TV/partition.cpp:
-// 103-104) unless the near ones share a count.  Returns the decision before
-// TV's clamps, (nets listing it << 13) | part; it tolerates no drift.
-__device__ __noinline__ int walk_pick_any(const DevInstance& I, float rC, const int* sz, int nc,
-                                          const unsigned long long* cl) {
+// nc of them, cl all of its entries.  Returns the decision before TV's clamps,
+// (nets listing it << 13) | part, and in *slack the drift of any part's size
+// from these that leaves it as it is.
+__device__ __noinline__ int walk_pick_any(const DevInstance& I, float rC, float Cf, const int* sz, int nc,
+                                          const unsigned long long* cl, int* slack) {
   const int lane = threadIdx.x & 31;
   const int K = I.K;
   const unsigned long long e0 = lane < nc ? lds(&cl[lane]) : 0;   // the first 32 stay in registers
-  float fb = 0.0f;
+  ScoreAcc A;
   for (int i = lane; i < nc; i += 32) {
     const unsigned long long e = i < 32 ? e0 : lds(&cl[i]);
-    const int c = (int)((e >> 36) & 0xffffull);
-    const float2 w = walk_pen(sz[(int)(e >> 52)], rC);
-    fb = fmaxf(fb, (float)c * w.x - (float)c * w.y);
+    const int p = (int)(e >> 52), c = (int)((e >> 36) & 0xffffull);
+    if (c > 0) A.add(p, c, pen_of(sz[p], rC));
   }
-  fb = warp_max_nonneg(fb);
-  int np = -1, nsz = 0, cmin = 0x7fffffff, cmax = 0;
-  unsigned nf = ~0u;
-  for (int i = lane; i < nc; i += 32) {
-    const unsigned long long e = i < 32 ? e0 : lds(&cl[i]);
-    const int p = (int)(e >> 52), c = (int)((e >> 36) & 0xffffull), s = sz[p];
-    const float2 w = walk_pen(s, rC);
-    if (c == 0 || (float)c * w.x + (float)c * w.y < fb) continue;
-    cmin = min(cmin, c);
-    cmax = max(cmax, c);
-    if (np < 0 || s < nsz || (s == nsz && (unsigned)e < nf)) { np = p; nsz = s; nf = (unsigned)e; }
-  }
-  cmin = warp_min(cmin);
-  cmax = warp_max(cmax);
-  int dn = -1, cd = 0;
-  if (fb > 0.0f && cmin == cmax) {
-    dn = least_size_first<unsigned>(nsz, nf, np);
-    cd = cmax;
-  } else if (cmax > 0) {
-    LdgKey best{-1.0, 0, -1, ~0ull};
-    int bc = 0;
-    for (int i = lane; i < nc; i += 32) {
-      const unsigned long long e = i < 32 ? e0 : lds(&cl[i]);
-      const int p = (int)(e >> 52), c = (int)((e >> 36) & 0xffffull), s = sz[p];
-      const float2 w = walk_pen(s, rC);
-      if (c == 0 || (float)c * w.x + (float)c * w.y < fb) continue;
-      const LdgKey k{ldg_score(c, s, I.C), s, p, e & 0xffffffffull};
-      if (ldg_better(k, best)) { best = k; bc = c; }
-    }
-    const int mine = best.part;
-    best = warp_ldg_argmax(best);
-    if (best.part >= 0) {
-      dn = best.part;
-      cd = __shfl_sync(kAll, bc, __ffs(__ballot_sync(kAll, mine == dn)) - 1);
-    }
-  }
-  if (dn < 0) {
+  A.meet(32);
+  int nd = -1, sl = -1;
+  if (A.one()) {
+    nd = (int)A.be;
+    sl = A.slack_one(Cf);
+  } else if (A.none()) {
     // no part scores: the least-loaded one, and the nets listing it all the same
-    int ms, cx = 0;
-    dn = warp_least_loaded(sz, K, &ms);
+    int ms, cx = 0, s2 = 0x7fffffff;
+    const int dn = warp_least_loaded(sz, K, &ms);
+    for (int p = lane; p < K; p += 32)
+      if (p != dn) s2 = min(s2, sz[p]);
+    sl = min(A.slack_none(Cf), (warp_min(s2) - ms - 1) / 2);
     for (int i = lane; i < nc; i += 32) {
       const unsigned long long e = i < 32 ? e0 : lds(&cl[i]);
       if ((int)(e >> 52) == dn) cx = (int)((e >> 36) & 0xffffull);
     }
-    cd = warp_max(cx);
+    nd = (warp_max(cx) << 13) | dn;
+  } else {
+    const float fb = fmaxf(A.blo, 0.0f);
+    int np = -1, nsz = 0, cmin = 0x7fffffff, cmax = 0;
+    unsigned nf = ~0u;
+    for (int i = lane; i < nc; i += 32) {
+      const unsigned long long e = i < 32 ? e0 : lds(&cl[i]);
+      const int p = (int)(e >> 52), c = (int)((e >> 36) & 0xffffull), s = sz[p];
+      const float2 w = pen_of(s, rC);
+      if (c == 0 || (float)c * w.x + (float)c * w.y < fb) continue;
+      cmin = min(cmin, c);
+      cmax = max(cmax, c);
+      if (np < 0 || s < nsz || (s == nsz && (unsigned)e < nf)) { np = p; nsz = s; nf = (unsigned)e; }
+    }
+    cmin = warp_min(cmin);
+    cmax = warp_max(cmax);
+    if (fb > 0.0f && cmin == cmax) {
+      nd = (cmax << 13) | least_size_first<unsigned>(nsz, nf, np);
+    } else {
+      LdgKey best{-1.0, 0, -1, ~0ull};
+      int bc = 0;
+      for (int i = lane; i < nc; i += 32) {
+        const unsigned long long e = i < 32 ? e0 : lds(&cl[i]);
+        const int p = (int)(e >> 52), c = (int)((e >> 36) & 0xffffull), s = sz[p];
+        const float2 w = pen_of(s, rC);
+        if (c == 0 || (float)c * w.x + (float)c * w.y < fb) continue;
+        const LdgKey k{ldg_score(c, s, I.C), s, p, e & 0xffffffffull};   // TV/partition.cpp:103-104
+        if (ldg_better(k, best)) { best = k; bc = c; }
+      }
+      const int mine = best.part;
+      best = warp_ldg_argmax(best);
+      if (best.part >= 0) {
+        nd = (__shfl_sync(kAll, bc, __ffs(__ballot_sync(kAll, mine == best.part)) - 1) << 13) | best.part;
+      } else {
+        int ms, cx = 0;
+        const int dn = warp_least_loaded(sz, K, &ms);
+        for (int i = lane; i < nc; i += 32) {
+          const unsigned long long e = i < 32 ? e0 : lds(&cl[i]);
+          if ((int)(e >> 52) == dn) cx = (int)((e >> 36) & 0xffffull);
+        }
+        nd = (warp_max(cx) << 13) | dn;
+      }
+    }
   }
-  return (cd << 13) | dn;
+  *slack = sl;
+  return nd;
+}
+
+// TV's clamps on the decision *d of a vertex of part own (TV/partition.cpp:
+// 135-143): returns the drift that leaves them as they are.
+__device__ __forceinline__ int tv_clamp(const DevInstance& I, const int* sz, int own, int* d, int sl) {
+  const int s0 = sz[*d];
+  sl = min(sl, s0 > I.max_pw ? s0 - I.max_pw - 1 : I.max_pw - s0);
+  if (s0 > I.max_pw) *d = own;
+  const int s1 = sz[*d];
+  sl = min(sl, s1 < I.min_pw ? I.min_pw - s1 - 1 : s1 - I.min_pw);
+  if (s1 < I.min_pw) *d = own;
+  return sl;
 }
 
 // A position's decision taken again with the sizes sz, TV's clamps included
-// (-1: it has no candidate list).  One warp.
-__device__ __forceinline__ int recheck(const DevInstance& I, float rC, const int* sz, int nc,
-                                       const unsigned long long* cl, bool tv, int own) {
+// (-1: it has no candidate list), and the drift from them it tolerates.  One warp.
+__device__ __forceinline__ int recheck(const DevInstance& I, float rC, float Cf, const int* sz, int nc,
+                                       const unsigned long long* cl, bool tv, int own, int* slack) {
+  *slack = -1;
   if (nc < 0) return -1;
-  int d = walk_pick_any(I, rC, sz, nc, cl) & 0x1fff;
-  if (tv) {
-    if (sz[d] > I.max_pw) d = own;
-    if (sz[d] < I.min_pw) d = own;
-  }
+  int d = walk_pick_any(I, rC, Cf, sz, nc, cl, slack) & 0x1fff;
+  if (tv) *slack = tv_clamp(I, sz, own, &d, *slack);
   __syncwarp();
   return d;
 }
@@ -772,7 +789,7 @@ __device__ __forceinline__ int recheck(const DevInstance& I, float rC, const int
 // candidates' scores and the largest upper bound of the others, three shuffles
 // meet them.  One candidate clear of the rest wins and tolerates the drift
 // that leaves it so; with none above zero the least-loaded part does.
-// Near-ties and long lists go to walk_pick_any, a warp each.
+// Near-ties of several counts and long lists go to walk_pick_any, a warp each.
 __device__ __forceinline__ void walk_eval(const DevInstance& I, const SpecBuf& B, const RoundCtx& R, bool tv, float rC,
                                           const int* sz, const float2* pen, WalkSmem& S, int i0, int sc, int ol) {
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -786,54 +803,20 @@ __device__ __forceinline__ void walk_eval(const DevInstance& I, const SpecBuf& B
   const bool todo = marked && !(mt.w & 8);
   const bool staged = todo && nc >= 0 && nc <= kWalkRow;
   const unsigned long long* row = S.ent + (size_t)(i0 - sc + l) * kWalkStride;
-  constexpr float kLow = -1e30f;
-  float blo = kLow, bhi = kLow, oh = kLow, up = kLow;
-  unsigned be = 0;
-  int cm = 0;
+  ScoreAcc A;
   const int ncl = staged ? nc : 0;
   for (int x = lane & 7; x < ncl; x += 8) {
-    const unsigned long long e = row[x];
-    const unsigned hi32 = (unsigned)(e >> 32);
+    const unsigned hi32 = (unsigned)(row[x] >> 32);
     const int p = (int)(hi32 >> 20), c = (int)((hi32 >> 4) & 0xffffu);
-    const float2 w = pen[p];
-    const float cf = (float)c;
-    const float v = cf * w.x;
-    const float lo = v - cf * w.y, hi = v + cf * w.y;
-    if (c > 0) {
-      up = fmaxf(up, w.x + w.y);
-      cm = max(cm, c);
-      if (lo > blo) {
-        oh = fmaxf(oh, bhi);
-        blo = lo;
-        bhi = hi;
-        be = ((unsigned)c << 13) | (unsigned)p;
-      } else {
-        oh = fmaxf(oh, hi);
-      }
-    }
+    if (c > 0) A.add(p, c, pen[p]);
   }
-#pragma unroll
-  for (int off = 1; off < 8; off <<= 1) {
-    const float xl = __shfl_xor_sync(kAll, blo, off), xh = __shfl_xor_sync(kAll, bhi, off);
-    const float xo = __shfl_xor_sync(kAll, oh, off);
-    const unsigned xe = __shfl_xor_sync(kAll, be, off);
-    oh = fmaxf(fmaxf(oh, xo), xl > blo ? bhi : xh);
-    if (xl > blo) {
-      blo = xl;
-      bhi = xh;
-      be = xe;
-    }
-    up = fmaxf(up, __shfl_xor_sync(kAll, up, off));
-    cm = max(cm, __shfl_xor_sync(kAll, cm, off));
-  }
-  const bool one = staged && blo > 0.0f && oh < blo;
-  const bool none = staged && !(fmaxf(bhi, oh) > 0.0f);
+  A.meet(8);
+  const bool one = staged && A.one();
+  const bool none = staged && A.none();
   int nd = nc < 0 ? -1 : 0, sl = -1;
   if (one) {
-    nd = (int)be;
-    const int cd = (int)(be >> 13);
-    const float diff = blo - oh - 1e-6f * (fabsf(blo) + fabsf(oh));
-    sl = min(walk_slack(diff * R.Cf, (float)(cd + cm)), walk_slack(blo * (1.0f - 1e-6f) * R.Cf, (float)cd));
+    nd = (int)A.be;
+    sl = A.slack_one(R.Cf);
   }
   if (__any_sync(kAll, none)) {
     int ms, s2 = 0x7fffffff;
@@ -852,24 +835,58 @@ __device__ __forceinline__ void walk_eval(const DevInstance& I, const SpecBuf& B
     }
     if (none) {
       nd = (cd << 13) | am;
-      sl = min((s2 - ms - 1) / 2, up <= kLow ? kBig : walk_slack(-up * R.Cf, 1.0f));
+      sl = min((s2 - ms - 1) / 2, A.slack_none(R.Cf));
     }
   }
-  const bool slow = todo && nc >= 0 && !one && !none;
+  // near-ties of one count, one of them positive for sure: by size and first
+  // sighting, as in ldg_decide
+  bool tied = staged && !one && !none && A.blo > 0.0f;
+  if (__any_sync(kAll, tied)) {
+    int cmin = 0x7fffffff, cmax = 0;
+    unsigned long long bk = ~0ull;
+    int bp = 0;
+    for (int x = lane & 7; x < ncl; x += 8) {
+      const unsigned long long e = row[x];
+      const unsigned hi32 = (unsigned)(e >> 32);
+      const int p = (int)(hi32 >> 20), c = (int)((hi32 >> 4) & 0xffffu);
+      const float2 w = pen[p];
+      if (c == 0 || (float)c * w.x + (float)c * w.y < A.blo) continue;
+      cmin = min(cmin, c);
+      cmax = max(cmax, c);
+      const unsigned long long k = ((unsigned long long)((unsigned)sz[p] ^ 0x80000000u) << 32) | (unsigned)e;
+      if (k < bk) {
+        bk = k;
+        bp = p;
+      }
+    }
+#pragma unroll
+    for (int off = 1; off < 8; off <<= 1) {
+      cmin = min(cmin, __shfl_xor_sync(kAll, cmin, off));
+      cmax = max(cmax, __shfl_xor_sync(kAll, cmax, off));
+      const unsigned long long k = __shfl_xor_sync(kAll, bk, off);
+      const int p = __shfl_xor_sync(kAll, bp, off);
+      if (k < bk) {
+        bk = k;
+        bp = p;
+      }
+    }
+    tied = tied && cmin == cmax;
+    if (tied) nd = (cmax << 13) | bp;
+  }
+  const bool slow = todo && nc >= 0 && !one && !none && !tied;
   for (unsigned sm = __ballot_sync(kAll, slow && (lane & 7) == 0); sm; sm &= sm - 1) {
     const int src = __ffs(sm) - 1;
-    const int r = walk_pick_any(I, rC, sz, __shfl_sync(kAll, nc, src),
-                                B.cand + (size_t)(ol + i0 + 4 * wib + (src >> 3)) * K);
-    if ((lane >> 3) == (src >> 3)) nd = r;
+    int rs;
+    const int r = walk_pick_any(I, rC, R.Cf, sz, __shfl_sync(kAll, nc, src),
+                                B.cand + (size_t)(ol + i0 + 4 * wib + (src >> 3)) * K, &rs);
+    if ((lane >> 3) == (src >> 3)) {
+      nd = r;
+      sl = rs;
+    }
   }
   if (todo && nc >= 0 && tv) {
     int dn = nd & 0x1fff;
-    const int s0 = sz[dn];
-    sl = min(sl, s0 > I.max_pw ? s0 - I.max_pw - 1 : I.max_pw - s0);
-    if (s0 > I.max_pw) dn = of;
-    const int s1 = sz[dn];
-    sl = min(sl, s1 < I.min_pw ? I.min_pw - s1 - 1 : s1 - I.min_pw);
-    if (s1 < I.min_pw) dn = of;
+    sl = tv_clamp(I, sz, of, &dn, sl);
     nd = (nd & ~0x1fff) | dn;
   }
   if (todo && (lane & 7) == 0) {
@@ -880,13 +897,16 @@ __device__ __forceinline__ void walk_eval(const DevInstance& I, const SpecBuf& B
 
 // The walk (block 0, every thread).  The positions [zs, end_w) are visited in
 // order with the exact sizes each would see: the window-start sizes plus the
-// moves before it (the window's movers before zs are in mlist).  A position is
-// decided again if the sizes may have drifted beyond its slack; the others
-// keep their decision.  A changed decision goes to dfix with the predicted
-// outcome: exact for TV (its accept test is a count of nets) and for vertices
-// without nets, else the old decision's, or a move (MSV) / no move (MSRV) if
-// that one stayed home.  The walk ends (ctl[0]) at a stale-marker risk or at a
-// changed vertex of a CTA or of the grid; ctl[1] counts the changes.
+// moves before it (the window's movers before zs are in mlist).  The
+// validation has checked every decision against the window's movers as they
+// are, so a position is decided again only if the decisions changed before it
+// may have drifted the sizes beyond what it tolerates on top of those; the
+// others keep their decision.  A changed decision goes to dfix with the
+// predicted outcome: exact for TV (its accept test is a count of nets) and for
+// vertices without nets, else the old decision's, or a move (MSV) / no move
+// (MSRV) if that one stayed home.  The walk ends (ctl[0]) at a stale-marker
+// risk or at a changed vertex of a CTA or of the grid; ctl[1] counts the
+// changes.
 //
 // It is bound by the latency of dependent instructions (about 5 cycles each in
 // a lone warp), so it speculates once more, inside the CTA: groups of 32
@@ -899,12 +919,15 @@ __device__ __forceinline__ void walk_eval(const DevInstance& I, const SpecBuf& B
 // least-loaded part, which its own kind moves with every step: those the
 // first warp decides one by one.
 __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const RoundCtx& R, int metric, int pos, int zs,
-                            int end_w, int nm, WalkSmem& S, int* sz, float2* pen) {
+                            int end_w, int nm, WalkSmem& S, int* sz, float2* pen, int* dl) {
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int K = I.K;
   const bool tv = metric == kTV;
   const float rC = __fdiv_rn(1.0f, R.Cf);
-  for (int p = threadIdx.x; p < K; p += blockDim.x) sz[p] = R.sizes[p];
+  for (int p = threadIdx.x; p < K; p += blockDim.x) {
+    sz[p] = R.sizes[p];
+    dl[p] = 0;   // what the changed decisions changed
+  }
   __syncthreads();
   for (int i = threadIdx.x; i < nm; i += blockDim.x) {
     const int4 m = lds(&B.mlist[i]);
@@ -913,8 +936,8 @@ __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const RoundC
     atomicAdd(&sz[m.z >> 16], -m.y);
   }
   __syncthreads();
-  for (int p = threadIdx.x; p < K; p += blockDim.x) pen[p] = walk_pen(sz[p], rC);
-  if (threadIdx.x == 0) S.drift = 0xffffffffu;   // not known: the first group takes it
+  for (int p = threadIdx.x; p < K; p += blockDim.x) pen[p] = pen_of(sz[p], rC);
+  if (threadIdx.x == 0) S.drift = 0;
   int hard = kNone, nchg = 0;   // warp 0
   bool stop = false;
   for (int zl = zs; zl < end_w && !stop; zl += kWalkLoad) {
@@ -923,30 +946,22 @@ __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const RoundC
       const int o = ol + i;
       const int nc = lds(&B.ncand[o]);
       S.meta[i] = make_int4(lds(&B.dec[o]), lds(&B.wt[o]), lds(&B.acc[o]), (nc << 8) | (int)lds(&B.flag[o]));
-      S.margin[i] = max(lds(&B.slack[o]), 0);
+      S.margin[i] = lds(&B.rel[o]);
     }
     __syncthreads();
     const int ng = (n + 31) >> 5;
     for (int g = wib; g < ng; g += kSWarps) {
       const int i = g * 32 + lane;
       const bool in = i < n;
-      const int4 m = in ? S.meta[i] : make_int4(0, 0, 0, 0);
-      const unsigned x = (m.w & 1) ? (unsigned)m.y : 0u;
-      unsigned incl = x;
-      if (__any_sync(kAll, x != 0))
-        for (int off = 1; off < 32; off <<= 1) {
-          const unsigned t = __shfl_up_sync(kAll, incl, off);
-          if (lane >= off) incl += t;
-        }
-      const bool always = (m.w & 32) || ((m.w & 2) && zl + i != pos);
-      const unsigned slk = in ? (unsigned)S.margin[i] : 0x7fffffffu;
-      const int mg = always || slk < incl - x ? -1 : (int)(slk - (incl - x));
-      if (in) S.margin[i] = mg;
-      const int gm = warp_min(mg);
-      if (lane == 31) {
-        S.gmin[g] = gm;
-        S.gsum[g] = incl;
+      int mg = 0x7fffffff;
+      if (in) {
+        const int fl = S.meta[i].w;
+        const int sl = S.margin[i];
+        mg = (fl & 32) || ((fl & 2) && zl + i != pos) || sl < -1 ? -1 : max(sl, 0);
+        S.margin[i] = mg;
       }
+      mg = warp_min(mg);
+      if (lane == 0) S.gmin[g] = mg;
     }
     __syncthreads();
     for (int sc = 0; sc < n && !stop; sc += kWalkSub) {
@@ -954,26 +969,37 @@ __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const RoundC
       const int g1 = (sc + ns + 31) >> 5;
       unsigned pot = 0;   // groups a drift may reach
       {
-        unsigned d = S.drift;
-        for (int g = sc >> 5; g < g1; g++) {
-          // (past the first such group, changed decisions may add to the drift)
-          if (pot || S.gmin[g] < 0 || d > (unsigned)S.gmin[g]) pot |= 1u << (g - (sc >> 5));
-          d += S.gsum[g];
-        }
+        // (past the first such group, changed decisions may add to the drift)
+        for (int g = sc >> 5; g < g1; g++)
+          if (pot || S.drift > S.gmin[g]) pot |= 1u << (g - (sc >> 5));
       }
       if (pot) {
-        const int row = min(K, kWalkRow);
-        for (int i = threadIdx.x; i < ns * kWalkRow; i += blockDim.x)
-          if ((i & (kWalkRow - 1)) < row && ((pot >> (i / (kWalkRow * 32))) & 1u))
-            S.ent[(i / kWalkRow) * kWalkStride + (i & (kWalkRow - 1))] =
-                lds(&B.cand[(size_t)(ol + sc + i / kWalkRow) * K + (i & (kWalkRow - 1))]);
+        // a warp per row, four rows' loads in flight (a load after each store
+        // measured 16 K cycles per 128 rows, this 3 K)
+        for (int r0 = wib; r0 < ns; r0 += 4 * kSWarps) {
+          unsigned long long e[4][2];
+          int nc[4];
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            const int r = r0 + u * kSWarps;
+            nc[u] = r < ns && ((pot >> (r >> 5)) & 1u) ? S.meta[sc + r].w >> 8 : 0;
+            const unsigned long long* cl = B.cand + (size_t)(ol + sc + min(r, ns - 1)) * K;
+#pragma unroll
+            for (int x = 0; x < 2; x++) e[u][x] = lane + 32 * x < nc[u] ? lds(&cl[lane + 32 * x]) : 0;
+          }
+#pragma unroll
+          for (int u = 0; u < 4; u++)
+#pragma unroll
+            for (int x = 0; x < 2; x++)
+              if (lane + 32 * x < nc[u]) S.ent[(r0 + u * kSWarps) * kWalkStride + lane + 32 * x] = e[u][x];
+        }
       }
       __syncthreads();   // also: every thread has read S.drift
       // warp 0: the group at hand, its lanes' positions and their present outcome
       int g = sc >> 5, j = 0, own = 0, d = 0, w = 0, mg = 0;
       int4 m = make_int4(0, 0, 0, 0);
       bool mv = false, in = false, fresh = true;
-      unsigned drift = S.drift, D = 0, extra = 0;
+      int drift = S.drift;
       // the moves own -> to of the lanes of mm applied
       auto apply = [&](unsigned mm, int to) {
         if (!mm) return;
@@ -984,8 +1010,8 @@ __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const RoundC
         }
         __syncwarp();
         if (me) {
-          pen[to] = walk_pen(sz[to], rC);
-          pen[own] = walk_pen(sz[own], rC);
+          pen[to] = pen_of(sz[to], rC);
+          pen[own] = pen_of(sz[own], rC);
         }
         __syncwarp();
       };
@@ -1005,25 +1031,21 @@ __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const RoundC
               w = m.y;
               mv = (m.w & 1) != 0;
               j = 0;
-              extra = 0;
-              const bool reach = S.gmin[g] < 0 || drift > (unsigned)S.gmin[g];
-              if (reach) {   // the exact drift here
+              if (drift > S.gmin[g]) {   // the exact drift here
                 int D0 = 0;
-                for (int p = lane; p < K; p += 32) D0 = max(D0, abs(sz[p] - R.sizes[p]));
-                drift = (unsigned)warp_max(D0);
+                for (int p = lane; p < K; p += 32) D0 = max(D0, abs(dl[p]));
+                drift = warp_max(D0);
               }
-              mg = in && reach ? S.margin[i0 + lane] : 0x7fffffff;
-              D = drift;
+              mg = in ? S.margin[i0 + lane] : 0x7fffffff;
               fresh = false;
             }
-            need = __ballot_sync(kAll, in && lane >= j && (mg < 0 || D > (unsigned)mg));
+            need = __ballot_sync(kAll, in && lane >= j && drift > mg);
             if (need) {
               task = g;
               break;
             }
             // the rest of the group keeps its outcome
             apply(__ballot_sync(kAll, mv && lane >= j), d);
-            drift += S.gsum[g] + extra;   // what the group's movers moved bounds the drift from here on
             fresh = true;
           }
           if (lane == 0) {
@@ -1054,30 +1076,29 @@ __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const RoundC
           }
           const bool chg = dn != d;
           // drift from these sizes before each position, and what the changed
-          // decisions before it add to its group's drift
+          // decisions before it add to the drift of the others
           const int x = mvn && lane >= j ? w : 0;
-          const int chgw = mvn == mv || lane < j ? 0 : mvn ? w : -w;
-          unsigned Dn = (unsigned)x;
-          int cn = chgw;
+          const int cw = chg && lane >= j ? (mvn ? w : 0) + (mv ? w : 0) : 0;
+          unsigned Dn = (unsigned)x, cn = (unsigned)cw;
           if (__any_sync(kAll, x != 0))
             for (int off = 1; off < 32; off <<= 1) {
               const unsigned t = __shfl_up_sync(kAll, Dn, off);
               if (lane >= off) Dn += t;
             }
           Dn -= (unsigned)x;
-          if (__any_sync(kAll, chgw != 0))
+          if (__any_sync(kAll, cw != 0))
             for (int off = 1; off < 32; off <<= 1) {
-              const int t = __shfl_up_sync(kAll, cn, off);
+              const unsigned t = __shfl_up_sync(kAll, cn, off);
               if (lane >= off) cn += t;
             }
-          cn -= chgw;
-          const long long lim = again ? (long long)nsl - Dn : (long long)mg - (long long)D - cn;
-          int more = 0;   // weight the vertices without nets add to both
+          cn -= (unsigned)cw;
+          const long long lim = again ? (long long)nsl - Dn : (long long)mg - drift - cn;
+          long long moren = 0, morec = 0;   // what the vertices without nets add to both
           while (true) {
             // the first position in doubt: decided again here and reached by the
             // moves since, or not decided again and reached now
             const unsigned db = __ballot_sync(
-                kAll, in && lane >= j && ((again && (hardf || iso)) || (long long)more > lim));
+                kAll, in && lane >= j && ((again && (hardf || iso)) || (again ? moren : morec) > lim));
             const int f = db ? __ffs(db) - 1 : nl;
             // ---- positions [j, f) stand; a changed vertex of a CTA or of the
             // grid ends the window
@@ -1090,12 +1111,12 @@ __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const RoundC
               if (keep && chg) {
                 B.dfix[ol + i0 + lane] = dn | (mvn ? 1 << 16 : 0);
                 B.flag[ol + i0 + lane] = (unsigned char)((m.w & 255) | 128);
+                if (mvn) { atomicAdd(&dl[dn], w); atomicAdd(&dl[own], -w); }
+                if (mv) { atomicAdd(&dl[d], -w); atomicAdd(&dl[own], w); }
               }
               nchg += __popc(cm);
-              const unsigned dx = (unsigned)warp_sum(keep ? chgw : 0);
-              extra += dx;
-              D += dx;
             }
+            if (keep && !chg && (m.w & 128)) B.flag[ol + i0 + lane] = (unsigned char)(m.w & 127);
             apply(__ballot_sync(kAll, keep && mvn), dn);
             if (hm) {
               hard = ((zl + i0 + fe) << 3) | 2;
@@ -1124,17 +1145,23 @@ __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const RoundC
                   B.flag[ol + i0 + j] = (unsigned char)((mt.w & 255) | 128);
                 }
                 nchg++;
-                const int dd = (m2 ? wf : 0) - ((mt.w & 1) ? wf : 0);
-                extra += (unsigned)dd;
-                D += (unsigned)dd;
-                more += dd;
+                const int wo = (mt.w & 1) ? wf : 0, wn = m2 ? wf : 0;
+                moren += wn - wo;   // (its old weight is in the others' Dn)
+                morec += wn + wo;
+                if (lane == 0) {
+                  dl[q] += wn;
+                  dl[df] -= wo;
+                  dl[of] += wo - wn;
+                }
+              } else if ((mt.w & 128) && lane == 0) {
+                B.flag[ol + i0 + j] = (unsigned char)(mt.w & 127);
               }
               if (m2) {
                 if (lane < 2) {
                   const int p = lane == 0 ? q : of;
                   const int s = sz[p] + (lane == 0 ? wf : -wf);
                   sz[p] = s;
-                  pen[p] = walk_pen(s, rC);
+                  pen[p] = pen_of(s, rC);
                 }
                 __syncwarp();
               }
@@ -1147,8 +1174,11 @@ __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const RoundC
             mv = mvn;
             d = dn;
           }
+          __syncwarp();
+          int D0 = 0;   // the drift from here on
+          for (int p = lane; p < K; p += 32) D0 = max(D0, abs(dl[p]));
+          drift = warp_max(D0);
           if (hard == kNone && j >= nl) {
-            drift += S.gsum[g] + extra;
             fresh = true;
             g++;
           }
@@ -1161,6 +1191,7 @@ __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const RoundC
   if (threadIdx.x == 0) {
     B.ctl[0] = hard;
     B.ctl[1] = nchg;
+    B.ctl[8] = kNone;   // the first mispredicted outcome (fix_position)
   }
 }
 
@@ -1168,12 +1199,12 @@ __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const RoundC
 // move records, the accept test and the claims are redone for the new
 // decision.  The replaced move's claims stay (a superset keeps every later
 // check conservative); their table slots go to rec_slot2 for the commit, so a
-// second replaced move ends the window here instead.  An outcome other than
-// the walk predicted lowers *mis: the positions after it are walked again.
+// second replaced move ends the window here instead (ctl[9]).  An outcome
+// other than the walk predicted lowers ctl[8]: the decisions after it are
+// validated again.
 // One warp, the one owning position z.
 __device__ void fix_position(const DevInstance& I, const SpecBuf& B, const RoundCtx& R, int metric, int z, int o,
-                             int fl, int par, int* mis, int* cut, int* loc, int* gains, int* losses, int* adelta,
-                             bool logp) {
+                             int fl, int par, int* loc, int* gains, int* losses, int* adelta, bool logp) {
   const int lane = threadIdx.x & 31;
   const bool vol = metric != kTV, rv = metric == kMSRV;
   const int K = I.K;
@@ -1186,7 +1217,7 @@ __device__ void fix_position(const DevInstance& I, const SpecBuf& B, const Round
   const bool had = (fl & 1) != 0;
   if (had && (fl & 64)) {
     if (lane == 0) {
-      atomicMin(cut, (z << 3) | 2);
+      atomicMin(&B.ctl[9], (z << 3) | 2);
       B.flag[o] = (unsigned char)(fl & ~128);
     }
     return;
@@ -1236,7 +1267,7 @@ __device__ void fix_position(const DevInstance& I, const SpecBuf& B, const Round
   }
   if (lane == 0) {
     if (logp) { B.rgain[o] = rg; B.rloss[o] = rl; }
-    if (mover != (fx >> 16 != 0)) atomicMin(mis, z);
+    if (mover != (fx >> 16 != 0)) atomicMin(&B.ctl[8], z);
     const int wv = mover ? __ldg(&I.w[v]) : 0;
     if (had) B.mlist[lds(&B.midx[o])] = make_int4(o, wv, (own << 16) | d, mover ? vdd : 0);   // the replaced mover's entry
     else if (mover) list_mover(B, par, o, wv, (own << 16) | d, vdd);
@@ -1247,6 +1278,11 @@ __device__ void fix_position(const DevInstance& I, const SpecBuf& B, const Round
   }
   __syncwarp();
 }
+
+// Changed decisions are taken at once, not walked, in a stretch longer than
+// this with at most so many of them: a walk costs about 2 us per 10 positions
+// it decides again, a validation of the whole window 12-25 us.
+constexpr int kJacobiSpan = 1024, kJacobiFlips = 64;
 
 static_assert(kMaxGridVerts <= kSWarps, "one warp decides each whole-grid vertex of a window");
 
@@ -1299,12 +1335,13 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
   // its exact sizes over the round's penalties (both rebuilt every round)
   WalkSmem& walk_s = *reinterpret_cast<WalkSmem*>(cnt_b);
   float2* walk_pn = reinterpret_cast<float2*>(cnt_b + sizeof(WalkSmem) / sizeof(int));
+  int* walk_dl = reinterpret_cast<int*>(walk_pn + K);
   const float rC = __fdiv_rn(1.0f, Cf);
   int* walk_sz = reinterpret_cast<int*>(penf_s);
 
   int round = 0;
   int heavy_round = 0;
-  int wr = 0;   // walks (parity selects the misprediction word)
+  int vr = 0;   // validations (parity selects the words of changed decisions)
   unsigned long long tA = gtimer();
   for (int it = 0; it < passes; it++) {
     const bool logp = I.recs != nullptr && it == passes - 1;   // decision records of the last pass
@@ -1319,7 +1356,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
       for (int p = threadIdx.x; p < K; p += blockDim.x) {
         const int sz = lds(&I.part_sizes[p]);
         sizes_s[p] = sz;
-        penf_s[p] = 1.0f - __fdiv_rn((float)sz, Cf);
+        penf_s[p] = pen_of(sz, rC).x;
         if (metric == kTV) {
           // a part scanned in the last window takes its last scanner as marker
           // (block 0 stores it; the others read only parts not scanned there)
@@ -1492,7 +1529,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         int slack;
         // candidates (part, count, first sighting) for an exact re-check of the
         // decision if the part sizes drift beyond its slack; TV's scanned parts
-        const int d = ldg_decide(I, R, cnt, first, sb, metric, v, own, z == pos, gains, B.cand + (size_t)o * K,
+        const int d = ldg_decide(I, R, cnt, first, sb, metric, v, own, z == pos, B.cand + (size_t)o * K,
                                  &B.ncand[o], metric == kTV ? B.scan + (size_t)o * words : nullptr, &special, &slack);
         const long long cD = clock64();
         // The accept outcome of a vertex without nets does not depend on the
@@ -1568,8 +1605,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         atomicAdd(&B.stats[26], (unsigned long long)nV);
       }
       // medium vertices of the window: one CTA each, dealt out from the end of
-      // the grid (their positions cluster; the CTAs that own them took up to 15
-      // each on the 1M-vertex Zipf workload while the others waited)
+      // the grid (a CTA with several among its own positions held the window up)
       __syncthreads();
       const long long cM = clock64();
       const int mend = midx + lower_bound_pos(B.mid_pos + midx, min(B.nmid - midx, span), end_w);
@@ -1607,7 +1643,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
           // block 0 keeps the candidates for an exact re-check, TV's scanned parts
           const int os = zs - pos;
           const bool b0 = blockIdx.x == 0;
-          const int d = ldg_decide(I, R, cj, fj, sb, metric, vsup, own_s, zs == pos, gains_b + (size_t)j * K,
+          const int d = ldg_decide(I, R, cj, fj, sb, metric, vsup, own_s, zs == pos,
                                    b0 ? B.cand + (size_t)os * K : nullptr, b0 ? &B.ncand[os] : nullptr,
                                    b0 && metric == kTV ? B.scan + (size_t)os * words : nullptr, &special, &slack);
           if (lane == 0) { s_gdec[j] = d; s_gspec[j] = special ? 1 : 0; s_gslk[j] = slack; }
@@ -1710,9 +1746,10 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
       // volumes and, with sizes, the part sizes (the decision taken again where
       // they drifted beyond its slack).  The first position that an earlier
       // one invalidates lowers *cut_w, the first whose decision the exact sizes
-      // change *flip_w.
+      // change *flip_w (dfix holds its new decision, flag bit 7); with sizes, rel
+      // receives the drift it tolerates beyond the window's movers as they are
+      // (-2: its decision changes).
       int* const cut_w = &B.ctl[4 + par];
-      int* const flip_w = &B.ctl[6 + par];
       const int cta_o0 = min(pos + blockIdx.x * kSWarps * q, end_w) - pos;
       int* dsz_cta = gains_b;   // (the evaluation's arrays are free here)
       // the size changes (in dsz) and volume drift (returned) of the window's
@@ -1740,7 +1777,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         __syncthreads();
         return x;
       };
-      auto validate = [&](int zfrom, int zto, bool sizes) {
+      auto validate = [&](int zfrom, int zto, bool sizes, int* flip_w, int* nflip_w) {
         const int mtpos = lds(&B.ctl[2 + par]);
         const bool ov = lds(&B.ctab_over[par]) != 0;
         if (sizes || vol) {
@@ -1769,7 +1806,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
               const uint32_t base = __ldg(&I.vptr[v]);
               const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
               const int own = pk >> 16;
-              if (sizes && Dw > max(slk, 0)) {
+              if (sizes && (Dw > max(slk, 0) || (fl & 32))) {
                 // the exact sizes here: this CTA's movers before z on top of dsz_cta
                 for (int p = lane; p < K; p += 32) cnt[p] = sizes_s[p] + dsz_cta[p];
                 __syncwarp();
@@ -1780,9 +1817,23 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
                     atomicAdd(&cnt[pk2 >> 16], -w2);
                   }
                 __syncwarp();
-                if (recheck(I, rC, cnt, lds(&B.ncand[o]), B.cand + (size_t)o * K, metric == kTV, own) != (pk & 0xffff) &&
-                    lane == 0)
-                  atomicMin(flip_w, (z << 3) | 2);
+                int ns1;
+                const int d2 = recheck(I, rC, Cf, cnt, lds(&B.ncand[o]), B.cand + (size_t)o * K, metric == kTV, own, &ns1);
+                const bool flip = d2 != (pk & 0xffff);
+                if (lane == 0) {
+                  if (flip) {
+                    atomicMin(flip_w, (z << 3) | 2);
+                    atomicAdd(nflip_w, 1);
+                    B.dfix[o] = d2;
+                    B.flag[o] = (unsigned char)(fl | 128);
+                  } else if (fl & 128) {
+                    B.flag[o] = (unsigned char)(fl & 127);
+                  }
+                  B.rel[o] = flip ? -2 : ns1;
+                }
+              } else if (sizes && lane == 0) {
+                B.rel[o] = max(slk, 0) - (int)Dw;
+                if (fl & 128) B.flag[o] = (unsigned char)(fl & 127);
               }
               // the max-volume parts enter only the accept test of a vertex whose
               // decision leaves its part (MSRV/partition.cpp:308-400,
@@ -1842,13 +1893,23 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
               if (sizes && wib == 0) {
                 int D0 = 0;
                 for (int p = lane; p < K; p += 32) D0 = max(D0, abs(cnt_b[p]));
-                if (warp_max(D0) > max(lds(&B.slack[o]), 0)) {
+                D0 = warp_max(D0);
+                const int slk = max(lds(&B.slack[o]), 0);
+                if (D0 > slk) {
                   for (int p = lane; p < K; p += 32) cnt_b[p] += sizes_s[p];
                   __syncwarp();
-                  const int nc = lds(&B.ncand[o]);
-                  if ((nc < 0 || recheck(I, rC, cnt_b, nc, B.cand + (size_t)o * K, metric == kTV, own) != (pk & 0xffff)) &&
-                      lane == 0)
-                    atomicMin(flip_w, (z << 3) | 2);
+                  int ns1;
+                  const bool flip = recheck(I, rC, Cf, cnt_b, lds(&B.ncand[o]), B.cand + (size_t)o * K, metric == kTV,
+                                            own, &ns1) != (pk & 0xffff);
+                  if (lane == 0) {
+                    if (flip) {
+                      atomicMin(flip_w, (z << 3) | 2);
+                      atomicAdd(nflip_w, kJacobiFlips + 1);   // the walk's: it ends the window there
+                    }
+                    B.rel[o] = flip ? -2 : ns1;
+                  }
+                } else if (lane == 0) {
+                  B.rel[o] = slk - D0;
                 }
               }
               __syncthreads();
@@ -1872,56 +1933,61 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
           if (z >= zfrom) check_big(z, gtid, gthreads, (int)blockIdx.x == j % (int)gridDim.x, true);
         }
       };
-      validate(pos, end_w, true);
-      if (!grid_barrier(B.bar, I.status)) return;
-      int cutw = lds(cut_w);
-      const int flipw = lds(flip_w);
-      int hard = kNone;
-      if ((flipw >> 3) < (cutw >> 3)) {
-        // ---- decisions change: walk from the first one to the cut with the exact
-        // sizes (block 0); the positions whose decision changed are redone by
-        // their warps, and the window is walked again behind an outcome that
-        // was mispredicted; then the rest of the window is validated again
-        const int zf = flipw >> 3, zc = min(end_w, cutw >> 3);
-        for (int zs = zf, nw = 1;; nw++) {
+      // ---- B: validate; while decisions change, take the changes and validate
+      // again from the first one.  Long stretches with few changes take them all
+      // at once, each as the exact sizes before it then were (the validation
+      // finds what that leaves wrong); otherwise one CTA walks them in order.
+      // Measured on the 1M-vertex Zipf workload under TV (windows of 1,500
+      // positions, five changes each): 315 us of walk per window, 75 us so.
+      int cutw, hard = kNone, fcut = kNone;
+      bool sizes = true;
+      for (int zf = pos, nfix = 0;; nfix++) {
+        int* const flip_w = &B.ctl[6 + (vr & 1)];
+        int* const nflip_w = &B.ctl[10 + (vr & 1)];
+        validate(zf, hard == kNone ? end_w : min(hard >> 3, end_w), sizes, flip_w, nflip_w);
+        if (!grid_barrier(B.bar, I.status)) return;
+        cutw = min(lds(cut_w), fcut);   // (no fix writes cut_w: CTAs ahead may be in theirs already)
+        if (hard != kNone && (hard >> 3) < end_w) cutw = min(cutw, hard);
+        const int flipw = lds(flip_w), nflip = lds(nflip_w);
+        if (blockIdx.x == 0 && threadIdx.x == 0) {   // the next validation's words
+          B.ctl[6 + ((vr & 1) ^ 1)] = kNone;
+          B.ctl[10 + ((vr & 1) ^ 1)] = 0;
+        }
+        vr++;
+        if (!sizes || (flipw >> 3) >= (cutw >> 3)) break;
+        zf = flipw >> 3;
+        const int zc = min(end_w, cutw >> 3);
+        if (nfix == B.maxfix) {
+          cutw = flipw;
+          break;
+        }
+        const bool at_once = zc - zf > kJacobiSpan && nflip <= kJacobiFlips;
+        if (!at_once) {
           const unsigned long long tW = gtimer();
-          if (blockIdx.x == 0) walk_window(I, B, R, metric, pos, zs, zc, lds(&B.mcnt[par]), walk_s, walk_sz, walk_pn);
+          if (blockIdx.x == 0)
+            walk_window(I, B, R, metric, pos, zf, zc, lds(&B.mcnt[par]), walk_s, walk_sz, walk_pn, walk_dl);
           if (!grid_barrier(B.bar, I.status)) return;
           hard = lds(&B.ctl[0]);
-          const int nchg = lds(&B.ctl[1]);
-          const unsigned long long tF = gtimer();
           if (blockIdx.x == 0 && threadIdx.x == 0) {
-            B.stats[44] += nchg;
-            B.stats[45] += tF - tW;
+            B.stats[44] += lds(&B.ctl[1]);
+            B.stats[45] += gtimer() - tW;
           }
-          if (nchg == 0) break;
-          int* const mis = &B.ctl[8 + (wr & 1)];
-          for (int z = max(z0, zs); z < z1; z++) {
-            const int fl = lds(&B.flag[z - pos]);
-            if (fl & 128)
-              fix_position(I, B, R, metric, z, z - pos, fl, par, mis, cut_w, loc, gains, losses, adelta, logp);
-          }
-          if (!grid_barrier(B.bar, I.status)) return;
-          const int zm = lds(mis);
-          if (blockIdx.x == 0 && threadIdx.x == 0) {
-            B.ctl[8 + ((wr & 1) ^ 1)] = kNone;   // the next walk's word
-            B.stats[46] += gtimer() - tF;
-          }
-          wr++;
-          if (zm == kNone) break;
-          // the outcome at zm is exact now; what follows it is walked again
-          zs = zm + 1;
-          if (nw == B.maxfix) {
-            hard = min(hard, (zs << 3) | 2);
-            break;
-          }
-          if (zs >= zc) break;
+        } else {
+          hard = kNone;
+          if (blockIdx.x == 0 && threadIdx.x == 0) B.stats[44] += nflip;
         }
-        const int lim = hard == kNone ? zc : min(hard >> 3, zc);
-        validate(zf, lim, false);
+        // the changed positions redone by their warps
+        for (int z = max(z0, zf); z < min(z1, hard == kNone ? zc : min(zc, hard >> 3)); z++) {
+          const int fl = lds(&B.flag[z - pos]);
+          if (fl & 128)
+            fix_position(I, B, R, metric, z, z - pos, fl, par, loc, gains, losses, adelta, logp);
+        }
         if (!grid_barrier(B.bar, I.status)) return;
-        cutw = lds(cut_w);
-        if (hard != kNone && (hard >> 3) < end_w) cutw = min(cutw, hard);
+        // a walk whose outcomes came as predicted leaves exact sizes; else the
+        // validation takes the decisions again
+        fcut = min(fcut, lds(&B.ctl[9]));
+        sizes = at_once || lds(&B.ctl[8]) != kNone;
+        if (sizes) hard = kNone;
       }
       // ---- C: commit every mover before the cut.
       const int cut = cutw == kNone ? end_w : min(cutw >> 3, end_w);
@@ -2138,7 +2204,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
       if (gw == 0 && lane == 0) {
         B.ctl[2 + (par ^ 1)] = kNone;
         B.ctl[4 + (par ^ 1)] = kNone;
-        B.ctl[6 + (par ^ 1)] = kNone;
+        B.ctl[9] = kNone;   // (read behind a fix's barrier, written by fixes alone)
         B.mcnt[par ^ 1] = 0;
         B.ctab_over[par ^ 1] = 0;
       }
@@ -2146,7 +2212,11 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
       if (cut == end_w) {
         if (end_w == pos + W) W = min(2 * W, B.wmax);
       } else {
-        // regrow from the last valid length
+        // regrow from the last valid length, by at most a factor of four down:
+        // every position past the cut is evaluated again, and walked (windows of
+        // at least one position per warp instead: 16K-vertex Zipf with unit
+        // weights under TV 47 -> 101 ms per pass, 256K degree weights MSV 243 ->
+        // 260, MSRV 47.2 -> 46.4)
         W = min(B.wmax, max(B.wmin > 0 ? B.wmin : 128, max(W / 4, B.wgrow * (cut - pos))));
       }
       pos = cut;
@@ -2174,7 +2244,7 @@ size_t spec_ldg_smem_bytes(int K) {
   auto a = [](size_t n) { return (n + 15) & ~size_t(15); };
   const size_t k4 = a(sizeof(int) * K);
   const size_t eval = 4 * a(sizeof(int) * (size_t)K * kSWarps) + a(sizeof(unsigned long long) * (size_t)K * kSWarps);
-  return 5 * k4 + std::max(eval, sizeof(WalkSmem) + sizeof(float2) * K);
+  return 5 * k4 + std::max(eval, sizeof(WalkSmem) + (sizeof(float2) + sizeof(int)) * K);
 }
 
 cudaError_t launch_spec_ldg(const DevInstance& I, const SpecBuf& B, int passes, int num_sms, cudaStream_t st,

@@ -52,3 +52,23 @@ def test_gpu_walk_matches_oracle(fp, orc, gpu_engine, metric, name, K, window):
         d = inst.decisions()
         for k in ("dest", "gain", "loss", "moved"):
             np.testing.assert_array_equal(d[k], o[f"rec_{k}"], err_msg=k)
+
+
+@pytest.mark.parametrize("metric", ["TV", "MSV"])
+def test_gpu_changes_taken_at_once_match_oracle(fp, orc, gpu_engine, metric):
+    """Windows of thousands of positions with few changed decisions: all of
+    them are redone at once and the window is validated again."""
+    hg = fp.generate(fp.GenSpec.zipf(100_003, 60_000, 2.1, 2, 10_000, beta=1.5, weight_rule=1, seed=7))
+    K = 256 if metric == "TV" else 64
+    o = orc.run_oracle(hg, K, metric, 2)
+    assert o["status"] == 0
+    with gpu_engine.instance(hg, K, metric) as inst:
+        inst.set_window(8192, 4)
+        inst.initial_partition()
+        inst.refine(2)
+        ln, pt, ct = inst.lists()
+        np.testing.assert_array_equal(inst.partition(), o["part_vec"])
+        np.testing.assert_array_equal(inst.moves(2), o["moves"])
+        np.testing.assert_array_equal(orc.flat_lists(hg, ln, pt), orc.flat_lists(hg, o["ep_len"], o["ep_part"]))
+        np.testing.assert_array_equal(ct, o["ep_cnt"])
+        assert inst.metrics() == o["metrics_final"]
