@@ -25,6 +25,7 @@ namespace {
 
 using namespace spec;
 
+constexpr int kMaxMsgWords = 4096 / 32;   // of the largest K
 constexpr int kStageK = 256;   // zero masks staged in shared memory up to this K
 
 // conn[a][b] += delta with the message count, the zero masks and the conn == 1
@@ -441,6 +442,8 @@ __device__ void msg_commit_grid(const DevInstance& I, int v, int own, int d, int
   }
 }
 
+constexpr int kMsgMinWindow = 512;
+
 // Three CTAs per SM (the compiler's own choice otherwise varies with the code
 // and can spill).
 __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, SpecBuf B, int passes) {
@@ -449,7 +452,8 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
   __shared__ unsigned long long uscr[kSWarps];
   __shared__ int iscr[kSWarps];
   __shared__ unsigned oc1m[kSWarps];
-  __shared__ int s_mx, s_nmax, s_stop;
+  __shared__ int s_mx, s_nmax, s_stop, s_ns;
+  __shared__ uint32_t okm_s[kMaxMsgWords];   // parts a vertex may leave this round (MSM)
   __shared__ int s_gz[kMaxGridVerts], s_go[kMaxGridVerts], s_gd[kMaxGridVerts];
   __shared__ uint32_t s_gb[kMaxGridVerts];
   const bool msm = I.metric == 3;
@@ -481,6 +485,8 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
   int heavy_round = 0;
   int round = 0;
   bool dirty = true;   // staged masks out of date (a move was committed)
+  // every vertex of part p may be evaluated (bit p of okm_s)
+  auto may_leave = [&](int p) { return ((okm_s[p >> 5] >> (p & 31)) & 1u) != 0u; };
   for (int it = 0; it < passes; it++) {
     // decision records of the last pass: a vertex evaluated before the window's
     // first mover saw the final state; one after it is evaluated again later
@@ -489,7 +495,7 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
     // window length: one position per warp to start, doubled after a window
     // without a mover, twice the distance to the mover after one
     int W = min(nwarps, B.wmax_msg);
-    int hidx = 0;
+    int hidx = 0, midx = 0;
     while (pos < I.nov) {
       // ------------------------------------------------------------ round state
       for (int p = threadIdx.x; p < K; p += blockDim.x) {
@@ -502,6 +508,7 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
           zc_s[x] = lds(&I.zcol[x]);
         }
       }
+      bool dirty_ok = dirty;
       dirty = false;
       __syncthreads();
       if (msm) {
@@ -523,8 +530,29 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
         }
         __syncthreads();
       }
+      if (dirty_ok || logp) {
+        // MSM: a vertex moves only if every max-message part gains, and a part m
+        // other than its own p gains only by conn[m][p] == 1 (msg_decide_warp):
+        // the parts where that holds for all of them.  On the 1M-vertex Zipf
+        // workload it leaves a few per cent of the vertices to evaluate.
+        // (Decision records need every vertex's gain.)
+        for (int x = wib; x < words; x += kSWarps) {
+          const int p = x * 32 + lane;
+          bool ok = p < K;
+          if (msm && !logp && ok)
+            for (int q = 0; q < s_nmax && ok; q++) {
+              const int m = maxl_s[q];
+              ok = m == p || ((lds(&I.c1col[(size_t)p * words + (m >> 5)]) >> (m & 31)) & 1u);
+            }
+          const unsigned b = __ballot_sync(kAll, ok);
+          if (lane == 0) okm_s[x] = b;
+        }
+        __syncthreads();
+        dirty_ok = false;
+      }
       const MsgRound Rd{sizes_s, msgs_s, maxl_s, msm ? s_nmax : 0, msm ? s_mx : 0};
       while (hidx < B.nheavy && __ldg(&B.heavy_pos[hidx]) < pos) hidx++;
+      midx += lower_bound_pos(B.mid_pos + midx, min(B.nmid - midx, B.wmax_msg), pos);
 
       // ================================================================= round
       // A window holds up to gmax whole-grid vertices and ends before the next
@@ -539,15 +567,23 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
       auto hslot = [&](int j) { return ((size_t)hp * kMaxGridVerts + j) * K; };
       auto hmslot = [&](int j) { return (hp * kMaxGridVerts + j) * 8; };
       const unsigned long long tR = gtimer();
-      if ((int)threadIdx.x < ns) {
-        const int v = __ldg(&B.heavy_pos[hidx + threadIdx.x]);
-        const uint32_t b = __ldg(&I.vptr[v]);
-        s_gz[threadIdx.x] = v;
-        s_go[threadIdx.x] = lds(&I.part_vec[v]);
-        s_gb[threadIdx.x] = b;
-        s_gd[threadIdx.x] = (int)(__ldg(&I.vptr[v + 1]) - b);
+      if (wib == 0) {   // those that may move
+        const int v = lane < ns ? __ldg(&B.heavy_pos[hidx + lane]) : 0;
+        const int own = lane < ns ? lds(&I.part_vec[v]) : 0;
+        const bool ok = lane < ns && may_leave(own);
+        const unsigned m = __ballot_sync(kAll, ok);
+        if (ok) {
+          const int j = __popc(m & ((1u << lane) - 1u));
+          const uint32_t b = __ldg(&I.vptr[v]);
+          s_gz[j] = v;
+          s_go[j] = own;
+          s_gb[j] = b;
+          s_gd[j] = (int)(__ldg(&I.vptr[v + 1]) - b);
+        }
+        if (lane == 0) s_ns = __popc(m);
       }
       __syncthreads();
+      ns = s_ns;
       // ---- tally slices of the whole-grid vertices, combined per CTA
       for (int j = 0; j < ns; j++) {
         const int v = s_gz[j], own = s_go[j], deg = s_gd[j];
@@ -582,38 +618,58 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
       const int q = (span + nwarps - 1) / nwarps;
       const int z0 = min(pos + gw * q, end_w);
       const int z1 = min(z0 + q, end_w);
-      for (int v = z0; v < z1; v++) {
-        if (__ldg(&B.vclass[v]) != 0) continue;   // medium vertex: evaluated by the whole CTA below
-        if (lds(&B.ctl[par]) < v) break;           // an earlier mover ends the window
-        const int own = lds(&I.part_vec[v]);
-        const uint32_t base = __ldg(&I.vptr[v]);
-        const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
-        msg_begin(I, Wk, own, msm);
-        int g = 0;
-        for (int nb = 0; nb < deg; nb += 32) g += msg_batch(I, v, own, base, nb, deg, Wk, &oc1m[wib]);
-        g = warp_sum(g);
-        int2 rec;
-        const int best = msg_decide_warp(I, M, Rd, Wk, own, g, msm, logp ? &rec : nullptr);
-        if (logp && lane == 0) I.recs[v] = make_int4(best, rec.x, rec.y, best >= 0);
-        if (best >= 0) {
-          if (lane == 0) {
-            B.dec[v - pos] = (own << 16) | best;
-            atomicMin(&B.ctl[par], v);
+      // light vertices, 32 at a time: those that can move are picked by the lanes
+      // (most have no nets or, for MSM, a part that cannot be left), then
+      // evaluated one by one
+      bool over = false;
+      for (int zb = z0; zb < z1 && !over; zb += 32) {
+        const int vl = zb + lane;
+        int own_l = 0, deg_l = 0;
+        uint32_t base_l = 0;
+        bool todo = vl < z1 && __ldg(&B.vclass[vl]) == 0;
+        if (todo) {
+          base_l = __ldg(&I.vptr[vl]);
+          deg_l = (int)(__ldg(&I.vptr[vl + 1]) - base_l);
+          own_l = lds(&I.part_vec[vl]);
+          if (logp && deg_l == 0) I.recs[vl] = make_int4(-1, 0, msm ? -1 : 0, 0);
+          todo = deg_l > 0 && may_leave(own_l);
+        }
+        for (unsigned tm = __ballot_sync(kAll, todo); tm; tm &= tm - 1) {
+          const int src = __ffs(tm) - 1, v = zb + src;
+          if (lds(&B.ctl[par]) < v) {   // an earlier mover ends the window
+            over = true;
+            break;
           }
-          break;
+          const int own = __shfl_sync(kAll, own_l, src);
+          const uint32_t base = __shfl_sync(kAll, base_l, src);
+          const int deg = __shfl_sync(kAll, deg_l, src);
+          msg_begin(I, Wk, own, msm);
+          int g = 0;
+          for (int nb = 0; nb < deg; nb += 32) g += msg_batch(I, v, own, base, nb, deg, Wk, &oc1m[wib]);
+          g = warp_sum(g);
+          int2 rec;
+          const int best = msg_decide_warp(I, M, Rd, Wk, own, g, msm, logp ? &rec : nullptr);
+          if (logp && lane == 0) I.recs[v] = make_int4(best, rec.x, rec.y, best >= 0);
+          if (best >= 0) {
+            if (lane == 0) {
+              B.dec[v - pos] = (own << 16) | best;
+              atomicMin(&B.ctl[par], v);
+            }
+            over = true;
+            break;
+          }
         }
       }
-      // medium vertices of this CTA's positions
-      const int cz0 = min(pos + blockIdx.x * kSWarps * q, end_w);
-      const int cz1 = min(cz0 + kSWarps * q, end_w);
-      for (int mi = lower_bound_pos(B.mid_pos, B.nmid, cz0); mi < B.nmid; mi++) {
+      // medium vertices of the window: one CTA each, dealt out from the end of the grid
+      const int mend = midx + lower_bound_pos(B.mid_pos + midx, min(B.nmid - midx, span), end_w);
+      for (int mi = midx + (int)(gridDim.x - 1 - blockIdx.x); mi < mend; mi += gridDim.x) {
         const int v = __ldg(&B.mid_pos[mi]);
-        if (v >= cz1) break;
         __syncthreads();
         if (threadIdx.x == 0) s_stop = lds(&B.ctl[par]) < v;
         __syncthreads();
         if (s_stop) break;
         const int own = lds(&I.part_vec[v]);
+        if (!may_leave(own)) continue;
         const uint32_t base = __ldg(&I.vptr[v]);
         const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
         msg_begin(I, Wk, own, msm);
@@ -718,7 +774,7 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
         B.stats[9] += end - pos;
         B.stats[f == kNone ? 3 : 8]++;
       }
-      W = f == kNone ? min(2 * W, B.wmax_msg) : max(min(nwarps, B.wmax_msg), min(B.wmax_msg, 2 * (end - pos)));
+      W = f == kNone ? min(2 * W, B.wmax_msg) : max(min(B.wmin > 0 ? B.wmin : kMsgMinWindow, B.wmax_msg), min(B.wmax_msg, 2 * (end - pos)));
       pos = end;
       round++;
       if (!grid_barrier(B.bar, I.status)) return;
