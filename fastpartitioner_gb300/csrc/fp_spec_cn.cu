@@ -6,16 +6,22 @@
 // A round covers a window of nets; every warp decides its nets against the
 // current state.  Claims are stamped with the round number, so they never need
 // to be cleared.  A net that will move pins ("acting") claims every net of
-// those pins (its write set); a later net is invalid if anything it read --
-// its own part list, the uncut net that kept it from acting, or the nets of
-// its smaller side -- was claimed by an earlier acting net.  The first invalid
-// net cuts the window; acting nets before the cut are applied concurrently
-// (their write sets are disjoint).
+// those pins (its write set).  An acting net takes at most one part off a
+// net (all its pins move old -> new), so behind n earlier acting nets a net of
+// more than 2 + n parts still has more than two, and one of at least 2 + n is
+// still cut.  A later net is therefore invalid only if an earlier acting net
+// claimed its own list and it has at most 2 + n parts, or claimed a net of its
+// smaller side that has fewer than 2 + n, or the uncut net that kept it from
+// acting.  The first invalid net cuts the window.
 //
 // An acting net moves its pins one at a time in the reference, each move
 // updating every net of the pin.  All of them move old -> new, so the k moves
 // that land on one net have a result that depends on k only (cn_apply_net);
-// the commit counts the moves per net, then updates each touched net once.
+// the commit counts the moves per net, then one warp updates each touched net:
+// the moves of the first acting net that claimed it, then those of the others,
+// in order.  Large nets are shared by most pairs of acting nets; with write
+// sets kept disjoint instead, a window of the 256K-net Zipf workload held 1.5
+// of them.
 
 #include "fp_spec_common.cuh"
 
@@ -24,6 +30,8 @@ namespace fp {
 namespace {
 
 using namespace spec;
+
+constexpr int kShared = 1 << 30;   // cn_kcnt: several acting nets move pins of the net
 
 // Round-stamped claim: the latest round wins, then the smallest position.
 __device__ __forceinline__ unsigned long long ckey(int round, int pos) {
@@ -41,13 +49,14 @@ __device__ __forceinline__ bool claim_before(const SpecBuf& B, int round, int x,
 //   kMode 0: returns a net of those pins that is not cut (-1: none);
 //   kMode 1: claims every such net for position e and records the pins to move
 //            (window offset o, round parity par); returns -1;
-//   kMode 2: returns 1 if an acting net before e claimed one of them, else -1.
+//   kMode 2: returns 1 if an acting net before e claimed one of them that has
+//            fewer than 2 + nb parts (nb acting nets before e), else -1.
 // Modes 0 and 2 stop early when *stop (shared by the warps splitting a net's
 // pins) is set.
 // gstop: the same in global memory (the grid's warps splitting a net).
 template <int kMode>
 __device__ int cn_walk_range(const DevInstance& I, const SpecBuf& B, int e, int pb, int pe, int oldp, int round,
-                             int o, int par, const volatile int* stop, const int* gstop = nullptr) {
+                             int o, int par, int nb, const volatile int* stop, const int* gstop = nullptr) {
   const int lane = threadIdx.x & 31;
   for (int b0 = pb; b0 < pe; b0 += 32) {
     if (kMode != 1 && stop && __shfl_sync(kAll, *stop, 0)) return -1;   // warp-uniform: lane 0's read
@@ -128,7 +137,7 @@ __device__ int cn_walk_range(const DevInstance& I, const SpecBuf& B, int e, int 
         bool c = false;
 #pragma unroll
         for (int q = 0; q < kU; q++)
-          if (xs[q] >= 0 && claim_before(B, round, xs[q], e)) c = true;
+          if (xs[q] >= 0 && claim_before(B, round, xs[q], e) && lds(&I.ep_len[xs[q]]) < 2 + nb) c = true;
         if (__any_sync(kAll, c)) return 1;
       }
     }
@@ -138,9 +147,26 @@ __device__ int cn_walk_range(const DevInstance& I, const SpecBuf& B, int e, int 
 
 template <int kMode>
 __device__ __forceinline__ int cn_walk(const DevInstance& I, const SpecBuf& B, int e, int oldp, int round, int o,
-                                       int par) {
-  return cn_walk_range<kMode>(I, B, e, (int)__ldg(&I.nptr[e]), (int)__ldg(&I.nptr[e + 1]), oldp, round, o, par,
+                                       int par, int nb = 0) {
+  return cn_walk_range<kMode>(I, B, e, (int)__ldg(&I.nptr[e]), (int)__ldg(&I.nptr[e + 1]), oldp, round, o, par, nb,
                               nullptr);
+}
+
+// Acting nets of the round before net e (one warp; midx holds their ids).
+__device__ __forceinline__ int cn_acting_before(const SpecBuf& B, int nact, int e) {
+  int n = 0;
+  for (int i = threadIdx.x & 31; i < nact; i += 32) n += lds(&B.midx[i]) < e;
+  return warp_sum(n);
+}
+__device__ __forceinline__ void cn_list_acting(const SpecBuf& B, int par, int e) {
+  B.midx[atomicAdd(&B.mcnt[par], 1)] = e;
+}
+
+// Did an acting net before e (nb of them) change what e's own list decides?
+__device__ __forceinline__ bool cn_own_conflict(const DevInstance& I, const SpecBuf& B, int round, int e, int unc,
+                                                int nb) {
+  return (claim_before(B, round, e, e) && lds(&I.ep_len[e]) <= 2 + nb) ||
+         (unc >= 0 && claim_before(B, round, unc, e));
 }
 
 // Warp gw's contiguous share (of nw warps) of net e's pins.
@@ -198,16 +224,17 @@ __device__ void cn_eval_cta(const DevInstance& I, const SpecBuf& B, int e, int o
   if (sh_two) {
     int pb, pe;
     cn_pin_share(I, e, &pb, &pe);
-    const int hit = cn_walk_range<0>(I, B, e, pb, pe, oldp, 0, 0, 0, &sh_stop);
+    const int hit = cn_walk_range<0>(I, B, e, pb, pe, oldp, 0, 0, 0, 0, &sh_stop);
     if (hit >= 0 && lane == 0) {
       atomicCAS(&sh_unc, -1, hit);   // any uncut net is a witness
       sh_stop = 1;
     }
     __syncthreads();
     act = sh_unc < 0;
-    if (act) cn_walk_range<1>(I, B, e, pb, pe, oldp, round, o, par, nullptr);
+    if (act) cn_walk_range<1>(I, B, e, pb, pe, oldp, round, o, par, 0, nullptr);
   }
   if (threadIdx.x == 0) {
+    if (act) cn_list_acting(B, par, e);
     B.dec[o] = (oldp << 16) | newp;
     B.flag[o] = (unsigned char)act;
     B.slack[o] = sh_unc;   // the uncut net that blocks the move (-1: none)
@@ -218,21 +245,17 @@ __device__ void cn_eval_cta(const DevInstance& I, const SpecBuf& B, int e, int o
 
 // Validation of a net with many pins by the whole CTA (the warp loop's rules);
 // a conflict lowers the cut word.
-__device__ void cn_validate_cta(const DevInstance& I, const SpecBuf& B, int e, int o, int round, int* cut) {
+__device__ void cn_validate_cta(const DevInstance& I, const SpecBuf& B, int e, int o, int round, int nact, int* cut) {
   __shared__ volatile int sh_conf;
   const int lane = threadIdx.x & 31;
   const int act = lds(&B.flag[o]);
-  if (threadIdx.x == 0) {
-    int c = claim_before(B, round, e, e) ? 1 : 0;
-    const int unc = lds(&B.slack[o]);
-    if (unc >= 0 && claim_before(B, round, unc, e)) c = 1;
-    sh_conf = c;
-  }
+  const int nb = cn_acting_before(B, nact, e);
+  if (threadIdx.x == 0) sh_conf = cn_own_conflict(I, B, round, e, lds(&B.slack[o]), nb) ? 1 : 0;
   __syncthreads();
   if (act && !sh_conf) {
     int pb, pe;
     cn_pin_share(I, e, &pb, &pe);
-    if (cn_walk_range<2>(I, B, e, pb, pe, lds(&B.dec[o]) >> 16, round, 0, 0, &sh_conf) > 0 && lane == 0) sh_conf = 1;
+    if (cn_walk_range<2>(I, B, e, pb, pe, lds(&B.dec[o]) >> 16, round, 0, 0, nb, &sh_conf) > 0 && lane == 0) sh_conf = 1;
   }
   __syncthreads();
   if (threadIdx.x == 0 && sh_conf) atomicMin(cut, (e << 3) | 5);
@@ -382,7 +405,7 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_cn_kernel(DevInstance I, Sp
         if (!s_gt[j]) continue;
         int pb, pe;
         cn_grid_share(I, s_ge[j], gw, nwarps, &pb, &pe);
-        const int hit = cn_walk_range<0>(I, B, s_ge[j], pb, pe, s_go[j], 0, 0, 0, nullptr, hm(j));
+        const int hit = cn_walk_range<0>(I, B, s_ge[j], pb, pe, s_go[j], 0, 0, 0, 0, nullptr, hm(j));
         if (hit >= 0 && lane == 0) atomicCAS(hm(j), 0, hit + 1);
       }
       const int span = end_w - pos;
@@ -397,6 +420,7 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_cn_kernel(DevInstance I, Sp
         const int act = cn_eval(I, B, e, &oldp, &newp, &unc, &oldc);
         if (act) cn_walk<1>(I, B, e, oldp, round, o, par);
         if (lane == 0) {
+          if (act) cn_list_acting(B, par, e);
           B.dec[o] = (oldp << 16) | newp;
           B.flag[o] = (unsigned char)act;
           B.slack[o] = unc;   // the uncut net that blocks the move (-1: none)
@@ -422,9 +446,10 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_cn_kernel(DevInstance I, Sp
           if (act) {
             int pb, pe;
             cn_grid_share(I, e, gw, nwarps, &pb, &pe);
-            cn_walk_range<1>(I, B, e, pb, pe, s_go[j], round, o, par, nullptr);
+            cn_walk_range<1>(I, B, e, pb, pe, s_go[j], round, o, par, 0, nullptr);
           }
           if (blockIdx.x == 0 && threadIdx.x == 0) {
+            if (act) cn_list_acting(B, par, e);
             B.dec[o] = s_gt[j] ? (s_go[j] << 16) | s_gn[j] : 0;
             B.flag[o] = (unsigned char)act;
             B.slack[o] = s_gt[j] ? unc : -1;
@@ -439,18 +464,17 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_cn_kernel(DevInstance I, Sp
         tA = tE;
       }
       // ---- B: validate against earlier acting nets' claims
+      const int nact = lds(&B.mcnt[par]);
       for (int e = z0; e < z1; e++) {
         const int o = e - pos;
         if ((int)(__ldg(&I.nptr[e + 1]) - __ldg(&I.nptr[e])) > B.cn_big) continue;   // validated by the CTA below
         const int act = lds(&B.flag[o]);
-        bool conf = false;
-        if (lane == 0) {
-          if (claim_before(B, round, e, e)) conf = true;
-          const int unc = lds(&B.slack[o]);
-          if (unc >= 0 && claim_before(B, round, unc, e)) conf = true;
-        }
+        if (nact == 0) break;
+        const int nb = cn_acting_before(B, nact, e);
+        if (nb == 0) continue;
+        bool conf = lane == 0 && cn_own_conflict(I, B, round, e, lds(&B.slack[o]), nb);
         conf = __any_sync(kAll, conf);   // warp-uniform before the pin loop's votes
-        if (act && !conf) conf = cn_walk<2>(I, B, e, lds(&B.dec[o]) >> 16, round, 0, 0) > 0;
+        if (act && !conf) conf = cn_walk<2>(I, B, e, lds(&B.dec[o]) >> 16, round, 0, 0, nb) > 0;
         conf = __any_sync(kAll, conf);
         if (conf) {
           if (lane == 0) atomicMin(&B.ctl[par], (e << 3) | 5);
@@ -461,18 +485,19 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_cn_kernel(DevInstance I, Sp
       for (int mi = lower_bound_pos(B.mid_pos, B.nmid, cz0); mi < B.nmid; mi++) {
         const int e = __ldg(&B.mid_pos[mi]);
         if (e >= cz1) break;
-        cn_validate_cta(I, B, e, e - pos, round, &B.ctl[par]);
+        cn_validate_cta(I, B, e, e - pos, round, nact, &B.ctl[par]);
       }
       for (int j = 0; j < ns; j++) {
         // a grid net: its own list and witness by every warp (cheap), its
         // moving pins' nets split across the grid
         const int e = s_ge[j], o = e - pos;
         const int unc = lds(&B.slack[o]);
-        bool conf = claim_before(B, round, e, e) || (unc >= 0 && claim_before(B, round, unc, e));
+        const int nb = cn_acting_before(B, nact, e);
+        bool conf = cn_own_conflict(I, B, round, e, unc, nb);
         if (!conf && lds(&B.flag[o])) {
           int pb, pe;
           cn_grid_share(I, e, gw, nwarps, &pb, &pe);
-          conf = cn_walk_range<2>(I, B, e, pb, pe, s_go[j], round, 0, 0, nullptr, hm(j) + 1) > 0;
+          conf = cn_walk_range<2>(I, B, e, pb, pe, s_go[j], round, 0, 0, nb, nullptr, hm(j) + 1) > 0;
           if (conf && lane == 0) atomicExch(hm(j) + 1, 1);
         }
         if (conf && lane == 0) atomicMin(&B.ctl[par], (e << 3) | 5);
@@ -511,7 +536,16 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_cn_kernel(DevInstance I, Sp
         const uint32_t ub = __ldg(&I.vptr[u]), ue = __ldg(&I.vptr[u + 1]);
         for (uint32_t j = ub + lane; j < ue; j += 32) {
           const int x = (int)__ldg(&I.vnets[j]);
-          if (atomicAdd(&B.cn_kcnt[x], 1) == 0) B.cn_nets[atomicAdd(&B.cn_cnt[2 + par], 1)] = make_int2(x, pk);
+          // the first acting net that claimed x counts its moves on it; those of
+          // the others are listed (kShared marks the net)
+          const int first = (int)(0xffffffffu - (unsigned)(lds(&B.claim64[x]) & 0xffffffffull));
+          if (first == pos + mv.y) {
+            if ((atomicAdd(&B.cn_kcnt[x], 1) & (kShared - 1)) == 0)
+              B.cn_nets[atomicAdd(&B.cn_cnt[2 + par], 1)] = make_int2(x, pk);
+          } else {
+            atomicOr(&B.cn_kcnt[x], kShared);
+            B.cn_more[atomicAdd(&B.cn_cnt[4 + par], 1)] = make_int2(x, mv.y);
+          }
         }
         if (lane == 0) {
           const int oldp = pk >> 16, newp = pk & 0xffff;
@@ -529,13 +563,33 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_cn_kernel(DevInstance I, Sp
       for (int i = gw; i < nnet; i += nwarps) {
         const int2 xe = lds(&B.cn_nets[i]);
         const int k = lds(&B.cn_kcnt[xe.x]);
-        cn_apply_net(I, xe.x, xe.y >> 16, xe.y & 0xffff, k);
+        cn_apply_net(I, xe.x, xe.y >> 16, xe.y & 0xffff, k & (kShared - 1));
+        if (k & kShared) {
+          // the other acting nets' moves on it, in their order
+          const int nmore = lds(&B.cn_cnt[4 + par]);
+          for (int last = -1;;) {
+            int o = kNone, c = 0;
+            for (int i2 = lane; i2 < nmore; i2 += 32) {
+              const int2 m2 = lds(&B.cn_more[i2]);
+              if (m2.x != xe.x || m2.y <= last || m2.y > o) continue;
+              c = m2.y == o ? c + 1 : 1;
+              o = m2.y;
+            }
+            const int o1 = warp_min(o);
+            if (o1 == kNone) break;
+            const int pk2 = lds(&B.dec[o1]);
+            cn_apply_net(I, xe.x, pk2 >> 16, pk2 & 0xffff, warp_sum(o == o1 ? c : 0));
+            last = o1;
+          }
+        }
         if (lane == 0) B.cn_kcnt[xe.x] = 0;
       }
       if (gw == 0 && lane == 0) {
         B.ctl[par ^ 1] = kNone;
         B.cn_cnt[par ^ 1] = 0;
         B.cn_cnt[2 + (par ^ 1)] = 0;
+        B.cn_cnt[4 + (par ^ 1)] = 0;
+        B.mcnt[par ^ 1] = 0;
       }
       if (ns) {
         // the other parity's grid-net words, for the next window with grid nets
