@@ -55,34 +55,43 @@ static bool spec_supported(int metric, int K, int max_smem, int nov, int noe) {
 // LDG metrics: vertex classes by work = sum over its nets of min(net size, K),
 // the list slots an evaluation reads at most.  Light: one warp; medium: one CTA;
 // above the super bound (or with 65536 nets or more, the limit of the candidate
-// encoding): all warps of the grid, all inside the window.  Windows that end
-// often (MSV moves nearly every vertex) favour a lower super bound, long ones
-// (TV, MSM) a higher one; bounds from a sweep on the 4M-vertex Zipf workload.
-// TM and MSM use the same classes in id order.
-constexpr int kLightWork = 2048;
+// encoding): a team of CTAs, all inside the window.  TM and MSM use the same
+// classes in id order.  A window holds at most default_grid_verts vertices of
+// the last class and ends before the next one; each one past the window's
+// eventual cut (first mover for TM / MSM) is evaluated again, so the bounds
+// follow from how early a metric's windows end.
+// Sweeps on Zipf workloads (K = 256, degree weights; milliseconds for the passes
+// swept, (super bound, vertices per window)):
+//   TV   1M vertices   (65536, 32) 14.9   (262144, 8) 17.4   (32768, 32) 21.0
+//   MSRV 256K          (16384, 16) 31.1   (32768, 4) 36.5    (65536, 16) 36.5
+//   MSV  256K          (32768, 4) 180     (16384, 2) 183     (262144, 2) 216
+//   TM   256K          (16384, 16) 56.1   (65536, 4) 66.8    (8192, 32) 57.2
+//                      and with light work up to 1024 52.6, 512 52.4
+//   MSM  1M            (262144, 16) 0.94  (65536, 32) 1.74
+constexpr int kLightWork = 2048, kLightWorkTm = 1024;
 constexpr int kCnLightPins = 128;   // CN: nets with more pins are evaluated by one CTA,
 constexpr int kCnGridPins = 1024;   //     with more than this by the whole grid
+int default_light_work(int metric) {
+  return metric == FP_METRIC_CN ? kCnLightPins : metric == FP_METRIC_TM ? kLightWorkTm : kLightWork;
+}
 int default_super_work(int metric) {
   switch (metric) {
-    case FP_METRIC_MSV: return 16384;
-    case FP_METRIC_MSRV: return 32768;
-    // measured on the 4M-vertex Zipf workload: passes 2-3 at 84 / 77 ms
-    // against 94 / 90 with 32768 (pass 1 152 against 140)
-    case FP_METRIC_TM: return 65536;
+    case FP_METRIC_CN: return kCnGridPins;
+    case FP_METRIC_TV: return 65536;
+    case FP_METRIC_MSV: return 32768;
+    case FP_METRIC_MSRV:
+    case FP_METRIC_TM: return 16384;
     default: return 262144;
   }
 }
-// Whole-grid vertices one window may hold.  Each one past the window's
-// eventual cut (first mover for TM / MSM) is evaluated again in a later window,
-// so metrics whose windows end early hold fewer.
 int default_grid_verts(int metric) {
   switch (metric) {
-    case FP_METRIC_TV:
-    case FP_METRIC_CN:
-    case FP_METRIC_MSM: return kMaxGridVerts;
+    case FP_METRIC_TV: return kMaxGridVerts;
+    case FP_METRIC_MSRV:
     case FP_METRIC_TM:
-    case FP_METRIC_MSRV: return 4;
-    default: return 2;
+    case FP_METRIC_MSM: return 16;
+    case FP_METRIC_CN: return kCnGridNets;
+    default: return 4;
   }
 }
 constexpr int kMaxSpecWarps = 16384;
@@ -789,8 +798,7 @@ int fp_instance_create(fp_ctx* ctx, const fp_hypergraph* h, int32_t K, int32_t m
       if (e != cudaSuccess) { fp_instance_destroy(in); return cuda_status(e); }
       if (ldg && (rc = build_positions(in))) { fp_instance_destroy(in); return rc; }
       if ((rc = build_stream_positions(in))) { fp_instance_destroy(in); return rc; }
-      rc = classify(in, metric == FP_METRIC_CN ? kCnLightPins : kLightWork,
-                    metric == FP_METRIC_CN ? kCnGridPins : default_super_work(metric));
+      rc = classify(in, default_light_work(metric), default_super_work(metric));
       if (rc) { fp_instance_destroy(in); return rc; }
     }
     if (in->in_arena) {   // the context's pinned words

@@ -88,7 +88,8 @@ constexpr int kMsgStreamCta = 1024;  // nets of a vertex one CTA places alone in
 constexpr int kNumStats = 48;
 
 // Whole-grid vertices one window may hold (slots of the whole-grid tallies).
-constexpr int kMaxGridVerts = 8;
+constexpr int kMaxGridVerts = 32;
+constexpr int kCnGridNets = 8;   // nets the whole grid evaluates in one CN window
 
 // Device buffers of the speculative engine (fp_spec.cu), allocated with the
 // instance.

@@ -34,8 +34,9 @@
 // (vertex, net); the gain / loss terms and the commit then take O(1) per net.
 // Vertices are classed by work (list slots over their nets, host-side): light
 // ones are evaluated by one warp, medium ones by one CTA, and the heaviest (up
-// to gmax per window) by all warps of the grid, which split the tally, the gain
-// / loss sums and the move in two extra grid phases of the window.
+// to gmax per window) by teams of CTAs sized by their nets, which split the
+// tally, the gain / loss sums and the move in two extra grid phases of the
+// window.
 
 #include "fp_spec_common.cuh"
 
@@ -323,16 +324,14 @@ __device__ __forceinline__ void net_terms(const DevInstance& I, bool rv, int v, 
   }
 }
 
-// Records of v's nets for the move own -> d; warp wi of a group of nw warps
-// takes a contiguous share of the nets (net_range).  With volumes (MSV / MSRV) the
-// gain / loss / volume terms are added to the warp's arrays.  loc: the warp's
-// 96 ints of scratch.  Returns this lane's counts of nets the move takes own
-// off (low 16 bits) and appends d to (high 16), TV's leave gain and arrival loss.
-__device__ int locate_all(const DevInstance& I, const SpecBuf& B, int metric, int v, int own, int d,
-                           uint32_t base, int deg, int wi, int nw, int* loc, int* gains, int* losses, int* adelta) {
+// Records of v's nets [n0, n1) for the move own -> d (one warp).  With volumes
+// (MSV / MSRV) the gain / loss / volume terms are added to the arrays.  loc: the
+// warp's 96 ints of scratch.  Returns this lane's counts of nets the move takes
+// own off (low 16 bits) and appends d to (high 16), TV's leave gain and arrival
+// loss (of a vertex one warp evaluates: fewer than 65536 nets).
+__device__ int locate_range(const DevInstance& I, const SpecBuf& B, int metric, int v, int own, int d, uint32_t base,
+                            int n0, int n1, int* loc, int* gains, int* losses, int* adelta) {
   const bool vol = metric != kTV, rv = metric == kMSRV;
-  int n0, n1;
-  net_range(deg, wi, nw, &n0, &n1);
   int ra = 0;
   for (int nb = n0; nb < n1; nb += 32) {
     int e;
@@ -341,6 +340,14 @@ __device__ int locate_all(const DevInstance& I, const SpecBuf& B, int metric, in
     if (vol && e >= 0) net_terms(I, rv, v, own, d, e, r, gains, losses, adelta);
   }
   return ra;
+}
+// The same for warp wi of nw warps splitting all of v's nets (net_range).
+__device__ __forceinline__ int locate_all(const DevInstance& I, const SpecBuf& B, int metric, int v, int own, int d,
+                                          uint32_t base, int deg, int wi, int nw, int* loc, int* gains, int* losses,
+                                          int* adelta) {
+  int n0, n1;
+  net_range(deg, wi, nw, &n0, &n1);
+  return locate_range(I, B, metric, v, own, d, base, n0, n1, loc, gains, losses, adelta);
 }
 
 // Count claims, exactly: an open-addressed table from (net, part) to the first
@@ -1284,8 +1291,6 @@ __device__ void fix_position(const DevInstance& I, const SpecBuf& B, const Round
 // it decides again, a validation of the whole window 12-25 us.
 constexpr int kJacobiSpan = 1024, kJacobiFlips = 64;
 
-static_assert(kMaxGridVerts <= kSWarps, "one warp decides each whole-grid vertex of a window");
-
 // Two CTAs per SM: without the hint the compiler trades registers for a third
 // CTA and spills, which measured slower.
 __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, SpecBuf B, int passes) {
@@ -1298,7 +1303,8 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
   // index, degree, decision, stale-marker risk, size slack
   __shared__ int s_gz[kMaxGridVerts], s_gv[kMaxGridVerts], s_go[kMaxGridVerts], s_gd[kMaxGridVerts];
   __shared__ uint32_t s_gb[kMaxGridVerts];
-  __shared__ int s_gdec[kMaxGridVerts], s_gspec[kMaxGridVerts], s_gslk[kMaxGridVerts];
+  __shared__ int s_gdec[kMaxGridVerts], s_gspec[kMaxGridVerts], s_gslk[kMaxGridVerts], s_gcnt[kMaxGridVerts];
+  __shared__ int s_t0[kMaxGridVerts], s_t1[kMaxGridVerts];   // their teams of CTAs
   __shared__ int loc_b[kSWarps * 96];   // per-warp locate scratch
   const int metric = I.metric;
   const bool vol = metric != kTV;
@@ -1464,45 +1470,46 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         s_gd[threadIdx.x] = (int)(__ldg(&I.vptr[v + 1]) - b);
       }
       __syncthreads();
-      // ---- A1: tally slices of the whole-grid vertices, pre-reduced per CTA
+      // ---- A1: tally slices of the whole-grid vertices by their teams of CTAs,
+      // one set of arrays per CTA
+      if (wib == 0 && ns) team_split(ns, s_gd, gridDim.x, s_t0, s_t1);
+      __syncthreads();
+      auto in_team = [&](int j) { return (int)blockIdx.x >= s_t0[j] && (int)blockIdx.x < s_t1[j]; };
+      auto leads = [&](int j) { return (int)blockIdx.x == s_t0[j]; };
+      // this CTA's share of vertex j's nets; its thread's first net and the step
+      auto team_nets = [&](int j, int* c0, int* c1) {
+        net_range(s_gd[j], (int)blockIdx.x - s_t0[j], s_t1[j] - s_t0[j], c0, c1);
+      };
+      auto team_tid = [&](int j) { return ((int)blockIdx.x - s_t0[j]) * (int)blockDim.x + (int)threadIdx.x; };
+      auto team_threads = [&](int j) { return (s_t1[j] - s_t0[j]) * (int)blockDim.x; };
       for (int j = 0; j < ns; j++) {
-        const int own_s = s_go[j], deg_s = s_gd[j];
+        if (!in_team(j)) continue;
+        const int own_s = s_go[j];
         const uint32_t base_s = s_gb[j];
         int* hcnt = B.hcnt + hslot(j);
         unsigned long long* hfirst = B.hfirst + hslot(j);
-        // a warp's share in pieces whose sighting keys fit 32 bits (all but always one)
-        const int share = (deg_s + nwarps - 1) / nwarps, piece = key_nets(sb);
-        for (int a0 = 0; a0 < share; a0 += piece) {
-          for (int p = lane; p < K; p += 32) { cnt[p] = 0; first[p] = ~0u; }
-          __syncwarp();
-          int c1 = 0;
-          {
-            int n0, n1;
-            net_range(deg_s, gw, nwarps, &n0, &n1);
-            const int b0 = n0 + min(a0, n1 - n0), b1 = b0 + min(piece, n1 - b0);
-            for (int nb = b0; nb < b1; nb += 32) c1 += tally_batch(I, own_s, base_s, nb, b1, b0, sb, cnt, first);
-          }
-          c1 = warp_sum(c1);
+        int c0, c1;
+        team_nets(j, &c0, &c1);
+        // in pieces whose sighting keys fit 32 bits (all but always one)
+        const int piece = key_nets(sb);
+        for (int a0 = c0, a1 = c0; a0 < c1; a0 = a1) {
+          a1 = a0 + min(piece, c1 - a0);
+          for (int p = threadIdx.x; p < K; p += blockDim.x) { cnt_b[p] = 0; first_b[p] = ~0u; }
+          __syncthreads();
+          int own1 = 0, n0, n1;
+          net_range(a1 - a0, wib, kSWarps, &n0, &n1);
+          for (int nb = a0 + n0; nb < a0 + n1; nb += 32)
+            own1 += tally_batch(I, own_s, base_s, nb, a0 + n1, a0, sb, cnt_b, first_b);
+          own1 = warp_sum(own1);
+          if (lane == 0 && own1) atomicAdd(&B.hmisc[hmslot(j)], own1);
           __syncthreads();
           for (int p = threadIdx.x; p < K; p += blockDim.x) {
-            int c = 0;
-            unsigned long long f = ~0ull;
-            for (int x = 0; x < kSWarps; x++) {
-              const int cx = cnt_b[(size_t)x * K + p];
-              if (cx && f == ~0ull) {   // the warps' shares ascend: the first that saw p saw it first
-                int n0, n1;
-                net_range(deg_s, blockIdx.x * kSWarps + x, nwarps, &n0, &n1);
-                f = wide_key(first_b[(size_t)x * K + p], sb, n0 + a0);
-              }
-              c += cx;
-            }
-            if (c) {
-              atomicAdd(&hcnt[p], c);
-              atomicMin(&hfirst[p], f);
+            if (cnt_b[p]) {
+              atomicAdd(&hcnt[p], cnt_b[p]);
+              atomicMin(&hfirst[p], wide_key(first_b[p], sb, a0));
             }
           }
-          if (lane == 0 && c1) atomicAdd(&B.hmisc[hmslot(j)], c1);
-          __syncthreads();   // the per-warp arrays serve the next vertex and the evaluations below
+          __syncthreads();   // the arrays serve the next piece and the evaluations below
         }
       }
       if (kTimingStats && ns && threadIdx.x == 0) atomicMax(&B.stats[38], gtimer() - tR);
@@ -1622,73 +1629,68 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
       if (ns) {
         if (!grid_barrier(B.bar, I.status)) return;
         const unsigned long long tG = gtimer();
-        // ---- A2: decisions of the whole-grid vertices, taken in every CTA from
-        // the global tallies (warp j decides vertex j; each is first of the
-        // window or not, like any position), then their locate / gain-loss slices
+        // ---- A2: decisions of the whole-grid vertices, taken in every CTA of their
+        // teams from the global tallies (each is first of the window or not, like
+        // any position), then their locate / gain-loss slices
         for (int j = 0; j < ns; j++) {
+          if (!in_team(j)) continue;
           const size_t hs = hslot(j);
-          for (int p = threadIdx.x; p < K; p += blockDim.x) {
-            cnt_b[(size_t)j * K + p] = lds(&B.hcnt[hs + p]);
-            first64_b[(size_t)j * K + p] = lds(&B.hfirst[hs + p]);
-          }
-        }
-        __syncthreads();
-        if (wib < ns) {
-          const int j = wib;
           const int zs = s_gz[j], vsup = s_gv[j], own_s = s_go[j];
-          const int* cj = cnt_b + (size_t)j * K;
-          const unsigned long long* fj = first64_b + (size_t)j * K;
-          bool special;
-          int slack;
-          // block 0 keeps the candidates for an exact re-check, TV's scanned parts
-          const int os = zs - pos;
-          const bool b0 = blockIdx.x == 0;
-          const int d = ldg_decide(I, R, cj, fj, sb, metric, vsup, own_s, zs == pos,
-                                   b0 ? B.cand + (size_t)os * K : nullptr, b0 ? &B.ncand[os] : nullptr,
-                                   b0 && metric == kTV ? B.scan + (size_t)os * words : nullptr, &special, &slack);
-          if (lane == 0) { s_gdec[j] = d; s_gspec[j] = special ? 1 : 0; s_gslk[j] = slack; }
-        }
-        __syncthreads();
-        for (int j = 0; j < ns; j++) {
-          const int d = s_gdec[j], own_s = s_go[j];
-          if (d == own_s) continue;   // records for every decision that moves (the validation reads own's slots)
-          const size_t hs = hslot(j);
-          if (vol) {
-            for (int p = lane; p < K; p += 32) { gains[p] = 0; losses[p] = 0; adelta[p] = 0; }
-            __syncwarp();
+          for (int p = threadIdx.x; p < K; p += blockDim.x) {
+            cnt_b[p] = lds(&B.hcnt[hs + p]);
+            first64_b[p] = lds(&B.hfirst[hs + p]);
+            if (vol) { gains_b[p] = 0; losses_b[p] = 0; adelta_b[p] = 0; }
           }
-          locate_all(I, B, metric, s_gv[j], own_s, d, s_gb[j], s_gd[j], gw, nwarps, loc, gains, losses, adelta);
-          if (vol) {
-            __syncthreads();
-            for (int p = threadIdx.x; p < K; p += blockDim.x) {
-              int g = 0, l = 0, a = 0;
-              for (int x = 0; x < kSWarps; x++) {
-                g += gains_b[(size_t)x * K + p];
-                l += losses_b[(size_t)x * K + p];
-                a += adelta_b[(size_t)x * K + p];
-              }
-              if (g) atomicAdd(&B.hgain[hs + p], g);
-              if (l) atomicAdd(&B.hloss[hs + p], l);
-              if (a) atomicAdd(&B.hadelta[hs + p], a);
+          __syncthreads();
+          if (wib == 0) {
+            bool special;
+            int slack;
+            // the first CTA keeps the candidates for an exact re-check, TV's scanned parts
+            const int os = zs - pos;
+            const bool b0 = leads(j);
+            const int d = ldg_decide(I, R, cnt_b, first64_b, sb, metric, vsup, own_s, zs == pos,
+                                     b0 ? B.cand + (size_t)os * K : nullptr, b0 ? &B.ncand[os] : nullptr,
+                                     b0 && metric == kTV ? B.scan + (size_t)os * words : nullptr, &special, &slack);
+            if (lane == 0) {
+              s_gdec[j] = d;
+              s_gspec[j] = special ? 1 : 0;
+              s_gslk[j] = slack;
+              s_gcnt[j] = cnt_b[d];
             }
-            __syncthreads();   // the per-warp arrays serve the next vertex
+          }
+          __syncthreads();
+          const int d = s_gdec[j];
+          if (d == own_s) continue;   // records for every decision that moves (the validation reads own's slots)
+          int c0, c1, n0, n1;
+          team_nets(j, &c0, &c1);
+          net_range(c1 - c0, wib, kSWarps, &n0, &n1);
+          locate_range(I, B, metric, vsup, own_s, d, s_gb[j], c0 + n0, c0 + n1, loc, gains_b, losses_b, adelta_b);
+          __syncthreads();
+          if (vol) {
+            for (int p = threadIdx.x; p < K; p += blockDim.x) {
+              if (gains_b[p]) atomicAdd(&B.hgain[hs + p], gains_b[p]);
+              if (losses_b[p]) atomicAdd(&B.hloss[hs + p], losses_b[p]);
+              if (adelta_b[p]) atomicAdd(&B.hadelta[hs + p], adelta_b[p]);
+            }
+            __syncthreads();   // the arrays serve the next vertex
           }
         }
         if (!grid_barrier(B.bar, I.status)) return;
-        // ---- A3: accept tests (MSV / MSRV) in every CTA, claims, the records
+        // ---- A3: accept tests (MSV / MSRV) in every CTA of the teams, claims, the records
         for (int j = 0; j < ns; j++) {
+          if (!in_team(j)) continue;
           const size_t hs = hslot(j);
           const int zs = s_gz[j], vsup = s_gv[j], own_s = s_go[j], deg_s = s_gd[j], d = s_gdec[j];
           const uint32_t base_s = s_gb[j];
           const int os = zs - pos;
           const bool need = d != own_s &&
-                            (metric == kTV ? lds(&B.hmisc[hmslot(j)]) >= deg_s - cnt_b[(size_t)j * K + d] : true);
+                            (metric == kTV ? lds(&B.hmisc[hmslot(j)]) >= deg_s - s_gcnt[j] : true);
           bool mover = metric == kTV && need, mt = false;
           int vs = kBig, vdd = 0;
           int rg = 0, rl = 0;   // decision record (with the log on)
           if (metric == kTV && d != own_s) {
             rg = lds(&B.hmisc[hmslot(j)]);
-            rl = deg_s - cnt_b[(size_t)j * K + d];
+            rl = deg_s - s_gcnt[j];
           }
           if (vol && need) {
             for (int p = threadIdx.x; p < K; p += blockDim.x) {
@@ -1715,8 +1717,8 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
               rl = block_reduce_sum(l, iscr);
             }
           }
-          if (mover) claim_nets(I, B, vol, zs, own_s, d, base_s, deg_s, gtid, gthreads, par);
-          if (blockIdx.x == 0 && threadIdx.x == 0) {
+          if (mover) claim_nets(I, B, vol, zs, own_s, d, base_s, deg_s, team_tid(j), team_threads(j), par);
+          if (leads(j) && threadIdx.x == 0) {
             if (logp) { B.rgain[os] = rg; B.rloss[os] = rl; }
             B.dec[os] = (own_s << 16) | d;
             B.flag[os] = (unsigned char)((mover ? 1 : 0) | (s_gspec[j] ? 2 : 0) | 4);
@@ -1930,7 +1932,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         for (int j = 0; j < ns; j++) {
           const int z = s_gz[j];
           if (z >= zto) break;
-          if (z >= zfrom) check_big(z, gtid, gthreads, (int)blockIdx.x == j % (int)gridDim.x, true);
+          if (z >= zfrom && in_team(j)) check_big(z, team_tid(j), team_threads(j), leads(j), true);
         }
       };
       // ---- B: validate; while decisions change, take the changes and validate
@@ -2067,7 +2069,9 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         unclaim_nets(I, B, vol, base, deg, threadIdx.x, blockDim.x);
       }
       for (int j = 0; j < ns; j++) {
-        // a whole-grid vertex, by every thread
+        // a whole-grid vertex, by its team
+        if (!in_team(j)) continue;
+        const int tt = team_tid(j), tn = team_threads(j);
         const int zs = s_gz[j], vsup = s_gv[j], own_s = s_go[j], deg_s = s_gd[j];
         const uint32_t base_s = s_gb[j];
         const int os = zs - pos;
@@ -2075,10 +2079,10 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
           const int pk = lds(&B.dec[os]);
           const int d = pk & 0xffff;
           if (zs < cut) {
-            for (int i = gtid; i < deg_s; i += gthreads)
+            for (int i = tt; i < deg_s; i += tn)
               commit_rec(I, vsup, own_s, d, (int)__ldg(&I.vnets[base_s + i]), lds(&B.rec[base_s + i]),
                          vol ? &V : nullptr);
-            if (gtid == 0) {
+            if (tt == 0) {
               atomicAdd(&B.stats[2], 1ull);
               I.part_vec[vsup] = d;
               const int wv = __ldg(&I.w[vsup]);
@@ -2087,7 +2091,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
               atomicAdd((unsigned long long*)&I.moves[it], 1ull);
             }
           }
-          unclaim_nets(I, B, vol, base_s, deg_s, gtid, gthreads);
+          unclaim_nets(I, B, vol, base_s, deg_s, tt, tn);
         }
       }
       if (B.niso && (metric != kMSRV || logp)) {

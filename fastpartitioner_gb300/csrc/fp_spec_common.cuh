@@ -152,6 +152,28 @@ __device__ __forceinline__ void net_range(int deg, int wi, int nw, int* b, int* 
   *e = min(*b + g, deg);
 }
 
+// Splits the grid's ncta CTAs among the window's ns whole-grid vertices (ns <=
+// 32) by their nets deg, at least a quarter of an even share each: vertex j's
+// team is the CTAs [t0[j], t1[j]) (one CTA of several teams when the grid is
+// small).  One warp.
+__device__ __forceinline__ void team_split(int ns, const int* deg, int ncta, int* t0, int* t1) {
+  const int lane = threadIdx.x & 31;
+  const long long d = lane < ns ? deg[lane] : 0;
+  const long long all = warp_sum64(d);
+  const long long w = lane < ns ? 3 * d + all / ns + 1 : 0;
+  long long incl = w;
+  for (int off = 1; off < 32; off <<= 1) {
+    const long long t = __shfl_up_sync(kAll, incl, off);
+    if (lane >= off) incl += t;
+  }
+  const long long total = __shfl_sync(kAll, incl, 31);
+  if (lane < ns) {
+    const int a = min((int)((incl - w) * ncta / total), ncta - 1);
+    t0[lane] = a;
+    t1[lane] = max((int)(incl * ncta / total), a + 1);
+  }
+}
+
 // Sighting keys: the reference breaks ties by the part seen first, in (net,
 // slot) order.  A key is the net's index from the start of the tallied range
 // above the slot, in 32 bits: shared-memory atomicMin has a native 32-bit form

@@ -13,9 +13,9 @@
 // vertex's own part, and conn == 0 (losses per candidate part,
 // TM/partition.cpp:408-450) staged in shared memory when K <= 256.  Vertices
 // are classed by work like the LDG engine: light ones are evaluated by one
-// warp, medium ones by one CTA, the heaviest (up to gmax per window) by all
-// warps of the grid, whose slices meet in global sets that one CTA per vertex
-// decides from after a grid barrier.
+// warp, medium ones by one CTA, the heaviest (up to gmax per window) by teams
+// of CTAs sized by their nets, whose slices meet in global sets that one CTA
+// per vertex decides from after a grid barrier.
 
 #include "fp_spec_common.cuh"
 
@@ -456,6 +456,7 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
   __shared__ uint32_t okm_s[kMaxMsgWords];   // parts a vertex may leave this round (MSM)
   __shared__ int s_gz[kMaxGridVerts], s_go[kMaxGridVerts], s_gd[kMaxGridVerts];
   __shared__ uint32_t s_gb[kMaxGridVerts];
+  __shared__ int s_t0[kMaxGridVerts], s_t1[kMaxGridVerts];   // their teams of CTAs
   const bool msm = I.metric == 3;
   const int K = I.K;
   const int words = (K + 31) >> 5;
@@ -485,6 +486,7 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
   int heavy_round = 0;
   int round = 0;
   bool dirty = true;   // staged masks out of date (a move was committed)
+  bool okm_set = false;
   // every vertex of part p may be evaluated (bit p of okm_s)
   auto may_leave = [&](int p) { return ((okm_s[p >> 5] >> (p & 31)) & 1u) != 0u; };
   for (int it = 0; it < passes; it++) {
@@ -508,7 +510,7 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
           zc_s[x] = lds(&I.zcol[x]);
         }
       }
-      bool dirty_ok = dirty;
+      const bool moved = dirty;
       dirty = false;
       __syncthreads();
       if (msm) {
@@ -530,7 +532,7 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
         }
         __syncthreads();
       }
-      if (dirty_ok || logp) {
+      if (!okm_set || logp || (msm && moved)) {
         // MSM: a vertex moves only if every max-message part gains, and a part m
         // other than its own p gains only by conn[m][p] == 1 (msg_decide_warp):
         // the parts where that holds for all of them.  On the 1M-vertex Zipf
@@ -548,7 +550,7 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
           if (lane == 0) okm_s[x] = b;
         }
         __syncthreads();
-        dirty_ok = false;
+        okm_set = true;
       }
       const MsgRound Rd{sizes_s, msgs_s, maxl_s, msm ? s_nmax : 0, msm ? s_mx : 0};
       while (hidx < B.nheavy && __ldg(&B.heavy_pos[hidx]) < pos) hidx++;
@@ -581,11 +583,15 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
           s_gd[j] = (int)(__ldg(&I.vptr[v + 1]) - b);
         }
         if (lane == 0) s_ns = __popc(m);
+        __syncwarp();
+        if (m) team_split(__popc(m), s_gd, gridDim.x, s_t0, s_t1);
       }
       __syncthreads();
+      const int nheld = ns;   // whole-grid vertices the window holds
       ns = s_ns;
-      // ---- tally slices of the whole-grid vertices, combined per CTA
+      // ---- tally slices of the whole-grid vertices by their teams, combined per CTA
       for (int j = 0; j < ns; j++) {
+        if ((int)blockIdx.x < s_t0[j] || (int)blockIdx.x >= s_t1[j]) continue;
         const int v = s_gz[j], own = s_go[j], deg = s_gd[j];
         const uint32_t base = s_gb[j];
         uint32_t* hR = reinterpret_cast<uint32_t*>(B.hloss + hslot(j));      // words <= K
@@ -595,7 +601,7 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
         int g = 0;
         {
           int n0, n1;
-          net_range(deg, gw, nwarps, &n0, &n1);
+          net_range(deg, ((int)blockIdx.x - s_t0[j]) * kSWarps + wib, (s_t1[j] - s_t0[j]) * kSWarps, &n0, &n1);
           for (int nb = n0; nb < n1; nb += 32) g += msg_batch(I, v, own, base, nb, n1, Wk, &oc1m[wib]);
         }
         g = warp_sum(g);
@@ -770,7 +776,7 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
       if (blockIdx.x == 0 && threadIdx.x == 0) {
         B.ctl[par ^ 1] = kNone;
         B.stats[0]++;
-        B.stats[1] += ns;
+        B.stats[1] += nheld;
         B.stats[9] += end - pos;
         B.stats[f == kNone ? 3 : 8]++;
       }
