@@ -658,21 +658,21 @@ __device__ void cta_eval_ldg(const DevInstance& I, const SpecBuf& B, const Round
 }
 
 // The window's positions as the walk stages them in shared memory: the words of
-// up to kWalkLoad positions, per 32 of them what a drift of the sizes has to
-// exceed to matter, and the first kWalkRow candidate entries of kWalkSub
-// positions (rows padded so that four rows read side by side meet no bank
+// up to kWalkLoad positions, per 32 of them (a group) what a drift of the sizes
+// has to exceed to matter, and the first kWalkRow candidate entries of the
+// group at hand (rows padded so that four rows read side by side meet no bank
 // conflict).
-constexpr int kWalkLoad = 1024, kWalkSub = 128, kWalkRow = 64, kWalkStride = kWalkRow + 8;
-static_assert(kWalkRow == 64, "two entries of a staged row per lane");
+constexpr int kWalkLoad = 1024, kWalkRow = 256, kWalkStride = kWalkRow + 8;
 struct WalkSmem {
-  unsigned long long ent[kWalkSub * kWalkStride];
+  unsigned long long ent[32 * kWalkStride];
   int4 meta[kWalkLoad];      // (own << 16) | decision, weight, acc, (ncand << 8) | flag
   int margin[kWalkLoad];     // drift the position tolerates (-1: always taken again)
   int gmin[kWalkLoad / 32];  // per group of 32: the smallest margin
   int nd[32], nslack[32];    // decisions taken again: (nets listing it << 13) | part (-1: no list), drift tolerated
   int drift;                 // largest change of one part's size so far by changed decisions (an upper bound)
-  int group;                 // group to decide again (-1: none left), and its positions
-  unsigned need;
+  int group;                 // group to decide again (-1: none left), its positions, and those
+  unsigned need, eval;       //   of them that have nets, in list
+  int list[32];
 };
 
 // Least-loaded part of sz, lowest index on ties (one warp); *ms its size.
@@ -791,33 +791,36 @@ __device__ __forceinline__ int recheck(const DevInstance& I, float rC, float Cf,
   return d;
 }
 
-// The marked positions of a group decided again with the sizes sz by the whole
-// CTA, eight lanes to a position: a lane keeps the best lower bound of its
-// candidates' scores and the largest upper bound of the others, three shuffles
-// meet them.  One candidate clear of the rest wins and tolerates the drift
-// that leaves it so; with none above zero the least-loaded part does.
-// Near-ties of several counts and long lists go to walk_pick_any, a warp each.
+// The marked positions of a group with nets decided again with the sizes sz by
+// the whole CTA, 8, 16 or 32 lanes to a position: a lane keeps the best lower
+// bound of its candidates' scores and the largest upper bound of the others,
+// shuffles meet them.  One candidate clear of the rest wins and tolerates the
+// drift that leaves it so; with none above zero the least-loaded part does.
+// Near-ties of several counts and lists beyond the staged rows go to
+// walk_pick_any, a warp each.
 __device__ __forceinline__ void walk_eval(const DevInstance& I, const SpecBuf& B, const RoundCtx& R, bool tv, float rC,
-                                          const int* sz, const float2* pen, WalkSmem& S, int i0, int sc, int ol) {
+                                          const int* sz, WalkSmem& S, int i0, int ol) {
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const unsigned need = S.need >> (4 * wib);
-  if (!(need & 15u)) return;
+  const int n = __popc(S.eval);
+  const int lg = n <= kSWarps ? 5 : n <= 2 * kSWarps ? 4 : 3;   // lanes to a position: 2^lg
+  const int lanes = 1 << lg, sub = lane & (lanes - 1);
+  if (wib * (32 >> lg) >= n) return;
   const int K = I.K;
-  const int q = lane >> 3, l = 4 * wib + q;
-  const bool marked = (need >> q) & 1u;
-  const int4 mt = marked ? S.meta[i0 + l] : make_int4(0, 0, 0, 8);
+  const int k = wib * (32 >> lg) + (lane >> lg);
+  const bool todo = k < n;
+  const int l = todo ? S.list[k] : 0;
+  const int4 mt = todo ? S.meta[i0 + l] : make_int4(0, 0, 0, 0);
   const int nc = mt.w >> 8, of = mt.x >> 16;
-  const bool todo = marked && !(mt.w & 8);
   const bool staged = todo && nc >= 0 && nc <= kWalkRow;
-  const unsigned long long* row = S.ent + (size_t)(i0 - sc + l) * kWalkStride;
+  const unsigned long long* row = S.ent + (size_t)l * kWalkStride;
   ScoreAcc A;
   const int ncl = staged ? nc : 0;
-  for (int x = lane & 7; x < ncl; x += 8) {
+  for (int x = sub; x < ncl; x += lanes) {
     const unsigned hi32 = (unsigned)(row[x] >> 32);
     const int p = (int)(hi32 >> 20), c = (int)((hi32 >> 4) & 0xffffu);
-    if (c > 0) A.add(p, c, pen[p]);
+    if (c > 0) A.add(p, c, pen_of(sz[p], rC));
   }
-  A.meet(8);
+  A.meet(lanes);
   const bool one = staged && A.one();
   const bool none = staged && A.none();
   int nd = nc < 0 ? -1 : 0, sl = -1;
@@ -833,12 +836,11 @@ __device__ __forceinline__ void walk_eval(const DevInstance& I, const SpecBuf& B
     s2 = warp_min(s2);
     int cd = 0;
     if (tv) {
-      for (int x = lane & 7; x < ncl; x += 8) {
+      for (int x = sub; x < ncl; x += lanes) {
         const unsigned hi32 = (unsigned)(row[x] >> 32);
         if ((int)(hi32 >> 20) == am) cd = (int)((hi32 >> 4) & 0xffffu);
       }
-#pragma unroll
-      for (int off = 1; off < 8; off <<= 1) cd = max(cd, __shfl_xor_sync(kAll, cd, off));
+      for (int off = 1; off < lanes; off <<= 1) cd = max(cd, __shfl_xor_sync(kAll, cd, off));
     }
     if (none) {
       nd = (cd << 13) | am;
@@ -852,28 +854,28 @@ __device__ __forceinline__ void walk_eval(const DevInstance& I, const SpecBuf& B
     int cmin = 0x7fffffff, cmax = 0;
     unsigned long long bk = ~0ull;
     int bp = 0;
-    for (int x = lane & 7; x < ncl; x += 8) {
+    for (int x = sub; x < ncl; x += lanes) {
       const unsigned long long e = row[x];
       const unsigned hi32 = (unsigned)(e >> 32);
       const int p = (int)(hi32 >> 20), c = (int)((hi32 >> 4) & 0xffffu);
-      const float2 w = pen[p];
+      const int s = sz[p];
+      const float2 w = pen_of(s, rC);
       if (c == 0 || (float)c * w.x + (float)c * w.y < A.blo) continue;
       cmin = min(cmin, c);
       cmax = max(cmax, c);
-      const unsigned long long k = ((unsigned long long)((unsigned)sz[p] ^ 0x80000000u) << 32) | (unsigned)e;
-      if (k < bk) {
-        bk = k;
+      const unsigned long long key = ((unsigned long long)((unsigned)s ^ 0x80000000u) << 32) | (unsigned)e;
+      if (key < bk) {
+        bk = key;
         bp = p;
       }
     }
-#pragma unroll
-    for (int off = 1; off < 8; off <<= 1) {
+    for (int off = 1; off < lanes; off <<= 1) {
       cmin = min(cmin, __shfl_xor_sync(kAll, cmin, off));
       cmax = max(cmax, __shfl_xor_sync(kAll, cmax, off));
-      const unsigned long long k = __shfl_xor_sync(kAll, bk, off);
+      const unsigned long long key = __shfl_xor_sync(kAll, bk, off);
       const int p = __shfl_xor_sync(kAll, bp, off);
-      if (k < bk) {
-        bk = k;
+      if (key < bk) {
+        bk = key;
         bp = p;
       }
     }
@@ -881,12 +883,12 @@ __device__ __forceinline__ void walk_eval(const DevInstance& I, const SpecBuf& B
     if (tied) nd = (cmax << 13) | bp;
   }
   const bool slow = todo && nc >= 0 && !one && !none && !tied;
-  for (unsigned sm = __ballot_sync(kAll, slow && (lane & 7) == 0); sm; sm &= sm - 1) {
+  for (unsigned sm = __ballot_sync(kAll, slow && sub == 0); sm; sm &= sm - 1) {
     const int src = __ffs(sm) - 1;
     int rs;
     const int r = walk_pick_any(I, rC, R.Cf, sz, __shfl_sync(kAll, nc, src),
-                                B.cand + (size_t)(ol + i0 + 4 * wib + (src >> 3)) * K, &rs);
-    if ((lane >> 3) == (src >> 3)) {
+                                B.cand + (size_t)(ol + i0 + __shfl_sync(kAll, l, src)) * K, &rs);
+    if ((lane >> lg) == (src >> lg)) {
       nd = r;
       sl = rs;
     }
@@ -896,10 +898,26 @@ __device__ __forceinline__ void walk_eval(const DevInstance& I, const SpecBuf& B
     sl = tv_clamp(I, sz, of, &dn, sl);
     nd = (nd & ~0x1fff) | dn;
   }
-  if (todo && (lane & 7) == 0) {
+  if (todo && sub == 0) {
     S.nd[l] = nd;
     S.nslack[l] = max(sl, 0);
   }
+}
+
+// Exclusive prefix over the lanes of x: by popcounts when the lanes with one
+// share it (unit weights), else a scan.
+__device__ __forceinline__ unsigned lane_prefix(unsigned x) {
+  const int lane = threadIdx.x & 31;
+  const unsigned m = __ballot_sync(kAll, x != 0u);
+  if (!m) return 0u;
+  const unsigned x0 = __shfl_sync(kAll, x, __ffs(m) - 1);
+  if (__all_sync(kAll, x == 0u || x == x0)) return x0 * (unsigned)__popc(m & ((1u << lane) - 1u));
+  unsigned incl = x;
+  for (int off = 1; off < 32; off <<= 1) {
+    const unsigned t = __shfl_up_sync(kAll, incl, off);
+    if (lane >= off) incl += t;
+  }
+  return incl - x;
 }
 
 // The walk (block 0, every thread).  The positions [zs, end_w) are visited in
@@ -926,7 +944,7 @@ __device__ __forceinline__ void walk_eval(const DevInstance& I, const SpecBuf& B
 // least-loaded part, which its own kind moves with every step: those the
 // first warp decides one by one.
 __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const RoundCtx& R, int metric, int pos, int zs,
-                            int end_w, int nm, WalkSmem& S, int* sz, float2* pen, int* dl) {
+                            int end_w, int nm, WalkSmem& S, int* sz, int* dl) {
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int K = I.K;
   const bool tv = metric == kTV;
@@ -942,13 +960,12 @@ __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const RoundC
     atomicAdd(&sz[m.z & 0xffff], m.y);
     atomicAdd(&sz[m.z >> 16], -m.y);
   }
-  __syncthreads();
-  for (int p = threadIdx.x; p < K; p += blockDim.x) pen[p] = pen_of(sz[p], rC);
   if (threadIdx.x == 0) S.drift = 0;
   int hard = kNone, nchg = 0;   // warp 0
   bool stop = false;
   for (int zl = zs; zl < end_w && !stop; zl += kWalkLoad) {
     const int n = min(kWalkLoad, end_w - zl), ol = zl - pos;
+    __syncthreads();   // the first warp has read the last positions' words
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
       const int o = ol + i;
       const int nc = lds(&B.ncand[o]);
@@ -971,105 +988,94 @@ __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const RoundC
       if (lane == 0) S.gmin[g] = mg;
     }
     __syncthreads();
-    for (int sc = 0; sc < n && !stop; sc += kWalkSub) {
-      const int ns = min(kWalkSub, n - sc);
-      const int g1 = (sc + ns + 31) >> 5;
-      unsigned pot = 0;   // groups a drift may reach
+    for (int g = 0; g < ng && !stop; g++) {
+      // groups that no drift reaches: the first warp applies their moves
       {
-        // (past the first such group, changed decisions may add to the drift)
-        for (int g = sc >> 5; g < g1; g++)
-          if (pot || S.drift > S.gmin[g]) pot |= 1u << (g - (sc >> 5));
-      }
-      if (pot) {
-        // a warp per row, four rows' loads in flight (a load after each store
-        // measured 16 K cycles per 128 rows, this 3 K)
-        for (int r0 = wib; r0 < ns; r0 += 4 * kSWarps) {
-          unsigned long long e[4][2];
-          int nc[4];
-#pragma unroll
-          for (int u = 0; u < 4; u++) {
-            const int r = r0 + u * kSWarps;
-            nc[u] = r < ns && ((pot >> (r >> 5)) & 1u) ? S.meta[sc + r].w >> 8 : 0;
-            const unsigned long long* cl = B.cand + (size_t)(ol + sc + min(r, ns - 1)) * K;
-#pragma unroll
-            for (int x = 0; x < 2; x++) e[u][x] = lane + 32 * x < nc[u] ? lds(&cl[lane + 32 * x]) : 0;
+        int gn = g;
+        for (const int dr = S.drift; gn < ng && dr <= S.gmin[gn]; gn++) {}
+        if (wib == 0)
+          for (; g < gn; g++) {
+            const int i = g * 32 + lane;
+            const int4 m = i < n ? S.meta[i] : make_int4(0, 0, 0, 0);
+            if (m.w & 1) {
+              atomicAdd(&sz[m.x & 0xffff], m.y);
+              atomicAdd(&sz[m.x >> 16], -m.y);
+            }
           }
+        g = gn;
+        if (g >= ng) break;
+      }
+      const int i0 = g * 32, nl = min(32, n - i0);
+      // its candidates: a warp per row, two rows' loads in flight, only the
+      // entries there are
+      for (int r0 = wib; r0 < nl; r0 += 2 * kSWarps) {
+        int nc[2];
 #pragma unroll
-          for (int u = 0; u < 4; u++)
+        for (int u = 0; u < 2; u++) {
+          const int r = r0 + u * kSWarps;
+          nc[u] = r < nl ? min(S.meta[i0 + r].w >> 8, kWalkRow) : 0;
+        }
+        for (int x = lane; x < max(nc[0], nc[1]); x += 64) {
+          unsigned long long e[2][2];
 #pragma unroll
-            for (int x = 0; x < 2; x++)
-              if (lane + 32 * x < nc[u]) S.ent[(r0 + u * kSWarps) * kWalkStride + lane + 32 * x] = e[u][x];
+          for (int u = 0; u < 2; u++)
+#pragma unroll
+            for (int y = 0; y < 2; y++)
+              e[u][y] = x + 32 * y < nc[u] ? lds(&B.cand[(size_t)(ol + i0 + r0 + u * kSWarps) * K + x + 32 * y]) : 0;
+#pragma unroll
+          for (int u = 0; u < 2; u++)
+#pragma unroll
+            for (int y = 0; y < 2; y++)
+              if (x + 32 * y < nc[u]) S.ent[(r0 + u * kSWarps) * kWalkStride + x + 32 * y] = e[u][y];
         }
       }
       __syncthreads();   // also: every thread has read S.drift
       // warp 0: the group at hand, its lanes' positions and their present outcome
-      int g = sc >> 5, j = 0, own = 0, d = 0, w = 0, mg = 0;
-      int4 m = make_int4(0, 0, 0, 0);
-      bool mv = false, in = false, fresh = true;
+      const bool in = lane < nl;
+      const int4 m = in ? S.meta[i0 + lane] : make_int4(0, 0, 0, 0);
+      const int own = m.x >> 16, w = m.y, mg = in ? S.margin[i0 + lane] : 0x7fffffff;
+      const bool iso = (m.w & 8) != 0;
+      int d = m.x & 0xffff, j = 0;
+      bool mv = (m.w & 1) != 0, done = false;
       int drift = S.drift;
+      auto exact_drift = [&]() {
+        int D0 = 0;
+        for (int p = lane; p < K; p += 32) D0 = max(D0, abs(dl[p]));
+        return warp_max(D0);
+      };
+      if (wib == 0) drift = exact_drift();
       // the moves own -> to of the lanes of mm applied
       auto apply = [&](unsigned mm, int to) {
         if (!mm) return;
-        const bool me = (mm >> lane) & 1u;
-        if (me) {
+        if ((mm >> lane) & 1u) {
           atomicAdd(&sz[to], w);
           atomicAdd(&sz[own], -w);
-        }
-        __syncwarp();
-        if (me) {
-          pen[to] = pen_of(sz[to], rC);
-          pen[own] = pen_of(sz[own], rC);
         }
         __syncwarp();
       };
       while (true) {
         if (wib == 0) {
-          // on to the next group with positions to decide again
-          int task = -1;
           unsigned need = 0;
-          for (; g < g1 && hard == kNone; g++) {
-            const int i0 = g * 32;
-            const int nl = min(32, n - i0);
-            if (fresh) {
-              in = lane < nl;
-              m = in ? S.meta[i0 + lane] : make_int4(0, 0, 0, 0);
-              own = m.x >> 16;
-              d = m.x & 0xffff;
-              w = m.y;
-              mv = (m.w & 1) != 0;
-              j = 0;
-              if (drift > S.gmin[g]) {   // the exact drift here
-                int D0 = 0;
-                for (int p = lane; p < K; p += 32) D0 = max(D0, abs(dl[p]));
-                drift = warp_max(D0);
-              }
-              mg = in ? S.margin[i0 + lane] : 0x7fffffff;
-              fresh = false;
-            }
+          if (!done && hard == kNone) {
             need = __ballot_sync(kAll, in && lane >= j && drift > mg);
-            if (need) {
-              task = g;
-              break;
-            }
-            // the rest of the group keeps its outcome
-            apply(__ballot_sync(kAll, mv && lane >= j), d);
-            fresh = true;
+            if (!need) apply(__ballot_sync(kAll, mv && lane >= j), d);   // the rest keeps its outcome
           }
+          const unsigned ev = __ballot_sync(kAll, ((need >> lane) & 1u) && !iso);
+          if ((ev >> lane) & 1u) S.list[__popc(ev & ((1u << lane) - 1u))] = lane;
           if (lane == 0) {
-            S.group = task;
+            S.group = need ? g : -1;
             S.need = need;
+            S.eval = ev;
           }
         }
         __syncthreads();
-        const int tg = S.group;
-        if (tg < 0) break;
-        walk_eval(I, B, R, tv, rC, sz, pen, S, tg * 32, sc, ol);
+        if (S.group < 0) break;
+        walk_eval(I, B, R, tv, rC, sz, S, i0, ol);
         __syncthreads();
         if (wib == 0) {
           // ---- take them in order
           const unsigned need = S.need;
-          const int i0 = g * 32, nl = min(32, n - i0);
-          const bool again = (need >> lane) & 1u, iso = (m.w & 8) != 0;
+          const bool again = (need >> lane) & 1u;
           const int nd = again && !iso ? S.nd[lane] : 0, nsl = again && !iso ? S.nslack[lane] : 0;
           const bool stale = (m.w & 2) && zl + i0 + lane != pos;
           const bool hardf = again && (stale || nd < 0);
@@ -1084,21 +1090,8 @@ __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const RoundC
           const bool chg = dn != d;
           // drift from these sizes before each position, and what the changed
           // decisions before it add to the drift of the others
-          const int x = mvn && lane >= j ? w : 0;
-          const int cw = chg && lane >= j ? (mvn ? w : 0) + (mv ? w : 0) : 0;
-          unsigned Dn = (unsigned)x, cn = (unsigned)cw;
-          if (__any_sync(kAll, x != 0))
-            for (int off = 1; off < 32; off <<= 1) {
-              const unsigned t = __shfl_up_sync(kAll, Dn, off);
-              if (lane >= off) Dn += t;
-            }
-          Dn -= (unsigned)x;
-          if (__any_sync(kAll, cw != 0))
-            for (int off = 1; off < 32; off <<= 1) {
-              const unsigned t = __shfl_up_sync(kAll, cn, off);
-              if (lane >= off) cn += t;
-            }
-          cn -= (unsigned)cw;
+          const unsigned Dn = lane_prefix(mvn && lane >= j ? (unsigned)w : 0u);
+          const unsigned cn = lane_prefix(chg && lane >= j ? (mvn ? (unsigned)w : 0u) + (mv ? (unsigned)w : 0u) : 0u);
           const long long lim = again ? (long long)nsl - Dn : (long long)mg - drift - cn;
           long long moren = 0, morec = 0;   // what the vertices without nets add to both
           while (true) {
@@ -1136,44 +1129,36 @@ __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const RoundC
               hard = ((zl + i0 + f) << 3) | (__shfl_sync(kAll, stale ? 1 : 0, f) ? 1 : 2);
               break;
             }
-            if (!af || !(S.meta[i0 + f].w & 8)) break;   // decided again from here
+            if (!af || !__shfl_sync(kAll, iso ? 1 : 0, f)) break;   // decided again from here
             // ---- vertices without nets, one by one (and their like after them)
+            const unsigned im = need & __ballot_sync(kAll, iso);
             do {
               const int4 mt = S.meta[i0 + j];
               const int of = mt.x >> 16, df = mt.x & 0xffff, wf = mt.y;
               int ms;
               int q = warp_least_loaded(sz, K, &ms);
               if (tv && (ms > I.max_pw || ms < I.min_pw)) q = of;   // the clamps keep it home
-              bool m2 = (mt.w & 1) != 0;
+              const bool m1 = (mt.w & 1) != 0;
+              const bool m2 = q == df ? m1 : q != of && (tv || (mt.w & 16));
               if (q != df) {
-                m2 = q != of && (tv || (mt.w & 16));
+                const int wo = m1 ? wf : 0, wn = m2 ? wf : 0;
+                moren += wn - wo;   // (its old weight is in the others' Dn)
+                morec += wn + wo;
+                nchg++;
                 if (lane == 0) {
                   B.dfix[ol + i0 + j] = q | (m2 ? 1 << 16 : 0);
                   B.flag[ol + i0 + j] = (unsigned char)((mt.w & 255) | 128);
                 }
-                nchg++;
-                const int wo = (mt.w & 1) ? wf : 0, wn = m2 ? wf : 0;
-                moren += wn - wo;   // (its old weight is in the others' Dn)
-                morec += wn + wo;
-                if (lane == 0) {
-                  dl[q] += wn;
-                  dl[df] -= wo;
-                  dl[of] += wo - wn;
-                }
+                if (lane < 3) atomicAdd(&dl[lane == 0 ? q : lane == 1 ? df : of], lane == 0 ? wn : lane == 1 ? -wo : wo - wn);
               } else if ((mt.w & 128) && lane == 0) {
                 B.flag[ol + i0 + j] = (unsigned char)(mt.w & 127);
               }
               if (m2) {
-                if (lane < 2) {
-                  const int p = lane == 0 ? q : of;
-                  const int s = sz[p] + (lane == 0 ? wf : -wf);
-                  sz[p] = s;
-                  pen[p] = pen_of(s, rC);
-                }
+                if (lane < 2) atomicAdd(&sz[lane == 0 ? q : of], lane == 0 ? wf : -wf);
                 __syncwarp();
               }
               j++;
-            } while (j < nl && ((need >> j) & 1u) && (S.meta[i0 + j].w & 8));
+            } while (j < nl && ((im >> j) & 1u));
             if (j >= nl) break;
           }
           // the positions taken keep what was decided
@@ -1182,13 +1167,8 @@ __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const RoundC
             d = dn;
           }
           __syncwarp();
-          int D0 = 0;   // the drift from here on
-          for (int p = lane; p < K; p += 32) D0 = max(D0, abs(dl[p]));
-          drift = warp_max(D0);
-          if (hard == kNone && j >= nl) {
-            fresh = true;
-            g++;
-          }
+          drift = exact_drift();   // from here on
+          done = j >= nl;
         }
       }
       if (threadIdx.x == 0) S.drift = drift;
@@ -1337,11 +1317,10 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
   int* adelta = adelta_b + (size_t)wib * K;
   int* loc = loc_b + wib * 96;
   Vol V{I.send, rv ? I.recv : nullptr};
-  // the walk's staged positions and penalties lie over the evaluation's arrays,
-  // its exact sizes over the round's penalties (both rebuilt every round)
+  // the walk's staged positions lie over the evaluation's arrays, its exact
+  // sizes over the round's penalties (both rebuilt every round)
   WalkSmem& walk_s = *reinterpret_cast<WalkSmem*>(cnt_b);
-  float2* walk_pn = reinterpret_cast<float2*>(cnt_b + sizeof(WalkSmem) / sizeof(int));
-  int* walk_dl = reinterpret_cast<int*>(walk_pn + K);
+  int* walk_dl = cnt_b + sizeof(WalkSmem) / sizeof(int);
   const float rC = __fdiv_rn(1.0f, Cf);
   int* walk_sz = reinterpret_cast<int*>(penf_s);
 
@@ -1967,7 +1946,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         if (!at_once) {
           const unsigned long long tW = gtimer();
           if (blockIdx.x == 0)
-            walk_window(I, B, R, metric, pos, zf, zc, lds(&B.mcnt[par]), walk_s, walk_sz, walk_pn, walk_dl);
+            walk_window(I, B, R, metric, pos, zf, zc, lds(&B.mcnt[par]), walk_s, walk_sz, walk_dl);
           if (!grid_barrier(B.bar, I.status)) return;
           hard = lds(&B.ctl[0]);
           if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -2248,7 +2227,7 @@ size_t spec_ldg_smem_bytes(int K) {
   auto a = [](size_t n) { return (n + 15) & ~size_t(15); };
   const size_t k4 = a(sizeof(int) * K);
   const size_t eval = 4 * a(sizeof(int) * (size_t)K * kSWarps) + a(sizeof(unsigned long long) * (size_t)K * kSWarps);
-  return 5 * k4 + std::max(eval, sizeof(WalkSmem) + (sizeof(float2) + sizeof(int)) * K);
+  return 5 * k4 + std::max(eval, sizeof(WalkSmem) + sizeof(int) * K);
 }
 
 cudaError_t launch_spec_ldg(const DevInstance& I, const SpecBuf& B, int passes, int num_sms, cudaStream_t st,
