@@ -526,11 +526,10 @@ static int build_stream_positions(fp_instance* in) {
   in->sa.actm = in->st_actm_d;
   in->sa.ownm = in->st_ownm_d;
   in->sa.msg_wmax = msg_stream_window(g.nov);
-  // Walking the changed decisions of a window on one warp (instead of ending
-  // the window at the first) pays where most windows end at a change: CN
-  // 8.9 -> 3.3 s on the 4M-vertex Zipf workload; the LDG streams, whose
-  // windows end at conflicts as often, went 1.05 -> 1.33 s, so they cut.
-  in->sa.walk = pb.metric == FP_METRIC_CN ? 1 : 0;
+  // Walking the changed decisions of a window (instead of ending the window at
+  // the first): Zipf streams at K = 256, TV 262144 vertices 177 -> 131 ms, 1M
+  // 321 -> 301, 30000 (K = 64) 43 -> 36.
+  in->sa.walk = 1;
   cudaStream_t s0 = in->ctx->stream;
   cudaError_t e0 = cudaSuccess;
   if (in->stream_dev) {

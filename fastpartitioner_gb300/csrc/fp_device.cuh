@@ -78,7 +78,10 @@ struct StreamArgs {
 };
 constexpr int kStreamHeavy = 4096;   // nets of a vertex the whole grid places in the device stream
 // List entries a position's evaluation may read (the sum of min(|e|, K) over
-// its nets) from which one CTA, or the whole grid, evaluates it.
+// its nets) from which a team of CTAs, or the whole grid in a window of its
+// own, evaluates it.  Zipf stream of 262144 vertices, K = 256: 122-124 ms at
+// 2048, 4096 and 8192; of 1M: 267 ms with kStreamGridWork 65536 and 277 with
+// 262144 (and 8192 nets).
 constexpr long long kStreamCtaWork = 4096;
 constexpr long long kStreamGridWork = 65536;
 constexpr int kStreamMaxK = 1024;    // shared memory of the device stream's CTAs

@@ -25,25 +25,32 @@
 //                window appends to one of its nets and the decision taken again
 //                with the exact sizes at its place (the window-start sizes plus
 //                the earlier placements) is the same.  The window ends at the
-//                first conflict; at the first changed decision it either ends
+//                first conflict.  At the first changed decision it either ends
 //                too (that position commits last, with its exact decision) or,
-//                with StreamArgs::walk, one warp walks on in order with exact
-//                sizes, taking every change (a change that appends where the
-//                old decision did not claims those nets, and the later
-//                positions are checked against the claims again);
+//                with StreamArgs::walk, one CTA walks on in order with exact
+//                sizes (walk_window), the changed positions' warps find their
+//                slots and claim their appends again (the old claims stay), and
+//                the rest of the window is checked against the claims again;
 //   C  commit    the positions before the cut are applied at once: on any net
 //                at most one of them appends (a later reader of that net is
 //                invalid), the others increment counts at their recorded slots
-//                (changed decisions locate theirs again).
+//                (a changed decision that ends the window locates its own).
 //
 // Vertices without nets read only the sizes.  When all of them weigh 0 (vertex
 // weight = degree) they are not positions: after each window's commit they take
-// the least-loaded part of the sizes at their place.  A position is evaluated
-// by a warp, by a CTA when its lists are long (kStreamCtaWork entries or more),
-// and a vertex with many nets (kStreamHeavy or more, or kStreamGridWork list
-// entries) is a window of its own, evaluated and committed by the whole grid.
+// the least-loaded part of the sizes at their place.
+//
+// A window of 262144 vertices' Zipf stream (K = 256) keeps some 21 positions
+// and is bound by the latency of its phases (a round trip to L2 280 cycles, a
+// grid barrier 1.4 us), so a window of no more positions than CTAs gives each
+// a CTA, whose warps share its nets, and a position with long lists
+// (kStreamCtaWork entries or more) a team of the CTAs: evaluation 28.5 us ->
+// 16, with the walk 228 ms -> 117 for the whole stream.  A longer window gives
+// its positions a warp each.  A vertex with many nets (kStreamHeavy or more, or
+// kStreamGridWork list entries) is a window of its own, evaluated and committed
+// by the whole grid.
 
-#include "fp_spec_common.cuh"
+#include "fp_walk.cuh"
 
 #include <algorithm>
 
@@ -57,6 +64,7 @@ constexpr int kCN = 0;
 constexpr int kTV = 1;
 constexpr int kMSV = 4;
 constexpr int kMSRV = 5;
+constexpr int kStreamTeams = kMaxGridVerts;   // positions of a window with a team of CTAs each
 
 // CN's tally of the nets [nb, min(nb + 32, deg)) of a vertex: the part of
 // every net with exactly one listed part, the number of such nets per part and
@@ -91,34 +99,6 @@ __device__ __forceinline__ unsigned long long skey(int round, int pos) {
 __device__ __forceinline__ bool claimed_before(const SpecBuf& B, int round, int e, int pos) {
   const unsigned long long c = lds(&B.claim64[e]);
   return (int)(c >> 32) == round && (int)(0xffffffffu - (unsigned)(c & 0xffffffffu)) < pos;
-}
-
-// Candidate entry: part (12 bits), nets listing it (16), first sighting: net
-// index (16) and slot (20).  Positions hold fewer than kStreamHeavy nets.
-__device__ __forceinline__ unsigned long long sc_entry(int p, int c, unsigned long long f) {
-  return ((unsigned long long)p << 52) | ((unsigned long long)c << 36) | (((f >> 32) & 0xffffull) << 20) |
-         (f & 0xfffffull);
-}
-
-// Exact LDG pick of one warp over candidate entries (part, count, first),
-// sizes sz0[p] + (dsz ? dsz[p] : 0): the best positive score, ties to the
-// smaller part, then the first seen; -1 if no part scores (TV/partition.cpp:
-// 98-117).
-__device__ int pick_entries(const DevInstance& I, const unsigned long long* cl, int nc, const int* sz0,
-                            const int* dsz) {
-  const int lane = threadIdx.x & 31;
-  LdgKey best{-1.0, 0, -1, ~0ull};
-  for (int i = lane; i < nc; i += 32) {
-    const unsigned long long ent = lds(&cl[i]);
-    const int p = (int)(ent >> 52);
-    const int c = (int)((ent >> 36) & 0xffffull);
-    const unsigned long long f = (((ent >> 20) & 0xffffull) << 32) | (ent & 0xfffffull);
-    const int sz = sz0[p] + (dsz ? dsz[p] : 0);
-    const LdgKey k{ldg_score(c, sz, I.C), sz, p, f};
-    if (ldg_better(k, best)) best = k;
-  }
-  best = warp_ldg_argmax(best);
-  return best.part;
 }
 
 // Least-loaded part of sz0 + dsz, lowest index on ties (one warp).
@@ -212,39 +192,63 @@ __device__ __forceinline__ void place_net(const DevInstance& I, int e, int d, in
 }
 
 // Candidates of window offset o from a tally (cnt / first over K parts), in
-// ascending part order, and its decision with the window-start sizes (the
-// least-loaded part minpart when no part scores); writes cand, ncand, dec, wt
-// and the weight's mlist entry.  One warp; returns the decision.
-__device__ int decide_position(const DevInstance& I, const SpecBuf& B, const int* sizes_s, int minpart,
-                               const int* cnt, const unsigned* first, int sb, int o, int wv, int par, int* nc_out) {
+// ascending part order, and its decision with the window-start sizes (penf:
+// their penalties; the least-loaded part minpart, with the second smallest
+// size, when no part scores); writes cand, ncand, dec, wt, the drift it
+// tolerates and the weight's mlist entry (if `write`).  One warp; returns the
+// decision.
+// Scores in float first (ScoreAcc): exact ones take 722 cycles each.
+__device__ int decide_position(const DevInstance& I, const SpecBuf& B, const int* sizes_s, const float* penf, float Cf,
+                               int minpart, int minsize, int second, const int* cnt, const unsigned* first, int sb,
+                               int o, int wv, int par, bool write, int* nc_out) {
   const int lane = threadIdx.x & 31;
   const int K = I.K;
   unsigned long long* cl = B.cand + (size_t)o * K;
   int nc = 0;
-  LdgKey best{-1.0, 0, -1, ~0ull};
+  ScoreAcc A;
+#pragma unroll 4
   for (int p0 = 0; p0 < K; p0 += 32) {
     const int p = p0 + lane;
     const int c = p < K ? cnt[p] : 0;
     const unsigned m = __ballot_sync(kAll, c > 0);
     if (c > 0) {
-      const unsigned long long f = wide_key(first[p], sb, 0);
-      cl[nc + __popc(m & ((1u << lane) - 1u))] = sc_entry(p, c, f);
-      const LdgKey k{ldg_score(c, sizes_s[p], I.C), sizes_s[p], p, f};
-      if (ldg_better(k, best)) best = k;
+      if (write) cl[nc + __popc(m & ((1u << lane) - 1u))] = cand_entry(p, c, first[p]);
+      A.add(p, c, make_float2(penf[p], tol_of(penf[p])));
     }
     nc += __popc(m);
   }
-  best = warp_ldg_argmax(best);
-  const int d = best.part >= 0 ? best.part : minpart;
+  A.meet(32);
+  int d = minpart, sl = -1;
+  if (A.one()) {
+    d = (int)(A.be & 0x1fffu);
+    sl = A.slack_one(Cf);
+  } else if (A.none()) {
+    sl = min(A.slack_none(Cf), (second - minsize - 1) / 2);
+  } else {
+    const float fb = fmaxf(A.blo, 0.0f);
+    LdgKey best{-1.0, 0, -1, ~0ull};
+    for (int p = lane; p < K; p += 32) {
+      const int c = cnt[p];
+      if (c == 0 || (float)c * penf[p] + (float)c * tol_of(penf[p]) < fb) continue;
+      const LdgKey k{ldg_score(c, sizes_s[p], I.C), sizes_s[p], p, first[p]};
+      if (ldg_better(k, best)) best = k;
+    }
+    best = warp_ldg_argmax(best);
+    if (best.part >= 0) d = best.part;
+  }
+  sl = max(sl, 0);
+  // TV's reference has no part for a vertex that chooses one above max_pw (-2: here)
+  if (I.metric == kTV) sl = sizes_s[d] > I.max_pw ? -2 : min(sl, I.max_pw - sizes_s[d]);
   *nc_out = nc;
-  if (lane == 0) {
+  if (write && lane == 0) {
     B.ncand[o] = nc;
-    B.dec[o] = d;
+    B.dec[o] = (K << 16) | d;
     B.wt[o] = wv;
-    B.flag[o] = 0;
+    B.slack[o] = sl;
+    B.flag[o] = nc ? 1 : 9;   // every position is placed; 8: always in the least-loaded part
     if (wv) {
       const int i = atomicAdd(&B.mcnt[par], 1);
-      B.mlist[i] = make_int4(o, wv, d, 0);
+      B.mlist[i] = make_int4(o, wv, (K << 16) | d, 0);
       B.midx[o] = i;
     }
   }
@@ -253,24 +257,19 @@ __device__ int decide_position(const DevInstance& I, const SpecBuf& B, const int
 }
 
 // The records of d in the nets [n0, n1) of a vertex (one warp) and the claims
-// of the nets d is appended to.
-// With claim_all every net is claimed (and counted as appended to): any
-// other decision's appends are then a subset.
-__device__ int record_slots(const DevInstance& I, const SpecBuf& B, const StreamArgs& S, uint32_t base, int n0,
-                            int n1, int d, int round, int z, int* sd, bool claim_all) {
+// of the nets d is appended to.  With claim_all every net is claimed: any other
+// decision's appends are then a subset.
+__device__ void record_slots(const DevInstance& I, const SpecBuf& B, const StreamArgs& S, uint32_t base, int n0,
+                             int n1, int d, int round, int z, int* sd, bool claim_all) {
   const int lane = threadIdx.x & 31;
-  int napp = 0;
   for (int nb = n0; nb < n1; nb += 32) {
     const int j = locate_part(I, base, nb, n1, d, sd);
     const int k = nb + lane;
-    const bool app = k < n1 && (j < 0 || claim_all);
     if (k < n1) {
       S.rec[base + k] = j >= 0 ? (uint32_t)j : kNoSlot;
-      if (app) atomicMax(&B.claim64[(int)__ldg(&I.vnets[base + k])], skey(round, z));
+      if (j < 0 || claim_all) atomicMax(&B.claim64[(int)__ldg(&I.vnets[base + k])], skey(round, z));
     }
-    napp += __popc(__ballot_sync(kAll, app));
   }
-  return napp;   // every lane
 }
 
 // The walk takes a changed decision d of position z that appends where the old
@@ -299,20 +298,6 @@ __device__ bool conflicts_now(const DevInstance& I, const SpecBuf& B, int v, int
   return __any_sync(kAll, conf);
 }
 
-// Nets of window offset o listing part d (its candidate entry's count; 0 if d
-// is not a candidate).  One warp.
-__device__ int cand_count(const SpecBuf& B, int K, int o, int d) {
-  const int lane = threadIdx.x & 31;
-  const unsigned long long* cl = B.cand + (size_t)o * K;
-  const int nc = lds(&B.ncand[o]);
-  int c = 0;
-  for (int i = lane; i < nc; i += 32) {
-    const unsigned long long ent = lds(&cl[i]);
-    if ((int)(ent >> 52) == d) c = (int)((ent >> 36) & 0xffffull);
-  }
-  return warp_max(c);
-}
-
 // The vertices without nets [k0, k1) of the iso list take the least-loaded
 // part of sz (TV: the size of that part above max_pw would make the reference
 // use part -1: unsupported).  One warp; *amin caches the argmin (-1: stale).
@@ -332,7 +317,8 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
   barrier_start();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ unsigned long long uscr[kSWarps];
-  __shared__ int s_minpart, s_minsize, s_second, s_dec, s_napp, s_nc;
+  __shared__ int s_minpart, s_minsize, s_second, s_dec, s_nc;
+  __shared__ int s_loc[32 * kSWarps];
   const int K = I.K;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int gw = blockIdx.x * kSWarps + wib;
@@ -342,13 +328,18 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
   const bool cn = I.metric == kCN;   // no marker and no TV clamp
   Carve cv{smem_raw};
   int* sizes_s = cv.take<int>(K);
-  int* dsz_cta = cv.take<int>(K);
+  int* dsz_cta = cv.take<int>(K + 1);
+  float* penf = cv.take<float>(K + 1);
   int* cnt_b = cv.take<int>((size_t)K * kSWarps);
-  unsigned* first_b = reinterpret_cast<unsigned*>(cv.take<unsigned long long>((size_t)K * kSWarps));
-  int* sd_b = cv.take<int>(32 * kSWarps);
+  unsigned* first_b = cv.take<unsigned>((size_t)K * kSWarps);
+  int* sd_b = s_loc;
   int* cnt = cnt_b + (size_t)wib * K;
   unsigned* first = first_b + (size_t)wib * K;
   const int sb = slot_bits(K);
+  const float Cf = (float)I.C, rC = __fdiv_rn(1.0f, Cf);
+  // the walk's staged positions lie over the evaluation's arrays, its exact
+  // sizes over the penalties, what it changed over the CTA's prefix
+  WalkSmem& walk_s = *reinterpret_cast<WalkSmem*>(cnt_b);
   int* sd = sd_b + 32 * wib;
   const bool stats = blockIdx.x == 0 && threadIdx.x == 0;
   unsigned long long t0 = stats ? gtimer() : 0ull;
@@ -360,12 +351,15 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
     }
   };
 
-  int pos = 0, round = 1, hidx = 0;
+  int pos = 0, round = 1, hidx = 0, mi0 = 0;
   int W = min(nwarps, B.wmax);
   while (pos < S.npos) {
     const int par = round & 1;
     // ------------------------------------------------------------ round state
-    for (int p = threadIdx.x; p < K; p += blockDim.x) sizes_s[p] = lds(&I.part_sizes[p]);
+    for (int p = threadIdx.x; p < K; p += blockDim.x) {
+      sizes_s[p] = lds(&I.part_sizes[p]);
+      penf[p] = pen_of(sizes_s[p], rC).x;
+    }
     __syncthreads();
     block_min_part(sizes_s, K, uscr, &s_minpart, &s_minsize, &s_second);
     __syncthreads();
@@ -409,15 +403,26 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
       if (!grid_barrier(B.bar, I.status)) return;
       if (blockIdx.x == 0) {
         if (wib == 0) {
-          LdgKey best{-1.0, 0, -1, ~0ull};
+          ScoreAcc A;
           for (int p = lane; p < K; p += 32) {
             const int c = lds(&B.hcnt[p]);
-            if (c <= 0) continue;
-            const LdgKey k{ldg_score(c, sizes_s[p], I.C), sizes_s[p], p, lds(&B.hfirst[p])};
-            if (ldg_better(k, best)) best = k;
+            if (c > 0) A.add(p, c, make_float2(penf[p], tol_of(penf[p])));
           }
-          best = warp_ldg_argmax(best);
-          const int d = best.part >= 0 ? best.part : s_minpart;
+          A.meet(32);
+          int d = s_minpart;
+          if (A.one()) {
+            d = (int)(A.be & 0x1fffu);
+          } else if (!A.none()) {
+            LdgKey best{-1.0, 0, -1, ~0ull};
+            for (int p = lane; p < K; p += 32) {
+              const int c = lds(&B.hcnt[p]);
+              if (c <= 0 || (float)c * penf[p] + (float)c * tol_of(penf[p]) < fmaxf(A.blo, 0.0f)) continue;
+              const LdgKey k{ldg_score(c, sizes_s[p], I.C), sizes_s[p], p, lds(&B.hfirst[p])};
+              if (ldg_better(k, best)) best = k;
+            }
+            best = warp_ldg_argmax(best);
+            if (best.part >= 0) d = best.part;
+          }
           if (lane == 0) {
             if (tv && sizes_s[d] > I.max_pw) dev_fail(I.status, kDevErrUnsupported);
             B.dec[0] = d;
@@ -476,12 +481,89 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
     int end_w = min(pos + W, S.npos);
     if (hidx < S.nheavy) end_w = min(end_w, (int)__ldg(&S.heavy_pos[hidx]));
     const int span = end_w - pos;
-    const int q = (span + nwarps - 1) / nwarps;
-    const int z0 = min(pos + gw * q, end_w);
+    // the others: a CTA each in a window of no more positions than CTAs (a
+    // share of the nets per warp), else q to a warp
+    const bool wide = span <= (int)gridDim.x;
+    const int q = wide ? 1 : (span + nwarps - 1) / nwarps;
+    const int z0 = min(pos + (wide ? (int)blockIdx.x : gw * q), end_w);
     const int z1 = min(z0 + q, end_w);
-    // ---- A: evaluate: light positions by their warps, medium positions by
-    // CTAs from the end of the grid
-    for (int z = z0; z < z1; z++) {
+    const bool owner = !wide || wib == 0;   // the warp that decides its positions
+    auto warp_nets = [&](int deg, int* n0, int* n1) {
+      if (wide) {
+        net_range(deg, wib, kSWarps, n0, n1);
+      } else {
+        *n0 = 0;
+        *n1 = deg;
+      }
+    };
+    // the positions with long lists: each gets an equal team of the CTAs (from
+    // the end of the grid, a share of its nets per CTA), or, in a window with
+    // more than kStreamTeams of them, a CTA
+    while (mi0 < S.nmid) {   // those before pos are placed
+      const unsigned m = __ballot_sync(kAll, mi0 + lane < S.nmid && __ldg(&S.mid_pos[min(mi0 + lane, S.nmid - 1)]) < pos);
+      mi0 += __popc(m);
+      if (m != kAll) break;
+    }
+    int nmid = 0;
+    while (mi0 + nmid < S.nmid) {
+      const int i = mi0 + nmid + lane;
+      const unsigned m = __ballot_sync(kAll, i < S.nmid && __ldg(&S.mid_pos[min(i, S.nmid - 1)]) < end_w);
+      nmid += __popc(m);
+      if (m != kAll) break;
+    }
+    const bool teams = nmid <= min(kStreamTeams, (int)gridDim.x);
+    const int tsize = teams && nmid ? (int)gridDim.x / nmid : 1;
+    const int bmid = (int)(gridDim.x - 1 - blockIdx.x);
+    // f(m, z, v, base, deg, c0, c1) for this CTA's shares: nets [c0, c1) of the
+    // window's m-th position with long lists, if it lies in [za, zb)
+    auto for_mid = [&](int za, int zb, auto&& f) {
+      for (int m = bmid / tsize; m < nmid; m += (int)gridDim.x) {
+        const int z = __ldg(&S.mid_pos[mi0 + m]);
+        if (z < za || z >= zb) continue;
+        const int v = __ldg(&S.porder[z]);
+        const uint32_t base = __ldg(&I.vptr[v]);
+        const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
+        int c0, c1;
+        net_range(deg, bmid % tsize, tsize, &c0, &c1);
+        f(m, z, v, base, deg, c0, c1);
+      }
+    };
+    // ---- A: evaluate: light positions by their warps, the others by CTAs
+    // one set of arrays for the CTA's warps (a position has fewer than kStreamHeavy nets)
+    auto tally_share = [&](int, int, int, uint32_t base, int, int c0, int c1) {
+      int n0, n1;
+      net_range(c1 - c0, wib, kSWarps, &n0, &n1);
+      n0 += c0;
+      n1 += c0;
+      __syncthreads();   // the CTA's previous tallies are read
+      for (int p = threadIdx.x; p < K; p += blockDim.x) { cnt_b[p] = 0; first_b[p] = ~0u; }
+      __syncthreads();
+      for (int nb = n0; nb < n1; nb += 32) tally_stream(I, cn, base, nb, n1, 0, sb, cnt_b, first_b);
+      __syncthreads();
+    };
+    auto decide_cta = [&](int, int z, int v, uint32_t base, int, int c0, int c1) {
+      if (wib == 0) {
+        int nc;
+        const int d = decide_position(I, B, sizes_s, penf, Cf, s_minpart, s_minsize, s_second, cnt_b, first_b, sb,
+                                      z - pos, __ldg(&I.w[v]), par, c0 == 0, &nc);
+        if (lane == 0) {
+          s_dec = d;
+          s_nc = nc;
+        }
+      }
+      __syncthreads();
+      int n0, n1;
+      net_range(c1 - c0, wib, kSWarps, &n0, &n1);
+      record_slots(I, B, S, base, c0 + n0, c0 + n1, s_dec, round, z, sd, cn && s_nc == 0);
+    };
+    if (wide && z0 < z1 && __ldg(&S.pclass[z0]) == 0) {
+      const int v = __ldg(&S.porder[z0]);
+      const uint32_t base = __ldg(&I.vptr[v]);
+      const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
+      tally_share(0, z0, v, base, deg, 0, deg);
+      decide_cta(0, z0, v, base, deg, 0, deg);
+    }
+    for (int z = z0; z < z1 && !wide; z++) {
       if (__ldg(&S.pclass[z]) != 0) continue;
       const int o = z - pos;
       const int v = __ldg(&S.porder[z]);
@@ -492,106 +574,133 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
       for (int nb = 0; nb < deg; nb += 32) tally_stream(I, cn, base, nb, deg, 0, sb, cnt, first);
       __syncwarp();
       int nc;
-      const int d = decide_position(I, B, sizes_s, s_minpart, cnt, first, sb, o, __ldg(&I.w[v]), par, &nc);
+      const int d = decide_position(I, B, sizes_s, penf, Cf, s_minpart, s_minsize, s_second, cnt, first, sb, o,
+                                    __ldg(&I.w[v]), par, true, &nc);
       // CN: a position without candidates decides by the sizes alone; it
       // claims all its nets, so that a changed decision adds no claim
-      const int napp = record_slots(I, B, S, base, 0, deg, d, round, z, sd, cn && nc == 0);
-      if (lane == 0) B.slack[o] = napp;   // nets the decision appends to
+      record_slots(I, B, S, base, 0, deg, d, round, z, sd, cn && nc == 0);
       __syncwarp();
     }
-    if (S.nmid) {
-      const int i0 = lower_bound_pos(S.mid_pos, S.nmid, pos);
-      const int i1 = lower_bound_pos(S.mid_pos, S.nmid, end_w);
-      for (int i = i0 + (int)(gridDim.x - 1 - blockIdx.x); i < i1; i += gridDim.x) {
-        const int z = __ldg(&S.mid_pos[i]);
-        const int o = z - pos;
-        const int v = __ldg(&S.porder[z]);
-        const uint32_t base = __ldg(&I.vptr[v]);
-        const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
-        int n0, n1;
-        net_range(deg, wib, kSWarps, &n0, &n1);
-        __syncthreads();   // the tallies of the CTA's previous position are read
-        // one set of arrays for the CTA's warps (a vertex here has fewer than kStreamHeavy nets)
-        for (int p = threadIdx.x; p < K; p += blockDim.x) { cnt_b[p] = 0; first_b[p] = ~0u; }
-        __syncthreads();
-        for (int nb = n0; nb < n1; nb += 32) tally_stream(I, cn, base, nb, n1, 0, sb, cnt_b, first_b);
-        __syncthreads();
-        if (wib == 0) {
-          int nc;
-          const int d = decide_position(I, B, sizes_s, s_minpart, cnt_b, first_b, sb, o, __ldg(&I.w[v]), par, &nc);
-          if (lane == 0) {
-            s_dec = d;
-            s_nc = nc;
+    if (nmid) {
+      if (!teams) {
+        for_mid(pos, end_w, [&](int m, int z, int v, uint32_t base, int deg, int c0, int c1) {
+          tally_share(m, z, v, base, deg, c0, c1);
+          decide_cta(m, z, v, base, deg, c0, c1);
+        });
+      } else {
+        // the team's tallies meet in global memory; each CTA decides from them
+        // and records its share
+        for_mid(pos, end_w, [&](int m, int z, int v, uint32_t base, int deg, int c0, int c1) {
+          tally_share(m, z, v, base, deg, c0, c1);
+          for (int p = threadIdx.x; p < K; p += blockDim.x)
+            if (cnt_b[p]) {
+              atomicAdd(&B.hcnt[(size_t)m * K + p], cnt_b[p]);
+              atomicMin(&B.hfirst[(size_t)m * K + p], (unsigned long long)first_b[p]);
+            }
+        });
+        if (!grid_barrier(B.bar, I.status)) return;
+        for_mid(pos, end_w, [&](int m, int z, int v, uint32_t base, int deg, int c0, int c1) {
+          for (int p = threadIdx.x; p < K; p += blockDim.x) {
+            cnt_b[p] = lds(&B.hcnt[(size_t)m * K + p]);
+            first_b[p] = (unsigned)lds(&B.hfirst[(size_t)m * K + p]);
           }
-        }
-        if (threadIdx.x == 0) s_napp = 0;
-        __syncthreads();
-        const int napp = record_slots(I, B, S, base, n0, n1, s_dec, round, z, sd, cn && s_nc == 0);
-        if (lane == 0) atomicAdd(&s_napp, napp);
-        __syncthreads();
-        if (threadIdx.x == 0) B.slack[o] = s_napp;
+          __syncthreads();
+          decide_cta(m, z, v, base, deg, c0, c1);
+        });
       }
     }
     if (!grid_barrier(B.bar, I.status)) return;
     lap(16);
-    // ---- B: validate.  B1 (every warp): the first position with a claim
-    // conflict, and the first whose decision changes with the exact sizes
-    // (or needs a TV part above max_pw) if every earlier one keeps its own.
-    // B2 (one warp, only if such a change comes before the first conflict):
-    // walk the positions from it in order with exact sizes, taking each
-    // changed decision whose appends are a subset of the old one's (no new
-    // claims), and end the window at the first change that is not -- that
-    // position commits last, with its exact decision -- or at the conflict.
+    // ---- B1: validate (every warp): the first position with a claim conflict,
+    // and the first whose decision the exact sizes change (or that needs a TV
+    // part above max_pw) if every earlier one keeps its own
     int* const cut_w = &B.ctl[4 + par];
     int* const flip_w = &B.ctl[2 + par];
-    const int cz0 = min(pos + blockIdx.x * kSWarps * q, end_w);
-    const int cta_o0 = cz0 - pos;
-    {
+    const int cta_o0 = min((int)blockIdx.x * (wide ? 1 : kSWarps * q), span);
+    // the placements of the window before this CTA's positions, per part
+    auto placed_before = [&]() {
       for (int p = threadIdx.x; p < K; p += blockDim.x) dsz_cta[p] = 0;
       __syncthreads();
       const int nm = lds(&B.mcnt[par]);
       for (int i = threadIdx.x; i < nm; i += blockDim.x) {
         const int4 m = lds(&B.mlist[i]);
-        if (m.x < cta_o0) atomicAdd(&dsz_cta[m.z], m.y);
+        if (m.x < cta_o0) atomicAdd(&dsz_cta[m.z & 0xffff], m.y);
       }
       __syncthreads();
-      bool decided = false;   // this warp found its first change: later ones only check conflicts
-      for (int z = z0; z < z1; z++) {
-        const int o = z - pos;
-        const int v = __ldg(&S.porder[z]);
-        const uint32_t base = __ldg(&I.vptr[v]);
-        const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
-        bool conf = false;
-        for (int k = lane; k < deg && !conf; k += 32)
-          conf = claimed_before(B, round, (int)__ldg(&I.vnets[base + k]), z);
-        if (__any_sync(kAll, conf)) {
-          if (lane == 0) atomicMin(cut_w, (z << 3) | 5);
-          break;
+    };
+    // the first conflict of the positions [za, zb) lowers *cut_w; a warp's
+    // positions before its first are taken again by `again`
+    auto conflict = [&](int z, uint32_t base, int n0, int n1) {
+      bool conf = false;
+      for (int k = n0 + lane; k < n1 && !conf; k += 32)
+        conf = claimed_before(B, round, (int)__ldg(&I.vnets[base + k]), z);
+      conf = __any_sync(kAll, conf);
+      if (conf && lane == 0) atomicMin(cut_w, (z << 3) | 5);
+      return conf;
+    };
+    auto check_claims = [&](int za, int zb, auto&& again) {
+      for (int z = max(z0, za); z < min(z1, zb); z++) {
+        if (__ldg(&S.pclass[z]) == 0) {
+          const int v = __ldg(&S.porder[z]);
+          const uint32_t base = __ldg(&I.vptr[v]);
+          int n0, n1;
+          warp_nets((int)(__ldg(&I.vptr[v + 1]) - base), &n0, &n1);
+          if (conflict(z, base, n0, n1)) break;
         }
-        if (decided) continue;
+        if (owner) again(z);
+      }
+      for_mid(za, zb, [&](int, int z, int, uint32_t base, int, int c0, int c1) {
+        int n0, n1;
+        net_range(c1 - c0, wib, kSWarps, &n0, &n1);
+        conflict(z, base, c0 + n0, c0 + n1);
+      });
+    };
+    placed_before();
+    {
+      bool decided = false;   // this warp's first change ends the window: later ones only check conflicts
+      int D0 = 0;
+      if (z0 < z1) {
+        int wi = 0;
+        for (int p = lane; p < K; p += 32) D0 = max(D0, dsz_cta[p]);
+        for (int o2 = cta_o0 + lane; o2 < z0 - pos; o2 += 32) wi += lds(&B.wt[o2]);
+        D0 = warp_max(D0) + warp_sum(wi);
+      }
+      check_claims(pos, end_w, [&](int z) {
+        if (decided) return;
+        const int o = z - pos;
+        const int sl = lds(&B.slack[o]), wz = lds(&B.wt[o]);
+        if (D0 <= sl) {
+          if (lane == 0) B.rel[o] = sl - D0;
+          D0 += wz;
+          return;
+        }
+        D0 += wz;
         // the exact sizes here if no earlier decision changes: the window-start
         // sizes, the placements before this CTA's positions, those of this
         // CTA's positions before z
-        int* dsz = cnt;
-        for (int p = lane; p < K; p += 32) dsz[p] = dsz_cta[p];
+        int* sz = cnt;
+        for (int p = lane; p < K; p += 32) sz[p] = sizes_s[p] + dsz_cta[p];
         __syncwarp();
         for (int o2 = cta_o0 + lane; o2 < o; o2 += 32) {
           const int w = lds(&B.wt[o2]);
-          if (w) atomicAdd(&dsz[lds(&B.dec[o2])], w);
+          if (w) atomicAdd(&sz[lds(&B.dec[o2]) & 0xffff], w);
         }
         __syncwarp();
-        int d2 = pick_entries(I, B.cand + (size_t)o * K, lds(&B.ncand[o]), sizes_s, dsz);
-        if (d2 < 0) d2 = least_loaded(sizes_s, dsz, K);
-        const bool clamp = tv && sizes_s[d2] + dsz[d2] > I.max_pw;
-        if (d2 != lds(&B.dec[o]) || clamp) {
-          if (lane == 0) {
+        int rel;
+        const int d2 = walk_pick_any(I, rC, Cf, sz, lds(&B.ncand[o]), B.cand + (size_t)o * K, &rel) & 0x1fff;
+        const bool clamp = tv && sz[d2] > I.max_pw;
+        if (tv) rel = min(rel, I.max_pw - sz[d2]);
+        const bool flip = d2 != (lds(&B.dec[o]) & 0xffff) || clamp;
+        if (lane == 0) {
+          B.rel[o] = flip ? -2 : max(rel, 0);
+          if (flip) {
             B.dfix[o] = d2;
             atomicMin(flip_w, (z << 3) | (clamp ? 7 : 2));
           }
-          decided = true;
         }
+        if (flip && !S.walk) decided = true;
         __syncwarp();
-      }
+      });
     }
     if (!grid_barrier(B.bar, I.status)) return;
     lap(17);
@@ -605,109 +714,48 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
       cut = zf;
       cutc = (flipw & 7) == 2 ? zf + 1 : zf;
     } else if (zf < zc) {
-      if (blockIdx.x == 0 && wib == 0) {
-        int* sz = cnt;
-        for (int p = lane; p < K; p += 32) sz[p] = sizes_s[p];
-        __syncwarp();
-        const int nm = lds(&B.mcnt[par]);
-        for (int i = lane; i < nm; i += 32) {
-          const int4 m = lds(&B.mlist[i]);
-          if (m.x < zf - pos) atomicAdd(&sz[m.z], m.y);
-        }
-        __syncwarp();
-        int c1 = zc, c2 = zc;
-        bool stop = false, reclaim = false;
-        // 32 positions at a time: their scalar words one per lane, and the
-        // next position's first 32 candidates loaded while one is decided
-        for (int zb = zf; zb < zc && !stop; zb += 32) {
-          const int zl = zb + lane, ol = zl - pos;
-          const bool in = zl < zc;
-          const int nc_l = in ? lds(&B.ncand[ol]) : 0;
-          const int d_l = in ? lds(&B.dec[ol]) : 0;
-          const int w_l = in ? lds(&B.wt[ol]) : 0;
-          const int na_l = in ? lds(&B.slack[ol]) : 0;
-          int deg_l = 0, v_l = 0;
-          if (in) {
-            v_l = __ldg(&S.porder[zl]);
-            deg_l = (int)(__ldg(&I.vptr[v_l + 1]) - __ldg(&I.vptr[v_l]));
-          }
-          const int nb = min(32, zc - zb);
-          unsigned long long ent = 0;
-          {
-            const int nc0 = __shfl_sync(kAll, nc_l, 0);
-            if (lane < nc0) ent = lds(&B.cand[(size_t)(zb - pos) * K + lane]);
-          }
-          for (int j = 0; j < nb; j++) {
-            const int z = zb + j, o = z - pos;
-            const int nc = __shfl_sync(kAll, nc_l, j);
-            const int d = __shfl_sync(kAll, d_l, j);
-            const int w = __shfl_sync(kAll, w_l, j);
-            const int napp = __shfl_sync(kAll, na_l, j);
-            const int deg = __shfl_sync(kAll, deg_l, j);
-            const int vz = __shfl_sync(kAll, v_l, j);
-            const int ncn = __shfl_sync(kAll, nc_l, (j + 1) & 31);
-            if (reclaim && conflicts_now(I, B, vz, round, z)) {   // a taken change appends to one of its nets
-              c1 = c2 = z;
-              stop = true;
-              break;
-            }
-            unsigned long long ent_next = 0;
-            if (j + 1 < nb && lane < ncn) ent_next = lds(&B.cand[(size_t)(o + 1) * K + lane]);
-            LdgKey best{-1.0, 0, -1, ~0ull};
-            for (int i = lane; i < nc; i += 32) {
-              const unsigned long long e = i < 32 ? ent : lds(&B.cand[(size_t)o * K + i]);
-              const int p = (int)(e >> 52);
-              const int c = (int)((e >> 36) & 0xffffull);
-              const unsigned long long f = (((e >> 20) & 0xffffull) << 32) | (e & 0xfffffull);
-              const LdgKey k{ldg_score(c, sz[p], I.C), sz[p], p, f};
-              if (ldg_better(k, best)) best = k;
-            }
-            best = warp_ldg_argmax(best);
-            const int d2 = best.part >= 0 ? best.part : least_loaded(sz, nullptr, K);
-            ent = ent_next;
-            if (tv && sz[d2] > I.max_pw) {   // the reference would use part -1
-              c1 = c2 = z;
-              stop = true;
-              break;
-            }
-            if (d2 != d) {
-              // the old decision appended to every net, or the new one to none:
-              // no new claim; else the new appends are claimed
-              const bool safe = napp == deg || (!cn && cand_count(B, K, o, d2) == deg);
-              if (!safe) {
-                claim_appends(I, B, vz, round, z, d2, sd);
-                reclaim = true;
-              }
-              if (lane == 0) {
-                B.dec[o] = d2;
-                B.flag[o] = 1;   // its records are d's: located again at commit
-                if (w) B.mlist[lds(&B.midx[o])].z = d2;
-                B.stats[9]++;
-              }
-            }
-            __syncwarp();
-            if (lane == 0 && w) sz[d2] += w;
-            __syncwarp();
-          }
-        }
-        if (lane == 0) {
-          B.ctl[6] = c1;
-          B.ctl[7] = c2;
-        }
-      }
+      // ---- B2: walk from the first change to the conflict with the exact sizes
+      // (block 0); the changed positions' warps and CTAs record their slots and
+      // claims again; the rest of the window is checked against the claims
+      if (blockIdx.x == 0)
+        walk_window<true>(I, B, sizes_s, Cf, tv, false, pos, zf, zc, lds(&B.mcnt[par]), walk_s,
+                          reinterpret_cast<int*>(penf), dsz_cta);
       if (!grid_barrier(B.bar, I.status)) return;
       lap(20);
-      cut = lds(&B.ctl[6]);
-      cutc = lds(&B.ctl[7]);
-      // the placements before each CTA's positions, with the changed decisions
-      for (int p = threadIdx.x; p < K; p += blockDim.x) dsz_cta[p] = 0;
-      __syncthreads();
-      const int nm = lds(&B.mcnt[par]);
-      for (int i = threadIdx.x; i < nm; i += blockDim.x) {
-        const int4 m = lds(&B.mlist[i]);
-        if (m.x < cta_o0) atomicAdd(&dsz_cta[m.z], m.y);
+      const int hard = lds(&B.ctl[0]);
+      const int lim = hard == kNone ? zc : min(hard >> 3, zc);
+      if (stats) B.stats[9] += lds(&B.ctl[1]);
+      auto redo = [&](int z, int n0, int n1, uint32_t base, bool first_warp) {
+        const int o = z - pos;
+        if (!(lds(&B.flag[o]) & 128)) return;
+        const int d = lds(&B.dfix[o]) & 0xffff;
+        record_slots(I, B, S, base, n0, n1, d, round, z, sd, cn && lds(&B.ncand[o]) == 0);
+        if (first_warp && lane == 0) {
+          B.dec[o] = (K << 16) | d;
+          const int w = lds(&B.wt[o]);
+          if (w) B.mlist[lds(&B.midx[o])] = make_int4(o, w, (K << 16) | d, 0);
+        }
+      };
+      for (int z = max(z0, zf); z < min(z1, lim); z++) {
+        if (__ldg(&S.pclass[z]) != 0) continue;
+        const int v = __ldg(&S.porder[z]);
+        const uint32_t base = __ldg(&I.vptr[v]);
+        int n0, n1;
+        warp_nets((int)(__ldg(&I.vptr[v + 1]) - base), &n0, &n1);
+        redo(z, n0, n1, base, owner);
       }
-      __syncthreads();
+      for_mid(zf, lim, [&](int, int z, int, uint32_t base, int, int c0, int c1) {
+        int n0, n1;
+        net_range(c1 - c0, wib, kSWarps, &n0, &n1);
+        redo(z, c0 + n0, c0 + n1, base, c0 == 0 && wib == 0);
+      });
+      if (!grid_barrier(B.bar, I.status)) return;
+      check_claims(zf, lim, [](int) {});
+      if (!grid_barrier(B.bar, I.status)) return;
+      lap(20);
+      const int cw2 = lds(cut_w);
+      cut = cutc = cw2 == kNone ? lim : min(cw2 >> 3, lim);
+      placed_before();   // with the changed decisions
     }
     if (cut <= pos) {
       // the window's first position needs a part above max_pw: the reference
@@ -716,21 +764,40 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
       return;
     }
     // ---- C: commit the positions before the cut (and a flip at the cut)
+    auto place = [&](int z, uint32_t base, int n0, int n1) {
+      const int d = (z == cut ? lds(&B.dfix[z - pos]) : lds(&B.dec[z - pos])) & 0xffff;
+      if (z == cut) {
+        for (int nb = n0; nb < n1; nb += 32) {
+          const int j = locate_part(I, base, nb, n1, d, sd);
+          if (nb + lane < n1) place_net(I, (int)__ldg(&I.vnets[base + nb + lane]), d, j);
+        }
+      } else {
+        for (int k = n0 + lane; k < n1; k += 32)
+          place_net(I, (int)__ldg(&I.vnets[base + k]), d, (int)lds(&S.rec[base + k]));
+      }
+    };
+    for_mid(pos, cutc, [&](int, int z, int, uint32_t base, int, int c0, int c1) {
+      int n0, n1;
+      net_range(c1 - c0, wib, kSWarps, &n0, &n1);
+      place(z, base, c0 + n0, c0 + n1);
+    });
+    if (teams)
+      for (int i = gtid; i < nmid * K; i += gthreads) {
+        B.hcnt[i] = 0;
+        B.hfirst[i] = ~0ull;
+      }
     for (int z = z0; z < min(z1, cutc); z++) {
       const int o = z - pos;
       const int v = __ldg(&S.porder[z]);
       const uint32_t base = __ldg(&I.vptr[v]);
       const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
-      const int d = z == cut ? lds(&B.dfix[o]) : lds(&B.dec[o]);
-      if (z == cut || lds(&B.flag[o])) {
-        for (int nb = 0; nb < deg; nb += 32) {
-          const int j = locate_part(I, base, nb, deg, d, sd);
-          if (nb + lane < deg) place_net(I, (int)__ldg(&I.vnets[base + nb + lane]), d, j);
-        }
-      } else {
-        for (int k = lane; k < deg; k += 32)
-          place_net(I, (int)__ldg(&I.vnets[base + k]), d, (int)lds(&S.rec[base + k]));
+      const int d = (z == cut ? lds(&B.dfix[o]) : lds(&B.dec[o])) & 0xffff;
+      if (__ldg(&S.pclass[z]) == 0) {
+        int n0, n1;
+        warp_nets(deg, &n0, &n1);
+        place(z, base, n0, n1);
       }
+      if (!owner) continue;
       if (!cn) {
         const unsigned long long* cl = B.cand + (size_t)o * K;
         const int nc = lds(&B.ncand[o]);
@@ -746,14 +813,13 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
       // the vertices without nets between the committed positions: the
       // least-loaded part of the exact sizes at their place
       const int zb = min(z1, cutc);
-      if (z0 < zb || (pos == 0 && gw == 0)) {
-        const int cta_o0 = min(pos + blockIdx.x * kSWarps * q, end_w) - pos;
+      if ((owner && z0 < zb) || (pos == 0 && gw == 0)) {
         int* sz = cnt;
         for (int p = lane; p < K; p += 32) sz[p] = sizes_s[p] + dsz_cta[p];
         __syncwarp();
         for (int o2 = cta_o0 + lane; o2 < z0 - pos; o2 += 32) {
           const int w = lds(&B.wt[o2]);
-          if (w) atomicAdd(&sz[lds(&B.dec[o2])], w);
+          if (w) atomicAdd(&sz[lds(&B.dec[o2]) & 0xffff], w);
         }
         __syncwarp();
         int amin = -1;
@@ -763,7 +829,7 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
           const int w = lds(&B.wt[o]);
           if (w) {
             __syncwarp();
-            if (lane == 0) sz[z == cut ? lds(&B.dfix[o]) : lds(&B.dec[o])] += w;
+            if (lane == 0) sz[(z == cut ? lds(&B.dfix[o]) : lds(&B.dec[o])) & 0xffff] += w;
             __syncwarp();
             amin = -1;
           }
@@ -785,7 +851,9 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
     if (cutc >= end_w) {
       if (end_w == pos + W) W = min(2 * W, B.wmax);
     } else {
-      W = max(256, min(B.wmax, 2 * (cutc - pos)));
+      // at least 64: 256 takes 2% longer (more positions to wait for), and the
+      // next window grows where this one was all valid
+      W = max(64, min(B.wmax, 2 * (cutc - pos)));
     }
     pos = cutc;
     round++;
@@ -1561,8 +1629,8 @@ __global__ void stream_conn_masks_kernel(DevInstance I) {
 
 size_t stream_smem_bytes(int K) {
   auto a = [](size_t n) { return (n + 15) & ~size_t(15); };
-  return 2 * a(sizeof(int) * K) + a(sizeof(int) * (size_t)K * kSWarps) +
-         a(sizeof(unsigned long long) * (size_t)K * kSWarps) + a(sizeof(int) * 32 * kSWarps);
+  const size_t eval = 2 * a(sizeof(int) * (size_t)K * kSWarps);
+  return a(sizeof(int) * K) + 2 * a(sizeof(int) * (K + 1)) + std::max(eval, sizeof(WalkSmem));
 }
 
 size_t stream_msg_smem_bytes(int K) {
