@@ -704,6 +704,7 @@ int fp_instance_create(fp_ctx* ctx, const fp_hypergraph* h, int32_t K, int32_t m
     const bool msg = metric == FP_METRIC_TM || metric == FP_METRIC_MSM;
     const bool cn = metric == FP_METRIC_CN;
     const bool ldg = !msg && !cn;
+    const bool volm = metric == FP_METRIC_MSV || metric == FP_METRIC_MSRV;
     // exact count claims of the LDG engine: a table well above the entries of a
     // round (two per count-only net of a window's movers)
     size_t ctab = 4096;
@@ -722,6 +723,9 @@ int fp_instance_create(fp_ctx* ctx, const fp_hypergraph* h, int32_t K, int32_t m
         (rc = dalloc(in, &in->sb.ctl, kCtlWords)) || (rc = dalloc(in, &in->sb.bar, 4)) || (rc = dalloc(in, &in->sb.stats, kNumStats)) || (rc = dalloc(in, &in->sb.dec, std::max(kSpecWindow, kMsgWindow))) ||
         (rc = dalloc(in, &in->sb.flag, kSpecWindow)) || (rc = dalloc(in, &in->sb.slack, kSpecWindow)) ||
         (rc = dalloc(in, &in->sb.vslack, kSpecWindow)) || (rc = dalloc(in, &in->sb.wt, kSpecWindow)) ||
+        (rc = dalloc(in, &in->sb.vn, volm ? kSpecWindow : 1)) ||
+        (rc = dalloc(in, &in->sb.vterm, volm ? (size_t)kSpecWindow * kVolTerms : 1)) ||
+        (rc = dalloc(in, &in->sb.vpart, volm ? (size_t)kSpecWindow * kVolTerms : 1)) ||
         (rc = dalloc(in, &in->sb.vd, kSpecWindow)) || (rc = dalloc(in, &in->sb.scan, (size_t)kSpecWindow * words)) ||
         (rc = dalloc(in, &in->sb.rgain, std::max(kSpecWindow, kMsgWindow))) ||
         (rc = dalloc(in, &in->sb.rloss, std::max(kSpecWindow, kMsgWindow))) ||
@@ -849,6 +853,7 @@ int fp_instance_footprint(int32_t nov, int32_t noe, int64_t pins, int32_t K, int
     const bool msg = metric == FP_METRIC_TM || metric == FP_METRIC_MSM;
     const bool cn = metric == FP_METRIC_CN;
     const bool ldg = !msg && !cn;
+    const bool volm = metric == FP_METRIC_MSV || metric == FP_METRIC_MSRV;
     size_t ctab = 4096;
     while (ctab < (size_t)2 * noe && ctab < ((size_t)1 << 21)) ctab <<= 1;
     const size_t P = (size_t)pins, V = (size_t)nov, E = (size_t)noe, G2K = 2 * (size_t)kMaxGridVerts * K;
@@ -865,6 +870,7 @@ int fp_instance_footprint(int32_t nov, int32_t noe, int64_t pins, int32_t K, int
     // speculation scratch
     add(kCtlWords, 4); add(4, 4); add(kNumStats, 8); add(std::max(kSpecWindow, kMsgWindow), 4);
     add(W, 1); add(W, 4); add(W, 4); add(W, 4); add(W, 4);   // flag, slack, vslack, wt, vd
+    add(volm ? W : 1, 4); add(volm ? W * kVolTerms : 1, 8); add(volm ? W * kVolTerms : 1, 2);   // vn, vterm, vpart
     add(W * words, 4);                                       // scan
     add(std::max(kSpecWindow, kMsgWindow), 4); add(std::max(kSpecWindow, kMsgWindow), 4);   // rgain, rloss
     add(ldg ? P : 1, 4); add(ldg ? P : 1, 8);                // rec, rec_slot

@@ -84,6 +84,7 @@ constexpr int kStreamHeavy = 4096;   // nets of a vertex the whole grid places i
 // 262144 (and 8192 nets).
 constexpr long long kStreamCtaWork = 4096;
 constexpr long long kStreamGridWork = 65536;
+constexpr int kVolTerms = 64;         // parts whose volumes a listed decision touches at most
 constexpr int kStreamMaxK = 1024;    // shared memory of the device stream's CTAs
 constexpr int kMsgStreamCta = 1024;  // nets of a vertex one CTA places alone in the message-greedy stream
 
@@ -114,6 +115,10 @@ struct SpecBuf {
   int* vslack;           // [wmax] volume drift the accept/reject outcome tolerates
   int* wt;               // [wmax] vertex weight (streams: of the placed vertex)
   int* vd;               // [wmax] largest volume change of one part by a mover
+  int* vn;               // [wmax] volume terms of a decision that leaves its part (-1: more
+                         //     than kVolTerms)
+  int2* vterm;           // [wmax * kVolTerms] (loss - gain, exact change) of a part's volume
+  unsigned short* vpart; // [wmax * kVolTerms] that part (MSV / MSRV)
   int* rgain;            // [wmax] decision-record gain / loss of each window offset (with
   int* rloss;            //     the decision log on)
   uint32_t* scan;        // [wmax * words] parts scanned per window offset (TV)

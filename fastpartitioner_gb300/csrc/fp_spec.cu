@@ -14,10 +14,13 @@
 //                 changed: no earlier mover of the window changed the part set
 //                 of one of its nets, or the count of its own part there; the
 //                 weight moved before it stays within its size slack (the LDG
-//                 argmax, its tie-breaks and TV's clamps cannot flip); the
-//                 volumes stay within its volume slack; if it would leave its
-//                 part, no earlier mover touched a max-volume part; for TV, no
-//                 stale marker can apply.  The first invalid position cuts the
+//                 argmax, its tie-breaks and TV's clamps cannot flip); if it
+//                 would leave its part, MSV's / MSRV's accept test comes out
+//                 the same with the volumes and max-volume parts that the
+//                 earlier movers leave (taken again from the decision's listed
+//                 terms where they drifted beyond its slack or the max parts
+//                 changed); for TV, no stale marker can apply.  The first
+//                 invalid position cuts the
 //                 window.  Decisions that the size drift changes do not: they are
 //                 taken again -- a few in a long window all at once, otherwise by
 //                 a walk of one CTA over the positions in order (walk_window) --
@@ -305,11 +308,11 @@ __device__ __forceinline__ void claim_nets(const DevInstance& I, const SpecBuf& 
   }
 }
 
-// Appends a mover of window offset o (weight wv, largest volume change vd) to
-// the round's list.
-__device__ __forceinline__ void list_mover(const SpecBuf& B, int par, int o, int wv, int pk, int vd) {
+// Appends a mover of window offset o (weight wv, vn volume terms) to the
+// round's list.
+__device__ __forceinline__ void list_mover(const SpecBuf& B, int par, int o, int wv, int pk, int vn) {
   const int i = atomicAdd(&B.mcnt[par], 1);
-  B.mlist[i] = make_int4(o, wv, pk, vd);
+  B.mlist[i] = make_int4(o, wv, pk, vn);
   B.midx[o] = i;
 }
 
@@ -399,6 +402,85 @@ __device__ AcceptPart accept_partial(const RoundCtx& R, const int* gains, const 
   return a;
 }
 
+// The volume terms of window offset o (a decision that leaves its part): the
+// parts with a loss or gain or an exact change, in part order; one warp.
+// Returns their number, -1 if there are more than kVolTerms.
+__device__ int store_terms(const SpecBuf& B, int o, int K, const int* gains, const int* losses, const int* adelta) {
+  const int lane = threadIdx.x & 31;
+  int n = 0;
+  for (int p0 = 0; p0 < K; p0 += 32) {
+    const int p = p0 + lane;
+    const int df = p < K ? losses[p] - gains[p] : 0, ad = p < K ? adelta[p] : 0;
+    const unsigned m = __ballot_sync(kAll, df != 0 || ad != 0);
+    const int i = n + __popc(m & ((1u << lane) - 1u));
+    if (((m >> lane) & 1u) && i < kVolTerms) {
+      B.vterm[(size_t)o * kVolTerms + i] = make_int2(df, ad);
+      B.vpart[(size_t)o * kVolTerms + i] = (unsigned short)p;
+    }
+    n += __popc(m);
+  }
+  if (n > kVolTerms) n = -1;
+  if (lane == 0) B.vn[o] = n;
+  return n;
+}
+
+// Max-volume parts while the window's movers are applied: state x holds after x
+// of the movers that change the set (kVolEvents at most; the window ends at the
+// next).  Outcomes rarely change with the volumes (none in a pass of the Zipf
+// workloads, 2 on 10,000 mixed vertices), but a bound on the drift (the sum of the
+// movers' largest changes) and every change of a max part used to end the
+// window: 548 -> 145 windows per pass on 10,000 mixed vertices under MSV (K =
+// 64), 25.9 -> 17.5 ms; MSRV on 262144 Zipf vertices (K = 256) 244 -> 112, 15.5
+// -> 10.0 ms; MSV there 1546 -> 1220.
+constexpr int kVolEvents = 15;   // (kVolEvents + 1) * ceil(K / 32) <= 8 * K for K >= 2
+struct VolStates {
+  int n;                       // such movers found
+  int at[kVolEvents];          // their window offsets
+  int maxv[kVolEvents + 1], nm[kVolEvents + 1], count[kVolEvents + 1];
+  int over;                    // offset of the first mover without listed terms
+  int end;                     // first offset whose max parts are not known
+  int ne, next, m2, chg, add, off;   // scratch
+};
+
+// The accept test of window offset o (one warp) from its listed terms with the
+// max parts `bits` (nm of them, volume maxv) and the other volumes vx(p),
+// computed on the first call.  MGV/partition.cpp:339-362 and
+// MSRV/partition.cpp:352-376 over the parts the move touches: an untouched max
+// part fails MSRV's test; an untouched other part reaches maxv only under
+// MSRV, whose changes differ from gain and loss by the source's own pin.
+template <class Build, class Vx>
+__device__ bool accept_terms(const SpecBuf& B, int o, int n, int K, bool rv, const uint32_t* bits, int nm, int maxv,
+                             Build&& build, Vx&& vx) {
+  const int lane = threadIdx.x & 31;
+  bool fail = false, other = false;
+  int neg = 0;
+  for (int t = lane; t < n; t += 32) {
+    const int p = (int)__ldcg(&B.vpart[(size_t)o * kVolTerms + t]);
+    const int df = __ldcg(&B.vterm[(size_t)o * kVolTerms + t].x);
+    if ((bits[p >> 5] >> (p & 31)) & 1u) {
+      if (rv ? df >= 0 : df > 0) fail = true;
+      else neg++;
+    } else {
+      other = true;
+    }
+  }
+  if (__any_sync(kAll, fail)) return false;
+  if (rv && warp_sum(neg) != nm) return false;
+  if (!rv && !__any_sync(kAll, other)) return true;
+  build();
+  int high = 0;
+  for (int t = lane; t < n; t += 32) {
+    const int p = (int)__ldcg(&B.vpart[(size_t)o * kVolTerms + t]);
+    const int df = __ldcg(&B.vterm[(size_t)o * kVolTerms + t].x);
+    if ((bits[p >> 5] >> (p & 31)) & 1u) continue;
+    if (vx(p) + df >= maxv) fail = true;
+    high -= vx(p) >= maxv;
+  }
+  if (rv)
+    for (int p = lane; p < K; p += 32) high += !((bits[p >> 5] >> (p & 31)) & 1u) && vx(p) >= maxv;
+  return !__any_sync(kAll, fail) && (!rv || warp_sum(high) == 0);
+}
+
 // Outcome and volume slack: accepted -> stays accepted while no non-max part
 // rises by more than msl; rejected on a max part -> local, stays rejected;
 // rejected only on non-max parts -> stays rejected while the worst of them
@@ -484,7 +566,7 @@ __device__ void cta_eval_ldg(const DevInstance& I, const SpecBuf& B, const Round
   const bool special = sh[1] != 0;
   const int slack = sh[2];
   bool mover = false, mt = false;
-  int vs = kBig, vdd = 0;
+  int vs = kBig, vdd = 0, nt = 0;
   int rg = 0, rl = 0;   // decision record (with the log on)
   if (d != own) {
     // TV moves iff the leave gain covers the arrival loss; MSV / MSRV need the
@@ -506,6 +588,7 @@ __device__ void cta_eval_ldg(const DevInstance& I, const SpecBuf& B, const Round
         const int fsl = block_reduce_max(a.fsl, iscr);
         const int msl = block_reduce_min(a.msl, iscr);
         vdd = block_reduce_max(a.vd, iscr);
+        if (wib == 0) nt = store_terms(B, o, K, gains_b, losses_b, adelta_b);
         bool good;
         accept_final(fM, fN, fsl, msl, &good, &vs);
         mover = good;
@@ -523,7 +606,7 @@ __device__ void cta_eval_ldg(const DevInstance& I, const SpecBuf& B, const Round
     claim_nets(I, B, vol, z, own, d, base, deg, threadIdx.x, blockDim.x, par);
     if (threadIdx.x == 0) {
       if (mt) atomicMin(&B.ctl[2 + par], z);
-      list_mover(B, par, o, __ldg(&I.w[v]), (own << 16) | d, vdd);
+      list_mover(B, par, o, __ldg(&I.w[v]), (own << 16) | d, nt);
     }
   }
   if (threadIdx.x == 0) {
@@ -581,11 +664,12 @@ __device__ void fix_position(const DevInstance& I, const SpecBuf& B, const Round
     __syncwarp();
   }
   bool mover = false, mt = false, good = (fl & 16) != 0;
-  int vs = kBig, vdd = 0;
+  int vs = kBig, vdd = 0, nt = 0;
   int rg = 0, rl = 0;
   if (deg == 0) {
     mover = d != own && (!vol || good);
     vs = lds(&B.vslack[o]);
+    if (vol && lane == 0) B.vn[o] = 0;
   } else if (d != own) {
     if (vol) {
       for (int p = lane; p < K; p += 32) { gains[p] = 0; losses[p] = 0; adelta[p] = 0; }
@@ -601,6 +685,7 @@ __device__ void fix_position(const DevInstance& I, const SpecBuf& B, const Round
       mover = good;
       mt = mover && __any_sync(kAll, a.mt);
       vdd = warp_max(a.vd);
+      nt = store_terms(B, o, K, gains, losses, adelta);
       if (logp) {
         for (int p = lane; p < K; p += 32) { rg += gains[p]; rl += losses[p]; }
         rg = warp_sum(rg);
@@ -621,8 +706,8 @@ __device__ void fix_position(const DevInstance& I, const SpecBuf& B, const Round
     if (logp) { B.rgain[o] = rg; B.rloss[o] = rl; }
     if (mover != (fx >> 16 != 0)) atomicMin(&B.ctl[8], z);
     const int wv = mover ? __ldg(&I.w[v]) : 0;
-    if (had) B.mlist[lds(&B.midx[o])] = make_int4(o, wv, (own << 16) | d, mover ? vdd : 0);   // the replaced mover's entry
-    else if (mover) list_mover(B, par, o, wv, (own << 16) | d, vdd);
+    if (had) B.mlist[lds(&B.midx[o])] = make_int4(o, wv, (own << 16) | d, mover ? nt : 0);   // the replaced mover's entry
+    else if (mover) list_mover(B, par, o, wv, (own << 16) | d, nt);
     B.dec[o] = (own << 16) | d;
     B.flag[o] = (unsigned char)((fl & (2 | 8 | 64)) | (mover ? 1 : 0) | (good ? 16 : 0) | 32 | (had && deg > 0 ? 64 : 0));
     B.vslack[o] = vs;
@@ -651,6 +736,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
   __shared__ int s_gdec[kMaxGridVerts], s_gspec[kMaxGridVerts], s_gslk[kMaxGridVerts], s_gcnt[kMaxGridVerts];
   __shared__ int s_t0[kMaxGridVerts], s_t1[kMaxGridVerts];   // their teams of CTAs
   __shared__ int loc_b[kSWarps * 96];   // per-warp locate scratch
+  __shared__ VolStates vs_s;
   const int metric = I.metric;
   const bool vol = metric != kTV;
   const bool rv = metric == kMSRV;
@@ -794,8 +880,11 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
       int ns = 0;
       while (ns < B.gmax && hidx + ns < B.nheavy && __ldg(&B.heavy_pos[hidx + ns]) < end_w) ns++;
       const int span = end_w - pos;
+      // (a short window fills the first CTAs' warps: spread over all CTAs it kept
+      // those of the medium vertices waiting, MSRV 51.6 -> 59 us per window)
       const int q = (span + nwarps - 1) / nwarps;
-      const int z0 = min(pos + gw * q, end_w);
+      const int cta_o0 = min((int)blockIdx.x * kSWarps * q, span);
+      const int z0 = pos + min(gw * q, span);
       const int z1 = min(z0 + q, end_w);
       const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = gridDim.x * blockDim.x;
       const int hp = heavy_round & 1;   // whole-grid tallies, double-buffered by parity
@@ -887,7 +976,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         // destination (all gains and losses are zero).
         const bool iso = deg == 0;
         bool mover = false, mt = false, good = metric == kTV;
-        int vs = kBig, vdd = 0;
+        int vs = kBig, vdd = 0, nt = 0;
         if (metric == kTV) {
           if (d != own) {
             mover = c1 >= deg - cnt[d];
@@ -906,6 +995,8 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
           mover = good && d != own;
           mt = mover && __any_sync(kAll, a.mt);
           vdd = warp_max(a.vd);
+          if (d != own && deg) nt = store_terms(B, o, K, gains, losses, adelta);
+          else if (lane == 0) B.vn[o] = 0;
         }
         __syncwarp();
         if (logp) {
@@ -928,7 +1019,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
           claim_nets(I, B, vol, z, own, d, base, deg, lane, 32, par);
           if (lane == 0) {
             if (mt) atomicMin(&B.ctl[2 + par], z);
-            list_mover(B, par, o, __ldg(&I.w[v]), (own << 16) | d, vdd);
+            list_mover(B, par, o, __ldg(&I.w[v]), (own << 16) | d, nt);
           }
         }
         if (lane == 0) {
@@ -1030,7 +1121,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
           const bool need = d != own_s &&
                             (metric == kTV ? lds(&B.hmisc[hmslot(j)]) >= deg_s - s_gcnt[j] : true);
           bool mover = metric == kTV && need, mt = false;
-          int vs = kBig, vdd = 0;
+          int vs = kBig, vdd = 0, nt = 0;
           int rg = 0, rl = 0;   // decision record (with the log on)
           if (metric == kTV && d != own_s) {
             rg = lds(&B.hmisc[hmslot(j)]);
@@ -1050,6 +1141,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
             const int fsl = block_reduce_max(a.fsl, iscr);
             const int msl = block_reduce_min(a.msl, iscr);
             vdd = block_reduce_max(a.vd, iscr);
+            if (leads(j) && wib == 0) nt = store_terms(B, os, K, gains_b, losses_b, adelta_b);
             bool good;
             accept_final(fM, fN, fsl, msl, &good, &vs);
             mover = good;
@@ -1072,7 +1164,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
             B.acc[os] = lds(&B.hmisc[hmslot(j)]) - deg_s;
             B.vd[os] = mover ? vdd : 0;
             if (mover && mt) atomicMin(&B.ctl[2 + par], zs);
-            if (mover) list_mover(B, par, os, __ldg(&I.w[vsup]), (own_s << 16) | d, vdd);
+            if (mover) list_mover(B, par, os, __ldg(&I.w[vsup]), (own_s << 16) | d, nt);
           }
           __syncthreads();
         }
@@ -1096,39 +1188,199 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
       // receives the drift it tolerates beyond the window's movers as they are
       // (-2: its decision changes).
       int* const cut_w = &B.ctl[4 + par];
-      const int cta_o0 = min(pos + blockIdx.x * kSWarps * q, end_w) - pos;
-      int* dsz_cta = gains_b;   // (the evaluation's arrays are free here)
-      // the size changes (in dsz) and volume drift (returned) of the window's
-      // movers before offset o; every thread of the CTA
-      auto moved_before = [&](int o, int* dsz) {
-        for (int p = threadIdx.x; p < K; p += blockDim.x) dsz[p] = 0;
+      // (the evaluation's arrays are free here)
+      int* dsz_cta = gains_b;
+      uint32_t* vbits = reinterpret_cast<uint32_t*>(losses_b);   // max parts, words per state
+      int* dv_cta = adelta_b;                                    // volume changes before this CTA's positions,
+      int* vol_x = adelta_b + K;                                 //   volumes at the last change of the max parts,
+      int* dv_big = adelta_b + 2 * K;                            //   changes before a CTA's or the grid's vertex
+      // the movers' terms (offset << 12 | part, change): behind the evaluation's
+      // arrays where the walk's words reach beyond them, or in the half of the
+      // sighting keys that only whole-grid vertices use; 1600 at least
+      const int tail = (int)(sizeof(WalkSmem) / 8 + K / 2) - (int)((adelta_b + (size_t)K * kSWarps - cnt_b + 1) / 2) - 1;
+      const bool behind = tail > K * (kSWarps / 2);
+      int2* const stage = reinterpret_cast<int2*>(behind ? adelta_b + (((size_t)K * kSWarps + 3) & ~size_t(3))
+                                                         : (int*)first_b + (((size_t)K * kSWarps + 1) & ~size_t(1)));
+      const int stage_cap = behind ? tail - 2 : K * (kSWarps / 2);
+      // the size changes (in dsz) and, with dv, the volume changes of the
+      // window's movers before offset o (listed terms only: no position beyond the
+      // first mover without them is taken); every thread of the CTA
+      auto moved_before = [&](int o, int* dsz, int* dv) {
+        for (int p = threadIdx.x; p < K; p += blockDim.x) {
+          dsz[p] = 0;
+          if (dv) dv[p] = 0;
+        }
         __syncthreads();
         const int nm = lds(&B.mcnt[par]);
-        long long x = 0;
         for (int i = threadIdx.x; i < nm; i += blockDim.x) {
           const int4 m = lds(&B.mlist[i]);
           if (m.x >= o) continue;
-          x += m.w;
-          if (m.y == 0) continue;
-          atomicAdd(&dsz[m.z & 0xffff], m.y);
-          atomicAdd(&dsz[m.z >> 16], -m.y);
-        }
-        if (vol) {
-          x = warp_sum64(x);
-          if (lane == 0) uscr[wib] = (unsigned long long)x;
-          __syncthreads();
-          x = 0;
-          for (int y = 0; y < kSWarps; y++) x += (long long)uscr[y];
+          if (m.y != 0) {
+            atomicAdd(&dsz[m.z & 0xffff], m.y);
+            atomicAdd(&dsz[m.z >> 16], -m.y);
+          }
+          if (dv)
+            for (int t = 0; t < m.w; t++) {
+              const int ad = __ldcg(&B.vterm[(size_t)m.x * kVolTerms + t].y);
+              if (ad) atomicAdd(&dv[(int)__ldcg(&B.vpart[(size_t)m.x * kVolTerms + t])], ad);
+            }
         }
         __syncthreads();
-        return x;
+      };
+      // The max-volume parts between the window's movers (vs_s, vbits): applies
+      // the movers in order up to each one that changes the set.  MSV scans anew
+      // after every move (MGV/partition.cpp:453-472): only a move that touches a
+      // max part changes it, as no other part reaches the maximum.  MSRV scans
+      // when a listed part is off the old maximum (MSRV/partition.cpp:486-513),
+      // after any move once that holds.  Every CTA does it for itself.
+      auto vol_states = [&]() {
+        const int nm = lds(&B.mcnt[par]);
+        if (threadIdx.x == 0) {
+          vs_s.n = 0;
+          vs_s.over = kNone;
+          vs_s.end = kNone;
+          vs_s.maxv[0] = s_maxv;
+          vs_s.count[0] = s_count;
+        }
+        for (int w = wib; w < words; w += kSWarps) {
+          const int p = w * 32 + lane;
+          const unsigned m = __ballot_sync(kAll, p < K && mark_s[p] == s_cc);
+          if (lane == 0) vbits[w] = m;
+        }
+        for (int p = threadIdx.x; p < K; p += blockDim.x) vol_x[p] = vol_s[p];
+        __syncthreads();
+        int ovm = kNone, nmk = 0, off = 0;
+        for (int i = threadIdx.x; i < nm; i += blockDim.x) {
+          const int4 m = lds(&B.mlist[i]);
+          if (m.w < 0) ovm = min(ovm, m.x);
+        }
+        if (ovm != kNone) atomicMin(&vs_s.over, ovm);
+        for (int w = 0; w < words; w++) nmk += __popc(vbits[w]);
+        if (threadIdx.x == 0) vs_s.nm[0] = nmk;
+        if (rv)
+          for (int p = threadIdx.x; p < K; p += blockDim.x)
+            off |= mark_s[p] == s_cc && vol_s[p] != s_maxv;
+        off = __syncthreads_or(off);
+        if (lds(&B.ctl[2 + par]) == kNone && !off) return;   // no mover touches a max part
+        // the movers' terms, unordered (half the window at a time where they do
+        // not fit)
+        int lim = min(vs_s.over, span);
+        while (true) {
+          if (threadIdx.x == 0) vs_s.ne = 0;
+          __syncthreads();
+          for (int i = threadIdx.x; i < nm; i += blockDim.x) {
+            const int4 m = lds(&B.mlist[i]);
+            if (m.x >= lim || m.w <= 0 || !(lds(&B.flag[m.x]) & 1)) continue;
+            const int at = atomicAdd(&vs_s.ne, m.w);
+            for (int t = 0; t < m.w && at + t < stage_cap; t++)
+              stage[at + t] = make_int2((m.x << 12) | (int)__ldcg(&B.vpart[(size_t)m.x * kVolTerms + t]),
+                                        __ldcg(&B.vterm[(size_t)m.x * kVolTerms + t].y));
+          }
+          __syncthreads();
+          if (vs_s.ne <= stage_cap) break;
+          lim = max(1, lim / 2);
+          if (threadIdx.x == 0) vs_s.end = lim;
+          __syncthreads();
+        }
+        const int ne = vs_s.ne;
+        if (threadIdx.x == 0) {
+          vs_s.next = kNone;
+          vs_s.m2 = -2147483647 - 1;
+          vs_s.chg = vs_s.add = vs_s.off = 0;
+        }
+        __syncthreads();
+        int last = -1;
+        for (int x = 0;; x++) {
+          const uint32_t* bits = vbits + x * words;
+          auto marked = [&](int p) { return ((bits[p >> 5] >> (p & 31)) & 1u) != 0; };
+          int nx = kNone;
+          for (int i = threadIdx.x; i < ne; i += blockDim.x) {
+            const int2 t = stage[i];
+            const int o = t.x >> 12;
+            if (o > last && o < nx && (off || (t.y != 0 && marked(t.x & 0xfff)))) nx = o;
+          }
+          nx = warp_min(nx);
+          if (lane == 0 && nx != kNone) atomicMin(&vs_s.next, nx);
+          __syncthreads();
+          nx = vs_s.next;
+          if (nx == kNone) break;
+          if (x == kVolEvents) {
+            if (threadIdx.x == 0) vs_s.end = min(vs_s.end, nx);
+            break;
+          }
+          for (int i = threadIdx.x; i < ne; i += blockDim.x) {
+            const int2 t = stage[i];
+            if ((t.x >> 12) > last && (t.x >> 12) <= nx && t.y) atomicAdd(&vol_x[t.x & 0xfff], t.y);
+          }
+          __syncthreads();
+          last = nx;
+          if (threadIdx.x == 0) {
+            vs_s.next = kNone;
+            vs_s.add = vs_s.off = vs_s.nm[x + 1] = 0;
+          }
+          const int mv0 = vs_s.maxv[x];
+          int m2 = -2147483647 - 1;
+          bool chg = !rv;
+          for (int p = threadIdx.x; p < K; p += blockDim.x) {
+            m2 = max(m2, vol_x[p]);
+            if (marked(p) && vol_x[p] != mv0) chg = true;
+          }
+          m2 = warp_max(m2);
+          chg = __any_sync(kAll, chg);
+          if (lane == 0) {
+            atomicMax(&vs_s.m2, m2);
+            if (chg) vs_s.chg = 1;
+          }
+          __syncthreads();
+          m2 = vs_s.m2;
+          chg = vs_s.chg != 0;
+          const bool fresh = !rv || (chg && m2 > mv0), more = rv && chg && m2 == mv0;
+          const int mv1 = fresh ? m2 : mv0;
+          for (int w = wib; w < words; w += kSWarps) {
+            const int p = w * 32 + lane;
+            const unsigned m = __ballot_sync(kAll, p < K && vol_x[p] == m2);
+            const unsigned b = fresh ? m : more ? bits[w] | m : bits[w];
+            const bool o2 = __any_sync(kAll, rv && p < K && ((b >> lane) & 1u) && vol_x[p] != mv1);
+            if (lane == 0) {
+              vbits[(x + 1) * words + w] = b;
+              atomicAdd(&vs_s.nm[x + 1], __popc(b));
+              atomicAdd(&vs_s.add, __popc(m));
+              if (o2) vs_s.off = 1;
+            }
+          }
+          __syncthreads();
+          off = vs_s.off;
+          if (threadIdx.x == 0) {
+            vs_s.at[x] = nx;
+            vs_s.maxv[x + 1] = mv1;
+            vs_s.count[x + 1] = fresh ? vs_s.add : vs_s.count[x] + (more ? vs_s.add : 0);
+            vs_s.n = x + 1;
+            vs_s.m2 = -2147483647 - 1;
+            vs_s.chg = 0;
+          }
+        }
+        __syncthreads();
       };
       auto validate = [&](int zfrom, int zto, bool sizes, int* flip_w, int* nflip_w) {
-        const int mtpos = lds(&B.ctl[2 + par]);
         const bool ov = lds(&B.ctab_over[par]) != 0;
+        if (vol) {
+          vol_states();
+          // the window ends behind a mover without listed terms, and at a change
+          // of the max parts beyond those kept
+          if (blockIdx.x == 0 && threadIdx.x == 0) {
+            if (vs_s.over != kNone) atomicMin(cut_w, ((pos + vs_s.over + 1) << 3) | 3);
+            if (vs_s.end != kNone) atomicMin(cut_w, ((pos + vs_s.end) << 3) | 4);
+          }
+        }
+        auto vol_state = [&](int o) {   // of the max parts before offset o
+          int x = 0;
+          while (x < vs_s.n && vs_s.at[x] < o) x++;
+          return x;
+        };
         if (sizes || vol) {
           // the movers before this warp's first position
-          long long Vw = moved_before(cta_o0, dsz_cta);
+          moved_before(cta_o0, dsz_cta, vol ? dv_cta : nullptr);
+          long long Vw = 0;
           long long Dw = 0;
           if (z0 < z1) {
             int D0 = 0, wi = 0, vi = 0;
@@ -1138,7 +1390,11 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
               if (vol) vi += lds(&B.vd[o]);
             }
             Dw = (long long)warp_max(D0) + (unsigned)warp_sum(wi);
-            if (vol) Vw += warp_sum(vi);
+            if (vol) {
+              int V0 = 0;
+              for (int p = lane; p < K; p += 32) V0 = max(V0, abs(dv_cta[p]));
+              Vw = (long long)warp_max(V0) + warp_sum(vi);
+            }
           }
           for (int z = z0; z < min(z1, zto); z++) {
             const int o = z - pos;
@@ -1181,10 +1437,36 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
                 B.rel[o] = max(slk, 0) - (int)Dw;
                 if (fl & 128) B.flag[o] = (unsigned char)(fl & 127);
               }
-              // the max-volume parts enter only the accept test of a vertex whose
-              // decision leaves its part (MSRV/partition.cpp:308-400,
-              // MGV/partition.cpp:292-362), and they change only with a move
-              int why = ((fl & 2) && z != pos) ? 1 : Vw > max(vslk, 0) ? 3 : (mtpos < z && (pk & 0xffff) != own) ? 4 : 0;
+              // the volumes enter only the accept test of a vertex whose decision
+              // leaves its part (MSRV/partition.cpp:308-400, MGV/partition.cpp:
+              // 292-362): taken again where the max parts changed or the others
+              // drifted beyond what it tolerates
+              int why = ((fl & 2) && z != pos) ? 1 : 0;
+              if (vol && !why && (pk & 0xffff) != own) {
+                const int x = vol_state(o);
+                if (x || Vw > max(vslk, 0)) {
+                  const int nt = lds(&B.vn[o]);
+                  int* vx = (int*)first;
+                  const bool good = nt >= 0 && accept_terms(
+                      B, o, nt, K, rv, vbits + x * words, vs_s.nm[x], vs_s.maxv[x],
+                      [&]() {
+                        for (int p = lane; p < K; p += 32) vx[p] = vol_s[p] + dv_cta[p];
+                        __syncwarp();
+                        for (int o2 = cta_o0; o2 < o; o2++)
+                          if (lds(&B.flag[o2]) & 1) {
+                            const int n2 = lds(&B.vn[o2]);
+                            for (int t = lane; t < n2; t += 32) {
+                              const int ad = __ldcg(&B.vterm[(size_t)o2 * kVolTerms + t].y);
+                              if (ad) atomicAdd(&vx[(int)__ldcg(&B.vpart[(size_t)o2 * kVolTerms + t])], ad);
+                            }
+                          }
+                        __syncwarp();
+                      },
+                      [&](int p) { return vx[p]; });
+                  if (nt < 0 || good != ((fl & 1) != 0)) why = nt < 0 && x ? 4 : 3;
+                  __syncwarp();
+                }
+              }
               if (!why) {
                 const int c = conflicts(I, B, vol, z, own, (pk & 0xffff) != own, fl & 1, base, deg, lane, 32, ov);
                 const int c5 = __any_sync(kAll, c == 5), c6 = __any_sync(kAll, c == 6), c7 = __any_sync(kAll, c == 7);
@@ -1234,8 +1516,20 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
             why = ((fl & 2) && z != pos) ? 1 : 0;
             if (sizes || vol) {
               __syncthreads();   // dsz_cta and cnt_b are read
-              const long long Vz = moved_before(o, cnt_b);
-              if (!why) why = Vz > max(lds(&B.vslack[o]), 0) ? 3 : (mtpos < z && leaves) ? 4 : 0;
+              moved_before(o, cnt_b, vol ? dv_big : nullptr);
+              if (vol && !why && leaves && wib == 0) {
+                const int x = vol_state(o);
+                int V0 = 0;
+                for (int p = lane; p < K; p += 32) V0 = max(V0, abs(dv_big[p]));
+                if (x || warp_max(V0) > max(lds(&B.vslack[o]), 0)) {
+                  const int nt = lds(&B.vn[o]);
+                  const bool good = nt >= 0 && accept_terms(
+                      B, o, nt, K, rv, vbits + x * words, vs_s.nm[x], vs_s.maxv[x], []() {},
+                      [&](int p) { return vol_s[p] + dv_big[p]; });
+                  // (only the first thread reports it, below)
+                  if (nt < 0 || good != ((fl & 1) != 0)) why = nt < 0 && x ? 4 : 3;
+                }
+              }
               if (sizes && wib == 0) {
                 int D0 = 0;
                 for (int p = lane; p < K; p += 32) D0 = max(D0, abs(cnt_b[p]));
@@ -1356,7 +1650,6 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         if (threadIdx.x == 0) dev_fail(I.status, kDevErrInvalid);
         return;
       }
-      const int mt_c = lds(&B.ctl[2 + par]);
       if (logp) {
         // decision records of this warp's committed positions
         for (int z = z0 + lane; z < min(z1, cut); z += 32) {
@@ -1448,7 +1741,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         // there they are walked only for the decision records).
         int* dsz = gains_b;   // the committed movers' size changes before this CTA's first position
         __syncthreads();
-        moved_before(cta_o0, dsz);
+        moved_before(cta_o0, dsz, nullptr);
         const int zb = min(z1, cut);
         if (z0 < zb) {
           int* sz = cnt;   // this warp's sizes, at its current position
@@ -1557,7 +1850,29 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         B.mcnt[par ^ 1] = 0;
         B.ctab_over[par ^ 1] = 0;
       }
-      prev_maxtouch = mt_c < cut;
+      if (rv) {
+        // MSRV's list of max parts after the committed movers; a last one without
+        // listed terms is left to the next round's scan
+        __syncthreads();
+        int x = 0, c = 0;
+        while (x < vs_s.n && pos + vs_s.at[x] < cut) {
+          x++;
+          c = max(c, vs_s.count[x]);
+        }
+        prev_maxtouch = vs_s.over != kNone && pos + vs_s.over < cut;
+        const int cc0 = s_cc;
+        __syncthreads();
+        if (x) {
+          for (int p = threadIdx.x; p < K; p += blockDim.x)
+            mark_s[p] = (vbits[x * words + (p >> 5)] >> (p & 31)) & 1u ? cc0 : -1;
+          if (threadIdx.x == 0) {
+            s_maxv = vs_s.maxv[x];
+            s_count = vs_s.count[x];
+            if (c > K) dev_fail(I.status, kDevErrUnsupported);   // the reference overruns max_parts
+          }
+        }
+        __syncthreads();
+      }
       if (cut == end_w) {
         if (end_w == pos + W) W = min(2 * W, B.wmax);
       } else {
