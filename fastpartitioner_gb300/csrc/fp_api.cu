@@ -95,7 +95,7 @@ int default_grid_verts(int metric) {
   }
 }
 constexpr int kMaxSpecWarps = 16384;
-constexpr int kCtlWords = 12;   // SpecBuf::ctl
+constexpr int kCtlWords = 16;   // SpecBuf::ctl
 cudaError_t launch_metrics(const DevInstance& I, void* scratch, long long* out, int num_sms, cudaStream_t st,
                            int* launches);
 }  // namespace fp
@@ -733,7 +733,7 @@ int fp_instance_create(fp_ctx* ctx, const fp_hypergraph* h, int32_t K, int32_t m
         (rc = dalloc(in, &in->sb.ctab_key, ldg ? ctab : 1)) || (rc = dalloc(in, &in->sb.ctab_pos, ldg ? ctab : 1)) ||
         (rc = dalloc(in, &in->sb.ctab_cnt, ldg ? ctab : 1)) ||
         (rc = dalloc(in, &in->sb.ctab_over, 2)) || (rc = dalloc(in, &in->sb.dfix, kSpecWindow)) ||
-        (rc = dalloc(in, &in->sb.rec_slot2, ldg ? g.pins : 1)) ||
+        (rc = dalloc(in, &in->sb.rlist, ldg ? kReplaced : 1)) ||
         (rc = dalloc(in, &in->sb.cn_moved, cn ? g.pins : 1)) || (rc = dalloc(in, &in->sb.cn_kcnt, cn ? g.noe : 1)) ||
         (rc = dalloc(in, &in->sb.cn_nets, cn ? g.noe : 1)) || (rc = dalloc(in, &in->sb.cn_more, cn ? g.pins : 1)) || (rc = dalloc(in, &in->sb.cn_cnt, 6)) ||
         (rc = dalloc(in, &in->sb.cn_wit, cn ? g.nov : 1)) || (rc = dalloc(in, &in->vclass_d, g.nov)) ||
@@ -876,7 +876,7 @@ int fp_instance_footprint(int32_t nov, int32_t noe, int64_t pins, int32_t K, int
     add(ldg ? P : 1, 4); add(ldg ? P : 1, 8);                // rec, rec_slot
     add(ldg ? ctab : 1, 8); add(ldg ? ctab : 1, 4); add(ldg ? ctab : 1, 4);
     add(2, 4); add(W, 4);                                    // ctab_over, dfix
-    add(ldg ? P : 1, 8);                                     // rec_slot2
+    add(ldg ? kReplaced : 1, 16);                            // rlist
     add(cn ? P : 1, 8); add(cn ? E : 1, 4); add(cn ? E : 1, 8); add(cn ? P : 1, 8); add(6, 4); add(cn ? V : 1, 4);
     add(V, 1);                                               // vertex classes
     add(W * K, 8); add(W, 4); add(W, 16); add(W, 4); add(2, 4);   // cand, ncand, mlist, midx, mcnt
@@ -933,7 +933,7 @@ static int device_stream(fp_instance* in) {
   const int K = in->pb.K;
   DevInstance& d = in->d;
   static const int none[kCtlWords] = {0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff,
-                                      0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0, 0};
+                                      0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0, 0, 0, 0, 0, 0};
   cudaError_t e = cudaMemsetAsync(d.part_vec, 0xff, sizeof(int) * g.nov, s);
   auto zero = [&](void* p, size_t bytes, int val) {
     if (e == cudaSuccess && bytes) e = cudaMemsetAsync(p, val, bytes, s);
@@ -1078,7 +1078,7 @@ int fp_refine(fp_instance* in, int32_t passes) {
     in->recs_valid = false;
     if (spec) {
       static const int none[kCtlWords] = {0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff,
-                                      0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0, 0};
+                                      0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0, 0, 0, 0, 0, 0};
       if (e == cudaSuccess) e = cudaMemcpyAsync(in->sb.ctl, none, sizeof(none), cudaMemcpyHostToDevice, s);
       if (e == cudaSuccess) e = cudaMemsetAsync(in->sb.bar, 0, sizeof(unsigned) * 4, s);
       if (e == cudaSuccess && (in->fault_leave_at || in->fault_poll_limit)) {

@@ -84,6 +84,7 @@ constexpr int kStreamHeavy = 4096;   // nets of a vertex the whole grid places i
 // 262144 (and 8192 nets).
 constexpr long long kStreamCtaWork = 4096;
 constexpr long long kStreamGridWork = 65536;
+constexpr int kReplaced = 1 << 18;     // claims of replaced moves a window holds
 constexpr int kVolTerms = 64;         // parts whose volumes a listed decision touches at most
 constexpr int kStreamMaxK = 1024;    // shared memory of the device stream's CTAs
 constexpr int kMsgStreamCta = 1024;  // nets of a vertex one CTA places alone in the message-greedy stream
@@ -99,14 +100,16 @@ constexpr int kCnGridNets = 8;   // nets the whole grid evaluates in one CN wind
 // instance.
 struct SpecBuf {
   unsigned* bar;         // [4] grid barrier: arrivals, generation, abort
-  int* ctl;              // [12] [2,3] first max-touching mover, [4,5] cut (by round parity),
+  int* ctl;              // [16] [2,3] first max-touching mover, [4,5] cut (by round parity),
                          //     [6,7] first changed decision, [10,11] their number (by
                          //     validation parity), [0,1] the walk's end and changes, [8]
-                         //     first outcome it mispredicted, [9] first change without room
+                         //     first outcome it mispredicted, [9] first change without room,
+                         //     [12,13] counts are committed first, [14,15] entries of
+                         //     rlist (by round parity)
   int* dec;              // [wmax] (own part << 16) | decision per window offset
   unsigned char* flag;   // [wmax] bit0 mover, bit1 stale-marker risk, bit2 CTA / grid evaluated,
                          //     bit3 no nets, bit4 accepted, bit5 decision changed in the
-                         //     window, bit6 claims of a replaced move held (rec_slot2),
+                         //     window, bit6 unused,
                          //     bit7 the decision changes (dfix)
   int* dfix;             // [wmax] the changed decision; the walk's with (predicted mover << 16)
   int* slack;            // [wmax] part-size drift the decision tolerates (-1: none)
@@ -150,7 +153,8 @@ struct SpecBuf {
   int* ctab_pos;         // [ctab_mask + 1] first position of a count-only mover with that (net, part)
   int* ctab_cnt;         // [ctab_mask + 1] count-only movers of the round on that (net, part)
   uint2* rec_slot;       // [pins] table slots of a count-only move's (net, own) and (net, new part)
-  uint2* rec_slot2;      // [pins] those of a move that a changed decision replaced
+  int4* rlist;           // [kReplaced] claims of the moves that changed decisions replaced
+                         //     (net or -1, its two entries of the table), until the commit
   int* ctab_over;        // [2] a probe ran past its bound this round (by round parity)
   unsigned ctab_mask;
   const int* heavy_pos;  // positions (visiting order, ascending) of vertices evaluated by

@@ -321,25 +321,40 @@ __device__ __forceinline__ void ctab_clear(const SpecBuf& B, uint2 sl) {
   if (sl.y != ~0u) { B.ctab_key[sl.y] = ~0ull; B.ctab_pos[sl.y] = kNone; B.ctab_cnt[sl.y] = 0; }
 }
 
-// Clears the claims of a vertex on its nets k0, k0 + kstep, ... (commit phase):
-// cur, those of its current move (its records and rec_slot); old, those of a
-// move an in-window fix replaced (rec_slot2).
+// Clears the claims of a mover on its nets k0, k0 + kstep, ... (commit phase).
+__device__ __forceinline__ void unclaim_net(const SpecBuf& B, int e) {
+  B.claim_m[e] = kNone;
+  B.claim_c[e] = kNone;
+  B.mask_c[e] = 0;
+}
 __device__ __forceinline__ void unclaim_nets(const DevInstance& I, const SpecBuf& B, bool vol, uint32_t base, int deg,
-                                             int k0, int kstep, bool cur = true, bool old = false) {
+                                             int k0, int kstep) {
   for (int k = k0; k < deg; k += kstep) {
-    const int e = (int)__ldg(&I.vnets[base + k]);
-    B.claim_m[e] = kNone;
-    B.claim_c[e] = kNone;
-    B.mask_c[e] = 0;
-    if (cur && !rec_setchange(lds(&B.rec[base + k]), vol)) ctab_clear(B, lds(&B.rec_slot[base + k]));
-    if (old) ctab_clear(B, lds(&B.rec_slot2[base + k]));
+    unclaim_net(B, (int)__ldg(&I.vnets[base + k]));
+    if (!rec_setchange(lds(&B.rec[base + k]), vol)) ctab_clear(B, lds(&B.rec_slot[base + k]));
   }
+}
+
+// Lists the claims of a move about to be replaced, entries [at, at + deg) of
+// rlist (nets k0, k0 + kstep, ...); false if they do not fit.  The claims stay
+// until the commit: a superset keeps every later check conservative.
+__device__ __forceinline__ bool list_replaced(const DevInstance& I, const SpecBuf& B, bool vol, uint32_t base, int deg,
+                                              int k0, int kstep, int at) {
+  const bool fits = at + deg <= kReplaced;
+  for (int k = k0; k < deg && at + k < kReplaced; k += kstep) {
+    const uint2 sl = !fits || rec_setchange(lds(&B.rec[base + k]), vol) ? make_uint2(~0u, ~0u)
+                                                                        : lds(&B.rec_slot[base + k]);
+    B.rlist[at + k] = make_int4(fits ? (int)__ldg(&I.vnets[base + k]) : -1, (int)sl.x, (int)sl.y, 0);
+  }
+  return fits;
 }
 
 // Did an earlier mover of the window change something the vertex at z read on
 // its nets k0, k0 + kstep, ...?  0: nothing; 5: a part set; 6: the count of
-// z's own part where it matters; 7: z (a mover) changes the part set of a net
-// whose counts an earlier mover changes.
+// z's own part where it matters.  *after: z (a mover) changes the part set of a
+// net whose counts an earlier mover changes, so the counts are committed first
+// (a barrier more; the window used to end at z, 31 of 145 windows per pass on
+// 10,000 mixed vertices under MSV and 176 of 1220 on 262144 Zipf vertices).
 //
 // Counts enter a decision only through "own has exactly one pin on the net",
 // and only when the vertex would move (cand: decision != own; its move records
@@ -347,7 +362,7 @@ __device__ __forceinline__ void unclaim_nets(const DevInstance& I, const SpecBuf
 // earlier count-only moves can make it 1 only if c == 1 or if at least c - 1
 // of the round's count-only movers touch (net, own).
 __device__ __forceinline__ int conflicts(const DevInstance& I, const SpecBuf& B, bool vol, int z, int own,
-                                         bool cand, bool mover, uint32_t base, int deg, int k0, int kstep, bool ov) {
+                                         bool cand, bool mover, uint32_t base, int deg, int k0, int kstep, bool ov, bool* after) {
   const unsigned ob = 1u << (own & 31);
   int conf = 0;
   for (int k = k0; k < deg && !conf; k += kstep) {
@@ -371,7 +386,7 @@ __device__ __forceinline__ int conflicts(const DevInstance& I, const SpecBuf& B,
         }
       }
       if (hit) conf = 6;
-      else if (mover && rec_setchange(lds(&B.rec[base + k]), vol)) conf = 7;
+      else if (mover && rec_setchange(lds(&B.rec[base + k]), vol)) *after = true;
     }
   }
   return conf;
@@ -612,7 +627,7 @@ __device__ void cta_eval_ldg(const DevInstance& I, const SpecBuf& B, const Round
   if (threadIdx.x == 0) {
     if (logp) { B.rgain[o] = rg; B.rloss[o] = rl; }
     B.dec[o] = (own << 16) | d;
-    B.flag[o] = (unsigned char)((mover ? 1 : 0) | (special ? 2 : 0) | 4);
+    B.flag[o] = (unsigned char)((mover ? 1 : 0) | (special ? 2 : 0) | 4 | (!vol || mover ? 16 : 0));
     B.slack[o] = slack;
     B.vslack[o] = vs;
     B.wt[o] = __ldg(&I.w[v]);
@@ -632,11 +647,9 @@ __device__ void cta_eval_ldg(const DevInstance& I, const SpecBuf& B, const Round
 
 // The position z (window offset o) whose decision the last walk changed: the
 // move records, the accept test and the claims are redone for the new
-// decision.  The replaced move's claims stay (a superset keeps every later
-// check conservative); their table slots go to rec_slot2 for the commit, so a
-// second replaced move ends the window here instead (ctl[9]).  An outcome
-// other than the walk predicted lowers ctl[8]: the decisions after it are
-// validated again.
+// decision.  The replaced move's claims stay (list_replaced; where they do not
+// fit, the window ends here instead, ctl[9]).  An outcome other than the walk
+// predicted lowers ctl[8]: the decisions after it are validated again.
 // One warp, the one owning position z.
 __device__ void fix_position(const DevInstance& I, const SpecBuf& B, const RoundCtx& R, int metric, int z, int o,
                              int fl, int par, int* loc, int* gains, int* losses, int* adelta, bool logp) {
@@ -650,17 +663,15 @@ __device__ void fix_position(const DevInstance& I, const SpecBuf& B, const Round
   const int fx = lds(&B.dfix[o]);
   const int d = fx & 0xffff;
   const bool had = (fl & 1) != 0;
-  if (had && (fl & 64)) {
-    if (lane == 0) {
-      atomicMin(&B.ctl[9], (z << 3) | 2);
-      B.flag[o] = (unsigned char)(fl & ~128);
+  if (had && deg) {
+    const int at = __shfl_sync(kAll, lane == 0 ? atomicAdd(&B.ctl[14 + par], deg) : 0, 0);
+    if (!list_replaced(I, B, vol, base, deg, lane, 32, at)) {
+      if (lane == 0) {
+        atomicMin(&B.ctl[9], (z << 3) | 2);
+        B.flag[o] = (unsigned char)(fl & ~128);
+      }
+      return;
     }
-    return;
-  }
-  if (had) {
-    for (int k = lane; k < deg; k += 32)
-      B.rec_slot2[base + k] =
-          rec_setchange(lds(&B.rec[base + k]), vol) ? make_uint2(~0u, ~0u) : lds(&B.rec_slot[base + k]);
     __syncwarp();
   }
   bool mover = false, mt = false, good = (fl & 16) != 0;
@@ -709,11 +720,86 @@ __device__ void fix_position(const DevInstance& I, const SpecBuf& B, const Round
     if (had) B.mlist[lds(&B.midx[o])] = make_int4(o, wv, (own << 16) | d, mover ? nt : 0);   // the replaced mover's entry
     else if (mover) list_mover(B, par, o, wv, (own << 16) | d, nt);
     B.dec[o] = (own << 16) | d;
-    B.flag[o] = (unsigned char)((fl & (2 | 8 | 64)) | (mover ? 1 : 0) | (good ? 16 : 0) | 32 | (had && deg > 0 ? 64 : 0));
+    B.flag[o] = (unsigned char)((fl & (2 | 8)) | (mover ? 1 : 0) | (good ? 16 : 0) | 32);
     B.vslack[o] = vs;
     B.vd[o] = mover ? vdd : 0;
   }
   __syncwarp();
+}
+
+// The same for a medium vertex or one of the whole grid, by one CTA (deg > 0).
+__device__ void cta_fix(const DevInstance& I, const SpecBuf& B, const RoundCtx& R, int metric, int z, int o, int fl,
+                        int par, int* loc_b, int* gains_b, int* losses_b, int* adelta_b, int* iscr, bool logp) {
+  const int wib = threadIdx.x >> 5;
+  const bool vol = metric != kTV, rv = metric == kMSRV;
+  const int K = I.K;
+  const int v = __ldg(&B.porder[z]);
+  const uint32_t base = __ldg(&I.vptr[v]);
+  const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
+  const int own = lds(&B.dec[o]) >> 16;
+  const int fx = lds(&B.dfix[o]);
+  const int d = fx & 0xffff;
+  const bool had = (fl & 1) != 0;
+  if (had) {
+    if (threadIdx.x == 0) iscr[0] = atomicAdd(&B.ctl[14 + par], deg);
+    __syncthreads();
+    if (!list_replaced(I, B, vol, base, deg, threadIdx.x, blockDim.x, iscr[0])) {
+      if (threadIdx.x == 0) {
+        atomicMin(&B.ctl[9], (z << 3) | 2);
+        B.flag[o] = (unsigned char)(fl & ~128);
+      }
+      return;
+    }
+    __syncthreads();
+  }
+  if (vol)
+    for (int p = threadIdx.x; p < K; p += blockDim.x) { gains_b[p] = 0; losses_b[p] = 0; adelta_b[p] = 0; }
+  __syncthreads();
+  bool mover = false, mt = false;
+  int vs = kBig, vdd = 0, nt = 0, rg = 0, rl = 0;
+  if (d != own) {
+    const int ra = locate_all(I, B, metric, v, own, d, base, deg, wib, kSWarps, loc_b + wib * 96, gains_b, losses_b,
+                              adelta_b);
+    __syncthreads();
+    if (vol) {
+      const AcceptPart a = accept_partial(R, gains_b, losses_b, adelta_b, K, rv, threadIdx.x, blockDim.x);
+      const bool fM = __syncthreads_or(a.failM);
+      const bool fN = __syncthreads_or(a.failN);
+      const bool amt = __syncthreads_or(a.mt);
+      const int fsl = block_reduce_max(a.fsl, iscr);
+      const int msl = block_reduce_min(a.msl, iscr);
+      vdd = block_reduce_max(a.vd, iscr);
+      if (wib == 0) nt = store_terms(B, o, K, gains_b, losses_b, adelta_b);
+      accept_final(fM, fN, fsl, msl, &mover, &vs);
+      mt = mover && amt;
+      if (logp) {
+        int g = 0, l = 0;
+        for (int p = threadIdx.x; p < K; p += blockDim.x) { g += gains_b[p]; l += losses_b[p]; }
+        rg = block_reduce_sum(g, iscr);
+        rl = block_reduce_sum(l, iscr);
+      }
+    } else {
+      rg = block_reduce_sum(ra & 0xffff, iscr);
+      rl = block_reduce_sum(ra >> 16, iscr);
+      mover = rg >= rl;
+    }
+  }
+  if (mover) {
+    claim_nets(I, B, vol, z, own, d, base, deg, threadIdx.x, blockDim.x, par);
+    if (threadIdx.x == 0 && mt) atomicMin(&B.ctl[2 + par], z);
+  }
+  if (threadIdx.x == 0) {
+    if (logp) { B.rgain[o] = rg; B.rloss[o] = rl; }
+    if (mover != (fx >> 16 != 0)) atomicMin(&B.ctl[8], z);
+    const int wv = mover ? __ldg(&I.w[v]) : 0;
+    if (had) B.mlist[lds(&B.midx[o])] = make_int4(o, wv, (own << 16) | d, mover ? nt : 0);
+    else if (mover) list_mover(B, par, o, wv, (own << 16) | d, nt);
+    B.dec[o] = (own << 16) | d;
+    B.flag[o] = (unsigned char)((fl & (2 | 4)) | (mover ? 1 : 0) | (!vol || mover ? 16 : 0) | 32);
+    B.vslack[o] = vs;
+    B.vd[o] = mover ? vdd : 0;
+  }
+  __syncthreads();
 }
 
 // Changed decisions are taken at once, not walked, in a stretch longer than
@@ -1157,7 +1243,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
           if (leads(j) && threadIdx.x == 0) {
             if (logp) { B.rgain[os] = rg; B.rloss[os] = rl; }
             B.dec[os] = (own_s << 16) | d;
-            B.flag[os] = (unsigned char)((mover ? 1 : 0) | (s_gspec[j] ? 2 : 0) | 4);
+            B.flag[os] = (unsigned char)((mover ? 1 : 0) | (s_gspec[j] ? 2 : 0) | 4 | (!vol || mover ? 16 : 0));
             B.slack[os] = s_gslk[j];
             B.vslack[os] = vs;
             B.wt[os] = __ldg(&I.w[vsup]);
@@ -1363,6 +1449,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
       };
       auto validate = [&](int zfrom, int zto, bool sizes, int* flip_w, int* nflip_w) {
         const bool ov = lds(&B.ctab_over[par]) != 0;
+        bool after = false;
         if (vol) {
           vol_states();
           // the window ends behind a mover without listed terms, and at a change
@@ -1468,9 +1555,9 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
                 }
               }
               if (!why) {
-                const int c = conflicts(I, B, vol, z, own, (pk & 0xffff) != own, fl & 1, base, deg, lane, 32, ov);
-                const int c5 = __any_sync(kAll, c == 5), c6 = __any_sync(kAll, c == 6), c7 = __any_sync(kAll, c == 7);
-                why = c5 ? 5 : c6 ? 6 : c7 ? 7 : 0;
+                const int c = conflicts(I, B, vol, z, own, (pk & 0xffff) != own, fl & 1, base, deg, lane, 32, ov, &after);
+                const int c5 = __any_sync(kAll, c == 5), c6 = __any_sync(kAll, c == 6);
+                why = c5 ? 5 : c6 ? 6 : 0;
               }
               if (why) {
                 if (lane == 0) atomicMin(cut_w, (z << 3) | why);   // position, then cut reason
@@ -1491,9 +1578,9 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
             const int own = pk >> 16;
             int why = ((fl & 2) && z != pos) ? 1 : 0;
             if (!why) {
-              const int c = conflicts(I, B, vol, z, own, (pk & 0xffff) != own, fl & 1, base, deg, lane, 32, ov);
-              const int c5 = __any_sync(kAll, c == 5), c6 = __any_sync(kAll, c == 6), c7 = __any_sync(kAll, c == 7);
-              why = c5 ? 5 : c6 ? 6 : c7 ? 7 : 0;
+              const int c = conflicts(I, B, vol, z, own, (pk & 0xffff) != own, fl & 1, base, deg, lane, 32, ov, &after);
+              const int c5 = __any_sync(kAll, c == 5), c6 = __any_sync(kAll, c == 6);
+              why = c5 ? 5 : c6 ? 6 : 0;
             }
             if (why) {
               if (lane == 0) atomicMin(cut_w, (z << 3) | why);
@@ -1535,7 +1622,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
                 for (int p = lane; p < K; p += 32) D0 = max(D0, abs(cnt_b[p]));
                 D0 = warp_max(D0);
                 const int slk = max(lds(&B.slack[o]), 0);
-                if (D0 > slk) {
+                if (D0 > slk || (fl & 32)) {
                   for (int p = lane; p < K; p += 32) cnt_b[p] += sizes_s[p];
                   __syncwarp();
                   int ns1;
@@ -1544,19 +1631,22 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
                   if (lane == 0) {
                     if (flip) {
                       atomicMin(flip_w, (z << 3) | 2);
-                      atomicAdd(nflip_w, kJacobiFlips + 1);   // the walk's: it ends the window there
+                      atomicAdd(nflip_w, kJacobiFlips + 1);   // the walk's
+                    } else if (fl & 128) {
+                      B.flag[o] = (unsigned char)(fl & 127);
                     }
                     B.rel[o] = flip ? -2 : ns1;
                   }
                 } else if (lane == 0) {
                   B.rel[o] = slk - D0;
+                  if (fl & 128) B.flag[o] = (unsigned char)(fl & 127);
                 }
               }
               __syncthreads();
             }
           }
           if (!why || grid) {
-            const int c = conflicts(I, B, vol, z, own, leaves, fl & 1, base, deg, k0, kstep, ov);
+            const int c = conflicts(I, B, vol, z, own, leaves, fl & 1, base, deg, k0, kstep, ov, &after);
             if (c) atomicMin(cut_w, (z << 3) | c);
           }
           if (why && threadIdx.x == 0) atomicMin(cut_w, (z << 3) | why);
@@ -1572,6 +1662,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
           if (z >= zto) break;
           if (z >= zfrom && in_team(j)) check_big(z, team_tid(j), team_threads(j), leads(j), true);
         }
+        if (after) B.ctl[12 + par] = 1;
       };
       // ---- B: validate; while decisions change, take the changes and validate
       // again from the first one.  Long stretches with few changes take them all
@@ -1620,8 +1711,23 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         // the changed positions redone by their warps
         for (int z = max(z0, zf); z < min(z1, hard == kNone ? zc : min(zc, hard >> 3)); z++) {
           const int fl = lds(&B.flag[z - pos]);
-          if (fl & 128)
+          if ((fl & 132) == 128)
             fix_position(I, B, R, metric, z, z - pos, fl, par, loc, gains, losses, adelta, logp);
+        }
+        __syncthreads();
+        for (int mi = mi0; mi < mend; mi += gridDim.x) {
+          const int z = __ldg(&B.mid_pos[mi]);
+          if (z >= (hard == kNone ? zc : min(zc, hard >> 3))) break;
+          const int fl = z >= zf ? lds(&B.flag[z - pos]) : 0;
+          __syncthreads();   // every thread has read the flag
+          if (fl & 128) cta_fix(I, B, R, metric, z, z - pos, fl, par, loc_b, gains_b, losses_b, adelta_b, iscr, logp);
+        }
+        for (int j = 0; j < ns; j++) {   // a whole-grid vertex by the first CTA of its team
+          const int z = s_gz[j];
+          if (!leads(j) || z < zf || z >= (hard == kNone ? zc : min(zc, hard >> 3))) continue;
+          const int fl = lds(&B.flag[z - pos]);
+          __syncthreads();
+          if (fl & 128) cta_fix(I, B, R, metric, z, z - pos, fl, par, loc_b, gains_b, losses_b, adelta_b, iscr, logp);
         }
         if (!grid_barrier(B.bar, I.status)) return;
         // a walk whose outcomes came as predicted leaves exact sizes; else the
@@ -1659,78 +1765,80 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
               make_int4(lds(&B.dec[o]) & 0xffff, lds(&B.rgain[o]), lds(&B.rloss[o]), fl & 1);
         }
       }
-      for (int z = z0; z < z1; z++) {
-        const int o = z - pos;
-        const int fl = lds(&B.flag[o]);
-        if (!(fl & (1 | 64)) || (fl & 4)) continue;   // claims held: a mover or a replaced mover
-        const int v = __ldg(&B.porder[z]);
-        const int pk = lds(&B.dec[o]);
-        const int own = pk >> 16, d = pk & 0xffff;
-        const uint32_t base = __ldg(&I.vptr[v]);
-        const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
-        if ((fl & 1) && z < cut) {
-          for (int k = lane; k < deg; k += 32)
-            commit_rec(I, v, own, d, (int)__ldg(&I.vnets[base + k]), lds(&B.rec[base + k]), vol ? &V : nullptr);
-          if (lane == 0) {
-            atomicAdd(&B.stats[2], 1ull);
-            I.part_vec[v] = d;
-            const int wv = __ldg(&I.w[v]);
-            atomicAdd(&I.part_sizes[own], -wv);
-            atomicAdd(&I.part_sizes[d], wv);
-            atomicAdd((unsigned long long*)&I.moves[it], 1ull);
-          }
-        }
-        unclaim_nets(I, B, vol, base, deg, lane, 32, fl & 1, fl & 64);
+      // the committed movers' nets [k0, step): all of them, or (counts_first) the
+      // count-only ones and, behind a barrier, those whose part set changes
+      const bool counts_first = lds(&B.ctl[12 + par]) != 0;
+      for (int i = gtid, n = min(lds(&B.ctl[14 + par]), kReplaced); i < n; i += gthreads) {
+        const int4 x = lds(&B.rlist[i]);
+        if (x.x < 0) continue;
+        unclaim_net(B, x.x);
+        ctab_clear(B, make_uint2((unsigned)x.y, (unsigned)x.z));
       }
-      for (int mi = mi0; mi < mend; mi += gridDim.x) {
-        const int z = __ldg(&B.mid_pos[mi]);
-        const int o = z - pos;
-        const int fl = lds(&B.flag[o]);
-        if (!(fl & 1)) continue;
-        const int v = __ldg(&B.porder[z]);
-        const int pk = lds(&B.dec[o]);
-        const int own = pk >> 16, d = pk & 0xffff;
-        const uint32_t base = __ldg(&I.vptr[v]);
-        const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
-        if (z < cut) {
-          for (int k = threadIdx.x; k < deg; k += blockDim.x)
-            commit_rec(I, v, own, d, (int)__ldg(&I.vnets[base + k]), lds(&B.rec[base + k]), vol ? &V : nullptr);
-          if (threadIdx.x == 0) {
-            atomicAdd(&B.stats[2], 1ull);
-            I.part_vec[v] = d;
-            const int wv = __ldg(&I.w[v]);
-            atomicAdd(&I.part_sizes[own], -wv);
-            atomicAdd(&I.part_sizes[d], wv);
-            atomicAdd((unsigned long long*)&I.moves[it], 1ull);
+      for (int ph = counts_first ? 1 : 0;; ph++) {
+        auto commit_nets = [&](int v, int own, int d, uint32_t base, int deg, int k0, int kstep) {
+          for (int k = k0; k < deg; k += kstep) {
+            const uint32_t rc = lds(&B.rec[base + k]);
+            if (ph == 0 || rec_setchange(rc, vol) == (ph == 2))
+              commit_rec(I, v, own, d, (int)__ldg(&I.vnets[base + k]), rc, vol ? &V : nullptr);
           }
+        };
+        auto commit_vertex = [&](int v, int own, int d) {
+          atomicAdd(&B.stats[2], 1ull);
+          I.part_vec[v] = d;
+          const int wv = __ldg(&I.w[v]);
+          atomicAdd(&I.part_sizes[own], -wv);
+          atomicAdd(&I.part_sizes[d], wv);
+          atomicAdd((unsigned long long*)&I.moves[it], 1ull);
+        };
+        for (int z = z0; z < z1; z++) {
+          const int o = z - pos;
+          const int fl = lds(&B.flag[o]);
+          if ((fl & 5) != 1) continue;   // a mover that a warp evaluated
+          const int v = __ldg(&B.porder[z]);
+          const int pk = lds(&B.dec[o]);
+          const int own = pk >> 16, d = pk & 0xffff;
+          const uint32_t base = __ldg(&I.vptr[v]);
+          const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
+          if (z < cut) {
+            commit_nets(v, own, d, base, deg, lane, 32);
+            if (ph != 1 && lane == 0) commit_vertex(v, own, d);
+          }
+          if (ph != 1) unclaim_nets(I, B, vol, base, deg, lane, 32);
         }
-        unclaim_nets(I, B, vol, base, deg, threadIdx.x, blockDim.x);
-      }
-      for (int j = 0; j < ns; j++) {
-        // a whole-grid vertex, by its team
-        if (!in_team(j)) continue;
-        const int tt = team_tid(j), tn = team_threads(j);
-        const int zs = s_gz[j], vsup = s_gv[j], own_s = s_go[j], deg_s = s_gd[j];
-        const uint32_t base_s = s_gb[j];
-        const int os = zs - pos;
-        if (lds(&B.flag[os]) & 1) {
-          const int pk = lds(&B.dec[os]);
-          const int d = pk & 0xffff;
-          if (zs < cut) {
-            for (int i = tt; i < deg_s; i += tn)
-              commit_rec(I, vsup, own_s, d, (int)__ldg(&I.vnets[base_s + i]), lds(&B.rec[base_s + i]),
-                         vol ? &V : nullptr);
-            if (tt == 0) {
-              atomicAdd(&B.stats[2], 1ull);
-              I.part_vec[vsup] = d;
-              const int wv = __ldg(&I.w[vsup]);
-              atomicAdd(&I.part_sizes[own_s], -wv);
-              atomicAdd(&I.part_sizes[d], wv);
-              atomicAdd((unsigned long long*)&I.moves[it], 1ull);
+        for (int mi = mi0; mi < mend; mi += gridDim.x) {
+          const int z = __ldg(&B.mid_pos[mi]);
+          const int o = z - pos;
+          const int fl = lds(&B.flag[o]);
+          if (!(fl & 1)) continue;
+          const int v = __ldg(&B.porder[z]);
+          const int pk = lds(&B.dec[o]);
+          const int own = pk >> 16, d = pk & 0xffff;
+          const uint32_t base = __ldg(&I.vptr[v]);
+          const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
+          if (z < cut) {
+            commit_nets(v, own, d, base, deg, threadIdx.x, blockDim.x);
+            if (ph != 1 && threadIdx.x == 0) commit_vertex(v, own, d);
+          }
+          if (ph != 1) unclaim_nets(I, B, vol, base, deg, threadIdx.x, blockDim.x);
+        }
+        for (int j = 0; j < ns; j++) {
+          // a whole-grid vertex, by its team
+          if (!in_team(j)) continue;
+          const int tt = team_tid(j), tn = team_threads(j);
+          const int zs = s_gz[j], vsup = s_gv[j], own_s = s_go[j], deg_s = s_gd[j];
+          const uint32_t base_s = s_gb[j];
+          const int os = zs - pos;
+          if (lds(&B.flag[os]) & 1) {
+            const int d = lds(&B.dec[os]) & 0xffff;
+            if (zs < cut) {
+              commit_nets(vsup, own_s, d, base_s, deg_s, tt, tn);
+              if (ph != 1 && tt == 0) commit_vertex(vsup, own_s, d);
             }
+            if (ph != 1) unclaim_nets(I, B, vol, base_s, deg_s, tt, tn);
           }
-          unclaim_nets(I, B, vol, base_s, deg_s, tt, tn);
         }
+        if (ph != 1) break;
+        if (!grid_barrier(B.bar, I.status)) return;
       }
       if (B.niso && (metric != kMSRV || logp)) {
         // Vertices without nets, weight 0 (positions hold only the others):
@@ -1846,6 +1954,8 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
       if (gw == 0 && lane == 0) {
         B.ctl[2 + (par ^ 1)] = kNone;
         B.ctl[4 + (par ^ 1)] = kNone;
+        B.ctl[12 + (par ^ 1)] = 0;
+        B.ctl[14 + (par ^ 1)] = 0;
         B.ctl[9] = kNone;   // (read behind a fix's barrier, written by fixes alone)
         B.mcnt[par ^ 1] = 0;
         B.ctab_over[par ^ 1] = 0;

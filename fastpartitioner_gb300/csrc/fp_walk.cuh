@@ -399,8 +399,7 @@ __device__ __forceinline__ unsigned lane_prefix(unsigned x) {
 // predicted outcome: exact for TV (its accept test is a count of nets) and for
 // vertices without nets, else the old decision's, or a move (MSV) / no move
 // (MSRV) if that one stayed home.  The walk ends (ctl[0]) at a stale-marker
-// risk or at a changed vertex of a CTA or of the grid; ctl[1] counts the
-// changes.  The streams (kStream) place every vertex: it comes from part K,
+// risk or at a position without a candidate list; ctl[1] counts the changes.  The streams (kStream) place every vertex: it comes from part K,
 // its decision needs no accept test, and TV's walk ends at a part above max_pw.
 //
 // It is bound by the latency of dependent instructions (about 5 cycles each in
@@ -574,12 +573,8 @@ __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const int* s
             const unsigned db = __ballot_sync(
                 kAll, in && lane >= j && ((again && (hardf || iso)) || (again ? moren : morec) > lim));
             const int f = db ? __ffs(db) - 1 : nl;
-            // ---- positions [j, f) stand; a changed vertex of a CTA or of the
-            // grid ends the window
-            const bool take = lane >= j && lane < f;
-            const unsigned hm = __ballot_sync(kAll, take && chg && (m.w & 4));
-            const int fe = hm ? __ffs(hm) - 1 : f;
-            const bool keep = lane >= j && lane < fe;
+            // ---- positions [j, f) stand
+            const bool keep = lane >= j && lane < f;
             const unsigned cm = __ballot_sync(kAll, keep && chg);
             if (cm) {
               if (keep && chg) {
@@ -592,10 +587,6 @@ __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const int* s
             }
             if (keep && !chg && (m.w & 128)) B.flag[ol + i0 + lane] = (unsigned char)(m.w & 127);
             apply(__ballot_sync(kAll, keep && mvn), dn);
-            if (hm) {
-              hard = ((zl + i0 + fe) << 3) | 2;
-              break;
-            }
             j = f;
             if (f >= nl) break;
             const bool af = (need >> f) & 1u;
