@@ -36,6 +36,13 @@ __device__ __forceinline__ int slack_of(float a, float b) {
   return !(x > -1.0f) ? -1 : x > 1.0e9f ? kBig : (int)x;
 }
 
+// Floats as integers of the same order, and back.
+__device__ __forceinline__ int order_of(float f) {
+  const int b = __float_as_int(f);
+  return b ^ ((b >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ float float_of(int k) { return __int_as_float(k ^ ((k >> 31) & 0x7fffffff)); }
+
 // What one pass over scored parts keeps: the best lower bound (its upper bound,
 // part and count) and the largest upper bound of the others, the largest
 // penalty and count.
@@ -59,8 +66,22 @@ struct ScoreAcc {
     }
   }
   // meets the accumulators of the lanes whose ids differ in the low bits of
-  // `lanes` - 1 (8 lanes to a position, or the whole warp)
+  // `lanes` - 1 (8 or 16 lanes to a position, or the whole warp: by redux.sync,
+  // 22 cycles each, where the shuffles take some 80 per step)
   __device__ __forceinline__ void meet(int lanes) {
+    if (lanes == 32) {
+      const int kb = order_of(blo), mb = __reduce_max_sync(kAll, kb);
+      const unsigned e = __reduce_min_sync(kAll, kb == mb ? be : ~0u);
+      const int wl = __ffs(__ballot_sync(kAll, kb == mb && be == e)) - 1;
+      oh = (int)(threadIdx.x & 31) == wl ? oh : fmaxf(oh, bhi);
+      bhi = __shfl_sync(kAll, bhi, wl);
+      blo = float_of(mb);
+      be = e;
+      oh = float_of(__reduce_max_sync(kAll, order_of(oh)));
+      up = float_of(__reduce_max_sync(kAll, order_of(up)));
+      cm = __reduce_max_sync(kAll, cm);
+      return;
+    }
 #pragma unroll
     for (int off = 1; off < lanes; off <<= 1) {
       const float xl = __shfl_xor_sync(kAll, blo, off), xh = __shfl_xor_sync(kAll, bhi, off);
@@ -304,7 +325,9 @@ __device__ __forceinline__ void walk_eval(const DevInstance& I, const SpecBuf& B
         const unsigned hi32 = (unsigned)(row[x] >> 32);
         if ((int)(hi32 >> 20) == am) cd = (int)((hi32 >> 4) & 0xffffu);
       }
-      for (int off = 1; off < lanes; off <<= 1) cd = max(cd, __shfl_xor_sync(kAll, cd, off));
+      if (lanes == 32) cd = __reduce_max_sync(kAll, cd);
+      else
+        for (int off = 1; off < lanes; off <<= 1) cd = max(cd, __shfl_xor_sync(kAll, cd, off));
     }
     if (none) {
       nd = (cd << 13) | am;
@@ -333,14 +356,21 @@ __device__ __forceinline__ void walk_eval(const DevInstance& I, const SpecBuf& B
         bp = p;
       }
     }
-    for (int off = 1; off < lanes; off <<= 1) {
-      cmin = min(cmin, __shfl_xor_sync(kAll, cmin, off));
-      cmax = max(cmax, __shfl_xor_sync(kAll, cmax, off));
-      const unsigned long long key = __shfl_xor_sync(kAll, bk, off);
-      const int p = __shfl_xor_sync(kAll, bp, off);
-      if (key < bk) {
-        bk = key;
-        bp = p;
+    if (lanes == 32) {
+      cmin = __reduce_min_sync(kAll, cmin);
+      cmax = __reduce_max_sync(kAll, cmax);
+      const unsigned long long mk = warp_min_u64(bk);
+      bp = __shfl_sync(kAll, bp, __ffs(__ballot_sync(kAll, bk == mk)) - 1);
+    } else {
+      for (int off = 1; off < lanes; off <<= 1) {
+        cmin = min(cmin, __shfl_xor_sync(kAll, cmin, off));
+        cmax = max(cmax, __shfl_xor_sync(kAll, cmax, off));
+        const unsigned long long key = __shfl_xor_sync(kAll, bk, off);
+        const int p = __shfl_xor_sync(kAll, bp, off);
+        if (key < bk) {
+          bk = key;
+          bp = p;
+        }
       }
     }
     tied = tied && cmin == cmax;
@@ -373,20 +403,29 @@ __device__ __forceinline__ void walk_eval(const DevInstance& I, const SpecBuf& B
   }
 }
 
-// Exclusive prefix over the lanes of x: by popcounts when the lanes with one
-// share it (unit weights), else a scan.
-__device__ __forceinline__ unsigned lane_prefix(unsigned x) {
+// Exclusive prefixes over the lanes of x and y: by popcounts when the lanes
+// with one share it (unit weights), else by scans side by side.
+__device__ __forceinline__ void lane_prefixes(unsigned x, unsigned y, unsigned* px, unsigned* py) {
   const int lane = threadIdx.x & 31;
-  const unsigned m = __ballot_sync(kAll, x != 0u);
-  if (!m) return 0u;
-  const unsigned x0 = __shfl_sync(kAll, x, __ffs(m) - 1);
-  if (__all_sync(kAll, x == 0u || x == x0)) return x0 * (unsigned)__popc(m & ((1u << lane) - 1u));
-  unsigned incl = x;
-  for (int off = 1; off < 32; off <<= 1) {
-    const unsigned t = __shfl_up_sync(kAll, incl, off);
-    if (lane >= off) incl += t;
+  const unsigned below = (1u << lane) - 1u;
+  const unsigned mx = __ballot_sync(kAll, x != 0u), my = __ballot_sync(kAll, y != 0u);
+  const unsigned x0 = __shfl_sync(kAll, x, (__ffs(mx) - 1) & 31), y0 = __shfl_sync(kAll, y, (__ffs(my) - 1) & 31);
+  if (__all_sync(kAll, (x == 0u || x == x0) && (y == 0u || y == y0))) {
+    *px = x0 * (unsigned)__popc(mx & below);
+    *py = y0 * (unsigned)__popc(my & below);
+    return;
   }
-  return incl - x;
+  unsigned ix = x, iy = y;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const unsigned t = __shfl_up_sync(kAll, ix, off), u = __shfl_up_sync(kAll, iy, off);
+    if (lane >= off) {
+      ix += t;
+      iy += u;
+    }
+  }
+  *px = ix - x;
+  *py = iy - y;
 }
 
 // The walk (block 0, every thread).  The positions [zs, end_w) are visited in
@@ -411,7 +450,10 @@ __device__ __forceinline__ unsigned lane_prefix(unsigned x) {
 // the rest of the group is decided again (on 16K vertices of unit weight, K =
 // 8, about 9 positions stand per step).  A vertex without nets takes the
 // least-loaded part, which its own kind moves with every step: those the
-// first warp decides one by one.
+// first warp decides one by one.  Per window of 1M Zipf vertices under TV with
+// sizes near the capacity (1215 positions, 67 changes): 446 us with every row
+// staged and shuffles to meet the lanes, 293 us with the rows the drift reaches
+// and redux.sync.
 template <bool kStream>
 __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const int* sizes, float Cf, bool tv, bool msv,
                             int pos, int zs, int end_w, int nm, WalkSmem& S, int* sz, int* dl) {
@@ -479,29 +521,37 @@ __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const int* s
         if (g >= ng) break;
       }
       const int i0 = g * 32, nl = min(32, n - i0);
-      // its candidates: a warp per row, two rows' loads in flight, only the
-      // entries there are
-      for (int r0 = wib; r0 < nl; r0 += 2 * kSWarps) {
-        int nc[2];
+      // the candidates of the positions in mask: a warp per row, two rows' loads
+      // in flight, only the entries there are
+      const unsigned fits = __ballot_sync(kAll, lane < nl && (S.meta[i0 + lane].w >> 8) <= kWalkRow);
+      auto stage = [&](unsigned mask) {
+        for (int k = 0; k < wib && mask; k++) mask &= mask - 1;
+        while (mask) {
+          int rr[2], nc[2];
 #pragma unroll
-        for (int u = 0; u < 2; u++) {
-          const int r = r0 + u * kSWarps;
-          nc[u] = r < nl ? min(S.meta[i0 + r].w >> 8, kWalkRow) : 0;
+          for (int u = 0; u < 2; u++) {
+            rr[u] = mask ? __ffs(mask) - 1 : 0;
+            nc[u] = mask ? S.meta[i0 + rr[u]].w >> 8 : 0;
+            for (int k = 0; k < kSWarps && mask; k++) mask &= mask - 1;
+          }
+          for (int x = lane; x < max(nc[0], nc[1]); x += 64) {
+            unsigned long long e[2][2];
+#pragma unroll
+            for (int u = 0; u < 2; u++)
+#pragma unroll
+              for (int y = 0; y < 2; y++)
+                e[u][y] = x + 32 * y < nc[u] ? lds(&B.cand[(size_t)(ol + i0 + rr[u]) * K + x + 32 * y]) : 0;
+#pragma unroll
+            for (int u = 0; u < 2; u++)
+#pragma unroll
+              for (int y = 0; y < 2; y++)
+                if (x + 32 * y < nc[u]) S.ent[rr[u] * kWalkStride + x + 32 * y] = e[u][y];
+          }
         }
-        for (int x = lane; x < max(nc[0], nc[1]); x += 64) {
-          unsigned long long e[2][2];
-#pragma unroll
-          for (int u = 0; u < 2; u++)
-#pragma unroll
-            for (int y = 0; y < 2; y++)
-              e[u][y] = x + 32 * y < nc[u] ? lds(&B.cand[(size_t)(ol + i0 + r0 + u * kSWarps) * K + x + 32 * y]) : 0;
-#pragma unroll
-          for (int u = 0; u < 2; u++)
-#pragma unroll
-            for (int y = 0; y < 2; y++)
-              if (x + 32 * y < nc[u]) S.ent[(r0 + u * kSWarps) * kWalkStride + x + 32 * y] = e[u][y];
-        }
-      }
+      };
+      // those that the drift so far reaches; more as it grows
+      unsigned rows = fits & __ballot_sync(kAll, lane < nl && S.margin[i0 + lane] < 2 * S.drift + 4);
+      stage(rows);
       __syncthreads();   // also: every thread has read S.drift
       // warp 0: the group at hand, its lanes' positions and their present outcome
       const bool in = lane < nl;
@@ -543,6 +593,11 @@ __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const int* s
         }
         __syncthreads();
         if (S.group < 0) break;
+        if (const unsigned miss = S.eval & fits & ~rows) {
+          stage(miss);
+          rows |= miss;
+          __syncthreads();
+        }
         walk_eval<kStream>(I, B, Cf, tv, rC, sz, S, i0, ol);
         __syncthreads();
         if (wib == 0) {
@@ -563,8 +618,9 @@ __device__ void walk_window(const DevInstance& I, const SpecBuf& B, const int* s
           const bool chg = dn != d;
           // drift from these sizes before each position, and what the changed
           // decisions before it add to the drift of the others
-          const unsigned Dn = lane_prefix(mvn && lane >= j ? (unsigned)w : 0u);
-          const unsigned cn = lane_prefix(chg && lane >= j ? (mvn ? (unsigned)w : 0u) + (mv ? (unsigned)w : 0u) : 0u);
+          unsigned Dn, cn;
+          lane_prefixes(mvn && lane >= j ? (unsigned)w : 0u,
+                        chg && lane >= j ? (mvn ? (unsigned)w : 0u) + (mv ? (unsigned)w : 0u) : 0u, &Dn, &cn);
           const long long lim = again ? (long long)nsl - Dn : (long long)mg - drift - cn;
           long long moren = 0, morec = 0;   // what the vertices without nets add to both
           while (true) {
