@@ -727,6 +727,7 @@ int fp_instance_create(fp_ctx* ctx, const fp_hypergraph* h, int32_t K, int32_t m
         (rc = dalloc(in, &in->sb.vterm, volm ? (size_t)kSpecWindow * kVolTerms : 1)) ||
         (rc = dalloc(in, &in->sb.vpart, volm ? (size_t)kSpecWindow * kVolTerms : 1)) ||
         (rc = dalloc(in, &in->sb.vd, kSpecWindow)) || (rc = dalloc(in, &in->sb.scan, (size_t)kSpecWindow * words)) ||
+        (rc = dalloc(in, &in->sb.cmask, ldg ? kMaxSpecWarps / 8 * words : 1)) ||
         (rc = dalloc(in, &in->sb.rgain, std::max(kSpecWindow, kMsgWindow))) ||
         (rc = dalloc(in, &in->sb.rloss, std::max(kSpecWindow, kMsgWindow))) ||
         (rc = dalloc(in, &in->sb.rec, ldg ? g.pins : 1)) || (rc = dalloc(in, &in->sb.rec_slot, ldg ? g.pins : 1)) ||
@@ -872,6 +873,7 @@ int fp_instance_footprint(int32_t nov, int32_t noe, int64_t pins, int32_t K, int
     add(W, 1); add(W, 4); add(W, 4); add(W, 4); add(W, 4);   // flag, slack, vslack, wt, vd
     add(volm ? W : 1, 4); add(volm ? W * kVolTerms : 1, 8); add(volm ? W * kVolTerms : 1, 2);   // vn, vterm, vpart
     add(W * words, 4);                                       // scan
+    add(ldg ? kMaxSpecWarps / 8 * words : 1, 4);                 // cmask
     add(std::max(kSpecWindow, kMsgWindow), 4); add(std::max(kSpecWindow, kMsgWindow), 4);   // rgain, rloss
     add(ldg ? P : 1, 4); add(ldg ? P : 1, 8);                // rec, rec_slot
     add(ldg ? ctab : 1, 8); add(ldg ? ctab : 1, 4); add(ldg ? ctab : 1, 4);

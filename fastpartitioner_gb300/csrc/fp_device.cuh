@@ -125,6 +125,7 @@ struct SpecBuf {
   int* rgain;            // [wmax] decision-record gain / loss of each window offset (with
   int* rloss;            //     the decision log on)
   uint32_t* scan;        // [wmax * words] parts scanned per window offset (TV)
+  uint32_t* cmask;       // [CTAs * words] parts scanned by each CTA's positions (TV)
   uint32_t* rec;         // [pins] per (vertex, net) record of a move (spec::rec_pack),
                          //     at the pair's vnets index
   const unsigned char* vclass;  // [nov] 0: warp-evaluated, 1: CTA-evaluated (medium),

@@ -52,6 +52,7 @@ namespace {
 using namespace spec;
 
 constexpr int kTV = 1, kMSV = 4, kMSRV = 5;
+constexpr int kMaxWords = 4096 / 32;   // part masks of the largest K
 
 struct RoundCtx {
   const int* sizes;
@@ -823,6 +824,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
   __shared__ int s_t0[kMaxGridVerts], s_t1[kMaxGridVerts];   // their teams of CTAs
   __shared__ int loc_b[kSWarps * 96];   // per-warp locate scratch
   __shared__ VolStates vs_s;
+  __shared__ uint32_t cmask_s[kMaxWords];
   const int metric = I.metric;
   const bool vol = metric != kTV;
   const bool rv = metric == kMSRV;
@@ -1670,6 +1672,15 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
       // finds what that leaves wrong); otherwise one CTA walks them in order.
       // Measured on the 1M-vertex Zipf workload under TV (windows of 1,500
       // positions, five changes each): 315 us of walk per window, 75 us so.
+      if (metric == kTV) {   // the parts scanned by this CTA's positions, for the markers below
+        const int ctan = min(kSWarps * q, span - cta_o0);
+        for (int x = threadIdx.x; x < words; x += blockDim.x) cmask_s[x] = 0;
+        __syncthreads();
+        for (int x = threadIdx.x; x < ctan * words; x += blockDim.x)
+          if (const uint32_t m = lds(&B.scan[(size_t)cta_o0 * words + x])) atomicOr(&cmask_s[x % words], m);
+        __syncthreads();
+        for (int x = threadIdx.x; x < words; x += blockDim.x) B.cmask[(size_t)blockIdx.x * words + x] = cmask_s[x];
+      }
       int cutw, hard = kNone, fcut = kNone;
       bool sizes = true;
       for (int zf = pos, nfix = 0;; nfix++) {
@@ -1934,12 +1945,24 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
       }
       if (metric == kTV) {
         // marker = last scanner of each part among the committed positions: each
-        // warp offers the last of its own positions per part, stamped with the
-        // window (round + 1), and the next round state reads the maximum
+        // warp offers the last of its own positions per part that no later CTA
+        // scanned, stamped with the window (round + 1), and the next round state
+        // reads the maximum (with every warp offering every part it scanned the
+        // commit of a window of 4400 positions of 1M Zipf vertices took 67 us
+        // instead of 20: the atomics meet on K words)
+        __syncthreads();
+        for (int x = threadIdx.x; x < words; x += blockDim.x) cmask_s[x] = 0;
+        __syncthreads();
+        {
+          const int per = kSWarps * q, whole = min((cut - pos) / per, (int)gridDim.x);   // CTAs whose positions all count
+          for (int x = ((int)blockIdx.x + 1) * words + (int)threadIdx.x; x < whole * words; x += blockDim.x)
+            if (const uint32_t m = lds(&B.cmask[x])) atomicOr(&cmask_s[x % words], m);
+        }
+        __syncthreads();
         const int zc = min(z1, cut);
         const unsigned long long stamp = (unsigned long long)(round + 1) << 32;
         for (int wd = lane; wd < words; wd += 32) {
-          uint32_t seen = 0;
+          uint32_t seen = cmask_s[wd];
           for (int z = zc - 1; z >= z0 && seen != ~0u; z--) {
             uint32_t m = lds(&B.scan[(size_t)(z - pos) * words + wd]) & ~seen;
             seen |= m;
