@@ -33,7 +33,7 @@
 // Every committed outcome therefore equals the reference's sequential outcome.
 //
 // A mover's slots (own part, destination) in each of its nets' lists are found
-// once, by a flattened pass over the slots (locate_batch), and recorded per
+// once, by a flattened pass over the slots (locate_nets), and recorded per
 // (vertex, net); the gain / loss terms and the commit then take O(1) per net.
 // Vertices are classed by work (list slots over their nets, host-side): light
 // ones are evaluated by one warp, medium ones by one CTA, and the heaviest (up
@@ -227,12 +227,10 @@ __device__ int locate_range(const DevInstance& I, const SpecBuf& B, int metric, 
                             int n0, int n1, int* loc, int* gains, int* losses, int* adelta) {
   const bool vol = metric != kTV, rv = metric == kMSRV;
   int ra = 0;
-  for (int nb = n0; nb < n1; nb += 32) {
-    int e;
-    const uint32_t r = locate_batch(I, B.rec, v, own, d, base, nb, n1, loc, loc + 32, loc + 64, &e);
-    if (e >= 0) ra += (rec_rem(r) ? 1 : 0) + (rec_add(r) ? 1 << 16 : 0);
-    if (vol && e >= 0) net_terms(I, rv, v, own, d, e, r, gains, losses, adelta);
-  }
+  locate_nets(I, B.rec, v, own, d, base, n0, n1, loc, [&](int e, uint32_t r) {
+    ra += (rec_rem(r) ? 1 : 0) + (rec_add(r) ? 1 << 16 : 0);
+    if (vol) net_terms(I, rv, v, own, d, e, r, gains, losses, adelta);
+  });
   return ra;
 }
 // The same for warp wi of nw warps splitting all of v's nets (net_range).
@@ -558,7 +556,7 @@ __device__ void cta_eval_ldg(const DevInstance& I, const SpecBuf& B, const Round
   int c1 = 0;
   int n0, n1;
   net_range(deg, wib, kSWarps, &n0, &n1);
-  for (int nb = n0; nb < n1; nb += 32) c1 += tally_batch(I, own, base, nb, n1, 0, sb, cnt_b, first_b);
+  c1 = tally_range<true>(I, own, base, n0, n1, 0, sb, cnt_b, first_b);
   c1 = warp_sum(c1);
   if (lane == 0) iscr[wib] = c1;
   __syncthreads();
@@ -1019,8 +1017,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
           __syncthreads();
           int own1 = 0, n0, n1;
           net_range(a1 - a0, wib, kSWarps, &n0, &n1);
-          for (int nb = a0 + n0; nb < a0 + n1; nb += 32)
-            own1 += tally_batch(I, own_s, base_s, nb, a0 + n1, a0, sb, cnt_b, first_b);
+          own1 = tally_range<true>(I, own_s, base_s, a0 + n0, a0 + n1, a0, sb, cnt_b, first_b);
           own1 = warp_sum(own1);
           if (lane == 0 && own1) atomicAdd(&B.hmisc[hmslot(j)], own1);
           __syncthreads();
@@ -1049,7 +1046,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
         for (int p = lane; p < K; p += 32) { cnt[p] = 0; first[p] = ~0u; }
         __syncwarp();
         int c1 = 0;
-        for (int nb = 0; nb < deg; nb += 32) c1 += tally_batch(I, own, base, nb, deg, 0, sb, cnt, first);
+        c1 = tally_range<true>(I, own, base, 0, deg, 0, sb, cnt, first);
         __syncwarp();
         c1 = warp_sum(c1);
         const long long cT = clock64();

@@ -84,12 +84,15 @@ __device__ __forceinline__ void tally_uncut(const DevInstance& I, uint32_t base,
   atomicMin(&first[p], (unsigned)(k - n0) << sb);
 }
 
-// The stream's tally of nets [nb, min(nb + 32, deg)) of the range from n0 into
-// cnt / first (tally_batch's sighting keys).
-__device__ __forceinline__ void tally_stream(const DevInstance& I, bool cn, uint32_t base, int nb, int deg, int n0,
+// The stream's tally of the nets [n0, n1) into cnt / first (tally_range's
+// sighting keys, from net k0).
+__device__ __forceinline__ void tally_stream(const DevInstance& I, bool cn, uint32_t base, int n0, int n1, int k0,
                                              int sb, int* cnt, unsigned* first) {
-  if (cn) tally_uncut(I, base, nb, deg, n0, sb, cnt, first);
-  else tally_batch(I, -1, base, nb, deg, n0, sb, cnt, first);
+  if (cn) {
+    for (int nb = n0; nb < n1; nb += 32) tally_uncut(I, base, nb, n1, k0, sb, cnt, first);
+  } else {
+    tally_range<false>(I, -1, base, n0, n1, k0, sb, cnt, first);
+  }
 }
 
 __device__ __forceinline__ unsigned long long skey(int round, int pos) {
@@ -117,60 +120,35 @@ __device__ int least_loaded(const int* sz0, const int* dsz, int K) {
   return (int)(mk & 0xffffffffu);
 }
 
-// Slot of part d in each of the nets [nb, min(nb + 32, deg)) of a vertex, -1
-// where d is not listed; lane i gets net nb + i's.  The lists' entries are
-// walked flattened across the warp, kU loads per lane in flight, as in
-// tally_batch.  sd: 32 ints of per-warp scratch.
-__device__ int locate_part(const DevInstance& I, uint32_t base, int nb, int deg, int d, int* sd) {
+// Slot of part d in each of the nets [n0, n1) of a vertex, -1 where d is not
+// listed: each(k, e, slot) on the lane of net index k.  One warp; sd: 32 ints of
+// its scratch.
+template <class Each>
+__device__ __forceinline__ void locate_part(const DevInstance& I, uint32_t base, int n0, int n1, int d, int* sd,
+                                            Each&& each) {
   const int lane = threadIdx.x & 31;
-  const int k = nb + lane;
-  int s = 0, n = 0;
-  if (k < deg) {
-    const int e = (int)__ldg(&I.vnets[base + k]);
-    s = (int)__ldg(&I.nptr[e]);
-    const int cap = (int)__ldg(&I.nptr[e + 1]) - s;
-    n = lds(&I.ep_len[e]);
-    if (n < 0 || n > cap) { dev_fail(I.status, kDevErrInvalid); n = 0; }
-  }
-  sd[lane] = -1;
-  int incl = n;
-  for (int off = 1; off < 32; off <<= 1) {
-    const int t = __shfl_up_sync(kAll, incl, off);
-    if (lane >= off) incl += t;
-  }
-  const int total = __shfl_sync(kAll, incl, 31);
-  __syncwarp();
-  constexpr int kU = 4;
-  for (int f0 = 0; f0 < total; f0 += 32 * kU) {
-    int aa[kU], kn[kU], kj[kU];
-#pragma unroll
-    for (int u = 0; u < kU; u++) {
-      const int f = f0 + u * 32 + lane;
-      int lo = 0, hi = 31;
-#pragma unroll
-      for (int it = 0; it < 5; it++) {
-        const int mid = (lo + hi) >> 1;
-        const int val = __shfl_sync(kAll, incl, mid);
-        if (f < val) hi = mid; else lo = mid + 1;
-      }
-      const int sl = __shfl_sync(kAll, s, lo);
-      const int nl = __shfl_sync(kAll, n, lo);
-      const int il = __shfl_sync(kAll, incl, lo);
-      kn[u] = lo;
-      kj[u] = f - (il - nl);
-      aa[u] = f < total ? sl + kj[u] : -1;
-    }
-    int pp[kU];
-#pragma unroll
-    for (int u = 0; u < kU; u++) pp[u] = aa[u] >= 0 ? lds(&I.ep_part[aa[u]]) : -1;
-#pragma unroll
-    for (int u = 0; u < kU; u++)
-      if (aa[u] >= 0 && pp[u] == d) sd[kn[u]] = kj[u];   // d is listed once per net: one writer
-  }
-  __syncwarp();
-  const int j = sd[lane];
-  __syncwarp();
-  return k < deg ? j : -1;
+  for_slots<false>(
+      I, base, n0, n1,
+      [&](int, int) {
+        sd[lane] = -1;
+        __syncwarp();
+      },
+      [&](int lo, int j, int p, int) {
+        if (p == d) sd[lo] = j;   // d is listed once per net: one writer
+      },
+      [&](int nb, int e) {
+        __syncwarp();
+        const int j = sd[lane];
+        __syncwarp();
+        if (e >= 0) each(nb + lane, e, j);
+      });
+}
+
+// Lane i's slot of d in net nb + i (before n1), -1 where it is not listed.
+__device__ __forceinline__ int locate_part32(const DevInstance& I, uint32_t base, int nb, int n1, int d, int* sd) {
+  int slot = -1;
+  locate_part(I, base, nb, min(nb + 32, n1), d, sd, [&](int, int, int j) { slot = j; });
+  return slot;
 }
 
 // Adds one pin of part d to net e at slot `slot` (-1 / kNoSlot: append).
@@ -261,15 +239,10 @@ __device__ int decide_position(const DevInstance& I, const SpecBuf& B, const int
 // decision's appends are then a subset.
 __device__ void record_slots(const DevInstance& I, const SpecBuf& B, const StreamArgs& S, uint32_t base, int n0,
                              int n1, int d, int round, int z, int* sd, bool claim_all) {
-  const int lane = threadIdx.x & 31;
-  for (int nb = n0; nb < n1; nb += 32) {
-    const int j = locate_part(I, base, nb, n1, d, sd);
-    const int k = nb + lane;
-    if (k < n1) {
-      S.rec[base + k] = j >= 0 ? (uint32_t)j : kNoSlot;
-      if (j < 0 || claim_all) atomicMax(&B.claim64[(int)__ldg(&I.vnets[base + k])], skey(round, z));
-    }
-  }
+  locate_part(I, base, n0, n1, d, sd, [&](int k, int e, int j) {
+    S.rec[base + k] = j >= 0 ? (uint32_t)j : kNoSlot;
+    if (j < 0 || claim_all) atomicMax(&B.claim64[e], skey(round, z));
+  });
 }
 
 // The walk takes a changed decision d of position z that appends where the old
@@ -277,14 +250,11 @@ __device__ void record_slots(const DevInstance& I, const SpecBuf& B, const Strea
 // claim wins), and the walk checks every later position against the claims
 // again.  One warp.
 __device__ void claim_appends(const DevInstance& I, const SpecBuf& B, int v, int round, int z, int d, int* sd) {
-  const int lane = threadIdx.x & 31;
   const uint32_t base = __ldg(&I.vptr[v]);
   const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
-  for (int nb = 0; nb < deg; nb += 32) {
-    const int j = locate_part(I, base, nb, deg, d, sd);
-    const int k = nb + lane;
-    if (k < deg && j < 0) atomicMax(&B.claim64[(int)__ldg(&I.vnets[base + k])], skey(round, z));
-  }
+  locate_part(I, base, 0, deg, d, sd, [&](int, int e, int j) {
+    if (j < 0) atomicMax(&B.claim64[e], skey(round, z));
+  });
 }
 
 // Does an earlier position of the round claim one of position z's nets (v's)?
@@ -378,7 +348,7 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
           int n0, n1;
           net_range(deg, gw, nwarps, &n0, &n1);
           const int b0 = n0 + min(a0, n1 - n0), b1 = b0 + min(piece, n1 - b0);
-          for (int nb = b0; nb < b1; nb += 32) tally_stream(I, cn, base, nb, b1, b0, sb, cnt, first);
+          tally_stream(I, cn, base, b0, b1, b0, sb, cnt, first);
         }
         __syncthreads();
         for (int p = threadIdx.x; p < K; p += blockDim.x) {
@@ -438,10 +408,7 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
       {
         int n0, n1;
         net_range(deg, gw, nwarps, &n0, &n1);
-        for (int nb = n0; nb < n1; nb += 32) {
-          const int j = locate_part(I, base, nb, n1, d, sd);
-          if (nb + lane < n1) place_net(I, (int)__ldg(&I.vnets[base + nb + lane]), d, j);
-        }
+        locate_part(I, base, n0, n1, d, sd, [&](int, int e, int j) { place_net(I, e, d, j); });
       }
       if (gtid == 0) {
         I.part_vec[v] = d;
@@ -538,7 +505,7 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
       __syncthreads();   // the CTA's previous tallies are read
       for (int p = threadIdx.x; p < K; p += blockDim.x) { cnt_b[p] = 0; first_b[p] = ~0u; }
       __syncthreads();
-      for (int nb = n0; nb < n1; nb += 32) tally_stream(I, cn, base, nb, n1, 0, sb, cnt_b, first_b);
+      tally_stream(I, cn, base, n0, n1, 0, sb, cnt_b, first_b);
       __syncthreads();
     };
     auto decide_cta = [&](int, int z, int v, uint32_t base, int, int c0, int c1) {
@@ -571,7 +538,7 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
       const int deg = (int)(__ldg(&I.vptr[v + 1]) - base);
       for (int p = lane; p < K; p += 32) { cnt[p] = 0; first[p] = ~0u; }
       __syncwarp();
-      for (int nb = 0; nb < deg; nb += 32) tally_stream(I, cn, base, nb, deg, 0, sb, cnt, first);
+      tally_stream(I, cn, base, 0, deg, 0, sb, cnt, first);
       __syncwarp();
       int nc;
       const int d = decide_position(I, B, sizes_s, penf, Cf, s_minpart, s_minsize, s_second, cnt, first, sb, o,
@@ -767,10 +734,7 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
     auto place = [&](int z, uint32_t base, int n0, int n1) {
       const int d = (z == cut ? lds(&B.dfix[z - pos]) : lds(&B.dec[z - pos])) & 0xffff;
       if (z == cut) {
-        for (int nb = n0; nb < n1; nb += 32) {
-          const int j = locate_part(I, base, nb, n1, d, sd);
-          if (nb + lane < n1) place_net(I, (int)__ldg(&I.vnets[base + nb + lane]), d, j);
-        }
+        locate_part(I, base, n0, n1, d, sd, [&](int, int e, int j) { place_net(I, e, d, j); });
       } else {
         for (int k = n0 + lane; k < n1; k += 32)
           place_net(I, (int)__ldg(&I.vnets[base + k]), d, (int)lds(&S.rec[base + k]));
@@ -999,7 +963,7 @@ __device__ int msg_records(const DevInstance& I, const SpecBuf& B, const StreamA
   const int lane = threadIdx.x & 31;
   int napp = 0;
   for (int nb = n0; nb < n1; nb += 32) {
-    const int j = locate_part(I, base, nb, n1, d, sd);
+    const int j = locate_part32(I, base, nb, n1, d, sd);
     const int k = nb + lane;
     if (k < n1) {
       const int e = (int)__ldg(&I.vnets[base + k]);
@@ -1050,7 +1014,7 @@ __device__ void msg_commit_act(const DevInstance& I, const StreamArgs& S, int wo
   const int K = I.K;
   for (int nb = n0; nb < n1; nb += 32) {
     // d's slot: the record's, or located again (a flip committed with another part)
-    const int jl = slot_override_d ? locate_part(I, base, nb, n1, d, sd) : 0;
+    const int jl = slot_override_d ? locate_part32(I, base, nb, n1, d, sd) : 0;
     const int k = nb + lane;
     if (k >= n1) continue;
     const uint32_t r = lds(&S.rec[base + k]);
@@ -1531,7 +1495,7 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_msg_kernel(DevInstance I,
       __syncwarp();
       if (fl) {
         for (int nb = 0; nb < deg; nb += 32) {
-          const int j = locate_part(I, base, nb, deg, d, sd);
+          const int j = locate_part32(I, base, nb, deg, d, sd);
           if (nb + lane < deg) place_net(I, (int)__ldg(&I.vnets[base + nb + lane]), d, j);
         }
       } else {
