@@ -96,7 +96,8 @@ int default_grid_verts(int metric) {
 }
 constexpr int kMaxSpecWarps = 16384;
 constexpr int kCtlWords = 16;   // SpecBuf::ctl
-cudaError_t launch_metrics(const DevInstance& I, void* scratch, long long* out, int num_sms, cudaStream_t st,
+int metrics_grid(int K, int noe, int num_sms);
+cudaError_t launch_metrics(const DevInstance& I, void* scratch, long long* out, int grid, cudaStream_t st,
                            int* launches);
 }  // namespace fp
 
@@ -133,7 +134,7 @@ struct fp_instance {
   long long dev_bytes = 0;        // bytes of the device allocations in `allocs`
   bool in_arena = false;          // buffers taken from ctx->arena (nothing in allocs)
   void* metric_scratch = nullptr;
-  long long* metric_out = nullptr;
+  int metric_grid = 1;
   long long* h_moves = nullptr;   // pinned
   int* h_status = nullptr;        // pinned
   long long* h_metrics = nullptr; // pinned
@@ -762,8 +763,7 @@ int fp_instance_create(fp_ctx* ctx, const fp_hypergraph* h, int32_t K, int32_t m
         (rc = dalloc(in, &in->st_rowpos_d, msg ? 2 * K : 1)) || (rc = dalloc(in, &in->st_colpos_d, msg ? 2 * K : 1)) ||
         (rc = dalloc(in, &in->st_saved_d, msg ? (size_t)msg_stream_window(g.nov) * K : 1)) ||
         (rc = dalloc(in, &in->st_actm_d, msg ? (size_t)msg_stream_window(g.nov) * words : 1)) ||
-        (rc = dalloc(in, &in->st_ownm_d, msg ? (size_t)msg_stream_window(g.nov) * words : 1)) ||
-        (rc = dalloc(in, &in->metric_out, 8))) {
+        (rc = dalloc(in, &in->st_ownm_d, msg ? (size_t)msg_stream_window(g.nov) * words : 1))) {
       fp_instance_destroy(in);
       return rc;
     }
@@ -780,6 +780,9 @@ int fp_instance_create(fp_ctx* ctx, const fp_hypergraph* h, int32_t K, int32_t m
       in->dev_bytes += (long long)metrics_scratch_bytes(K);
     }
     in->metric_scratch = ms;
+    in->metric_grid = metrics_grid(K, g.noe, ctx->num_sms);
+    e = cudaMemsetAsync(ms, 0, metrics_scratch_bytes(K), ctx->stream);   // (each evaluation leaves it so)
+    if (e != cudaSuccess) { fp_instance_destroy(in); return cuda_status(e); }
     in->sb.wmax = kSpecWindow;
     in->sb.ctab_mask = ldg ? (unsigned)(ctab - 1) : 0u;
     in->sb.wmax_msg = kMsgWindow;
@@ -898,7 +901,6 @@ int fp_instance_footprint(int32_t nov, int32_t noe, int64_t pins, int32_t K, int
       add(msg ? 2 * (size_t)K : 1, 4); add(msg ? 2 * (size_t)K : 1, 4);               //   saved messages,
       add(msg ? mw * K : 1, 4); add(msg ? mw * words : 1, 4); add(msg ? mw * words : 1, 4);   // part masks
     }
-    add(8, 8);                                               // metric_out
     b += (long long)metrics_scratch_bytes(K);
     *bytes = b;
     return FP_OK;
@@ -1205,9 +1207,8 @@ int fp_metrics(fp_instance* in, int64_t out[6]) {
     cudaSetDevice(in->ctx->device);
     cudaStream_t s = in->ctx->stream;
     int launches = 0;
-    cudaError_t e = launch_metrics(in->d, in->metric_scratch, in->metric_out, in->ctx->num_sms, s, &launches);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(in->h_metrics, in->metric_out, sizeof(long long) * 6, cudaMemcpyDeviceToHost, s);
+    // (the kernel writes the six values to pinned host memory)
+    cudaError_t e = launch_metrics(in->d, in->metric_scratch, in->h_metrics, in->metric_grid, s, &launches);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_status(e);
     for (int i = 0; i < 6; i++) out[i] = in->h_metrics[i];

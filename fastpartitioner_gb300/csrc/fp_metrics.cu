@@ -17,6 +17,7 @@
 #include "fp_device.cuh"
 #include "../../include/fastpart.h"
 
+#include <algorithm>
 #include <mutex>
 
 namespace fp {
@@ -24,13 +25,62 @@ namespace fp {
 namespace {
 
 struct MetricScratch {
-  unsigned long long* acc;   // [0]=TV [1]=CN
+  unsigned long long* acc;   // [0]=TV [1]=CN [2]=CTAs done
   long long* send;           // K, send volume per part (MSV = MSRV send)
   long long* recv;           // K
   uint32_t* pairs;           // K*words bits
 };
 
-__global__ void metrics_nets_kernel(DevInstance I, MetricScratch M) {
+// TM = popcount of the pair matrix, MSM = max row popcount, MSV = max send, MSRV
+// = max send + received, by one CTA of up to 32 warps; kHere: of the kernel that
+// made the totals (read past L1).
+template <bool kHere>
+__device__ void metrics_final(const DevInstance& I, const MetricScratch& M, long long* out) {
+  __shared__ long long red[4][32];
+  const int K = I.K;
+  const int words = (K + 31) >> 5;
+  auto get = [](const auto* x) { return kHere ? __ldcg(x) : *x; };
+  long long tm = 0, msm = -1, msv = -1, msrv = -1;
+  for (int p = threadIdx.x; p < K; p += blockDim.x) {
+    long long row = 0;
+    for (int x = 0; x < words; x++) row += __popc(get(&M.pairs[(size_t)p * words + x]));
+    tm += row;
+    msm = max(msm, row);
+    const long long send = get(&M.send[p]);
+    msv = max(msv, send);
+    msrv = max(msrv, send + get(&M.recv[p]));
+  }
+  for (int off = 16; off; off >>= 1) {
+    tm += __shfl_xor_sync(0xffffffffu, tm, off);
+    msm = max(msm, __shfl_xor_sync(0xffffffffu, msm, off));
+    msv = max(msv, __shfl_xor_sync(0xffffffffu, msv, off));
+    msrv = max(msrv, __shfl_xor_sync(0xffffffffu, msrv, off));
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0) { red[0][warp] = tm; red[1][warp] = msm; red[2][warp] = msv; red[3][warp] = msrv; }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const int nw = blockDim.x >> 5;
+    for (int w = 1; w < nw; w++) {
+      tm += red[0][w];
+      msm = max(msm, red[1][w]);
+      msv = max(msv, red[2][w]);
+      msrv = max(msrv, red[3][w]);
+    }
+    out[0] = (long long)get(&M.acc[0]);
+    out[1] = (long long)get(&M.acc[1]);
+    out[2] = tm;
+    out[3] = msm;
+    out[4] = msv;
+    out[5] = msrv;
+  }
+}
+
+// With `last`, the last CTA to finish reduces the totals into out and leaves the
+// scratch zeroed for the next call: one launch instead of a fill, two kernels
+// and a copy, which is what a small evaluation costs (1000 nets, K = 8: 30.8 -> 20.5
+// us, 8000 nets and K = 512 43 -> 32, 262144 and K = 256 68 -> 65).
+__global__ void metrics_nets_kernel(DevInstance I, MetricScratch M, long long* out, bool last) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int K = I.K;
   const int words = (K + 31) >> 5;
@@ -67,49 +117,29 @@ __global__ void metrics_nets_kernel(DevInstance I, MetricScratch M) {
     if (send_s[p]) atomicAdd((unsigned long long*)&M.send[p], (unsigned long long)send_s[p]);
     if (recv_s[p]) atomicAdd((unsigned long long*)&M.recv[p], (unsigned long long)recv_s[p]);
   }
+  if (!last) return;
+  __shared__ bool s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(&M.acc[2], 1ull) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  metrics_final<true>(I, M, out);
+  __syncthreads();
+  for (int p = threadIdx.x; p < 2 * K; p += blockDim.x) M.send[p] = 0;   // (and recv behind it)
+  for (int x = threadIdx.x; x < K * words; x += blockDim.x) M.pairs[x] = 0;
+  if (threadIdx.x < 3) M.acc[threadIdx.x] = 0;
 }
 
-// One CTA: TM = popcount of the pair matrix, MSM = max row popcount,
-// MSV = max send, MSRV = max send + recv.
 __global__ void metrics_final_kernel(DevInstance I, MetricScratch M, long long* out) {
-  __shared__ long long red[4][32];
-  const int K = I.K;
-  const int words = (K + 31) >> 5;
-  long long tm = 0, msm = -1, msv = -1, msrv = -1;
-  for (int p = threadIdx.x; p < K; p += blockDim.x) {
-    long long row = 0;
-    for (int x = 0; x < words; x++) row += __popc(M.pairs[(size_t)p * words + x]);
-    tm += row;
-    msm = row > msm ? row : msm;
-    msv = M.send[p] > msv ? M.send[p] : msv;
-    const long long sr = M.send[p] + M.recv[p];
-    msrv = sr > msrv ? sr : msrv;
-  }
-  for (int off = 16; off; off >>= 1) {
-    tm += __shfl_xor_sync(0xffffffffu, tm, off);
-    msm = max(msm, __shfl_xor_sync(0xffffffffu, msm, off));
-    msv = max(msv, __shfl_xor_sync(0xffffffffu, msv, off));
-    msrv = max(msrv, __shfl_xor_sync(0xffffffffu, msrv, off));
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) { red[0][warp] = tm; red[1][warp] = msm; red[2][warp] = msv; red[3][warp] = msrv; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int nw = blockDim.x >> 5;
-    for (int w = 1; w < nw; w++) {
-      tm += red[0][w];
-      msm = max(msm, red[1][w]);
-      msv = max(msv, red[2][w]);
-      msrv = max(msrv, red[3][w]);
-    }
-    out[0] = (long long)M.acc[0];
-    out[1] = (long long)M.acc[1];
-    out[2] = tm;
-    out[3] = msm;
-    out[4] = msv;
-    out[5] = msrv;
-  }
+  metrics_final<false>(I, M, out);
 }
+
+// Up to this K the last CTA reduces the K x K bit matrix (K * K / 32 words) itself;
+// above, a second launch of 1024 threads does.
+constexpr int kMetricsOneLaunchK = 512;
+constexpr int kMetricsThreads = 256;
 
 }  // namespace
 
@@ -118,33 +148,37 @@ size_t metrics_scratch_bytes(int K) {
   return 64 + 2 * sizeof(long long) * (size_t)K + sizeof(uint32_t) * words * (size_t)K;
 }
 
-// `scratch` must hold metrics_scratch_bytes(K) bytes (zeroed here);
-// `out` receives 6 values on the device.
-cudaError_t launch_metrics(const DevInstance& I, void* scratch, long long* out, int num_sms, cudaStream_t st,
+// CTAs of the evaluation of noe nets.
+int metrics_grid(int K, int noe, int num_sms) {
+  const size_t smem = 2 * sizeof(long long) * (size_t)K;
+  if (smem > 48 * 1024)
+    cudaFuncSetAttribute(metrics_nets_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int per_sm = 1;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, metrics_nets_kernel, kMetricsThreads, smem);
+  const long long want = ((long long)noe + kMetricsThreads / 32 - 1) / (kMetricsThreads / 32);
+  return (int)std::max(1ll, std::min((long long)num_sms * std::max(per_sm, 1), want));
+}
+
+// `scratch` must hold metrics_scratch_bytes(K) bytes, zeroed before the first
+// call; `grid` from metrics_grid; `out` receives 6 values (device or pinned host
+// memory).
+cudaError_t launch_metrics(const DevInstance& I, void* scratch, long long* out, int grid, cudaStream_t st,
                            int* launches) {
   const int K = I.K;
-  const size_t words = (size_t)(K + 31) / 32;
   MetricScratch M;
   unsigned char* b = static_cast<unsigned char*>(scratch);
   M.acc = reinterpret_cast<unsigned long long*>(b);
   M.send = reinterpret_cast<long long*>(b + 64);
   M.recv = M.send + K;
   M.pairs = reinterpret_cast<uint32_t*>(M.recv + K);
-  cudaError_t err = cudaMemsetAsync(scratch, 0, 64 + 2 * sizeof(long long) * K + sizeof(uint32_t) * words * K, st);
-  if (err != cudaSuccess) return err;
-  const int threads = 256;
-  const size_t smem = 2 * sizeof(long long) * (size_t)K;
-  err = cudaFuncSetAttribute(metrics_nets_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (err != cudaSuccess) return err;
-  int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, metrics_nets_kernel, threads, smem);
-  if (per_sm < 1) per_sm = 1;
-  long long want = ((long long)I.noe + (threads / 32) - 1) / (threads / 32);
-  long long grid = (long long)num_sms * per_sm;
-  if (grid > want) grid = want > 0 ? want : 1;
-  metrics_nets_kernel<<<(int)grid, threads, smem, st>>>(I, M);
-  metrics_final_kernel<<<1, 1024, 0, st>>>(I, M, out);
-  if (launches) *launches = 2;
+  const bool one = K <= kMetricsOneLaunchK;
+  if (!one) {
+    const cudaError_t err = cudaMemsetAsync(scratch, 0, metrics_scratch_bytes(K), st);
+    if (err != cudaSuccess) return err;
+  }
+  metrics_nets_kernel<<<grid, kMetricsThreads, 2 * sizeof(long long) * (size_t)K, st>>>(I, M, out, one);
+  if (!one) metrics_final_kernel<<<1, 1024, 0, st>>>(I, M, out);
+  if (launches) *launches = one ? 1 : 2;
   return cudaGetLastError();
 }
 
