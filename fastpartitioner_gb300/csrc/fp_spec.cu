@@ -955,16 +955,15 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
       if (blockIdx.x == 0 && threadIdx.x == 0) B.stats[20] += gtimer() - tA;
       pass_start = false;
       prev_maxtouch = false;
-      while (hidx < B.nheavy && __ldg(&B.heavy_pos[hidx]) < pos) hidx++;
-      midx += lower_bound_pos(B.mid_pos + midx, min(B.nmid - midx, B.wmax), pos);
+      hidx = seek_pos(B.heavy_pos, B.nheavy, hidx, pos);
+      midx = seek_pos(B.mid_pos, B.nmid, midx, pos);
 
       // ================================================================= round
       // A window holds up to gmax whole-grid vertices and ends before the next
       // one.
       int end_w = min(pos + W, B.npos);
       if (hidx + B.gmax < B.nheavy) end_w = min(end_w, (int)__ldg(&B.heavy_pos[hidx + B.gmax]));
-      int ns = 0;
-      while (ns < B.gmax && hidx + ns < B.nheavy && __ldg(&B.heavy_pos[hidx + ns]) < end_w) ns++;
+      const int ns = min(B.gmax, seek_pos(B.heavy_pos, B.nheavy, hidx, end_w) - hidx);
       const int span = end_w - pos;
       // (a short window fills the first CTAs' warps: spread over all CTAs it kept
       // those of the medium vertices waiting, MSRV 51.6 -> 59 us per window)
@@ -1135,7 +1134,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
       // the grid (a CTA with several among its own positions held the window up)
       __syncthreads();
       const long long cM = clock64();
-      const int mend = midx + lower_bound_pos(B.mid_pos + midx, min(B.nmid - midx, span), end_w);
+      const int mend = seek_pos(B.mid_pos, B.nmid, midx, end_w);
       const int mi0 = midx + (int)(gridDim.x - 1 - blockIdx.x);
       for (int mi = mi0; mi < mend; mi += gridDim.x)
         cta_eval_ldg(I, B, R, metric, __ldg(&B.mid_pos[mi]), pos, par, sb, cnt_b, first_b, gains_b, losses_b,

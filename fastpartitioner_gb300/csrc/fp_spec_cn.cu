@@ -378,15 +378,15 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_cn_kernel(DevInstance I, Sp
     const bool logp = I.recs != nullptr && it == passes - 1;
     int pos = 0;
     int W = min(nwarps * 4, B.wmax);
-    int hidx = 0;
+    int hidx = 0, midx = 0;
     while (pos < I.noe) {
       const int par = round & 1;
       // a window holds up to gmax nets evaluated by the grid and ends before the next
-      while (hidx < B.nheavy && __ldg(&B.heavy_pos[hidx]) < pos) hidx++;
+      hidx = seek_pos(B.heavy_pos, B.nheavy, hidx, pos);
+      midx = seek_pos(B.mid_pos, B.nmid, midx, pos);
       int end_w = min(pos + W, I.noe);
       if (hidx + B.gmax < B.nheavy) end_w = min(end_w, (int)__ldg(&B.heavy_pos[hidx + B.gmax]));
-      int ns = 0;
-      while (ns < B.gmax && hidx + ns < B.nheavy && __ldg(&B.heavy_pos[hidx + ns]) < end_w) ns++;
+      const int ns = min(B.gmax, seek_pos(B.heavy_pos, B.nheavy, hidx, end_w) - hidx);
       const int hp = heavy_round & 1;
       // slot j of this parity in hmisc: [0] uncut witness + 1 (0: none), [1] conflict
       auto hm = [&](int j) { return B.hmisc + (hp * kMaxGridVerts + j) * 8; };
@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_cn_kernel(DevInstance I, Sp
       // nets with many pins of this CTA's positions: the whole CTA each
       const int cz0 = min(pos + blockIdx.x * kSWarps * q, end_w);
       const int cz1 = min(cz0 + kSWarps * q, end_w);
-      for (int mi = lower_bound_pos(B.mid_pos, B.nmid, cz0); mi < B.nmid; mi++) {
+      for (int mi = seek_pos(B.mid_pos, B.nmid, midx, cz0); mi < B.nmid; mi++) {
         const int e = __ldg(&B.mid_pos[mi]);
         if (e >= cz1) break;
         cn_eval_cta(I, B, e, e - pos, round, par, logp);
@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_cn_kernel(DevInstance I, Sp
         }
       }
       __syncthreads();
-      for (int mi = lower_bound_pos(B.mid_pos, B.nmid, cz0); mi < B.nmid; mi++) {
+      for (int mi = seek_pos(B.mid_pos, B.nmid, midx, cz0); mi < B.nmid; mi++) {
         const int e = __ldg(&B.mid_pos[mi]);
         if (e >= cz1) break;
         cn_validate_cta(I, B, e, e - pos, round, nact, &B.ctl[par]);

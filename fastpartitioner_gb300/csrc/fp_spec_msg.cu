@@ -553,16 +553,15 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
         okm_set = true;
       }
       const MsgRound Rd{sizes_s, msgs_s, maxl_s, msm ? s_nmax : 0, msm ? s_mx : 0};
-      while (hidx < B.nheavy && __ldg(&B.heavy_pos[hidx]) < pos) hidx++;
-      midx += lower_bound_pos(B.mid_pos + midx, min(B.nmid - midx, B.wmax_msg), pos);
+      hidx = seek_pos(B.heavy_pos, B.nheavy, hidx, pos);
+      midx = seek_pos(B.mid_pos, B.nmid, midx, pos);
 
       // ================================================================= round
       // A window holds up to gmax whole-grid vertices and ends before the next
       // one, or at its first mover.
       int end_w = min(pos + W, I.nov);
       if (hidx + B.gmax < B.nheavy) end_w = min(end_w, (int)__ldg(&B.heavy_pos[hidx + B.gmax]));
-      int ns = 0;
-      while (ns < B.gmax && hidx + ns < B.nheavy && __ldg(&B.heavy_pos[hidx + ns]) < end_w) ns++;
+      int ns = min(B.gmax, seek_pos(B.heavy_pos, B.nheavy, hidx, end_w) - hidx);
       const int hp = heavy_round & 1;   // whole-grid sets, double-buffered by parity
       // slot j of this parity: K words at hslot(j) (receivers in hloss, senders in
       // hadelta, first non-source nets in hfirst), 8 words of hmisc at hmslot(j)
@@ -667,7 +666,7 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
         }
       }
       // medium vertices of the window: one CTA each, dealt out from the end of the grid
-      const int mend = midx + lower_bound_pos(B.mid_pos + midx, min(B.nmid - midx, span), end_w);
+      const int mend = seek_pos(B.mid_pos, B.nmid, midx, end_w);
       for (int mi = midx + (int)(gridDim.x - 1 - blockIdx.x); mi < mend; mi += gridDim.x) {
         const int v = __ldg(&B.mid_pos[mi]);
         __syncthreads();

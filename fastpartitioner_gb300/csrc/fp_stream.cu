@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
     __syncthreads();
     block_min_part(sizes_s, K, uscr, &s_minpart, &s_minsize, &s_second);
     __syncthreads();
-    while (hidx < S.nheavy && __ldg(&S.heavy_pos[hidx]) < pos) hidx++;
+    hidx = seek_pos(S.heavy_pos, S.nheavy, hidx, pos);
     if (hidx < S.nheavy && __ldg(&S.heavy_pos[hidx]) == pos) {
       // ================================================ a vertex with many nets
       const int v = __ldg(&S.porder[pos]);
@@ -466,18 +466,8 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_ldg_kernel(DevInstance I,
     // the positions with long lists: each gets an equal team of the CTAs (from
     // the end of the grid, a share of its nets per CTA), or, in a window with
     // more than kStreamTeams of them, a CTA
-    while (mi0 < S.nmid) {   // those before pos are placed
-      const unsigned m = __ballot_sync(kAll, mi0 + lane < S.nmid && __ldg(&S.mid_pos[min(mi0 + lane, S.nmid - 1)]) < pos);
-      mi0 += __popc(m);
-      if (m != kAll) break;
-    }
-    int nmid = 0;
-    while (mi0 + nmid < S.nmid) {
-      const int i = mi0 + nmid + lane;
-      const unsigned m = __ballot_sync(kAll, i < S.nmid && __ldg(&S.mid_pos[min(i, S.nmid - 1)]) < end_w);
-      nmid += __popc(m);
-      if (m != kAll) break;
-    }
+    mi0 = seek_pos(S.mid_pos, S.nmid, mi0, pos);
+    const int nmid = seek_pos(S.mid_pos, S.nmid, mi0, end_w) - mi0;
     const bool teams = nmid <= min(kStreamTeams, (int)gridDim.x);
     const int tsize = teams && nmid ? (int)gridDim.x / nmid : 1;
     const int bmid = (int)(gridDim.x - 1 - blockIdx.x);
@@ -1086,7 +1076,7 @@ __global__ void __launch_bounds__(kSThreads, 2) stream_msg_kernel(DevInstance I,
     __syncthreads();
     block_min_part(sizes_s, K, uscr, &s_minpart, &s_minsize, &s_second);
     __syncthreads();
-    while (hidx < S.nheavy && __ldg(&S.heavy_pos[hidx]) < pos) hidx++;
+    hidx = seek_pos(S.heavy_pos, S.nheavy, hidx, pos);
     if (hidx < S.nheavy && __ldg(&S.heavy_pos[hidx]) == pos) {
       // ======================= a vertex with many nets: CTA 0 places it alone
       if (blockIdx.x == 0) {
