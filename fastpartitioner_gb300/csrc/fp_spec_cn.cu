@@ -282,28 +282,44 @@ __device__ int cn_eval(const DevInstance& I, const SpecBuf& B, int e, int* oldp_
   return *uncut < 0 ? 1 : 0;
 }
 
-// k moves oldp -> newp of pins of net x, each the reference's REMOVAL then
-// ADDING on x's list (CN/partition.cpp:311-370), applied at once by one warp:
-// the lanes find the two slots, lane 0 replays the k steps.  Only the first
-// step can append newp and only the last can remove oldp, so the k-fold result
-// follows from the counts.
-__device__ void cn_apply_net(const DevInstance& I, int x, int oldp, int newp, int k) {
+// A net's list where it lies, or staged in shared memory.
+struct ListHere {
+  const DevInstance& I;
+  int s;
+  __device__ int part(int j) const { return lds(&I.ep_part[s + j]); }
+  __device__ int cnt(int j) const { return lds(&I.ep_cnt[s + j]); }
+  __device__ void set_part(int j, int p) const { I.ep_part[s + j] = p; }
+  __device__ void set_cnt(int j, int c) const { I.ep_cnt[s + j] = c; }
+};
+struct ListStaged {
+  int2* l;
+  __device__ int part(int j) const { return l[j].x; }
+  __device__ int cnt(int j) const { return l[j].y; }
+  __device__ void set_part(int j, int p) const { l[j].x = p; }
+  __device__ void set_cnt(int j, int c) const { l[j].y = c; }
+};
+
+// k moves oldp -> newp of pins of a net with list L (n parts, room for cap), each
+// the reference's REMOVAL then ADDING (CN/partition.cpp:311-370), applied at once
+// by one warp: the lanes find the two slots, lane 0 replays the k steps.  Only
+// the first step can append newp and only the last can remove oldp, so the
+// k-fold result follows from the counts.  Returns the new length (every lane).
+template <class List>
+__device__ int cn_apply_moves(const DevInstance& I, const List& L, int n, int cap, int oldp, int newp, int k) {
   const int lane = threadIdx.x & 31;
-  const int s = (int)__ldg(&I.nptr[x]);
-  const int cap = (int)__ldg(&I.nptr[x + 1]) - s;
-  int n = lds(&I.ep_len[x]);
   int jo = -1, jd = -1;
   for (int j0 = 0; j0 < n; j0 += 32) {
     const int j = j0 + lane;
-    const int p = j < n ? lds(&I.ep_part[s + j]) : -1;
+    const int p = j < n ? L.part(j) : -1;
     const unsigned mo = __ballot_sync(kAll, p == oldp);
     const unsigned md = __ballot_sync(kAll, p == newp);
     if (mo && jo < 0) jo = j0 + __ffs(mo) - 1;
     if (md && jd < 0) jd = j0 + __ffs(md) - 1;
   }
+  __syncwarp();
   if (lane == 0) {
-    int co = jo >= 0 ? lds(&I.ep_cnt[s + jo]) : 0;
-    int cd = jd >= 0 ? lds(&I.ep_cnt[s + jd]) : 0;
+    int co = jo >= 0 ? L.cnt(jo) : 0;
+    int cd = jd >= 0 ? L.cnt(jd) : 0;
     if (jo < 0 || n > cap || co < k || k < 1) {
       dev_fail(I.status, kDevErrInvalid);
     } else {
@@ -313,15 +329,15 @@ __device__ void cn_apply_net(const DevInstance& I, int x, int oldp, int newp, in
         const int last = n - 1;
         if (last != jo) {
           if (last == jd) {
-            I.ep_part[s + jo] = newp;
+            L.set_part(jo, newp);
             jd = jo;
           } else {
-            I.ep_part[s + jo] = lds(&I.ep_part[s + last]);
-            I.ep_cnt[s + jo] = lds(&I.ep_cnt[s + last]);
+            L.set_part(jo, L.part(last));
+            L.set_cnt(jo, L.cnt(last));
           }
         }
-        I.ep_part[s + last] = -1;
-        I.ep_cnt[s + last] = 0;
+        L.set_part(last, -1);
+        L.set_cnt(last, 0);
         n = last;
         jo = -1;
       };
@@ -329,7 +345,7 @@ __device__ void cn_apply_net(const DevInstance& I, int x, int oldp, int newp, in
         if (n >= cap) { ok = false; return; }
         jd = n;
         cd = 1;
-        I.ep_part[s + jd] = newp;
+        L.set_part(jd, newp);
         n++;
       };
       if (jd >= 0) {
@@ -351,14 +367,79 @@ __device__ void cn_apply_net(const DevInstance& I, int x, int oldp, int newp, in
       if (!ok) {
         dev_fail(I.status, kDevErrInvalid);
       } else {
-        if (jo >= 0) I.ep_cnt[s + jo] = co;
-        I.ep_cnt[s + jd] = cd;
-        I.ep_len[x] = n;
+        if (jo >= 0) L.set_cnt(jo, co);
+        L.set_cnt(jd, cd);
       }
     }
   }
   __syncwarp();
+  return __shfl_sync(kAll, n, 0);
 }
+
+// The same on net x's list in global memory.
+__device__ void cn_apply_net(const DevInstance& I, int x, int oldp, int newp, int k) {
+  const int s = (int)__ldg(&I.nptr[x]);
+  const int cap = (int)__ldg(&I.nptr[x + 1]) - s;
+  const int n = cn_apply_moves(I, ListHere{I, s}, lds(&I.ep_len[x]), cap, oldp, newp, k);
+  if ((threadIdx.x & 31) == 0) I.ep_len[x] = n;
+  __syncwarp();
+}
+
+// The moves of several acting nets on net x in their order: k0 of the first one
+// (pk0: old and new part), then those listed in cn_more (nmore entries), one warp.
+// The list is staged in shared memory (list) and the acting nets gathered once
+// (acts): a shared net of 262144 Zipf vertices (K = 256) has dozens, and each took
+// a scan of cn_more and of the list in L2: 53 us of commit per window, 28 so.
+// False if either does not fit.
+constexpr int kCnStage = 256, kCnActs = 256;
+__device__ bool cn_apply_shared(const DevInstance& I, const SpecBuf& B, int x, int pk0, int k0, int nmore, int2* list,
+                                int2* acts) {
+  const int lane = threadIdx.x & 31;
+  int na = 0;
+  for (int i0 = 0; i0 < nmore; i0 += 32) {
+    const int2 m2 = i0 + lane < nmore ? lds(&B.cn_more[i0 + lane]) : make_int2(-1, 0);
+    const unsigned m = __ballot_sync(kAll, m2.x == x);
+    const int at = na + __popc(m & ((1u << lane) - 1u));
+    if (m2.x == x && at < kCnActs) acts[at] = make_int2(m2.y, lds(&B.dec[m2.y]));
+    na += __popc(m);
+  }
+  const int s = (int)__ldg(&I.nptr[x]);
+  const int cap = (int)__ldg(&I.nptr[x + 1]) - s;
+  const int n0 = lds(&I.ep_len[x]);
+  const int room = min(min(cap, I.K), n0 + na + 1);   // each acting net adds a part at most
+  if (na > kCnActs || n0 > cap || room > kCnStage) return false;
+  for (int j = lane; j < room; j += 32) list[j] = j < n0 ? make_int2(lds(&I.ep_part[s + j]), lds(&I.ep_cnt[s + j])) : make_int2(-1, 0);
+  __syncwarp();
+  const ListStaged L{list};
+  int n = cn_apply_moves(I, L, n0, room, pk0 >> 16, pk0 & 0xffff, k0);
+  for (int last = -1;;) {
+    int o = kNone, c = 0, pk = 0;
+    for (int j = lane; j < na; j += 32) {
+      const int2 t = acts[j];
+      if (t.x <= last || t.x > o) continue;
+      c = t.x == o ? c + 1 : 1;
+      o = t.x;
+      pk = t.y;
+    }
+    const int o1 = warp_min(o);
+    if (o1 == kNone) break;
+    pk = __shfl_sync(kAll, pk, __ffs(__ballot_sync(kAll, o == o1)) - 1);
+    n = cn_apply_moves(I, L, n, room, pk >> 16, pk & 0xffff, warp_sum(o == o1 ? c : 0));
+    last = o1;
+  }
+  for (int j = lane; j < max(n, n0); j += 32) {
+    I.ep_part[s + j] = list[j].x;
+    I.ep_cnt[s + j] = list[j].y;
+  }
+  if (lane == 0) I.ep_len[x] = n;
+  __syncwarp();
+  return true;
+}
+
+// A window that moves few pins (27 on average on 262144 Zipf vertices) spreads
+// each one's nets over the warps: a hub's thousands of nets took one warp 60 us,
+// C1 takes 10 so.  More pins keep the warps busy as they are.
+constexpr int kCnSpreadMoves = 256, kCnChunk = 128, kCnStep = 37;
 
 // Three CTAs per SM: without the hint the compiler spills to fit more.
 __global__ void __launch_bounds__(kSThreads, 3) spec_cn_kernel(DevInstance I, SpecBuf B, int passes) {
@@ -372,6 +453,8 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_cn_kernel(DevInstance I, Sp
   int round = 1;   // claims of round 0 (the cleared array) never match
   int heavy_round = 0;
   __shared__ int s_gc[kMaxGridVerts];
+  __shared__ int2 list_b[kSWarps * kCnStage];   // per-warp staged list and acting nets of a shared net
+  __shared__ int2 acts_b[kSWarps * kCnActs];
   for (int it = 0; it < passes; it++) {
     // decision records of the last pass: (new part, pins moved, old part,
     // acting) of a two-part net, (-1, 0, -1, 0) of any other net
@@ -528,13 +611,9 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_cn_kernel(DevInstance I, Sp
       }
       // ---- C1: pins of acting nets before the cut: part, sizes, moves per net
       const int nmv = lds(&B.cn_cnt[par]);
-      for (int i = gw; i < nmv; i += nwarps) {
-        const int2 mv = lds(&B.cn_moved[i]);
-        if (pos + mv.y >= cut) continue;
-        const int u = mv.x;
+      auto move_nets = [&](int2 mv, uint32_t j0, uint32_t j1) {
         const int pk = lds(&B.dec[mv.y]);
-        const uint32_t ub = __ldg(&I.vptr[u]), ue = __ldg(&I.vptr[u + 1]);
-        for (uint32_t j = ub + lane; j < ue; j += 32) {
+        for (uint32_t j = j0 + lane; j < j1; j += 32) {
           const int x = (int)__ldg(&I.vnets[j]);
           // the first acting net that claimed x counts its moves on it; those of
           // the others are listed (kShared marks the net)
@@ -547,14 +626,49 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_cn_kernel(DevInstance I, Sp
             B.cn_more[atomicAdd(&B.cn_cnt[4 + par], 1)] = make_int2(x, mv.y);
           }
         }
-        if (lane == 0) {
-          const int oldp = pk >> 16, newp = pk & 0xffff;
-          I.part_vec[u] = newp;
-          const int wv = __ldg(&I.w[u]);
-          atomicAdd(&I.part_sizes[oldp], -wv);
-          atomicAdd(&I.part_sizes[newp], wv);
-          atomicAdd((unsigned long long*)&I.moves[it], 1ull);
-          atomicAdd(&B.stats[2], 1ull);
+      };
+      auto move_pin = [&](int2 mv) {
+        const int u = mv.x, pk = lds(&B.dec[mv.y]);
+        const int oldp = pk >> 16, newp = pk & 0xffff;
+        I.part_vec[u] = newp;
+        const int wv = __ldg(&I.w[u]);
+        atomicAdd(&I.part_sizes[oldp], -wv);
+        atomicAdd(&I.part_sizes[newp], wv);
+        atomicAdd((unsigned long long*)&I.moves[it], 1ull);
+        atomicAdd(&B.stats[2], 1ull);
+      };
+      if (nmv > kCnSpreadMoves) {
+        for (int i = gw; i < nmv; i += nwarps) {
+          const int2 mv = lds(&B.cn_moved[i]);
+          if (pos + mv.y >= cut) continue;
+          move_nets(mv, __ldg(&I.vptr[mv.x]), __ldg(&I.vptr[mv.x + 1]));
+          if (lane == 0) move_pin(mv);
+        }
+      } else {
+        // few pins: kCnChunk nets of one per warp, chunk c of pin i to warp
+        // i * kCnStep + c; the lanes look for this warp's chunks among 32 pins
+        for (int i0 = 0; i0 < nmv; i0 += 32) {
+          const int i = i0 + lane;
+          int2 mv = make_int2(0, 0);
+          uint32_t ub = 0, ue = 0;
+          bool mine = false;
+          if (i < nmv) {
+            mv = lds(&B.cn_moved[i]);
+            ub = __ldg(&I.vptr[mv.x]);
+            ue = __ldg(&I.vptr[mv.x + 1]);
+            mine = pos + mv.y < cut;
+          }
+          const int c0 = (gw + nwarps - i * kCnStep % nwarps) % nwarps;
+          mine = mine && (c0 == 0 || c0 * (long long)kCnChunk < (long long)(ue - ub));
+          for (unsigned m = __ballot_sync(kAll, mine); m; m &= m - 1) {
+            const int src = __ffs(m) - 1;
+            const int2 mvs = make_int2(__shfl_sync(kAll, mv.x, src), __shfl_sync(kAll, mv.y, src));
+            const uint32_t b = __shfl_sync(kAll, ub, src), e = __shfl_sync(kAll, ue, src);
+            const int c1 = __shfl_sync(kAll, c0, src);
+            for (long long c = c1; b + c * kCnChunk < e; c += nwarps)
+              move_nets(mvs, (uint32_t)(b + c * kCnChunk), (uint32_t)min((long long)e, b + (c + 1) * kCnChunk));
+            if (c1 == 0 && lane == 0) move_pin(mvs);
+          }
         }
       }
       if (!grid_barrier(B.bar, I.status)) return;
@@ -563,11 +677,12 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_cn_kernel(DevInstance I, Sp
       for (int i = gw; i < nnet; i += nwarps) {
         const int2 xe = lds(&B.cn_nets[i]);
         const int k = lds(&B.cn_kcnt[xe.x]);
-        cn_apply_net(I, xe.x, xe.y >> 16, xe.y & 0xffff, k & (kShared - 1));
-        if (k & kShared) {
+        const int nmore = (k & kShared) ? lds(&B.cn_cnt[4 + par]) : 0;
+        if (!(k & kShared) ||
+            !cn_apply_shared(I, B, xe.x, xe.y, k & (kShared - 1), nmore, list_b + wib * kCnStage, acts_b + wib * kCnActs)) {
+          cn_apply_net(I, xe.x, xe.y >> 16, xe.y & 0xffff, k & (kShared - 1));
           // the other acting nets' moves on it, in their order
-          const int nmore = lds(&B.cn_cnt[4 + par]);
-          for (int last = -1;;) {
+          for (int last = -1; k & kShared;) {
             int o = kNone, c = 0;
             for (int i2 = lane; i2 < nmore; i2 += 32) {
               const int2 m2 = lds(&B.cn_more[i2]);
