@@ -990,7 +990,9 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
       __syncthreads();
       // ---- A1: tally slices of the whole-grid vertices by their teams of CTAs,
       // one set of arrays per CTA
-      if (wib == 0 && ns) team_split(ns, s_gd, gridDim.x, s_t0, s_t1);
+      const int mend = seek_pos(B.mid_pos, B.nmid, midx, end_w);
+      if (wib == 0 && ns)
+        team_split(ns, s_gd, gridDim.x, (span + kSWarps * q - 1) / (kSWarps * q), mend - midx, s_t0, s_t1);
       __syncthreads();
       auto in_team = [&](int j) { return (int)blockIdx.x >= s_t0[j] && (int)blockIdx.x < s_t1[j]; };
       auto leads = [&](int j) { return (int)blockIdx.x == s_t0[j]; };
@@ -1134,7 +1136,6 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
       // the grid (a CTA with several among its own positions held the window up)
       __syncthreads();
       const long long cM = clock64();
-      const int mend = seek_pos(B.mid_pos, B.nmid, midx, end_w);
       const int mi0 = midx + (int)(gridDim.x - 1 - blockIdx.x);
       for (int mi = mi0; mi < mend; mi += gridDim.x)
         cta_eval_ldg(I, B, R, metric, __ldg(&B.mid_pos[mi]), pos, par, sb, cnt_b, first_b, gains_b, losses_b,

