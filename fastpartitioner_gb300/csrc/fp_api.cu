@@ -61,34 +61,38 @@ static bool spec_supported(int metric, int K, int max_smem, int nov, int noe) {
 // eventual cut (first mover for TM / MSM) is evaluated again, so the bounds
 // follow from how early a metric's windows end.
 // Sweeps on Zipf workloads (K = 256, degree weights; milliseconds for the passes
-// swept, (super bound, vertices per window)):
-//   TV   1M vertices   (65536, 32) 14.9   (262144, 8) 17.4   (32768, 32) 21.0
-//   MSRV 256K          (16384, 16) 31.1   (32768, 4) 36.5    (65536, 16) 36.5
-//   MSV  256K          (32768, 4) 180     (16384, 2) 183     (262144, 2) 216
-//   TM   256K          (16384, 16) 56.1   (65536, 4) 66.8    (8192, 32) 57.2
-//                      and with light work up to 1024 52.6, 512 52.4
-//   MSM  1M            (262144, 16) 0.94  (65536, 32) 1.74
-constexpr int kLightWork = 2048, kLightWorkTm = 1024;
+// in brackets at (light bound, super bound, vertices per window)):
+//   TV   1M   [3]   (2048, 65536, 32) 15.5    (2048, 32768, 32) 21.1    (2048, 65536, 16) 21.0
+//   MSRV 256K [10]  (2048, 32768, 32) 42-63   (2048, 16384, 16) 57-68   (1024, 32768, 32) 45-66
+//   MSV  256K [3]   (1024, 16384, 4) 305-370  (2048, 32768, 4) 312-379  (1024, 8192, 8) 306-372
+//   TM   256K [5]   (512, 8192, 32) 41-49     (1024, 16384, 16) 44-52   (512, 4096, 16) 52-57
+//   MSM  1M         (2048, 262144, 16) 0.94   (2048, 65536, 32) 1.74
+constexpr int kLightWork = 2048, kLightWorkMsv = 1024, kLightWorkTm = 512;
 constexpr int kCnLightPins = 128;   // CN: nets with more pins are evaluated by one CTA,
 constexpr int kCnGridPins = 1024;   //     with more than this by the whole grid
 int default_light_work(int metric) {
-  return metric == FP_METRIC_CN ? kCnLightPins : metric == FP_METRIC_TM ? kLightWorkTm : kLightWork;
+  switch (metric) {
+    case FP_METRIC_CN: return kCnLightPins;
+    case FP_METRIC_TM: return kLightWorkTm;
+    case FP_METRIC_MSV: return kLightWorkMsv;
+    default: return kLightWork;
+  }
 }
 int default_super_work(int metric) {
   switch (metric) {
     case FP_METRIC_CN: return kCnGridPins;
     case FP_METRIC_TV: return 65536;
-    case FP_METRIC_MSV: return 32768;
-    case FP_METRIC_MSRV:
-    case FP_METRIC_TM: return 16384;
+    case FP_METRIC_MSV: return 16384;
+    case FP_METRIC_MSRV: return 32768;
+    case FP_METRIC_TM: return 8192;
     default: return 262144;
   }
 }
 int default_grid_verts(int metric) {
   switch (metric) {
-    case FP_METRIC_TV: return kMaxGridVerts;
+    case FP_METRIC_TV:
     case FP_METRIC_MSRV:
-    case FP_METRIC_TM:
+    case FP_METRIC_TM: return kMaxGridVerts;
     case FP_METRIC_MSM: return 16;
     case FP_METRIC_CN: return kCnGridNets;
     default: return 4;
