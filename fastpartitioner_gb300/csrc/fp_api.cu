@@ -63,7 +63,8 @@ static bool spec_supported(int metric, int K, int max_smem, int nov, int noe) {
 // Sweeps on Zipf workloads (K = 256, degree weights; milliseconds for the passes
 // in brackets at (light bound, super bound, vertices per window)):
 //   TV   1M   [3]   (2048, 65536, 32) 15.5    (2048, 32768, 32) 21.1    (2048, 65536, 16) 21.0
-//   MSRV 256K [10]  (2048, 32768, 32) 42-63   (2048, 16384, 16) 57-68   (1024, 32768, 32) 45-66
+//   MSRV 256K [10]  (2048, 24576, 16) 51-53   (2048, 16384, 16) 59      (2048, 32768, 32) 44-49
+//             [2]   (2048, 24576, 16) 20-34   (2048, 16384, 16) 20-30   (2048, 32768, 32) 23-37
 //   MSV  256K [3]   (1024, 16384, 4) 305-370  (2048, 32768, 4) 312-379  (1024, 8192, 8) 306-372
 //   TM   256K [5]   (512, 8192, 32) 41-49     (1024, 16384, 16) 44-52   (512, 4096, 16) 52-57
 //   MSM  1M         (2048, 262144, 16) 0.94   (2048, 65536, 32) 1.74
@@ -83,7 +84,7 @@ int default_super_work(int metric) {
     case FP_METRIC_CN: return kCnGridPins;
     case FP_METRIC_TV: return 65536;
     case FP_METRIC_MSV: return 16384;
-    case FP_METRIC_MSRV: return 32768;
+    case FP_METRIC_MSRV: return 24576;
     case FP_METRIC_TM: return 8192;
     default: return 262144;
   }
@@ -91,8 +92,8 @@ int default_super_work(int metric) {
 int default_grid_verts(int metric) {
   switch (metric) {
     case FP_METRIC_TV:
-    case FP_METRIC_MSRV:
     case FP_METRIC_TM: return kMaxGridVerts;
+    case FP_METRIC_MSRV:
     case FP_METRIC_MSM: return 16;
     case FP_METRIC_CN: return kCnGridNets;
     default: return 4;
@@ -570,7 +571,8 @@ static int build_positions(fp_instance* in) {
   for (int v = 0; v < g.nov; v++)
     if (g.vptr[v + 1] == g.vptr[v]) {
       any_iso = true;
-      if (pb.w[v] != 0) compact = false;
+      // (MSRV never moves one, whatever it weighs: 0 <= 0 fails on every max part)
+      if (pb.w[v] != 0 && pb.metric != FP_METRIC_MSRV) compact = false;
     }
   // Measured on Zipf workloads (degree weights): TV 75 -> 48 ms per pass (4M
   // vertices), MSV 243 -> 207 and MSRV 47.2 -> 45.3 (256K vertices, one and two

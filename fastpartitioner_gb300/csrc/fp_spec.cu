@@ -804,7 +804,15 @@ __device__ void cta_fix(const DevInstance& I, const SpecBuf& B, const RoundCtx& 
 // Changed decisions are taken at once, not walked, in a stretch longer than
 // this with at most so many of them: a walk costs about 2 us per 10 positions
 // it decides again, a validation of the whole window 12-25 us.
-constexpr int kJacobiSpan = 1024, kJacobiFlips = 64;
+// Up to kJacobiFew are tried so at first in any stretch (7564 uniform vertices, K =
+// 24, MSV: 9.7 -> 9.0 ms for three passes).
+constexpr int kJacobiSpan = 1024, kJacobiFlips = 64, kJacobiFew = 4;
+
+// MSRV: a window with more changed decisions than this ends behind its first
+// change of the max-volume parts: walking them costs more than a new window, and
+// most change nothing (three passes over 41936 mixed vertices of unit weight, K =
+// 32: 10.6 ms with every change walked, 8.5 so).
+constexpr int kWalkOverEvent = 8;
 
 // Two CTAs per SM: without the hint the compiler trades registers for a third
 // CTA and spills, which measured slower.
@@ -1693,6 +1701,10 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
           B.ctl[10 + ((vr & 1) ^ 1)] = 0;
         }
         vr++;
+        if (rv && sizes && nflip > kWalkOverEvent && vs_s.n > 0) {
+          fcut = min(fcut, ((pos + vs_s.at[0] + 1) << 3) | 4);
+          cutw = min(cutw, fcut);
+        }
         if (!sizes || (flipw >> 3) >= (cutw >> 3)) break;
         zf = flipw >> 3;
         const int zc = min(end_w, cutw >> 3);
@@ -1700,7 +1712,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
           cutw = flipw;
           break;
         }
-        const bool at_once = zc - zf > kJacobiSpan && nflip <= kJacobiFlips;
+        const bool at_once = (nfix == 0 && nflip <= kJacobiFew) || (zc - zf > kJacobiSpan && nflip <= kJacobiFlips);
         if (!at_once) {
           const unsigned long long tW = gtimer();
           if (blockIdx.x == 0)

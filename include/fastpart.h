@@ -180,15 +180,16 @@ int fp_set_engine(fp_instance* inst, int32_t engine);
 /* Tuning of the speculative engine (no effect on results).  TV / MSV / MSRV /
  * TM / MSM: a vertex whose work -- the sum over its nets of min(net size, K) --
  * is at most light_work is evaluated by one warp, at most super_work by one
- * CTA, above it by the whole grid.  Defaults: 2048 and 262144 (MSV 16384,
- * MSRV 32768, TM 65536).  CN: a net with more than light_work pins is evaluated
- * by one CTA, with more than super_work pins by the whole grid (defaults 128
- * and 1024). */
+ * CTA, above it by a team of CTAs.  Defaults: TV 2048 and 65536, MSV 1024 and
+ * 16384, MSRV 2048 and 24576, TM 512 and 8192, MSM 2048 and 262144.  CN: a net
+ * with more than light_work pins is evaluated by one CTA, with more than
+ * super_work pins by the whole grid (defaults 128 and 1024). */
 int fp_set_classes(fp_instance* inst, int64_t light_work, int64_t super_work);
-/* Tuning of the speculative engine's window lengths (no effect on results;
- * TV / MSV / MSRV): after a window ends early, the next one is `grow` times
- * the committed length, at least `min_len` positions (0: one per warp of the
- * grid).  Defaults 0 and 2 (MSV) or 4 (TV, MSRV). */
+/* Tuning of the speculative engine's window lengths (no effect on results):
+ * after a window ends early, the next one is `grow` times the committed length
+ * (TV / MSV / MSRV; TM / MSM always twice), at least a quarter of the last one and
+ * `min_len` positions (0: 128, TM 1024, MSM 512).  Defaults 0 and 2 (MSV) or 4 (TV,
+ * MSRV). */
 int fp_set_window(fp_instance* inst, int32_t min_len, int32_t grow);
 int fp_metrics(fp_instance* inst, int64_t out[6]);
 
@@ -272,25 +273,24 @@ int fp_debug_barrier_fault(fp_instance* inst, int32_t leave_at, int32_t poll_lim
 /* Statistics of the last fp_refine on the grid-wide engine (up to 48 values):
  * [0] windows, [1] whole-grid evaluations of heavy vertices (CN: nets), [2] moves
  * committed from windows, [3..8] windows ended by: nothing (fully valid), a
- * possibly stale TV marker, part-size drift, volume drift, a max-volume part
- * changing, a shared net; [9] vertices walked in windows; [16..19] nanoseconds
+ * possibly stale TV marker, a changed decision that could not be redone, a changed
+ * MSV / MSRV accept outcome, more changes of the max-volume parts than a window
+ * keeps, a shared net; [9] vertices walked in windows; [16..19] nanoseconds
  * in evaluate, validate, commit phases and (TM / MSM) whole-grid decisions; TV / MSV /
  * MSRV also: [20] nanoseconds computing the round state, [21] / [23] SM cycles
  * summed over windows of the slowest warp / CTA evaluation, [25] / [26] SM
  * cycles and count of warp evaluations, [27] / [28] windows ended by an earlier
- * mover changing the count of the position's own part on a shared net / by a
- * part-set change after earlier count changes ([8] then counts part-set
- * changes only), [29..31] SM cycles of CTA evaluations in tally, decision and
- * the rest; nanoseconds summed over windows of: [32] the slowest CTA's
+ * mover changing the count of the position's own part on a shared net ([8] then
+ * counts part-set changes only) / unused, [29..31] SM cycles of CTA evaluations
+ * in tally, decision and the rest; nanoseconds summed over windows of: [32] the slowest CTA's
  * evaluation of its own positions (light and medium), [33] the whole-grid
  * vertices' decision and accept phases, [34] the slowest CTA's tally of
  * whole-grid vertex slices, [35] the slowest CTA's validation; [40] CTA
  * evaluations; [41..43] SM cycles of warp evaluations in tally, decision and
- * the rest; [44] decisions fixed inside a window (MSV / MSRV); [45..47]
- * nanoseconds summed over CTAs and validation passes in prefix sums, light
- * positions and the rest (medium and whole-grid vertices).  The per-warp and
- * per-CTA timings ([21..26], [29..43] except the [33] phase time, [45..47]) are
- * collected only by a library built with FP_TIMING_STATS defined, and are zero
+ * the rest; [44] decisions changed inside a window; [45] nanoseconds of the walks
+ * over changed decisions; [35], [46], [47] unused.  The per-warp and per-CTA
+ * timings ([21..26], [29..43] except the [33] phase time) are collected only by a
+ * library built with FP_TIMING_STATS defined, and are zero
  * otherwise. */
 int fp_get_stats(fp_instance* inst, int64_t* out, int32_t n);
 /* Number of kernel launches the last fp_refine / fp_metrics call enqueued. */
