@@ -811,8 +811,8 @@ constexpr int kJacobiSpan = 1024, kJacobiFlips = 64, kJacobiFew = 4;
 // MSRV: a window with more changed decisions than this ends behind its first
 // change of the max-volume parts: walking them costs more than a new window, and
 // most change nothing (three passes over 41936 mixed vertices of unit weight, K =
-// 32: 10.6 ms with every change walked, 8.5 so).
-constexpr int kWalkOverEvent = 8;
+// 32: 10.6 ms with every change walked, 8.6 so, 8.9 with none).
+constexpr int kWalkOverEvent = 4;
 
 // Two CTAs per SM: without the hint the compiler trades registers for a third
 // CTA and spills, which measured slower.
