@@ -101,7 +101,7 @@ int default_grid_verts(int metric) {
 }
 constexpr int kMaxSpecWarps = 16384;
 constexpr int kCtlWords = 16;   // SpecBuf::ctl
-int metrics_grid(int K, int noe, int num_sms);
+cudaError_t metrics_grid(int K, int noe, int num_sms, int* grid);
 cudaError_t launch_metrics(const DevInstance& I, void* scratch, long long* out, int grid, cudaStream_t st,
                            int* launches);
 }  // namespace fp
@@ -786,8 +786,9 @@ int fp_instance_create(fp_ctx* ctx, const fp_hypergraph* h, int32_t K, int32_t m
       in->dev_bytes += (long long)metrics_scratch_bytes(K);
     }
     in->metric_scratch = ms;
-    in->metric_grid = metrics_grid(K, g.noe, ctx->num_sms);
-    e = cudaMemsetAsync(ms, 0, metrics_scratch_bytes(K), ctx->stream);   // (each evaluation leaves it so)
+    e = metrics_grid(K, g.noe, ctx->num_sms, &in->metric_grid);
+    if (e == cudaSuccess)
+      e = cudaMemsetAsync(ms, 0, metrics_scratch_bytes(K), ctx->stream);   // (each evaluation leaves it zeroed)
     if (e != cudaSuccess) { fp_instance_destroy(in); return cuda_status(e); }
     in->sb.wmax = kSpecWindow;
     in->sb.ctab_mask = ldg ? (unsigned)(ctab - 1) : 0u;

@@ -148,15 +148,23 @@ size_t metrics_scratch_bytes(int K) {
   return 64 + 2 * sizeof(long long) * (size_t)K + sizeof(uint32_t) * words * (size_t)K;
 }
 
-// CTAs of the evaluation of noe nets.
-int metrics_grid(int K, int noe, int num_sms) {
+// CTAs of the evaluation of noe nets (*grid).  The kernel's static arrays count
+// against the 48 KB that a launch may have without the opt-in: it is due from K =
+// 3008 on, where the send and receive totals alone still fit.
+cudaError_t metrics_grid(int K, int noe, int num_sms, int* grid) {
   const size_t smem = 2 * sizeof(long long) * (size_t)K;
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(metrics_nets_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, metrics_nets_kernel, kMetricsThreads, smem);
+  cudaFuncAttributes a;
+  cudaError_t err = cudaFuncGetAttributes(&a, metrics_nets_kernel);
+  if (err == cudaSuccess && a.sharedSizeBytes + smem > 48 * 1024)
+    err = cudaFuncSetAttribute(metrics_nets_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int per_sm = 0;
+  if (err == cudaSuccess)
+    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, metrics_nets_kernel, kMetricsThreads, smem);
+  if (err != cudaSuccess) return err;
+  if (per_sm < 1) return cudaErrorInvalidConfiguration;
   const long long want = ((long long)noe + kMetricsThreads / 32 - 1) / (kMetricsThreads / 32);
-  return (int)std::max(1ll, std::min((long long)num_sms * std::max(per_sm, 1), want));
+  *grid = (int)std::max(1ll, std::min((long long)num_sms * per_sm, want));
+  return cudaSuccess;
 }
 
 // `scratch` must hold metrics_scratch_bytes(K) bytes, zeroed before the first

@@ -1,0 +1,23 @@
+"""fp_metrics at the part counts where its shared memory crosses the 48 KB that
+a launch may have without the opt-in (static and dynamic together: K = 3008 on;
+dynamic alone: K = 3073 on) and at the largest K, against the oracle."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def hg(fp):
+    return fp.generate(fp.GenSpec.column_net(6000, 2500, 2, 16, seed=91))
+
+
+def expected(orc, hg, K):
+    return orc.run_oracle(hg, K, "TV", 0)["metrics_init"]
+
+
+@pytest.mark.parametrize("K", (3007, 3008, 3072, 3073, 4096))
+def test_metrics_at_shared_memory_limits(orc, gpu_engine, hg, K):
+    with gpu_engine.instance(hg, K, "TV") as inst:
+        inst.initial_partition()
+        for _ in range(2):
+            assert inst.metrics() == expected(orc, hg, K)
