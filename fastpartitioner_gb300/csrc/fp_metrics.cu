@@ -15,6 +15,7 @@
 // arithmetic is integer and order-independent, hence exact.
 
 #include "fp_device.cuh"
+#include "fp_internal.h"
 #include "../../include/fastpart.h"
 
 #include <algorithm>
@@ -143,20 +144,23 @@ constexpr int kMetricsThreads = 256;
 
 }  // namespace
 
+// Dynamic shared memory of metrics_nets_kernel: a CTA's send and receive totals.
+static size_t metrics_smem_bytes(int K) { return 2 * sizeof(long long) * (size_t)K; }
+
 size_t metrics_scratch_bytes(int K) {
   const size_t words = (size_t)(K + 31) / 32;
   return 64 + 2 * sizeof(long long) * (size_t)K + sizeof(uint32_t) * words * (size_t)K;
 }
 
-// CTAs of the evaluation of noe nets (*grid).  The kernel's static arrays count
-// against the 48 KB that a launch may have without the opt-in: it is due from K =
-// 3008 on, where the send and receive totals alone still fit.
+// CTAs of the evaluation of noe nets (*grid).  Also raises the kernel's limit of
+// dynamic shared memory: the static arrays count against the 48 KB that a launch
+// may have without, so it is due from K = 3008 on.  The limit belongs to the
+// kernel on this device, not to an instance: it is always what the largest K
+// needs, whichever instance sets it last.
 cudaError_t metrics_grid(int K, int noe, int num_sms, int* grid) {
-  const size_t smem = 2 * sizeof(long long) * (size_t)K;
-  cudaFuncAttributes a;
-  cudaError_t err = cudaFuncGetAttributes(&a, metrics_nets_kernel);
-  if (err == cudaSuccess && a.sharedSizeBytes + smem > 48 * 1024)
-    err = cudaFuncSetAttribute(metrics_nets_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const size_t smem = metrics_smem_bytes(K);
+  cudaError_t err = cudaFuncSetAttribute(metrics_nets_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)metrics_smem_bytes(kMaxK));
   int per_sm = 0;
   if (err == cudaSuccess)
     err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, metrics_nets_kernel, kMetricsThreads, smem);
@@ -184,7 +188,7 @@ cudaError_t launch_metrics(const DevInstance& I, void* scratch, long long* out, 
     const cudaError_t err = cudaMemsetAsync(scratch, 0, metrics_scratch_bytes(K), st);
     if (err != cudaSuccess) return err;
   }
-  metrics_nets_kernel<<<grid, kMetricsThreads, 2 * sizeof(long long) * (size_t)K, st>>>(I, M, out, one);
+  metrics_nets_kernel<<<grid, kMetricsThreads, metrics_smem_bytes(K), st>>>(I, M, out, one);
   if (!one) metrics_final_kernel<<<1, 1024, 0, st>>>(I, M, out);
   if (launches) *launches = one ? 1 : 2;
   return cudaGetLastError();
