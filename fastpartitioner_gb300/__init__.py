@@ -594,7 +594,7 @@ class Instance:
                  grid_tally_ms=x[34] / 1e6, local_validate_ms=x[35] / 1e6, cta_evals=int(x[40]),
                  light_tally_cycles=int(x[41]), light_decide_cycles=int(x[42]), light_rest_cycles=int(x[43]),
                  window_fixes=int(x[44]), val_prefix_cta_ns=int(x[45]), val_light_cta_ns=int(x[46]),
-                 val_rest_cta_ns=int(x[47]))
+                 val_rest_cta_ns=int(x[47]), relisted=int(x[10]))
         return d
 
     def last_launches(self) -> int:

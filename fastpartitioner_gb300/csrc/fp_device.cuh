@@ -109,8 +109,8 @@ struct SpecBuf {
   int* dec;              // [wmax] (own part << 16) | decision per window offset
   unsigned char* flag;   // [wmax] bit0 mover, bit1 stale-marker risk, bit2 CTA / grid evaluated,
                          //     bit3 no nets, bit4 accepted, bit5 decision changed in the
-                         //     window, bit6 unused,
-                         //     bit7 the decision changes (dfix)
+                         //     window, bit6 has an entry in mlist, bit7 the decision
+                         //     changes (dfix)
   int* dfix;             // [wmax] the changed decision; the walk's with (predicted mover << 16)
   int* slack;            // [wmax] part-size drift the decision tolerates (-1: none)
   int* rel;              // [wmax] drift it tolerates beyond the window's validated movers

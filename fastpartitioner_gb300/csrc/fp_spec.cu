@@ -53,6 +53,7 @@ using namespace spec;
 
 constexpr int kTV = 1, kMSV = 4, kMSRV = 5;
 constexpr int kMaxWords = 4096 / 32;   // part masks of the largest K
+constexpr int kListed = 64;            // flag bit: the offset has an entry in mlist
 
 struct RoundCtx {
   const int* sizes;
@@ -308,11 +309,33 @@ __device__ __forceinline__ void claim_nets(const DevInstance& I, const SpecBuf& 
 }
 
 // Appends a mover of window offset o (weight wv, vn volume terms) to the
-// round's list.
-__device__ __forceinline__ void list_mover(const SpecBuf& B, int par, int o, int wv, int pk, int vn) {
+// round's list.  An offset is appended once per round (flag bit 6), so the list,
+// with an entry per offset, is long enough.
+__device__ __forceinline__ void list_mover(const DevInstance& I, const SpecBuf& B, int par, int o, int wv, int pk,
+                                           int vn) {
   const int i = atomicAdd(&B.mcnt[par], 1);
+  if (i >= B.wmax) {
+    atomicSub(&B.mcnt[par], 1);
+    dev_fail(I.status, kDevErrInvalid);
+    return;
+  }
   B.mlist[i] = make_int4(o, wv, pk, vn);
   B.midx[o] = i;
+}
+// The same for an offset decided again (fl: its flag before): a mover's entry is
+// replaced, also that of one that an earlier change of the window made stay.
+// Returns the flag bit of a listed offset.  (Not inlined: inside the kernel, whose
+// registers are all taken, its statistic cost MSRV on 262144 Zipf vertices 6%.)
+__device__ __noinline__ int relist_mover(const DevInstance& I, const SpecBuf& B, int par, int o, int fl, bool mover,
+                                         int wv, int pk, int vn) {
+  if (fl & kListed) {
+    B.mlist[lds(&B.midx[o])] = make_int4(o, mover ? wv : 0, pk, mover ? vn : 0);
+    if (mover && !(fl & 1)) atomicAdd(&B.stats[10], 1ull);
+    return kListed;
+  }
+  if (!mover) return 0;
+  list_mover(I, B, par, o, wv, pk, vn);
+  return kListed;
 }
 
 __device__ __forceinline__ void ctab_clear(const SpecBuf& B, uint2 sl) {
@@ -620,13 +643,13 @@ __device__ void cta_eval_ldg(const DevInstance& I, const SpecBuf& B, const Round
     claim_nets(I, B, vol, z, own, d, base, deg, threadIdx.x, blockDim.x, par);
     if (threadIdx.x == 0) {
       if (mt) atomicMin(&B.ctl[2 + par], z);
-      list_mover(B, par, o, __ldg(&I.w[v]), (own << 16) | d, nt);
+      list_mover(I, B, par, o, __ldg(&I.w[v]), (own << 16) | d, nt);
     }
   }
   if (threadIdx.x == 0) {
     if (logp) { B.rgain[o] = rg; B.rloss[o] = rl; }
     B.dec[o] = (own << 16) | d;
-    B.flag[o] = (unsigned char)((mover ? 1 : 0) | (special ? 2 : 0) | 4 | (!vol || mover ? 16 : 0));
+    B.flag[o] = (unsigned char)((mover ? 1 | kListed : 0) | (special ? 2 : 0) | 4 | (!vol || mover ? 16 : 0));
     B.slack[o] = slack;
     B.vslack[o] = vs;
     B.wt[o] = __ldg(&I.w[v]);
@@ -715,11 +738,9 @@ __device__ void fix_position(const DevInstance& I, const SpecBuf& B, const Round
   if (lane == 0) {
     if (logp) { B.rgain[o] = rg; B.rloss[o] = rl; }
     if (mover != (fx >> 16 != 0)) atomicMin(&B.ctl[8], z);
-    const int wv = mover ? __ldg(&I.w[v]) : 0;
-    if (had) B.mlist[lds(&B.midx[o])] = make_int4(o, wv, (own << 16) | d, mover ? nt : 0);   // the replaced mover's entry
-    else if (mover) list_mover(B, par, o, wv, (own << 16) | d, nt);
+    const int listed = relist_mover(I, B, par, o, fl, mover, __ldg(&I.w[v]), (own << 16) | d, nt);
     B.dec[o] = (own << 16) | d;
-    B.flag[o] = (unsigned char)((fl & (2 | 8)) | (mover ? 1 : 0) | (good ? 16 : 0) | 32);
+    B.flag[o] = (unsigned char)((fl & (2 | 8)) | listed | (mover ? 1 : 0) | (good ? 16 : 0) | 32);
     B.vslack[o] = vs;
     B.vd[o] = mover ? vdd : 0;
   }
@@ -790,11 +811,9 @@ __device__ void cta_fix(const DevInstance& I, const SpecBuf& B, const RoundCtx& 
   if (threadIdx.x == 0) {
     if (logp) { B.rgain[o] = rg; B.rloss[o] = rl; }
     if (mover != (fx >> 16 != 0)) atomicMin(&B.ctl[8], z);
-    const int wv = mover ? __ldg(&I.w[v]) : 0;
-    if (had) B.mlist[lds(&B.midx[o])] = make_int4(o, wv, (own << 16) | d, mover ? nt : 0);
-    else if (mover) list_mover(B, par, o, wv, (own << 16) | d, nt);
+    const int listed = relist_mover(I, B, par, o, fl, mover, __ldg(&I.w[v]), (own << 16) | d, nt);
     B.dec[o] = (own << 16) | d;
-    B.flag[o] = (unsigned char)((fl & (2 | 4)) | (mover ? 1 : 0) | (!vol || mover ? 16 : 0) | 32);
+    B.flag[o] = (unsigned char)((fl & (2 | 4)) | listed | (mover ? 1 : 0) | (!vol || mover ? 16 : 0) | 32);
     B.vslack[o] = vs;
     B.vd[o] = mover ? vdd : 0;
   }
@@ -1113,12 +1132,12 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
           claim_nets(I, B, vol, z, own, d, base, deg, lane, 32, par);
           if (lane == 0) {
             if (mt) atomicMin(&B.ctl[2 + par], z);
-            list_mover(B, par, o, __ldg(&I.w[v]), (own << 16) | d, nt);
+            list_mover(I, B, par, o, __ldg(&I.w[v]), (own << 16) | d, nt);
           }
         }
         if (lane == 0) {
           B.dec[o] = (own << 16) | d;   // own read now: part_vec changes in the commit phase
-          B.flag[o] = (unsigned char)((mover ? 1 : 0) | (special ? 2 : 0) | (iso ? 8 : 0) | (good ? 16 : 0));
+          B.flag[o] = (unsigned char)((mover ? 1 | kListed : 0) | (special ? 2 : 0) | (iso ? 8 : 0) | (good ? 16 : 0));
           B.slack[o] = slack;
           B.vslack[o] = vs;
           B.wt[o] = __ldg(&I.w[v]);
@@ -1250,14 +1269,14 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
           if (leads(j) && threadIdx.x == 0) {
             if (logp) { B.rgain[os] = rg; B.rloss[os] = rl; }
             B.dec[os] = (own_s << 16) | d;
-            B.flag[os] = (unsigned char)((mover ? 1 : 0) | (s_gspec[j] ? 2 : 0) | 4 | (!vol || mover ? 16 : 0));
+            B.flag[os] = (unsigned char)((mover ? 1 | kListed : 0) | (s_gspec[j] ? 2 : 0) | 4 | (!vol || mover ? 16 : 0));
             B.slack[os] = s_gslk[j];
             B.vslack[os] = vs;
             B.wt[os] = __ldg(&I.w[vsup]);
             B.acc[os] = lds(&B.hmisc[hmslot(j)]) - deg_s;
             B.vd[os] = mover ? vdd : 0;
             if (mover && mt) atomicMin(&B.ctl[2 + par], zs);
-            if (mover) list_mover(B, par, os, __ldg(&I.w[vsup]), (own_s << 16) | d, nt);
+            if (mover) list_mover(I, B, par, os, __ldg(&I.w[vsup]), (own_s << 16) | d, nt);
           }
           __syncthreads();
         }

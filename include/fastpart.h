@@ -275,7 +275,8 @@ int fp_debug_barrier_fault(fp_instance* inst, int32_t leave_at, int32_t poll_lim
  * committed from windows, [3..8] windows ended by: nothing (fully valid), a
  * possibly stale TV marker, a changed decision that could not be redone, a changed
  * MSV / MSRV accept outcome, more changes of the max-volume parts than a window
- * keeps, a shared net; [9] vertices walked in windows; [16..19] nanoseconds
+ * keeps, a shared net; [9] vertices walked in windows; [10] movers that an earlier change of
+ * their window had made stay (TV / MSV / MSRV); [16..19] nanoseconds
  * in evaluate, validate, commit phases and (TM / MSM) whole-grid decisions; TV / MSV /
  * MSRV also: [20] nanoseconds computing the round state, [21] / [23] SM cycles
  * summed over windows of the slowest warp / CTA evaluation, [25] / [26] SM
