@@ -134,6 +134,7 @@ def lib():
             "fp_reset_state": ([vp], C.c_int),
             "fp_set_engine": ([vp, i32], C.c_int),
             "fp_debug_barrier_fault": ([vp, i32, i32], C.c_int),
+            "fp_debug_replaced_room": ([vp, i32], C.c_int),
             "fp_set_decision_log": ([vp, i32], C.c_int),
             "fp_get_decisions": ([vp, vp, vp, vp, vp], C.c_int),
             "fp_set_classes": ([vp, i64, i64], C.c_int),
@@ -578,6 +579,11 @@ class Instance:
         its leave_at-th grid barrier without arriving, and the others give up
         after poll_limit polls (0: the default limit); (0, 0) turns it off."""
         _check(lib().fp_debug_barrier_fault(self._h, int(leave_at), int(poll_limit)), "fp_debug_barrier_fault")
+
+    def debug_replaced_room(self, entries: int) -> None:
+        """fp_debug_replaced_room: room for the claims of moves that a window's
+        later changes replace (results do not depend on it)."""
+        _check(lib().fp_debug_replaced_room(self._h, int(entries)), "fp_debug_replaced_room")
 
     def stats(self) -> dict:
         """Round statistics of the last refine on the grid-wide engine."""

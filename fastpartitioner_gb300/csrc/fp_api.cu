@@ -800,6 +800,7 @@ int fp_instance_create(fp_ctx* ctx, const fp_hypergraph* h, int32_t K, int32_t m
     // 0: the kernels' own shortest window after a cut
     in->sb.wmin = 0;
     in->sb.maxfix = 32;
+    in->sb.rmax = kReplaced;
     in->sb.max_warps = kMaxSpecWarps;
     in->sb.heavy_pos = in->heavy_pos_d;
     in->sb.mid_pos = in->mid_pos_d;
@@ -1195,6 +1196,14 @@ int fp_debug_barrier_fault(fp_instance* in, int32_t leave_at, int32_t poll_limit
     if (!in || leave_at < 0 || poll_limit < 0) return FP_ERR_INVALID;
     in->fault_leave_at = (unsigned)leave_at;
     in->fault_poll_limit = (unsigned)poll_limit;
+    return FP_OK;
+  });
+}
+
+int fp_debug_replaced_room(fp_instance* in, int32_t entries) {
+  return fp::guarded([&]() -> int {
+    if (!in || entries < 0 || entries > kReplaced) return FP_ERR_INVALID;
+    in->sb.rmax = entries;
     return FP_OK;
   });
 }

@@ -156,6 +156,7 @@ struct SpecBuf {
   uint2* rec_slot;       // [pins] table slots of a count-only move's (net, own) and (net, new part)
   int4* rlist;           // [kReplaced] claims of the moves that changed decisions replaced
                          //     (net or -1, its two entries of the table), until the commit
+  int rmax;              // entries of rlist that a window may use (kReplaced)
   int* ctab_over;        // [2] a probe ran past its bound this round (by round parity)
   unsigned ctab_mask;
   const int* heavy_pos;  // positions (visiting order, ascending) of vertices evaluated by

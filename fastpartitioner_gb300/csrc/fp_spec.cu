@@ -357,13 +357,21 @@ __device__ __forceinline__ void unclaim_nets(const DevInstance& I, const SpecBuf
   }
 }
 
+// Takes deg entries of rlist for the claims of a move about to be replaced (one
+// thread): the first, or one from which they do not fit.  (A full list is not
+// counted on: the count stays far from overflow whatever the degrees.)
+__device__ __noinline__ int replaced_entries(const SpecBuf& B, int par, int deg) {
+  int* const n = &B.ctl[14 + par];
+  return lds(n) > B.rmax ? B.rmax : atomicAdd(n, min(deg, B.rmax + 1));
+}
+
 // Lists the claims of a move about to be replaced, entries [at, at + deg) of
 // rlist (nets k0, k0 + kstep, ...); false if they do not fit.  The claims stay
 // until the commit: a superset keeps every later check conservative.
 __device__ __forceinline__ bool list_replaced(const DevInstance& I, const SpecBuf& B, bool vol, uint32_t base, int deg,
                                               int k0, int kstep, int at) {
-  const bool fits = at + deg <= kReplaced;
-  for (int k = k0; k < deg && at + k < kReplaced; k += kstep) {
+  const bool fits = deg <= B.rmax - at;
+  for (int k = k0; k < min(deg, B.rmax - at); k += kstep) {
     const uint2 sl = !fits || rec_setchange(lds(&B.rec[base + k]), vol) ? make_uint2(~0u, ~0u)
                                                                         : lds(&B.rec_slot[base + k]);
     B.rlist[at + k] = make_int4(fits ? (int)__ldg(&I.vnets[base + k]) : -1, (int)sl.x, (int)sl.y, 0);
@@ -686,7 +694,7 @@ __device__ void fix_position(const DevInstance& I, const SpecBuf& B, const Round
   const int d = fx & 0xffff;
   const bool had = (fl & 1) != 0;
   if (had && deg) {
-    const int at = __shfl_sync(kAll, lane == 0 ? atomicAdd(&B.ctl[14 + par], deg) : 0, 0);
+    const int at = __shfl_sync(kAll, lane == 0 ? replaced_entries(B, par, deg) : 0, 0);
     if (!list_replaced(I, B, vol, base, deg, lane, 32, at)) {
       if (lane == 0) {
         atomicMin(&B.ctl[9], (z << 3) | 2);
@@ -761,7 +769,7 @@ __device__ void cta_fix(const DevInstance& I, const SpecBuf& B, const RoundCtx& 
   const int d = fx & 0xffff;
   const bool had = (fl & 1) != 0;
   if (had) {
-    if (threadIdx.x == 0) iscr[0] = atomicAdd(&B.ctl[14 + par], deg);
+    if (threadIdx.x == 0) iscr[0] = replaced_entries(B, par, deg);
     __syncthreads();
     if (!list_replaced(I, B, vol, base, deg, threadIdx.x, blockDim.x, iscr[0])) {
       if (threadIdx.x == 0) {
@@ -1807,7 +1815,7 @@ __global__ void __launch_bounds__(kSThreads, 2) spec_ldg_kernel(DevInstance I, S
       // the committed movers' nets [k0, step): all of them, or (counts_first) the
       // count-only ones and, behind a barrier, those whose part set changes
       const bool counts_first = lds(&B.ctl[12 + par]) != 0;
-      for (int i = gtid, n = min(lds(&B.ctl[14 + par]), kReplaced); i < n; i += gthreads) {
+      for (int i = gtid, n = min(lds(&B.ctl[14 + par]), B.rmax); i < n; i += gthreads) {
         const int4 x = lds(&B.rlist[i]);
         if (x.x < 0) continue;
         unclaim_net(B, x.x);

@@ -269,6 +269,10 @@ int fp_get_decisions(fp_instance* inst, int32_t* dest, int32_t* gain, int32_t* l
  * zero (the default) turns the hook off.  The refined state after a timeout is
  * partial: fp_reset_state restores the initial one. */
 int fp_debug_barrier_fault(fp_instance* inst, int32_t leave_at, int32_t poll_limit);
+/* Test hook (no effect on results; TV / MSV / MSRV): at most `entries` (net,
+ * vertex) pairs of moves that a window's later changes replace are kept, 2^18 by
+ * default; a change without room ends the window in front of it. */
+int fp_debug_replaced_room(fp_instance* inst, int32_t entries);
 
 /* Statistics of the last fp_refine on the grid-wide engine (up to 48 values):
  * [0] windows, [1] whole-grid evaluations of heavy vertices (CN: nets), [2] moves
