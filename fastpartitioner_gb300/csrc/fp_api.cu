@@ -434,6 +434,23 @@ int fp_ctx_set_stream(fp_ctx* ctx, void* stream) {
   });
 }
 
+// The scratch that starts a launch as zeros lies in one buffer (from hcnt on),
+// cleared by one fill: the whole-grid tallies, TV's marker words, the mover and
+// table counts.  (Eight fills of them took 33 us of a refinement at K = 24, 26 with
+// a quarter of the tallies' slots: 7220 uniform vertices under TM 207 -> 191 us for
+// one pass and its metrics.)
+static size_t zeroed_words(int K) { return 8 * (size_t)kMaxGridVerts * K + 16 * kMaxGridVerts + 2 * (size_t)K + 4; }
+static void place_zeroed(SpecBuf& b, int K) {
+  const size_t n = 2 * (size_t)kMaxGridVerts * K;
+  b.hgain = b.hcnt + n;
+  b.hloss = b.hgain + n;
+  b.hadelta = b.hloss + n;
+  b.hmisc = b.hadelta + n;
+  b.mlast = reinterpret_cast<unsigned long long*>(b.hmisc + 16 * kMaxGridVerts);
+  b.mcnt = reinterpret_cast<int*>(b.mlast + K);
+  b.ctab_over = b.mcnt + 2;
+}
+
 // Claims (no claim: a value above every position) and both parities of the
 // whole-grid tallies start clear for every speculative launch: a launch leaves
 // the tallies of its last window with whole-grid vertices, and an aborted
@@ -443,15 +460,8 @@ static cudaError_t clear_spec_scratch(const SpecBuf& b, int noe, int K, cudaStre
   cudaError_t e = cudaMemsetAsync(b.claim_m, 0x7f, sizeof(int) * ne, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(b.claim_c, 0x7f, sizeof(int) * ne, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(b.mask_c, 0, sizeof(uint32_t) * ne, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(b.hcnt, 0, sizeof(int) * 2 * kMaxGridVerts * K, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(b.hcnt, 0, sizeof(int) * zeroed_words(K), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(b.hfirst, 0xff, sizeof(unsigned long long) * 2 * kMaxGridVerts * K, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(b.hgain, 0, sizeof(int) * 2 * kMaxGridVerts * K, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(b.hloss, 0, sizeof(int) * 2 * kMaxGridVerts * K, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(b.hadelta, 0, sizeof(int) * 2 * kMaxGridVerts * K, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(b.hmisc, 0, sizeof(int) * 16 * kMaxGridVerts, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(b.mlast, 0, sizeof(unsigned long long) * K, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(b.mcnt, 0, sizeof(int) * 2, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(b.ctab_over, 0, sizeof(int) * 2, s);
   if (e == cudaSuccess && b.ctab_mask) {
     const size_t n = (size_t)b.ctab_mask + 1;
     e = cudaMemsetAsync(b.ctab_key, 0xff, sizeof(unsigned long long) * n, s);
@@ -740,22 +750,18 @@ int fp_instance_create(fp_ctx* ctx, const fp_hypergraph* h, int32_t K, int32_t m
         (rc = dalloc(in, &in->sb.rec, ldg ? g.pins : 1)) || (rc = dalloc(in, &in->sb.rec_slot, ldg ? g.pins : 1)) ||
         (rc = dalloc(in, &in->sb.ctab_key, ldg ? ctab : 1)) || (rc = dalloc(in, &in->sb.ctab_pos, ldg ? ctab : 1)) ||
         (rc = dalloc(in, &in->sb.ctab_cnt, ldg ? ctab : 1)) ||
-        (rc = dalloc(in, &in->sb.ctab_over, 2)) || (rc = dalloc(in, &in->sb.dfix, kSpecWindow)) ||
+        (rc = dalloc(in, &in->sb.dfix, kSpecWindow)) ||
         (rc = dalloc(in, &in->sb.rlist, ldg ? kReplaced : 1)) ||
         (rc = dalloc(in, &in->sb.cn_moved, cn ? g.pins : 1)) || (rc = dalloc(in, &in->sb.cn_kcnt, cn ? g.noe : 1)) ||
         (rc = dalloc(in, &in->sb.cn_nets, cn ? g.noe : 1)) || (rc = dalloc(in, &in->sb.cn_more, cn ? g.pins : 1)) || (rc = dalloc(in, &in->sb.cn_cnt, 6)) ||
         (rc = dalloc(in, &in->sb.cn_wit, cn ? g.nov : 1)) || (rc = dalloc(in, &in->vclass_d, g.nov)) ||
         (rc = dalloc(in, &in->sb.cand, (size_t)kSpecWindow * K)) || (rc = dalloc(in, &in->sb.ncand, kSpecWindow)) ||
         (rc = dalloc(in, &in->sb.mlist, kSpecWindow)) || (rc = dalloc(in, &in->sb.midx, kSpecWindow)) ||
-        (rc = dalloc(in, &in->sb.mcnt, 2)) ||
         (rc = dalloc(in, &in->sb.acc, kSpecWindow)) || (rc = dalloc(in, &in->sb.rel, kSpecWindow)) ||
         (rc = dalloc(in, &in->sb.claim_m, g.noe)) || (rc = dalloc(in, &in->sb.claim64, g.noe)) || (rc = dalloc(in, &in->sb.claim_c, g.noe)) ||
-        (rc = dalloc(in, &in->sb.mask_c, g.noe)) || (rc = dalloc(in, &in->sb.hcnt, 2 * kMaxGridVerts * K)) ||
+        (rc = dalloc(in, &in->sb.mask_c, g.noe)) || (rc = dalloc(in, &in->sb.hcnt, zeroed_words(K))) ||
         (rc = dalloc(in, &in->sb.hfirst, 2 * kMaxGridVerts * K)) ||
-        (rc = dalloc(in, &in->sb.hgain, 2 * kMaxGridVerts * K)) ||
-        (rc = dalloc(in, &in->sb.hloss, 2 * kMaxGridVerts * K)) ||
-        (rc = dalloc(in, &in->sb.hadelta, 2 * kMaxGridVerts * K)) ||
-        (rc = dalloc(in, &in->sb.hmisc, 16 * kMaxGridVerts)) || (rc = dalloc(in, &in->sb.mlast, K)) || (rc = dalloc(in, &in->heavy_pos_d, std::max(g.nov, g.noe))) ||
+        (rc = dalloc(in, &in->heavy_pos_d, std::max(g.nov, g.noe))) ||
         (rc = dalloc(in, &in->mid_pos_d, std::max(g.nov, g.noe))) ||
         (rc = dalloc(in, &in->porder_d, ldg ? g.nov : 1)) || (rc = dalloc(in, &in->iso_list_d, ldg ? g.nov : 1)) ||
         (rc = dalloc(in, &in->iso_before_d, ldg ? g.nov + 1 : 1)) ||
@@ -773,6 +779,7 @@ int fp_instance_create(fp_ctx* ctx, const fp_hypergraph* h, int32_t K, int32_t m
       fp_instance_destroy(in);
       return rc;
     }
+    place_zeroed(in->sb, K);
     void* ms = nullptr;
     cudaError_t e = cudaSuccess;
     if (in->in_arena) {
@@ -888,15 +895,14 @@ int fp_instance_footprint(int32_t nov, int32_t noe, int64_t pins, int32_t K, int
     add(std::max(kSpecWindow, kMsgWindow), 4); add(std::max(kSpecWindow, kMsgWindow), 4);   // rgain, rloss
     add(ldg ? P : 1, 4); add(ldg ? P : 1, 8);                // rec, rec_slot
     add(ldg ? ctab : 1, 8); add(ldg ? ctab : 1, 4); add(ldg ? ctab : 1, 4);
-    add(2, 4); add(W, 4);                                    // ctab_over, dfix
+    add(W, 4);                                               // dfix
     add(ldg ? kReplaced : 1, 16);                            // rlist
     add(cn ? P : 1, 8); add(cn ? E : 1, 4); add(cn ? E : 1, 8); add(cn ? P : 1, 8); add(6, 4); add(cn ? V : 1, 4);
     add(V, 1);                                               // vertex classes
-    add(W * K, 8); add(W, 4); add(W, 16); add(W, 4); add(2, 4);   // cand, ncand, mlist, midx, mcnt
+    add(W * K, 8); add(W, 4); add(W, 16); add(W, 4);         // cand, ncand, mlist, midx
     add(W, 4); add(W, 4);                                    // acc, rel
     add(E, 4); add(E, 8); add(E, 4); add(E, 4);              // claim_m, claim64, claim_c, mask_c
-    add(G2K, 4); add(G2K, 8); add(G2K, 4); add(G2K, 4); add(G2K, 4);
-    add(16 * (size_t)kMaxGridVerts, 4); add(K, 8);           // hmisc, mlast
+    add(zeroed_words(K), 4); add(G2K, 8);                    // tallies and counts from hcnt on, hfirst
     add(VE, 4); add(VE, 4);                                  // heavy / medium positions
     add(ldg ? V : 1, 4); add(ldg ? V : 1, 4); add(ldg ? V + 1 : 1, 4);   // porder, iso_list, iso_before
     add(V, 4); add(V, 4); add(V + 1, 4); add(V, 4);          // device stream: positions, iso, before,
