@@ -753,7 +753,7 @@ int fp_instance_create(fp_ctx* ctx, const fp_hypergraph* h, int32_t K, int32_t m
         (rc = dalloc(in, &in->sb.dfix, kSpecWindow)) ||
         (rc = dalloc(in, &in->sb.rlist, ldg ? kReplaced : 1)) ||
         (rc = dalloc(in, &in->sb.cn_moved, cn ? g.pins : 1)) || (rc = dalloc(in, &in->sb.cn_kcnt, cn ? g.noe : 1)) ||
-        (rc = dalloc(in, &in->sb.cn_nets, cn ? g.noe : 1)) || (rc = dalloc(in, &in->sb.cn_more, cn ? g.pins : 1)) || (rc = dalloc(in, &in->sb.cn_cnt, 6)) ||
+        (rc = dalloc(in, &in->sb.cn_nets, cn ? g.noe : 1)) || (rc = dalloc(in, &in->sb.cn_more, cn ? g.pins : 1)) || (rc = dalloc(in, &in->sb.cn_cnt, 8)) ||
         (rc = dalloc(in, &in->sb.cn_wit, cn ? g.nov : 1)) || (rc = dalloc(in, &in->vclass_d, g.nov)) ||
         (rc = dalloc(in, &in->sb.cand, (size_t)kSpecWindow * K)) || (rc = dalloc(in, &in->sb.ncand, kSpecWindow)) ||
         (rc = dalloc(in, &in->sb.mlist, kSpecWindow)) || (rc = dalloc(in, &in->sb.midx, kSpecWindow)) ||
@@ -897,7 +897,7 @@ int fp_instance_footprint(int32_t nov, int32_t noe, int64_t pins, int32_t K, int
     add(ldg ? ctab : 1, 8); add(ldg ? ctab : 1, 4); add(ldg ? ctab : 1, 4);
     add(W, 4);                                               // dfix
     add(ldg ? kReplaced : 1, 16);                            // rlist
-    add(cn ? P : 1, 8); add(cn ? E : 1, 4); add(cn ? E : 1, 8); add(cn ? P : 1, 8); add(6, 4); add(cn ? V : 1, 4);
+    add(cn ? P : 1, 8); add(cn ? E : 1, 4); add(cn ? E : 1, 8); add(cn ? P : 1, 8); add(8, 4); add(cn ? V : 1, 4);
     add(V, 1);                                               // vertex classes
     add(W * K, 8); add(W, 4); add(W, 16); add(W, 4);         // cand, ncand, mlist, midx
     add(W, 4); add(W, 4);                                    // acc, rel
@@ -1110,7 +1110,7 @@ int fp_refine(fp_instance* in, int32_t passes) {
         if (in->pb.metric == FP_METRIC_CN) {
           e = cudaMemsetAsync(in->sb.claim64, 0, sizeof(unsigned long long) * std::max(in->g.noe, 1), s);
           if (e == cudaSuccess) e = cudaMemsetAsync(in->sb.cn_kcnt, 0, sizeof(int) * std::max(in->g.noe, 1), s);
-          if (e == cudaSuccess) e = cudaMemsetAsync(in->sb.cn_cnt, 0, sizeof(int) * 6, s);
+          if (e == cudaSuccess) e = cudaMemsetAsync(in->sb.cn_cnt, 0, sizeof(int) * 8, s);
           if (e == cudaSuccess) e = launch_spec_cn(in->d, in->sb, passes, in->ctx->num_sms, s, &in->last_grid);
         } else if (in->pb.metric == FP_METRIC_TM || in->pb.metric == FP_METRIC_MSM) {
           e = launch_spec_msg(in->d, in->sb, passes, in->ctx->num_sms, s, &in->last_grid);

@@ -144,8 +144,8 @@ struct SpecBuf {
   int2* cn_nets;         // [noe] CN: (net, packed old/new part) of the nets those moves touch
   int2* cn_more;         // [pins] CN: (net, window offset) of the moves of acting nets after the
                          //     first on a net
-  int* cn_cnt;           // [6] CN: counts of cn_moved [0,1], cn_nets [2,3] and cn_more [4,5] by
-                         //     round parity
+  int* cn_cnt;           // [8] CN: counts of cn_moved [0,1], cn_nets [2,3] and cn_more [4,5], a
+                         //     moved pin has many nets [6,7], by round parity
   int* cn_wit;           // [nov] CN: a net of the vertex found uncut before (-1: none)
   int* claim_m;          // [noe] first mover position changing the net's part set
   int* claim_c;          // [noe] first mover position changing only counts

@@ -31,6 +31,12 @@ namespace {
 
 using namespace spec;
 
+// A window that moves few pins (27 on average on 262144 Zipf vertices), one of them
+// on more than kCnChunk nets, spreads each one's nets over the warps: a hub's
+// thousands of nets took one warp 60 us, C1 takes 10 so.  More pins keep the warps
+// busy as they are, and pins of few nets need no search for shares (a commit on 86565
+// mixed vertices 12.0 us with it, 10.7 without).
+constexpr int kCnSpreadMoves = 256, kCnChunk = 128, kCnStep = 37;
 constexpr int kShared = 1 << 30;   // cn_kcnt: several acting nets move pins of the net
 
 // Round-stamped claim: the latest round wins, then the smallest position.
@@ -82,7 +88,10 @@ __device__ int cn_walk_range(const DevInstance& I, const SpecBuf& B, int e, int 
       const unsigned m = __ballot_sync(kAll, hit >= 0);
       if (m) return __shfl_sync(kAll, hit, __ffs(m) - 1);
     }
-    if (kMode == 1 && u >= 0) B.cn_moved[atomicAdd(&B.cn_cnt[par], 1)] = make_int2(u, o);
+    if (kMode == 1 && u >= 0) {
+      B.cn_moved[atomicAdd(&B.cn_cnt[par], 1)] = make_int2(u, o);
+      if (d > kCnChunk) B.cn_cnt[6 + par] = 1;
+    }
     int incl = d;
     for (int off = 1; off < 32; off <<= 1) {
       const int t = __shfl_up_sync(kAll, incl, off);
@@ -162,11 +171,15 @@ __device__ __forceinline__ void cn_list_acting(const SpecBuf& B, int par, int e)
   B.midx[atomicAdd(&B.mcnt[par], 1)] = e;
 }
 
-// Did an acting net before e (nb of them) change what e's own list decides?
-__device__ __forceinline__ bool cn_own_conflict(const DevInstance& I, const SpecBuf& B, int round, int e, int unc,
-                                                int nb) {
-  return (claim_before(B, round, e, e) && lds(&I.ep_len[e]) <= 2 + nb) ||
-         (unc >= 0 && claim_before(B, round, unc, e));
+// What the acting nets before e may have changed of what e's own list decides: e
+// conflicts with nb of them if the result is at most 2 + nb (0: one claimed its
+// witness; its parts: one claimed e itself; kNone: neither).  It does not depend
+// on nb, so that its loads and those of the count are under way together.
+__device__ __forceinline__ int cn_own_claims(const DevInstance& I, const SpecBuf& B, int round, int e, int unc) {
+  const int n = lds(&I.ep_len[e]);
+  const bool own = claim_before(B, round, e, e);
+  if (unc >= 0 && claim_before(B, round, unc, e)) return 0;
+  return own ? n : kNone;
 }
 
 // Warp gw's contiguous share (of nw warps) of net e's pins.
@@ -249,8 +262,9 @@ __device__ void cn_validate_cta(const DevInstance& I, const SpecBuf& B, int e, i
   __shared__ volatile int sh_conf;
   const int lane = threadIdx.x & 31;
   const int act = lds(&B.flag[o]);
+  const int own = cn_own_claims(I, B, round, e, lds(&B.slack[o]));
   const int nb = cn_acting_before(B, nact, e);
-  if (threadIdx.x == 0) sh_conf = cn_own_conflict(I, B, round, e, lds(&B.slack[o]), nb) ? 1 : 0;
+  if (threadIdx.x == 0) sh_conf = own <= 2 + nb ? 1 : 0;
   __syncthreads();
   if (act && !sh_conf) {
     int pb, pe;
@@ -436,11 +450,6 @@ __device__ bool cn_apply_shared(const DevInstance& I, const SpecBuf& B, int x, i
   return true;
 }
 
-// A window that moves few pins (27 on average on 262144 Zipf vertices) spreads
-// each one's nets over the warps: a hub's thousands of nets took one warp 60 us,
-// C1 takes 10 so.  More pins keep the warps busy as they are.
-constexpr int kCnSpreadMoves = 256, kCnChunk = 128, kCnStep = 37;
-
 // Three CTAs per SM: without the hint the compiler spills to fit more.
 __global__ void __launch_bounds__(kSThreads, 3) spec_cn_kernel(DevInstance I, SpecBuf B, int passes) {
   barrier_start();
@@ -548,15 +557,18 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_cn_kernel(DevInstance I, Sp
       }
       // ---- B: validate against earlier acting nets' claims
       const int nact = lds(&B.mcnt[par]);
-      for (int e = z0; e < z1; e++) {
+      // (the acting nets before a warp's first net are counted once, beside its
+      // words' loads; counted for each net, after them, a window of 86565 mixed
+      // vertices, K = 128, took 8.7 us to validate instead of 8.0)
+      for (int e = z0, before = -1; e < z1; e++) {
         const int o = e - pos;
-        if ((int)(__ldg(&I.nptr[e + 1]) - __ldg(&I.nptr[e])) > B.cn_big) continue;   // validated by the CTA below
         const int act = lds(&B.flag[o]);
-        if (nact == 0) break;
-        const int nb = cn_acting_before(B, nact, e);
+        const int own = cn_own_claims(I, B, round, e, lds(&B.slack[o]));
+        const int nb = before < 0 ? cn_acting_before(B, nact, e) : before;
+        before = nb + act;
+        if ((int)(__ldg(&I.nptr[e + 1]) - __ldg(&I.nptr[e])) > B.cn_big) continue;   // validated by the CTA below
         if (nb == 0) continue;
-        bool conf = lane == 0 && cn_own_conflict(I, B, round, e, lds(&B.slack[o]), nb);
-        conf = __any_sync(kAll, conf);   // warp-uniform before the pin loop's votes
+        bool conf = own <= 2 + nb;
         if (act && !conf) conf = cn_walk<2>(I, B, e, lds(&B.dec[o]) >> 16, round, 0, 0, nb) > 0;
         conf = __any_sync(kAll, conf);
         if (conf) {
@@ -574,9 +586,9 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_cn_kernel(DevInstance I, Sp
         // a grid net: its own list and witness by every warp (cheap), its
         // moving pins' nets split across the grid
         const int e = s_ge[j], o = e - pos;
-        const int unc = lds(&B.slack[o]);
+        const int own = cn_own_claims(I, B, round, e, lds(&B.slack[o]));
         const int nb = cn_acting_before(B, nact, e);
-        bool conf = cn_own_conflict(I, B, round, e, unc, nb);
+        bool conf = own <= 2 + nb;
         if (!conf && lds(&B.flag[o])) {
           int pb, pe;
           cn_grid_share(I, e, gw, nwarps, &pb, &pe);
@@ -637,7 +649,7 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_cn_kernel(DevInstance I, Sp
         atomicAdd((unsigned long long*)&I.moves[it], 1ull);
         atomicAdd(&B.stats[2], 1ull);
       };
-      if (nmv > kCnSpreadMoves) {
+      if (nmv > kCnSpreadMoves || !lds(&B.cn_cnt[6 + par])) {
         for (int i = gw; i < nmv; i += nwarps) {
           const int2 mv = lds(&B.cn_moved[i]);
           if (pos + mv.y >= cut) continue;
@@ -704,6 +716,7 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_cn_kernel(DevInstance I, Sp
         B.cn_cnt[par ^ 1] = 0;
         B.cn_cnt[2 + (par ^ 1)] = 0;
         B.cn_cnt[4 + (par ^ 1)] = 0;
+        B.cn_cnt[6 + (par ^ 1)] = 0;
         B.mcnt[par ^ 1] = 0;
       }
       if (ns) {
