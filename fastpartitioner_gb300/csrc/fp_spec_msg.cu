@@ -442,6 +442,59 @@ __device__ void msg_commit_grid(const DevInstance& I, int v, int own, int d, int
   }
 }
 
+// The max-message parts, recomputed for every vertex by the reference
+// (MSM/partition.cpp:368-386); they change only with moves.  In part order (maxl,
+// *nmax of them) and as a mask (maxm).  The whole CTA.
+__device__ __noinline__ void msm_max_parts(const int* msgs, int K, int* maxl, uint32_t* maxm, int* iscr, int* mx_out,
+                                           int* nmax) {
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  int mx = -2147483647 - 1;
+  for (int p = threadIdx.x; p < K; p += blockDim.x) mx = max(mx, msgs[p]);
+  mx = warp_max(mx);
+  if (lane == 0) iscr[wib] = mx;
+  __syncthreads();
+  if (wib == 0) {
+    mx = warp_max(iscr[lane & (kSWarps - 1)]);
+    int c = 0;
+    for (int p0 = 0; p0 < K; p0 += 32) {
+      const int p = p0 + lane;
+      const unsigned b = __ballot_sync(kAll, p < K && msgs[p] == mx);
+      if ((b >> lane) & 1u) maxl[c + __popc(b & ((1u << lane) - 1u))] = p;
+      if (lane == 0) maxm[p0 >> 5] = b;
+      c += __popc(b);
+    }
+    if (lane == 0) {
+      *mx_out = mx;
+      *nmax = c;
+    }
+  }
+  __syncthreads();
+}
+
+// Parts whose vertices can move at all (bits of okm).  MSM (limited): a vertex
+// moves only if every max-message part gains, and a part m other than its own p
+// gains only by conn[m][p] == 1 (msg_decide_warp): the parts where that holds for
+// all of them.  On the 1M-vertex Zipf workload it leaves a few per cent of the
+// vertices to evaluate.  By whole words of the max parts' mask: part by part, and
+// with one thread listing them, a window of 16981 mixed vertices, K = 512, took 86
+// us to evaluate instead of 75.
+__device__ __noinline__ void msg_may_leave(const DevInstance& I, bool limited, const uint32_t* maxm, uint32_t* okm) {
+  const int lane = threadIdx.x & 31, K = I.K, words = (K + 31) >> 5;
+  for (int x = threadIdx.x >> 5; x < words; x += kSWarps) {
+    const int p = x * 32 + lane;
+    uint32_t miss = p < K ? 0u : 1u;
+    if (limited && p < K) {
+#pragma unroll 4
+      for (int y = 0; y < words; y++)
+        if (const uint32_t m = maxm[y])
+          miss |= m & ~lds(&I.c1col[(size_t)p * words + y]) & ~(y == x ? 1u << lane : 0u);
+    }
+    const unsigned b = __ballot_sync(kAll, miss == 0u);
+    if (lane == 0) okm[x] = b;
+  }
+  __syncthreads();
+}
+
 // Shortest window after a mover: 512, 1024 and 2048 positions within 2% of each
 // other for TM on Zipf workloads; longer ones suit uniform nets, MSM's evaluations
 // of large K shorter ones (16981 mixed vertices, K = 512: 3.97 ms, 4.87 at 3648).
@@ -457,6 +510,7 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
   __shared__ unsigned oc1m[kSWarps];
   __shared__ int s_mx, s_nmax, s_stop, s_ns;
   __shared__ uint32_t okm_s[kMaxMsgWords];   // parts a vertex may leave this round (MSM)
+  __shared__ uint32_t maxm_s[kMaxMsgWords];  // the max-message parts (MSM)
   __shared__ int s_gz[kMaxGridVerts], s_go[kMaxGridVerts], s_gd[kMaxGridVerts];
   __shared__ uint32_t s_gb[kMaxGridVerts];
   __shared__ int s_t0[kMaxGridVerts], s_t1[kMaxGridVerts];   // their teams of CTAs
@@ -516,43 +570,10 @@ __global__ void __launch_bounds__(kSThreads, 3) spec_msg_kernel(DevInstance I, S
       const bool moved = dirty;
       dirty = false;
       __syncthreads();
-      if (msm) {
-        // max-message parts, recomputed for every vertex by the reference
-        // (MSM/partition.cpp:368-386); they change only with moves.
-        int mx = -2147483647 - 1;
-        for (int p = threadIdx.x; p < K; p += blockDim.x) mx = max(mx, msgs_s[p]);
-        mx = warp_max(mx);
-        if (lane == 0) iscr[wib] = mx;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-          int m = iscr[0];
-          for (int x = 1; x < kSWarps; x++) m = max(m, iscr[x]);
-          s_mx = m;
-          int c = 0;
-          for (int p = 0; p < K; p++)
-            if (msgs_s[p] == m) maxl_s[c++] = p;
-          s_nmax = c;
-        }
-        __syncthreads();
-      }
+      if (msm) msm_max_parts(msgs_s, K, maxl_s, maxm_s, iscr, &s_mx, &s_nmax);
       if (!okm_set || logp || (msm && moved)) {
-        // MSM: a vertex moves only if every max-message part gains, and a part m
-        // other than its own p gains only by conn[m][p] == 1 (msg_decide_warp):
-        // the parts where that holds for all of them.  On the 1M-vertex Zipf
-        // workload it leaves a few per cent of the vertices to evaluate.
-        // (Decision records need every vertex's gain.)
-        for (int x = wib; x < words; x += kSWarps) {
-          const int p = x * 32 + lane;
-          bool ok = p < K;
-          if (msm && !logp && ok)
-            for (int q = 0; q < s_nmax && ok; q++) {
-              const int m = maxl_s[q];
-              ok = m == p || ((lds(&I.c1col[(size_t)p * words + (m >> 5)]) >> (m & 31)) & 1u);
-            }
-          const unsigned b = __ballot_sync(kAll, ok);
-          if (lane == 0) okm_s[x] = b;
-        }
-        __syncthreads();
+        // (decision records need every vertex's gain)
+        msg_may_leave(I, msm && !logp, maxm_s, okm_s);
         okm_set = true;
       }
       const MsgRound Rd{sizes_s, msgs_s, maxl_s, msm ? s_nmax : 0, msm ? s_mx : 0};
