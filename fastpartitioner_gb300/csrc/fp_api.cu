@@ -101,8 +101,8 @@ int default_grid_verts(int metric) {
 }
 constexpr int kMaxSpecWarps = 16384;
 constexpr int kCtlWords = 16;   // SpecBuf::ctl
-cudaError_t metrics_grid(int K, int noe, int num_sms, int* grid);
-cudaError_t launch_metrics(const DevInstance& I, void* scratch, long long* out, int grid, cudaStream_t st,
+cudaError_t metrics_per_sm(int K, int* per_sm);
+cudaError_t launch_metrics(const DevInstance& I, void* scratch, long long* out, int max_ctas, cudaStream_t st,
                            int* launches);
 }  // namespace fp
 
@@ -139,7 +139,7 @@ struct fp_instance {
   long long dev_bytes = 0;        // bytes of the device allocations in `allocs`
   bool in_arena = false;          // buffers taken from ctx->arena (nothing in allocs)
   void* metric_scratch = nullptr;
-  int metric_grid = 1;
+  int metric_per_sm = 1;
   long long* h_moves = nullptr;   // pinned
   int* h_status = nullptr;        // pinned
   long long* h_metrics = nullptr; // pinned
@@ -793,7 +793,7 @@ int fp_instance_create(fp_ctx* ctx, const fp_hypergraph* h, int32_t K, int32_t m
       in->dev_bytes += (long long)metrics_scratch_bytes(K);
     }
     in->metric_scratch = ms;
-    e = metrics_grid(K, g.noe, ctx->num_sms, &in->metric_grid);
+    e = metrics_per_sm(K, &in->metric_per_sm);
     if (e == cudaSuccess)
       e = cudaMemsetAsync(ms, 0, metrics_scratch_bytes(K), ctx->stream);   // (each evaluation leaves it zeroed)
     if (e != cudaSuccess) { fp_instance_destroy(in); return cuda_status(e); }
@@ -1230,7 +1230,8 @@ int fp_metrics(fp_instance* in, int64_t out[6]) {
     cudaStream_t s = in->ctx->stream;
     int launches = 0;
     // (the kernel writes the six values to pinned host memory)
-    cudaError_t e = launch_metrics(in->d, in->metric_scratch, in->h_metrics, in->metric_grid, s, &launches);
+    cudaError_t e = launch_metrics(in->d, in->metric_scratch, in->h_metrics, in->ctx->num_sms * in->metric_per_sm, s,
+                                   &launches);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_status(e);
     for (int i = 0; i < 6; i++) out[i] = in->h_metrics[i];

@@ -152,31 +152,30 @@ size_t metrics_scratch_bytes(int K) {
   return 64 + 2 * sizeof(long long) * (size_t)K + sizeof(uint32_t) * words * (size_t)K;
 }
 
-// CTAs of the evaluation of noe nets (*grid).  Also raises the kernel's limit of
-// dynamic shared memory: the static arrays count against the 48 KB that a launch
+// CTAs of the evaluation that an SM holds (*per_sm).  Also raises the kernel's limit
+// of dynamic shared memory: the static arrays count against the 48 KB that a launch
 // may have without, so it is due from K = 3008 on.  The limit belongs to the
 // kernel on this device, not to an instance: it is always what the largest K
 // needs, whichever instance sets it last.
-cudaError_t metrics_grid(int K, int noe, int num_sms, int* grid) {
+cudaError_t metrics_per_sm(int K, int* per_sm) {
   const size_t smem = metrics_smem_bytes(K);
   cudaError_t err = cudaFuncSetAttribute(metrics_nets_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)metrics_smem_bytes(kMaxK));
-  int per_sm = 0;
+  *per_sm = 0;
   if (err == cudaSuccess)
-    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, metrics_nets_kernel, kMetricsThreads, smem);
+    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, metrics_nets_kernel, kMetricsThreads, smem);
   if (err != cudaSuccess) return err;
-  if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  const long long want = ((long long)noe + kMetricsThreads / 32 - 1) / (kMetricsThreads / 32);
-  *grid = (int)std::max(1ll, std::min((long long)num_sms * per_sm, want));
-  return cudaSuccess;
+  return *per_sm < 1 ? cudaErrorInvalidConfiguration : cudaSuccess;
 }
 
 // `scratch` must hold metrics_scratch_bytes(K) bytes, zeroed before the first
-// call; `grid` from metrics_grid; `out` receives 6 values (device or pinned host
-// memory).
-cudaError_t launch_metrics(const DevInstance& I, void* scratch, long long* out, int grid, cudaStream_t st,
+// call; `out` receives 6 values (device or pinned host memory).  At most max_ctas CTAs
+// (metrics_per_sm for each SM in use).
+cudaError_t launch_metrics(const DevInstance& I, void* scratch, long long* out, int max_ctas, cudaStream_t st,
                            int* launches) {
   const int K = I.K;
+  const long long want = ((long long)I.noe + kMetricsThreads / 32 - 1) / (kMetricsThreads / 32);
+  const int grid = (int)std::max(1ll, std::min((long long)max_ctas, want));
   MetricScratch M;
   unsigned char* b = static_cast<unsigned char*>(scratch);
   M.acc = reinterpret_cast<unsigned long long*>(b);

@@ -36,3 +36,16 @@ def test_metrics_of_instances_alive_together(orc, gpu_engine, hg, Ks):
     finally:
         for inst in insts:
             inst.close()
+
+
+@pytest.mark.parametrize("K", (16, 700))
+def test_metrics_under_changed_sm_limits(fp, orc, hg, K):
+    eng = fp.Engine(0)   # (its own context: the limit is the context's)
+    try:
+        with eng.instance(hg, K, "TV") as inst:
+            inst.initial_partition()
+            for sms in (1, 7, 0):   # limits set after the instance was made
+                eng.set_sm_limit(sms)
+                assert inst.metrics() == expected(orc, hg, K)
+    finally:
+        eng.close()
