@@ -9,6 +9,20 @@ namespace fp {
 constexpr int kThreads = 512;                 // refinement CTA size
 constexpr int kWarps = kThreads / 32;
 
+// Raises a kernel's limit of dynamic shared memory to all that a CTA of the
+// current device can have beside the kernel's static arrays.  The limit belongs to
+// the kernel, not to a launch: set to each launch's own size, a thread that
+// refined for a small K lowered it between another's set and launch for a large one.
+inline cudaError_t allow_shared_memory(const void* kernel) {
+  int device = 0, most = 0;
+  cudaFuncAttributes a;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes);
+}
+
 // Everything the refinement kernels read or write, as device pointers.
 struct DevInstance {
   int nov, noe;

@@ -15,7 +15,6 @@
 // arithmetic is integer and order-independent, hence exact.
 
 #include "fp_device.cuh"
-#include "fp_internal.h"
 #include "../../include/fastpart.h"
 
 #include <algorithm>
@@ -154,13 +153,10 @@ size_t metrics_scratch_bytes(int K) {
 
 // CTAs of the evaluation that an SM holds (*per_sm).  Also raises the kernel's limit
 // of dynamic shared memory: the static arrays count against the 48 KB that a launch
-// may have without, so it is due from K = 3008 on.  The limit belongs to the
-// kernel on this device, not to an instance: it is always what the largest K
-// needs, whichever instance sets it last.
+// may have without, so it is due from K = 3008 on.
 cudaError_t metrics_per_sm(int K, int* per_sm) {
   const size_t smem = metrics_smem_bytes(K);
-  cudaError_t err = cudaFuncSetAttribute(metrics_nets_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)metrics_smem_bytes(kMaxK));
+  cudaError_t err = allow_shared_memory((const void*)metrics_nets_kernel);
   *per_sm = 0;
   if (err == cudaSuccess)
     err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, metrics_nets_kernel, kMetricsThreads, smem);

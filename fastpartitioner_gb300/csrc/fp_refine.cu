@@ -741,17 +741,17 @@ cudaError_t launch_refine(const DevInstance& I, int passes, cudaStream_t st) {
   cudaError_t err = cudaSuccess;
   switch (I.metric) {
     case 1:
-      err = cudaFuncSetAttribute(refine_tv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      err = allow_shared_memory((const void*)refine_tv_kernel);
       if (err == cudaSuccess) refine_tv_kernel<<<1, kThreads, smem, st>>>(I, passes);
       break;
     case 4:
     case 5:
-      err = cudaFuncSetAttribute(refine_vol_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      err = allow_shared_memory((const void*)refine_vol_kernel);
       if (err == cudaSuccess) refine_vol_kernel<<<1, kThreads, smem, st>>>(I, passes, I.metric == 5);
       break;
     case 2:
     case 3:
-      err = cudaFuncSetAttribute(refine_msg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      err = allow_shared_memory((const void*)refine_msg_kernel);
       if (err == cudaSuccess) refine_msg_kernel<<<1, kThreads, smem, st>>>(I, passes, I.metric == 3);
       break;
     case 0:

@@ -2084,7 +2084,7 @@ cudaError_t launch_spec_ldg(const DevInstance& I, const SpecBuf& B, int passes, 
                             int* grid_out) {
   const size_t smem = spec_ldg_smem_bytes(I.K);
   const void* fn = (const void*)spec_ldg_kernel;
-  cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t err = allow_shared_memory(fn);
   if (err != cudaSuccess) return err;
   int per_sm = 0;
   err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kSThreads, smem);

@@ -1599,7 +1599,7 @@ cudaError_t launch_stream_msg(const DevInstance& I, const SpecBuf& B, const Stre
                               cudaStream_t st) {
   const size_t smem = stream_msg_smem_bytes(I.K);
   const void* fn = (const void*)stream_msg_kernel;
-  cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t err = allow_shared_memory(fn);
   if (err != cudaSuccess) return err;
   int per_sm = 0;
   err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kSThreads, smem);
@@ -1622,7 +1622,7 @@ cudaError_t launch_stream_ldg(const DevInstance& I, const SpecBuf& B, const Stre
                               cudaStream_t st) {
   const size_t smem = stream_smem_bytes(I.K);
   const void* fn = (const void*)stream_ldg_kernel;
-  cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t err = allow_shared_memory(fn);
   if (err != cudaSuccess) return err;
   int per_sm = 0;
   err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kSThreads, smem);
