@@ -586,7 +586,9 @@ class Instance:
         _check(lib().fp_debug_replaced_room(self._h, int(entries)), "fp_debug_replaced_room")
 
     def stats(self) -> dict:
-        """Round statistics of the last refine on the grid-wide engine."""
+        """Round statistics of the last refine on the grid-wide engine (see
+        fp_get_stats: val_prefix_cta_ns is word 45, the nanoseconds of walks;
+        local_validate_ms, val_light_cta_ns and val_rest_cta_ns are unused words)."""
         x = np.zeros(48, np.int64)
         _check(lib().fp_get_stats(self._h, _ptr(x), 48), "fp_get_stats")
         names = ["windows", "heavy_rounds", "window_moves", "cut_none", "cut_stale", "cut_size", "cut_volume",

@@ -79,7 +79,7 @@ struct StreamArgs {
   const unsigned char* pclass;   // [npos] 0 a warp evaluates, 1 a CTA, 2 the grid
   int* mark_pos;          // [K] last position whose vertex saw the part, -1: none
   uint32_t* rec;          // [pins] slot of the chosen part in each (vertex, net) pair
-  // message-greedy stream (TM, MSM; csrc/fp_stream_msg.cu)
+  // message-greedy stream (TM, MSM; csrc/fp_stream.cu)
   uint32_t* prow;         // [K * words] conn > 0: bit b of row a
   uint32_t* pcol;         // [K * words] conn > 0: bit a of column b
   int* rowpos;            // [2 * K] by round parity: first position that makes an entry of row a positive

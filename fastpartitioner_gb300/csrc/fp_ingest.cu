@@ -616,8 +616,10 @@ int create_inverse_device(int device, cudaStream_t st, int num_sms, int nov, int
   if (!vertex_csr_ok(nov, noe, pins, vptr_h, vnets_h) || !nptr_h || (pins > 0 && !npins_h)) return FP_ERR_INVALID;
   cudaError_t e = cudaSetDevice(device);
   if (e != cudaSuccess) return status_of(e);
-  // one allocation for all buffers: with it and the vectorised checks 5.3M pins
-  // take 2.7 ms instead of 3.9 (1.5M 1.0 instead of 1.65), mostly the copies
+  // one allocation for all buffers: with it and the vectorised checks a repeated
+  // call on 5.3M pins takes 2.6 ms instead of 3.8 (checks 1.4, kernels 0.7,
+  // allocation 0.2, copies 0.35).  A first call, into host pages that nothing has
+  // touched, pays for those in its copies: 2.6 to 26 ms with either form
   DevBufs M;
   size_t words = 0;
   for (size_t n : {(size_t)nov + 1, (size_t)pins, (size_t)noe + 1, (size_t)pins, (size_t)noe,

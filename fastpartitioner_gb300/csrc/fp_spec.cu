@@ -343,12 +343,14 @@ __device__ __forceinline__ void ctab_clear(const SpecBuf& B, uint2 sl) {
   if (sl.y != ~0u) { B.ctab_key[sl.y] = ~0ull; B.ctab_pos[sl.y] = kNone; B.ctab_cnt[sl.y] = 0; }
 }
 
-// Clears the claims of a mover on its nets k0, k0 + kstep, ... (commit phase).
+// Clears the claims on net e (commit phase: movers' nets, replaced claims).
 __device__ __forceinline__ void unclaim_net(const SpecBuf& B, int e) {
   B.claim_m[e] = kNone;
   B.claim_c[e] = kNone;
   B.mask_c[e] = 0;
 }
+// Clears the claims of a mover on its nets k0, k0 + kstep, ... and its entries of
+// the count table.
 __device__ __forceinline__ void unclaim_nets(const DevInstance& I, const SpecBuf& B, bool vol, uint32_t base, int deg,
                                              int k0, int kstep) {
   for (int k = k0; k < deg; k += kstep) {

@@ -101,10 +101,6 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, int* status) {
 __device__ __forceinline__ int warp_sum(int x) { return __reduce_add_sync(kAll, x); }
 __device__ __forceinline__ int warp_min(int x) { return __reduce_min_sync(kAll, x); }
 __device__ __forceinline__ int warp_max(int x) { return __reduce_max_sync(kAll, x); }
-// Maximum of non-negative floats (their bit patterns order like the values).
-__device__ __forceinline__ float warp_max_nonneg(float x) {
-  return __uint_as_float(__reduce_max_sync(kAll, __float_as_uint(x)));
-}
 // Minimum of a 64-bit key: the high words, then the low words of their holders.
 __device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long x) {
   const unsigned hi = __reduce_min_sync(kAll, (unsigned)(x >> 32));
