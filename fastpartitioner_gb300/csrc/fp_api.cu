@@ -434,6 +434,13 @@ int fp_ctx_set_stream(fp_ctx* ctx, void* stream) {
   });
 }
 
+// Window offsets that list volume terms (640 bytes each): a window holds no more
+// positions than there are vertices.  Entries for replaced claims (16 bytes each):
+// each change in a window lists its vertex's nets, a few times all pins at most.
+// An MSV instance of 1,000 vertices holds 5 MB, 18 with the full windows.
+static size_t term_window(int nov) { return (size_t)std::max(1, std::min(nov, kSpecWindow)); }
+static int replaced_room(long long pins) { return (int)std::max(64ll, std::min(8 * pins, (long long)kReplaced)); }
+
 // The scratch that starts a launch as zeros lies in one buffer (from hcnt on),
 // cleared by one fill: the whole-grid tallies, TV's marker words, the mover and
 // table counts.  (Eight fills of them took 33 us of a refinement at K = 24, 26 with
@@ -740,9 +747,9 @@ int fp_instance_create(fp_ctx* ctx, const fp_hypergraph* h, int32_t K, int32_t m
         (rc = dalloc(in, &in->sb.ctl, kCtlWords)) || (rc = dalloc(in, &in->sb.bar, 4)) || (rc = dalloc(in, &in->sb.stats, kNumStats)) || (rc = dalloc(in, &in->sb.dec, std::max(kSpecWindow, kMsgWindow))) ||
         (rc = dalloc(in, &in->sb.flag, kSpecWindow)) || (rc = dalloc(in, &in->sb.slack, kSpecWindow)) ||
         (rc = dalloc(in, &in->sb.vslack, kSpecWindow)) || (rc = dalloc(in, &in->sb.wt, kSpecWindow)) ||
-        (rc = dalloc(in, &in->sb.vn, volm ? kSpecWindow : 1)) ||
-        (rc = dalloc(in, &in->sb.vterm, volm ? (size_t)kSpecWindow * kVolTerms : 1)) ||
-        (rc = dalloc(in, &in->sb.vpart, volm ? (size_t)kSpecWindow * kVolTerms : 1)) ||
+        (rc = dalloc(in, &in->sb.vn, volm ? term_window(g.nov) : 1)) ||
+        (rc = dalloc(in, &in->sb.vterm, volm ? term_window(g.nov) * kVolTerms : 1)) ||
+        (rc = dalloc(in, &in->sb.vpart, volm ? term_window(g.nov) * kVolTerms : 1)) ||
         (rc = dalloc(in, &in->sb.vd, kSpecWindow)) || (rc = dalloc(in, &in->sb.scan, (size_t)kSpecWindow * words)) ||
         (rc = dalloc(in, &in->sb.cmask, ldg ? kMaxSpecWarps / 8 * words : 1)) ||
         (rc = dalloc(in, &in->sb.rgain, std::max(kSpecWindow, kMsgWindow))) ||
@@ -751,7 +758,7 @@ int fp_instance_create(fp_ctx* ctx, const fp_hypergraph* h, int32_t K, int32_t m
         (rc = dalloc(in, &in->sb.ctab_key, ldg ? ctab : 1)) || (rc = dalloc(in, &in->sb.ctab_pos, ldg ? ctab : 1)) ||
         (rc = dalloc(in, &in->sb.ctab_cnt, ldg ? ctab : 1)) ||
         (rc = dalloc(in, &in->sb.dfix, kSpecWindow)) ||
-        (rc = dalloc(in, &in->sb.rlist, ldg ? kReplaced : 1)) ||
+        (rc = dalloc(in, &in->sb.rlist, ldg ? replaced_room(g.pins) : 1)) ||
         (rc = dalloc(in, &in->sb.cn_moved, cn ? g.pins : 1)) || (rc = dalloc(in, &in->sb.cn_kcnt, cn ? g.noe : 1)) ||
         (rc = dalloc(in, &in->sb.cn_nets, cn ? g.noe : 1)) || (rc = dalloc(in, &in->sb.cn_more, cn ? g.pins : 1)) || (rc = dalloc(in, &in->sb.cn_cnt, 8)) ||
         (rc = dalloc(in, &in->sb.cn_wit, cn ? g.nov : 1)) || (rc = dalloc(in, &in->vclass_d, g.nov)) ||
@@ -807,7 +814,7 @@ int fp_instance_create(fp_ctx* ctx, const fp_hypergraph* h, int32_t K, int32_t m
     // 0: the kernels' own shortest window after a cut
     in->sb.wmin = 0;
     in->sb.maxfix = 32;
-    in->sb.rmax = kReplaced;
+    in->sb.rmax = replaced_room(g.pins);
     in->sb.max_warps = kMaxSpecWarps;
     in->sb.heavy_pos = in->heavy_pos_d;
     in->sb.mid_pos = in->mid_pos_d;
@@ -889,14 +896,15 @@ int fp_instance_footprint(int32_t nov, int32_t noe, int64_t pins, int32_t K, int
     // speculation scratch
     add(kCtlWords, 4); add(4, 4); add(kNumStats, 8); add(std::max(kSpecWindow, kMsgWindow), 4);
     add(W, 1); add(W, 4); add(W, 4); add(W, 4); add(W, 4);   // flag, slack, vslack, wt, vd
-    add(volm ? W : 1, 4); add(volm ? W * kVolTerms : 1, 8); add(volm ? W * kVolTerms : 1, 2);   // vn, vterm, vpart
+    const size_t T = term_window(nov);
+    add(volm ? T : 1, 4); add(volm ? T * kVolTerms : 1, 8); add(volm ? T * kVolTerms : 1, 2);   // vn, vterm, vpart
     add(W * words, 4);                                       // scan
     add(ldg ? kMaxSpecWarps / 8 * words : 1, 4);                 // cmask
     add(std::max(kSpecWindow, kMsgWindow), 4); add(std::max(kSpecWindow, kMsgWindow), 4);   // rgain, rloss
     add(ldg ? P : 1, 4); add(ldg ? P : 1, 8);                // rec, rec_slot
     add(ldg ? ctab : 1, 8); add(ldg ? ctab : 1, 4); add(ldg ? ctab : 1, 4);
     add(W, 4);                                               // dfix
-    add(ldg ? kReplaced : 1, 16);                            // rlist
+    add(ldg ? replaced_room(pins) : 1, 16);                  // rlist
     add(cn ? P : 1, 8); add(cn ? E : 1, 4); add(cn ? E : 1, 8); add(cn ? P : 1, 8); add(8, 4); add(cn ? V : 1, 4);
     add(V, 1);                                               // vertex classes
     add(W * K, 8); add(W, 4); add(W, 16); add(W, 4);         // cand, ncand, mlist, midx
@@ -1208,7 +1216,7 @@ int fp_debug_barrier_fault(fp_instance* in, int32_t leave_at, int32_t poll_limit
 
 int fp_debug_replaced_room(fp_instance* in, int32_t entries) {
   return fp::guarded([&]() -> int {
-    if (!in || entries < 0 || entries > kReplaced) return FP_ERR_INVALID;
+    if (!in || entries < 0 || entries > replaced_room(in->g.pins)) return FP_ERR_INVALID;
     in->sb.rmax = entries;
     return FP_OK;
   });

@@ -98,7 +98,7 @@ constexpr int kStreamHeavy = 4096;   // nets of a vertex the whole grid places i
 // 262144 (and 8192 nets).
 constexpr long long kStreamCtaWork = 4096;
 constexpr long long kStreamGridWork = 65536;
-constexpr int kReplaced = 1 << 18;     // claims of replaced moves a window holds
+constexpr int kReplaced = 1 << 18;     // claims of replaced moves a window holds at most
 constexpr int kVolTerms = 64;         // parts whose volumes a listed decision touches at most
 constexpr int kStreamMaxK = 1024;    // shared memory of the device stream's CTAs
 constexpr int kMsgStreamCta = 1024;  // nets of a vertex one CTA places alone in the message-greedy stream
@@ -132,10 +132,10 @@ struct SpecBuf {
   int* vslack;           // [wmax] volume drift the accept/reject outcome tolerates
   int* wt;               // [wmax] vertex weight (streams: of the placed vertex)
   int* vd;               // [wmax] largest volume change of one part by a mover
-  int* vn;               // [wmax] volume terms of a decision that leaves its part (-1: more
+  int* vn;               // [min(wmax, nov)] volume terms of a decision that leaves its part (-1: more
                          //     than kVolTerms)
-  int2* vterm;           // [wmax * kVolTerms] (loss - gain, exact change) of a part's volume
-  unsigned short* vpart; // [wmax * kVolTerms] that part (MSV / MSRV)
+  int2* vterm;           // [min(wmax, nov) * kVolTerms] (loss - gain, exact change) of a part's volume
+  unsigned short* vpart; // [min(wmax, nov) * kVolTerms] that part (MSV / MSRV)
   int* rgain;            // [wmax] decision-record gain / loss of each window offset (with
   int* rloss;            //     the decision log on)
   uint32_t* scan;        // [wmax * words] parts scanned per window offset (TV)
@@ -168,9 +168,9 @@ struct SpecBuf {
   int* ctab_pos;         // [ctab_mask + 1] first position of a count-only mover with that (net, part)
   int* ctab_cnt;         // [ctab_mask + 1] count-only movers of the round on that (net, part)
   uint2* rec_slot;       // [pins] table slots of a count-only move's (net, own) and (net, new part)
-  int4* rlist;           // [kReplaced] claims of the moves that changed decisions replaced
+  int4* rlist;           // [rmax] claims of the moves that changed decisions replaced
                          //     (net or -1, its two entries of the table), until the commit
-  int rmax;              // entries of rlist that a window may use (kReplaced)
+  int rmax;              // entries of rlist that a window may use (kReplaced or fewer)
   int* ctab_over;        // [2] a probe ran past its bound this round (by round parity)
   unsigned ctab_mask;
   const int* heavy_pos;  // positions (visiting order, ascending) of vertices evaluated by

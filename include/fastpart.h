@@ -270,8 +270,9 @@ int fp_get_decisions(fp_instance* inst, int32_t* dest, int32_t* gain, int32_t* l
  * partial: fp_reset_state restores the initial one. */
 int fp_debug_barrier_fault(fp_instance* inst, int32_t leave_at, int32_t poll_limit);
 /* Test hook (no effect on results; TV / MSV / MSRV): at most `entries` (net,
- * vertex) pairs of moves that a window's later changes replace are kept, 2^18 by
- * default; a change without room ends the window in front of it. */
+ * vertex) pairs of moves that a window's later changes replace are kept; a change
+ * without room ends the window in front of it.  The default and the most: 2^18,
+ * or eight times the pins if that is less. */
 int fp_debug_replaced_room(fp_instance* inst, int32_t entries);
 
 /* Statistics of the last fp_refine on the grid-wide engine (up to 48 values):
