@@ -63,11 +63,15 @@ static bool spec_supported(int metric, int K, int max_smem, int nov, int noe) {
 // Sweeps on Zipf workloads (K = 256, degree weights; milliseconds for the passes
 // in brackets at (light bound, super bound, vertices per window)):
 //   TV   1M   [3]   (2048, 65536, 32) 15.5    (2048, 32768, 32) 21.1    (2048, 65536, 16) 21.0
-//   MSRV 256K [10]  (2048, 24576, 16) 51-53   (2048, 16384, 16) 59      (2048, 32768, 32) 44-49
-//             [2]   (2048, 24576, 16) 20-34   (2048, 16384, 16) 20-30   (2048, 32768, 32) 23-37
+//   MSRV 256K [10]  (2048, 24576, 16) 51-74   (2048, 16384, 16) 59      (2048, 32768, 32) 44-72
+//             [2]   (2048, 24576, 16) 21-35   (2048, 16384, 16) 20-30   (2048, 32768, 32) 24-38
 //   MSV  256K [3]   (1024, 16384, 4) 305-370  (2048, 32768, 4) 312-379  (1024, 8192, 8) 306-372
 //   TM   256K [5]   (512, 8192, 32) 41-49     (1024, 16384, 16) 44-52   (512, 4096, 16) 52-57
 //   MSM  1M         (2048, 262144, 16) 0.94   (2048, 65536, 32) 1.74
+// MSRV: most passes of a short schedule move something, so windows end early and
+// fewer whole-grid vertices per window pay: over four seeds each of 16K (K = 64),
+// 64K, 256K and 1M vertices, passes 1, 2 and 3 take 3-17% longer with (32768, 32),
+// and so do ten passes at 16K and 1M; ten at 64K and 256K take 5-8% less.
 constexpr int kLightWork = 2048, kLightWorkMsv = 1024, kLightWorkTm = 512;
 constexpr int kCnLightPins = 128;   // CN: nets with more pins are evaluated by one CTA,
 constexpr int kCnGridPins = 1024;   //     with more than this by the whole grid
